@@ -1075,13 +1075,19 @@ int bm_verify_accept(const void *draft, const void *verify, int D, void *n_out, 
 int bm_pack_t2_g128(const void *w, int N, int K, void *packed, void *scale, void *frozen, void *stream) {
     if (!w || !packed || !scale || N < 1 || K < BM_GROUP || (K % BM_GROUP) != 0) return BM_EINVAL;
     if (!aligned16(w) || (frozen && !aligned16(frozen)) || (reinterpret_cast<uintptr_t>(packed) & 1u)) return BM_EINVAL;
-    const long long units = (long long)N * (K / BM_GROUP);
-    const long long blocks = (units + 15) / 16;                     // two (row, group) units per warp
+    const long long groups = (long long)N * (K / BM_GROUP);
+    const int per_cta = bm::kPackThreads / 32 * 2 * bm::kPackGroupPairs;
+    const long long blocks = (groups + per_cta - 1) / per_cta;
     if (blocks > 0x7fffffffLL) return BM_EINVAL;
     count_launch();
-    bm::pack_t2_g128_kernel<<<(unsigned)blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const uint16_t *>(w), N, K, static_cast<uint8_t *>(packed), static_cast<uint16_t *>(scale),
-        static_cast<uint16_t *>(frozen));
+    const uint16_t *src = static_cast<const uint16_t *>(w);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (frozen)
+        bm::pack_t2_g128_kernel<true><<<(unsigned)blocks, bm::kPackThreads, 0, st>>>(
+            src, groups, static_cast<uint8_t *>(packed), static_cast<uint16_t *>(scale), static_cast<uint16_t *>(frozen));
+    else
+        bm::pack_t2_g128_kernel<false><<<(unsigned)blocks, bm::kPackThreads, 0, st>>>(
+            src, groups, static_cast<uint8_t *>(packed), static_cast<uint16_t *>(scale), nullptr);
     return cuda_status(cudaGetLastError());
 }
 

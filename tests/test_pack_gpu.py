@@ -62,6 +62,30 @@ def test_degenerate_groups():
     assert float(scale[0].abs().max()) == 0.0
 
 
+def test_tail_groups_and_values_that_are_not_finite():
+    """Group counts that leave a warp's share unfinished; a NaN packs as 0 and leaves its group's scale alone, an
+    infinity gives its group scale 0 and codes 0; the frozen values round either side of s / 2 correctly."""
+    gen = torch.Generator().manual_seed(11)
+    for n in (1, 7, 8, 9, 63, 65):
+        _same((torch.randn(n, 128, generator=gen) * 0.02).to(torch.bfloat16))
+    mags = torch.arange(1, 2 ** 15 - 2 ** 7, 37, dtype=torch.int32).to(torch.int16).view(torch.bfloat16).float()
+    top = mags[:, None].expand(-1, 128).clone()
+    half = (top[:, 1:65] / 2).to(torch.bfloat16).view(torch.int16).int() + torch.arange(-32, 32)   # neighbours of s / 2
+    top[:, 1:65] = half.clamp(0, 0x7f7f).to(torch.int16).view(torch.bfloat16).float()
+    top[:, 65:] *= -0.25
+    _same(top.to(torch.bfloat16))
+    w = (torch.randn(4, 128, generator=gen) * 0.02).to(torch.bfloat16)
+    w[1, 3] = float("nan")
+    w[2, 5] = float("-inf")
+    codes, scale, frozen = (t.cpu() for t in ops.pack_t2_g128(w.to(DEV), want_frozen=True))
+    clean = w.clone()
+    clean[1, 3] = 0
+    want_codes, want_scale = pack_t2_g128(CV.freeze_ternary_g128(clean))
+    assert torch.equal(codes[[0, 1, 3]], want_codes[[0, 1, 3]]) and torch.equal(scale[[0, 1, 3]], want_scale[[0, 1, 3]])
+    assert bool(frozen[1, 3].isnan()) and int(frozen[1].isnan().sum()) == 1 and bool(frozen[2].isnan().all())
+    assert bool((codes[2].view(torch.uint8) == 0xAA).all()) and float(scale[2]) == 0.0
+
+
 def test_rejects_what_the_packer_cannot_take():
     w = torch.zeros(4, 128, dtype=torch.bfloat16, device=DEV)
     with pytest.raises(RuntimeError):
