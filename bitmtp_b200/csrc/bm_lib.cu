@@ -14,6 +14,7 @@
 #include "t2_gemv.cuh"
 #include "fused_ops.cuh"
 #include "verify_attn.cuh"
+#include "prompt_attn.cuh"
 #include "t2_gemv_rowwarp.cuh"
 #include "t2_gemv_direct.cuh"
 #include "dense_head.cuh"
@@ -1158,7 +1159,19 @@ int bm_prompt_attention(const void *q, const void *k_base, const void *v_base, i
     p.pdl = pdl & BM_PDL_OVERLAP;
     p.slab_rows = slab_rows;
     p.slab_hist0 = hist0;
-    const dim3 grid(pl.units, Hkv, pl.Z);
+    if (bm::prompt_hist_fits(slab_rows, H, Hkv)) {
+        // history super-chunks by tiles of 64 query vectors, then one CTA set per slab for its own rows and the merge
+        const int hist_end = hist0 + (pl.n_slabs - 1) * slab_rows, G = H / Hkv;
+        if (hist_end > 0) {
+            const bm::PromptHistParams hp{p.q, p.k_base, p.v_base, p.pm, p.pl, p.po, T, H, Hkv, G, kv_rows, hist0, pl.NJ, p.pdl};
+            const dim3 hgrid((hist_end + BM_ATTN_SUPER - 1) / BM_ATTN_SUPER, Hkv, (T * G + bm::kPaQueries - 1) / bm::kPaQueries);
+            const int rc = launch_ex(bm::prompt_hist_kernel, hgrid, dim3(bm::kPaThreads), bm::kPaSmem,
+                                     static_cast<cudaStream_t>(stream), p.pdl, hp);
+            if (rc != BM_OK) return rc;
+        }
+        p.hist_done = 1;
+    }
+    const dim3 grid(p.hist_done ? pl.n_slabs : pl.units, Hkv, pl.Z);
     return launch_attention<false>(pl.nq, grid, bm::attn_smem_bytes(pl.nq), static_cast<cudaStream_t>(stream), p.pdl, p);
 }
 

@@ -1,0 +1,228 @@
+// History part of the prompt attention: the super-chunk partials of MANY query rows at once.
+//
+// The prompt's causal attention runs in slabs of 16 rows: every row of slab s attends to the history
+// [0, h_s), h_s = hist0 + 16 s, cut into super-chunks of 128 keys, and to the rows of its own slab (the
+// reference's prompt forward: src/bonsai_sft/gpu/model.py:1306-1340).  attn_fused_kernel serves 8 query vectors
+// per CTA, so it reads 64 KB of K / V per 262 K multiply-adds and repeats the staging, the waits and the
+// level-1 merge for every eighth vector.  Here one CTA serves kPaQueries = 64 query vectors against one
+// super-chunk as a register-blocked product on the CUDA cores (8 x 8 outputs per thread): scores S = Q K^T, the
+// softmax of each 32-key sub-chunk, numerators O = P V and the merge of the four sub-chunks.  It writes the
+// partials (max, sum, 128 numerators) that the slab's own CTA of attn_fused_kernel then merges in order.
+//
+// Bound by the fp32 pipe: 2 * 128 multiply-adds per (query vector, key).  Every one of them is the fma of
+// attn_sub_pass, in the same chain (scores ascending in d, numerators ascending in the key, sub-chunks
+// ascending, the weight sum as the butterfly over the 32 keys), so the partials are the same bits; tensor
+// cores would not give that order.
+#pragma once
+
+#include "verify_attn.cuh"
+
+namespace bm {
+
+constexpr int kPaThreads = 128;
+constexpr int kPaQueries = 64;           // query vectors per CTA: 64 / G rows x G heads of a kv head
+constexpr int kPaSlab = 16;              // rows per slab; a thread's 8 vectors and a warp's 16 lie in one slab
+constexpr int kPaQStride = kPaQueries + 4;       // fp32 per d row of Q^T
+constexpr int kPaKStride = BM_ATTN_SUPER + 8;    // bf16 per d row of K^T
+
+struct PromptHistParams {
+    const uint16_t *q;                   // [T, H, 128] rotated queries
+    const uint16_t *k_base, *v_base;     // [Hkv, kv_rows, 128]
+    float *pm, *pl, *po;                 // [T, H, NJ] and [T, H, NJ, 128]
+    int T, H, Hkv, G, kv_rows, hist0, NJ, pdl;
+};
+
+// Q^T fp32 [128][kPaQStride] (after the scores its space holds P^T fp32 [128][64], see pa_weight), K^T bf16
+// [128][kPaKStride], V bf16 [128][128], m and l fp32 [4][64].
+constexpr int kPaQBytes = 128 * kPaQStride * 4, kPaKBytes = 128 * kPaKStride * 2, kPaVBytes = BM_ATTN_SUPER * 256;
+constexpr int kPaSmem = kPaQBytes + kPaKBytes + kPaVBytes + 2 * kAttnSub * kPaQueries * 4;
+
+// Whether the tile kernel takes a call; the launcher keeps attn_fused_kernel for every other slab height or
+// head grouping.
+__host__ __device__ inline bool prompt_hist_fits(int slab_rows, int H, int Hkv) {
+    const int G = H / Hkv;
+    return slab_rows == kPaSlab && (G == 1 || G == 2 || G == 4 || G == 8);
+}
+
+// History length of the slab that holds prompt row r.
+__device__ __forceinline__ int pa_history(int hist0, int r) { return hist0 + r / kPaSlab * kPaSlab; }
+
+// Word of weight (key, vector 8 vg) in P^T, whose 16-byte pieces are swizzled by the key's group of eight: the
+// threads of a warp, eight keys apart, then store to different banks.  Vectors 8 vg + 4 .. + 7 are at ^ 4 words.
+__device__ __forceinline__ int pa_weight(int key, int vg) { return key * kPaQueries + 4 * ((2 * vg) ^ (key >> 3)); }
+
+// One step of the register-blocked products: acc[t][j] = fma(a[t], b[j], acc[t][j]).
+__device__ __forceinline__ void pa_step(float (&acc)[8][8], const float4 &a0, const float4 &a1, const uint4 &braw) {
+    float b[8];
+    unpack8(braw, b);
+    const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+#pragma unroll
+    for (int t = 0; t < 8; ++t)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[t][j] = fmaf(a[t], b[j], acc[t][j]);
+}
+
+// grid (super-chunks of the longest history, Hkv, ceil(T * G / 64)), 128 threads = 8 vector groups x 16 key
+// (then dim) groups.
+__global__ void __launch_bounds__(kPaThreads, 2) prompt_hist_kernel(const PromptHistParams p) {
+    extern __shared__ __align__(16) unsigned char pa_smem[];
+    pdl_launch_dependents();
+    if (p.pdl) pdl_wait();
+    const int J = blockIdx.x, hk = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int rows = kPaQueries / p.G, row0 = blockIdx.z * rows;      // this tile's prompt rows
+    const int row_end = min(row0 + rows, p.T);
+    const int key0 = J * BM_ATTN_SUPER;
+    const int keys_max = min(BM_ATTN_SUPER, pa_history(p.hist0, row_end - 1) - key0);
+    if (keys_max <= 0) return;
+    float *Qt = reinterpret_cast<float *>(pa_smem), *Pt = Qt;
+    uint16_t *Kt = reinterpret_cast<uint16_t *>(pa_smem + kPaQBytes);
+    uint16_t *Vs = reinterpret_cast<uint16_t *>(pa_smem + kPaQBytes + kPaKBytes);
+    float *mc = reinterpret_cast<float *>(pa_smem + kPaQBytes + kPaKBytes + kPaVBytes), *lc = mc + kAttnSub * kPaQueries;
+
+    // V as it is (16-byte asynchronous copies); K two rows per lane, transposed as bf16 pairs; Q one vector per
+    // lane, transposed as fp32.  Consecutive lanes store consecutive words: no bank conflicts.
+    const uint16_t *kg = p.k_base + ((size_t)hk * p.kv_rows + key0) * 128;
+    const uint16_t *vg = p.v_base + ((size_t)hk * p.kv_rows + key0) * 128;
+    for (int i = tid; i < BM_ATTN_SUPER * 16; i += kPaThreads) {
+        if ((i >> 4) < keys_max) cp_async16(Vs + 8 * i, reinterpret_cast<const uint4 *>(vg) + i);
+    }
+    {
+        const int k0 = 2 * (lane + 32 * (warp & 1));                  // keys k0, k0 + 1
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int d0 = 8 * ((warp >> 1) + 2 * j);
+            uint4 a = make_uint4(0u, 0u, 0u, 0u), b = a;
+            if (k0 < keys_max) a = *reinterpret_cast<const uint4 *>(kg + (size_t)k0 * 128 + d0);
+            if (k0 + 1 < keys_max) b = *reinterpret_cast<const uint4 *>(kg + (size_t)(k0 + 1) * 128 + d0);
+            const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+                *reinterpret_cast<uint32_t *>(Kt + (d0 + 2 * w) * kPaKStride + k0) = __byte_perm(aw[w], bw[w], 0x5410);
+                *reinterpret_cast<uint32_t *>(Kt + (d0 + 2 * w + 1) * kPaKStride + k0) = __byte_perm(aw[w], bw[w], 0x7632);
+            }
+        }
+        const int v = lane + 32 * (warp & 1);                         // vector v of the tile: row v / G, head v % G
+        const int r = row0 + v / p.G, head = hk * p.G + v % p.G;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int d0 = 8 * ((warp >> 1) + 2 * j);
+            float f[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+            if (r < p.T) unpack8(*reinterpret_cast<const uint4 *>(p.q + ((size_t)r * p.H + head) * 128 + d0), f);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) Qt[(d0 + e) * kPaQStride + v] = f[e];
+        }
+    }
+    cp_async_wait_all();
+    __syncthreads();
+
+    const int vgp = tid >> 4, kgp = tid & 15;                         // vector group, key / dim group
+    const int v0 = 8 * vgp;
+    // keys of this super-chunk that this thread's vectors see (one slab, the same for the whole warp)
+    const int my_row = row0 + v0 / p.G;
+    const int lim = my_row < p.T ? min(BM_ATTN_SUPER, pa_history(p.hist0, my_row) - key0) : 0;
+
+    float acc[8][8];                                                  // [vector][key]
+#pragma unroll
+    for (int t = 0; t < 8; ++t)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[t][j] = 0.0f;
+    if (lim > 0) {
+        const float *qp = Qt + v0;
+        const uint16_t *kp = Kt + 8 * kgp;
+#pragma unroll 4
+        for (int d = 0; d < 128; ++d)
+            pa_step(acc, *reinterpret_cast<const float4 *>(qp + d * kPaQStride),
+                    *reinterpret_cast<const float4 *>(qp + d * kPaQStride + 4),
+                    *reinterpret_cast<const uint4 *>(kp + d * kPaKStride));
+    }
+    __syncthreads();                                                  // Q^T is spent: its space takes P^T
+    const int c = kgp >> 2;                                           // sub-chunk of this thread's keys
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+        float mj = -INFINITY;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            acc[t][j] = 8 * kgp + j < lim ? acc[t][j] * 0.08838834764831845f : -INFINITY;
+            mj = fmaxf(mj, acc[t][j]);
+        }
+        mj = fmaxf(mj, __shfl_xor_sync(0xffffffffu, mj, 1));
+        mj = fmaxf(mj, __shfl_xor_sync(0xffffffffu, mj, 2));
+        float s[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float pr = 8 * kgp + j < lim ? bm_expf(acc[t][j] - mj) : 0.0f;
+            acc[t][j] = bm_bf16_rn(pr);
+            // butterfly over the 32 keys of the sub-chunk: offsets 16 and 8 lie across the four threads
+            s[j] = pr + __shfl_xor_sync(0xffffffffu, pr, 2);
+            s[j] = s[j] + __shfl_xor_sync(0xffffffffu, s[j], 1);
+        }
+        const float lj = ((s[0] + s[4]) + (s[2] + s[6])) + ((s[1] + s[5]) + (s[3] + s[7]));
+        if ((kgp & 3) == 0) {
+            mc[c * kPaQueries + v0 + t] = mj;
+            lc[c * kPaQueries + v0 + t] = lj;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const int w = pa_weight(8 * kgp + j, vgp);
+        *reinterpret_cast<float4 *>(Pt + w) = make_float4(acc[0][j], acc[1][j], acc[2][j], acc[3][j]);
+        *reinterpret_cast<float4 *>(Pt + (w ^ 4)) = make_float4(acc[4][j], acc[5][j], acc[6][j], acc[7][j]);
+    }
+    __syncthreads();
+    if (lim <= 0) return;
+
+    // numerators: this thread's 8 vectors x dims 8 kgp .. 8 kgp + 7, one chain per sub-chunk, then the merge
+    float O[8][8], L[8], MJ[8];
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+        L[t] = 0.0f;
+        MJ[t] = -INFINITY;
+#pragma unroll
+        for (int s = 0; s < kAttnSub; ++s) MJ[t] = fmaxf(MJ[t], mc[s * kPaQueries + v0 + t]);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) O[t][e] = 0.0f;
+    }
+    for (int s = 0; s < kAttnSub; ++s) {
+#pragma unroll
+        for (int t = 0; t < 8; ++t)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) acc[t][e] = 0.0f;
+        const int cn = min(BM_ATTN_CHUNK, lim - s * BM_ATTN_CHUNK);
+        for (int k8 = 0; k8 < cn; k8 += 8) {
+            const int key = s * BM_ATTN_CHUNK + k8, w = pa_weight(key, vgp);
+            const uint16_t *vp = Vs + key * 128 + 8 * kgp;
+            if (cn - k8 >= 8) {
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                    pa_step(acc, *reinterpret_cast<const float4 *>(Pt + w + k * kPaQueries),
+                            *reinterpret_cast<const float4 *>(Pt + (w ^ 4) + k * kPaQueries),
+                            *reinterpret_cast<const uint4 *>(vp + k * 128));
+            } else {                                                  // a history that ends inside the eight keys
+                for (int k = 0; k < cn - k8; ++k)
+                    pa_step(acc, *reinterpret_cast<const float4 *>(Pt + w + k * kPaQueries),
+                            *reinterpret_cast<const float4 *>(Pt + (w ^ 4) + k * kPaQueries),
+                            *reinterpret_cast<const uint4 *>(vp + k * 128));
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+            const float m = mc[s * kPaQueries + v0 + t];
+            const float w = m > -INFINITY ? bm_expf(m - MJ[t]) : 0.0f;
+            L[t] = fmaf(lc[s * kPaQueries + v0 + t], w, L[t]);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) O[t][e] = fmaf(acc[t][e], w, O[t][e]);
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+        const int r = row0 + (v0 + t) / p.G, head = hk * p.G + (v0 + t) % p.G;
+        if (r >= p.T) continue;
+        const size_t pb = ((size_t)r * p.H + head) * p.NJ + J;
+        float *dst = p.po + pb * 128 + 8 * kgp;
+        *reinterpret_cast<float4 *>(dst) = make_float4(O[t][0], O[t][1], O[t][2], O[t][3]);
+        *reinterpret_cast<float4 *>(dst + 4) = make_float4(O[t][4], O[t][5], O[t][6], O[t][7]);
+        if (kgp == 0) { p.pm[pb] = MJ[t]; p.pl[pb] = L[t]; }
+    }
+}
+
+}  // namespace bm

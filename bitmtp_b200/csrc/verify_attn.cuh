@@ -67,7 +67,9 @@ struct AttnParams {
     // sees history [0, slab_hist0 + s * slab_rows) and its own rows.  blockIdx.x runs over the
     // (slab, super-chunk) pairs in slab order; `state` is not read; q, att, amax and the partials are
     // indexed by prompt row; tickets [slabs][Hkv][gridDim.z].
-    int slab_rows, slab_hist0;
+    // hist_done: the history super-chunks' partials are in pm / pl / po already (prompt_hist_kernel); blockIdx.x is
+    // the slab, its CTAs make the partial of the slab's own rows and merge at once, without a ticket.
+    int slab_rows, slab_hist0, hist_done;
     int slots;       // CTAs the device holds at once (0: keep the coarse query split)
 };
 
@@ -255,7 +257,11 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_fused_kernel(const AttnP
     if (!ROPE && p.slab_rows > 0) {
         // prompt mode: find this CTA's slab; a slab with history h has ceil(h / 128) + 1 super-chunks
         int s = 0, rem = J, h = p.slab_hist0;
-        for (;;) {
+        if (p.hist_done) {
+            s = J;
+            h += s * p.slab_rows;
+            rem = (h + BM_ATTN_SUPER - 1) / BM_ATTN_SUPER;
+        } else for (;;) {
             const int units = (h + BM_ATTN_SUPER - 1) / BM_ATTN_SUPER + 1;
             if (rem < units) break;
             rem -= units;
@@ -463,11 +469,12 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_fused_kernel(const AttnP
     __syncthreads();
 
     // level 1: the four sub-chunk partials of query vector qi, merged in ascending sub-chunk order
+    const bool merge_now = !ROPE && p.hist_done;       // the partial below stays in this warp's registers
+    float MJ = -INFINITY, L = 0.0f, O[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     if (q_live) {
-        float mm[kAttnSub], MJ = -INFINITY;
+        float mm[kAttnSub];
 #pragma unroll
         for (int c = 0; c < kAttnSub; ++c) { mm[c] = mc[c * QC + qi]; MJ = fmaxf(MJ, mm[c]); }
-        float L = 0.0f, O[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
         for (int c = 0; c < kAttnSub; ++c) {
             const float w = mm[c] > -INFINITY ? bm_expf(mm[c] - MJ) : 0.0f;
@@ -483,7 +490,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_fused_kernel(const AttnP
             // vector, both spent since the CTA barrier after level 0
             *reinterpret_cast<float4 *>(Ps + qi * BM_ATTN_SUPER + 4 * lane) = make_float4(O[0], O[1], O[2], O[3]);
             if (lane == 0) *reinterpret_cast<float2 *>(Qs + qi * 128) = make_float2(MJ, L);
-        } else {
+        } else if (!merge_now) {
             const size_t pb = ((size_t)(r0 + qm) * p.H + hk * G + qg_) * p.NJ + J;
             *reinterpret_cast<float4 *>(p.po + pb * 128 + 4 * lane) = make_float4(O[0], O[1], O[2], O[3]);
             if (lane == 0) { p.pm[pb] = MJ; p.pl[pb] = L; }
@@ -548,14 +555,16 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_fused_kernel(const AttnP
         cluster_wait();
         return;
     }
-    // ticket: the last CTA of this (kv head, query group) to get here merges the super-chunks
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) sh_ticket = atomicAdd(ticket, 1u);
-    __syncthreads();
-    if (sh_ticket != (unsigned int)n_hs) return;                  // n_hs + 1 CTAs take part
-    __threadfence();
-    if (tid == 0) *ticket = 0u;                                   // ready for the next launch
+    if (!merge_now) {
+        // ticket: the last CTA of this (kv head, query group) to get here merges the super-chunks
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) sh_ticket = atomicAdd(ticket, 1u);
+        __syncthreads();
+        if (sh_ticket != (unsigned int)n_hs) return;              // n_hs + 1 CTAs take part
+        __threadfence();
+        if (tid == 0) *ticket = 0u;                               // ready for the next launch
+    }
     if (!q_live) return;
 
     // level 2: super-chunk partials of query vector qi in ascending order (history, then the replay's rows)
@@ -563,20 +572,28 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_fused_kernel(const AttnP
     const size_t pb = ((size_t)(r0 + qm) * p.H + hk * G + qg_) * p.NJ;
     constexpr int kBatch = 8;
     float4 part[kBatch];
+    const float4 own_o = make_float4(O[0], O[1], O[2], O[3]);
     // the first batch of numerators is requested together with the maxima and sums: one round trip
 #pragma unroll
     for (int i = 0; i < kBatch; ++i) {
         const int j = i < n_hs ? i : p.NJ - 1;
-        part[i] = i < nv ? __ldcg(reinterpret_cast<const float4 *>(p.po + (pb + j) * 128 + 4 * lane))
-                         : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        part[i] = merge_now && i == n_hs ? own_o
+                  : i < nv ? __ldcg(reinterpret_cast<const float4 *>(p.po + (pb + j) * 128 + 4 * lane))
+                           : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
     float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.0f, l1 = 0.0f;
-    if (lane < nv) {
+    if (merge_now && lane == n_hs) {
+        m0 = MJ;
+        l0 = L;
+    } else if (lane < nv) {
         const int j = lane < n_hs ? lane : p.NJ - 1;
         m0 = __ldcg(p.pm + pb + j);
         l0 = __ldcg(p.pl + pb + j);
     }
-    if (lane + 32 < nv) {
+    if (merge_now && lane + 32 == n_hs) {
+        m1 = MJ;
+        l1 = L;
+    } else if (lane + 32 < nv) {
         const int j = lane + 32 < n_hs ? lane + 32 : p.NJ - 1;
         m1 = __ldcg(p.pm + pb + j);
         l1 = __ldcg(p.pl + pb + j);
@@ -591,8 +608,9 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_fused_kernel(const AttnP
             for (int i = 0; i < kBatch; ++i) {
                 const int c = b0 + i;
                 const int j = c < n_hs ? c : p.NJ - 1;
-                part[i] = c < nv ? __ldcg(reinterpret_cast<const float4 *>(p.po + (pb + j) * 128 + 4 * lane))
-                                 : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                part[i] = merge_now && c == n_hs ? own_o
+                          : c < nv ? __ldcg(reinterpret_cast<const float4 *>(p.po + (pb + j) * 128 + 4 * lane))
+                                   : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             }
         }
 #pragma unroll

@@ -1,0 +1,66 @@
+"""The many-row paths of a prompt against the decode operators, row for row and bit for bit: the prompt attention
+(history tiles + one merge per slab) against slab-by-slab verify attention, and the packed linear module against the
+GEMV in slabs."""
+import pytest
+import torch
+
+from bitmtp_b200 import native, ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+SLAB = 16
+
+
+def _attention_inputs(T, hist0, H, Hkv, seed):
+    gen = torch.Generator(device=DEV).manual_seed(seed)
+    rows = hist0 + T + 40
+    q = torch.randn(T, H, 128, generator=gen, device=DEV).to(torch.bfloat16)
+    k = torch.randn(Hkv, rows, 128, generator=gen, device=DEV).to(torch.bfloat16)
+    v = torch.randn(Hkv, rows, 128, generator=gen, device=DEV).to(torch.bfloat16)
+    return q, k, v
+
+
+def _by_slab(q, k, v, hist0):
+    T, H, _ = q.shape
+    state = ops.new_step_state(torch.device(DEV))
+    att = torch.empty(T, H * 128, dtype=torch.bfloat16, device=DEV)
+    for r0 in range(0, T, SLAB):
+        n, h = min(SLAB, T - r0), hist0 + r0
+        ops.set_step_state(state, h, 0, native.ROLE_AR, 0)
+        att[r0:r0 + n] = ops.verify_attention(q[r0:r0 + n].contiguous(), k, v, h, state,
+                                              ops.attention_scratch(SLAB, H, h, DEV))[0]
+    return att
+
+
+def _prompt(q, k, v, hist0, calls=1):
+    T, H, _ = q.shape
+    scratch = ops.prompt_attention_scratch(T, hist0, SLAB, H, k.shape[0], DEV)
+    att = torch.full((T + 1, H * 128), 7.0, dtype=torch.bfloat16, device=DEV)
+    for _ in range(calls):
+        amax = torch.zeros(T, dtype=torch.int32, device=DEV)
+        ops.prompt_attention(q, k, v, hist0, SLAB, scratch, att=att[:T], amax=amax)
+    torch.cuda.synchronize()
+    assert native.lib().bm_device_error() == 0
+    assert bool((att[T] == 7.0).all())
+    finite = att[:T].float().isfinite().all(dim=1)
+    assert torch.equal(amax.view(torch.float32)[finite], att[:T].float().abs().amax(dim=1)[finite])
+    return att[:T]
+
+
+@pytest.mark.parametrize("H,Hkv", [(2, 2), (16, 8), (32, 8), (8, 1), (6, 2)])      # 1, 2, 4, 8 and (general kernel) 3 heads per group
+@pytest.mark.parametrize("T,hist0", [(1, 0), (16, 0), (17, 0), (33, 112), (64, 128), (100, 129), (31, 500), (256, 1024)])
+def test_prompt_attention_equals_the_slabs(T, hist0, H, Hkv):
+    q, k, v = _attention_inputs(T, hist0, H, Hkv, T + hist0 + H)
+    want = _by_slab(q, k, v, hist0)
+    assert torch.equal(_prompt(q, k, v, hist0, calls=2).view(torch.int16), want.view(torch.int16))
+
+
+def test_rows_past_a_history_do_not_reach_it():
+    """Infinities and NaN in K / V rows that a slab may not see stay out of its results."""
+    T, hist0 = 64, 160
+    q, k, v = _attention_inputs(T, hist0, 16, 8, 3)
+    clean = _prompt(q, k, v, hist0)
+    k[:, hist0 + 32:] = float("nan")
+    v[:, hist0 + 32:] = float("inf")
+    got = _prompt(q, k, v, hist0)[:32]
+    assert bool(clean.isfinite().all()) and torch.equal(got.view(torch.int16), clean[:32].view(torch.int16))
