@@ -1095,7 +1095,7 @@ int bm_pack_t2_g128(const void *w, int N, int K, void *packed, void *scale, void
 // ---------------------------------------------------------------------------- prompt (many-row) path
 int bm_t2_gemm_wide(const void *A_prep, const void *a_sums, const void *B, void *C, const void *s, const void *ws, int T,
                     int N, int K, int ldc, int pdl, void *stream) {
-    if (!A_prep || !a_sums || !B || !C || !s || !ws || T < 1 || N < bm::kWideRows || (N % bm::kWideRows) != 0 ||
+    if (!A_prep || !a_sums || !B || !C || !s || !ws || T < 1 || N < 8 || (N % 8) != 0 ||
         K < BM_GROUP || (K % BM_GROUP) != 0 || ldc < N)
         return BM_EINVAL;
     if (!aligned16(A_prep) || !aligned16(B)) return BM_EINVAL;
@@ -1109,7 +1109,7 @@ int bm_t2_gemm_wide(const void *A_prep, const void *a_sums, const void *B, void 
     p.ws = static_cast<const uint16_t *>(ws);
     p.C = static_cast<uint16_t *>(C);
     p.T = T; p.N = N; p.K = K; p.ldc = ldc; p.pdl = pdl & BM_PDL_OVERLAP;
-    const dim3 grid(N / bm::kWideRows, (T + bm::kWideTokens - 1) / bm::kWideTokens);
+    const dim3 grid((N + bm::kWideRows - 1) / bm::kWideRows, (T + bm::kWideTokens - 1) / bm::kWideTokens);
     if (grid.y > 65535) return BM_EINVAL;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (K == BM_SLOTS * BM_GROUP) return launch_ex(bm::t2_gemm_wide_kernel<true>, grid, dim3(bm::kWideThreads), smem, st, p.pdl, p);

@@ -192,7 +192,8 @@ __device__ __forceinline__ void wide_enter_stage(WidePipe &pp, int st) {
     }
 }
 
-// grid (N / 128, ceil(T / 32)), 256 threads.  K % 128 == 0, N % 128 == 0.
+// grid (ceil(N / 128), ceil(T / 32)), 256 threads.  K % 128 == 0, N % 8 == 0: weight rows past N in the last tile
+// repeat row N - 1 and are not stored.
 // ONE: K == 2048, one group per slot - the position in the sequence, its stage and its place in the stage are
 // compile-time constants and the loop over a slot's groups disappears.
 template <bool ONE>
@@ -207,7 +208,7 @@ __global__ void __launch_bounds__(kWideThreads, 2) t2_gemm_wide_kernel(const Wid
     int *nb_tab = reinterpret_cast<int *>(wsm + kWideStages * kWideStageBytes + (((size_t)kWideRows * scs * 2 + 15) & ~(size_t)15));
     float4 *parked = reinterpret_cast<float4 *>(reinterpret_cast<unsigned char *>(nb_tab) + (((size_t)ng * kWideNbStride * 4 + 15) & ~(size_t)15));
     // what this thread copies of every group: its half of a code row, its piece of a prompt row (null: past T)
-    const uint8_t *code_src = p.B + (size_t)(n0 + (tid >> 1)) * (p.K / 4) + 16 * (tid & 1);
+    const uint8_t *code_src = p.B + (size_t)min(n0 + (tid >> 1), p.N - 1) * (p.K / 4) + 16 * (tid & 1);
     const int8_t *row_src = t0 + (tid >> 3) < p.T ? p.A + (size_t)(t0 + (tid >> 3)) * p.K + 16 * (tid & 7) : nullptr;
 
     // Weights first: the codes of the whole ring and the scales do not depend on the previous kernel in
@@ -221,7 +222,7 @@ __global__ void __launch_bounds__(kWideThreads, 2) t2_gemm_wide_kernel(const Wid
 #pragma unroll
     for (int j = 0; j < kWideRows / 32; ++j) {
         const int r = (tid >> 3) + 32 * j;
-        for (int grp = tid & 7; grp < ng; grp += 8) sc_tab[r * scs + grp] = p.ws[(size_t)(n0 + r) * ng + grp];
+        for (int grp = tid & 7; grp < ng; grp += 8) sc_tab[r * scs + grp] = p.ws[(size_t)min(n0 + r, p.N - 1) * ng + grp];
     }
     if (p.pdl) pdl_wait();
     WidePipe pp = {ring, code_src, row_src, {0, 0}, 0, ng};
@@ -289,19 +290,20 @@ __global__ void __launch_bounds__(kWideThreads, 2) t2_gemm_wide_kernel(const Wid
     BM_WIDE_SLOT(13) BM_WIDE_SLOT(14) BM_WIDE_SLOT(15)
 #undef BM_WIDE_SLOT
     // times 1/s of the prompt row, to bf16
-    const int row = n0 + 16 * warp + g;
+    const int row = n0 + 16 * warp + g;                     // N % 8 == 0: the eight rows of a half are in or out together
+    const bool in0 = row < p.N, in8 = row + 8 < p.N;
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
         const int ta = t0 + 8 * b + 2 * q, tb = ta + 1;
         if (ta < p.T) {
             const float is = 1.0f / p.s[ta];
-            p.C[(size_t)ta * p.ldc + row] = bm_f32_to_bf16(tree[b][0][3] * is);
-            p.C[(size_t)ta * p.ldc + row + 8] = bm_f32_to_bf16(tree[b][2][3] * is);
+            if (in0) p.C[(size_t)ta * p.ldc + row] = bm_f32_to_bf16(tree[b][0][3] * is);
+            if (in8) p.C[(size_t)ta * p.ldc + row + 8] = bm_f32_to_bf16(tree[b][2][3] * is);
         }
         if (tb < p.T) {
             const float is = 1.0f / p.s[tb];
-            p.C[(size_t)tb * p.ldc + row] = bm_f32_to_bf16(tree[b][1][3] * is);
-            p.C[(size_t)tb * p.ldc + row + 8] = bm_f32_to_bf16(tree[b][3][3] * is);
+            if (in0) p.C[(size_t)tb * p.ldc + row] = bm_f32_to_bf16(tree[b][1][3] * is);
+            if (in8) p.C[(size_t)tb * p.ldc + row + 8] = bm_f32_to_bf16(tree[b][3][3] * is);
         }
     }
 }

@@ -32,6 +32,20 @@ def _require_cuda(*tensors: torch.Tensor) -> None:
             raise RuntimeError("bitmtp_b200 operators need all tensors on one CUDA device")
 
 
+def _check_packed_operands(a_int8: torch.Tensor, b_packed: torch.Tensor, s: torch.Tensor, ws: torch.Tensor):
+    """(W, N, K) of a packed product after the metadata checks."""
+    _require_cuda(a_int8, b_packed, s, ws)
+    W, K = a_int8.shape
+    N = b_packed.shape[0]
+    if b_packed.shape[1] * 4 != K or tuple(ws.shape) != (N, K // 128):
+        raise RuntimeError("t2_gemv: packed weight / scale shape mismatch")
+    if a_int8.dtype != torch.int8 or ws.dtype != torch.bfloat16 or s.dtype != torch.float32:
+        raise RuntimeError("t2_gemv: invalid activation, scale or multiplier dtype")
+    if s.numel() != W:
+        raise RuntimeError("t2_gemv: one activation multiplier per row is required")
+    return W, N, K
+
+
 def t2_gemv(a_int8: torch.Tensor, b_packed: torch.Tensor, s: torch.Tensor, ws: torch.Tensor, *,
             out_kind: int = native.OUT_BF16, path: int = native.PATH_AUTO,
             want_groups: bool = False, pdl: bool = False, out: Optional[torch.Tensor] = None,
@@ -42,15 +56,7 @@ def t2_gemv(a_int8: torch.Tensor, b_packed: torch.Tensor, s: torch.Tensor, ws: t
     ws [N, K/128] bf16.  Returns C ([W, N] bf16 or fp32 per `out_kind`), or
     (C, G) with G int32 [W, N, K/128] when `want_groups`.
     """
-    _require_cuda(a_int8, b_packed, s, ws)
-    W, K = a_int8.shape
-    N = b_packed.shape[0]
-    if b_packed.shape[1] * 4 != K or tuple(ws.shape) != (N, K // 128):
-        raise RuntimeError("t2_gemv: packed weight / scale shape mismatch")
-    if a_int8.dtype != torch.int8 or ws.dtype != torch.bfloat16 or s.dtype != torch.float32:
-        raise RuntimeError("t2_gemv: invalid activation, scale or multiplier dtype")
-    if s.numel() != W:
-        raise RuntimeError("t2_gemv: one activation multiplier per row is required")
+    W, N, K = _check_packed_operands(a_int8, b_packed, s, ws)
     dt = torch.bfloat16 if out_kind == native.OUT_BF16 else torch.float32
     if out is None:
         out = torch.empty((W, N), dtype=dt, device=a_int8.device)
@@ -271,6 +277,18 @@ def t2_gemm_wide(a_prep: torch.Tensor, a_sums: torch.Tensor, b_packed: torch.Ten
                                       out.stride(0), int(pdl), _stream(a_prep.device))
     check(rc, f"bm_t2_gemm_wide(T={T}, N={N}, K={K})")
     return out
+
+
+GEMM_WIDE_MAX_K = 51200            # its scale and C-operand tables fill the shared memory of an SM there
+GEMM_WIDE_MAX_ROWS = 32 * 65535    # grid.y
+
+
+def t2_linear_rows(x: torch.Tensor, b_packed: torch.Tensor, ws: torch.Tensor) -> torch.Tensor:
+    """Quantise bf16 rows [T, K] and multiply them by the packed weight in two launches, whatever T: bf16 [T, N],
+    every row what t2_gemv gives it."""
+    qp, sums, s = quant_rows(x, prepared=True)
+    T, N, _ = _check_packed_operands(qp, b_packed, s, ws)
+    return t2_gemm_wide(qp, sums, b_packed, s, ws, out=torch.empty((T, N), dtype=torch.bfloat16, device=x.device))
 
 
 def prompt_attention_scratch(T: int, hist0: int, slab_rows: int, H: int, Hkv: int, device) -> torch.Tensor:

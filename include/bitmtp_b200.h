@@ -345,7 +345,7 @@ int bm_pack_t2_g128(const void *w, int N, int K, void *packed, void *scale, void
 /* The packed product for MANY rows at once (a prompt): C bf16 [T, ldc] = the value bm_t2_gemv_prepared
  * gives every row alone, bit for bit, with each weight byte read once per 32 rows instead of once per
  * GEMV launch.  A_prep / a_sums / s: GEMV-ready INT8 rows, their group sums and multipliers for T rows;
- * N % 128 == 0, K % 128 == 0.  Tensor-core kernel (mma.sync int8, exact int32 group sums, the GEMV's
+ * N % 8 == 0, K % 128 == 0.  Tensor-core kernel (mma.sync int8, exact int32 group sums, the GEMV's
  * fp32 order).  Replaces the dense bf16 fallback of T2LinearKernel.forward behind forward_sdlm_prefill
  * (src/bonsai_sft/gpu/model.py:650-656, 1306-1340). */
 int bm_t2_gemm_wide(const void *A_prep, const void *a_sums, const void *B, void *C, const void *s, const void *ws,

@@ -4,7 +4,8 @@ GEMV in slabs."""
 import pytest
 import torch
 
-from bitmtp_b200 import native, ops
+from bitmtp_b200 import native, ops, synthetic
+from bitmtp_b200.model import T2LinearKernel
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -64,3 +65,21 @@ def test_rows_past_a_history_do_not_reach_it():
     v[:, hist0 + 32:] = float("inf")
     got = _prompt(q, k, v, hist0)[:32]
     assert bool(clean.isfinite().all()) and torch.equal(got.view(torch.int16), clean[:32].view(torch.int16))
+
+
+@pytest.mark.parametrize("N,K", [(8, 128), (136, 384), (200, 2048), (504, 2560), (1024, 9728), (512, 2048)])
+@pytest.mark.parametrize("rows", [16, 17, 33, 333])
+def test_linear_module_equals_the_gemv_in_slabs(N, K, rows):
+    """Row counts on both sides of the module's change to the many-row kernel, weights that end inside one of its
+    tiles of 128 rows, K with and without a whole number of its stages."""
+    gen = torch.Generator(device=DEV).manual_seed(N + K + rows)
+    packed, scale = synthetic.device_ternary(N, K, gen, torch.device(DEV))
+    layer = T2LinearKernel(K, N).to(DEV)
+    layer.weight.data, layer.weight_scale = packed, scale
+    x = torch.randn(1, rows, K, generator=gen, device=DEV).to(torch.bfloat16)
+    q, s = ops.quant_rows(x[0])
+    want = torch.cat([ops.t2_gemv(q[r:r + SLAB], packed, s[r:r + SLAB], scale) for r in range(0, rows, SLAB)])
+    got = layer(x)
+    torch.cuda.synchronize()
+    assert native.lib().bm_device_error() == 0
+    assert got.shape == (1, rows, N) and torch.equal(got[0].view(torch.int16), want.view(torch.int16))
