@@ -247,8 +247,9 @@ class _Session:
         self.sigma = atlas.select_segment(self.seq_len + self.max_gen_len + atlas.M_max)
         shared = atlas.kv_buffers[self.sigma]
         shared.zero_()
-        if getattr(atlas, "prefill_graphs", None) and self.seq_len <= self.sigma:
-            # captured slab graphs write the prompt's rows straight into the segment
+        takes_prompt = getattr(atlas, "takes_prompt", None)
+        if takes_prompt is not None and takes_prompt(self.seq_len, self.sigma):
+            # the prompt's rows go straight into the segment, and only the last one through the head
             logits = atlas.prefill(self.prompt_ids, self.sigma)
         else:
             cache = make_sdlm_cache(self.args, device=self.device)

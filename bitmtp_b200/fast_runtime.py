@@ -264,6 +264,14 @@ class GraphAtlas:
         sigma = verify_graph.sigma
         ops.kv_copy_rows(self.kv_buffers[sigma], sigma + self.M_max, sigma + 1, cache_len, n_accept)
 
+    def takes_prompt(self, seq: int, sigma: int) -> bool:
+        """Whether `prefill` serves a prompt of `seq` rows in segment `sigma`: by the many-row kernels, whatever
+        widths the atlas holds, or by the slab graph, which an atlas of at least PREFILL_CHUNK rows captures."""
+        graphs = getattr(self, "prefill_graphs", None)
+        if graphs is None or not 1 <= seq <= sigma:
+            return False
+        return bool(graphs) or (seq > PREFILL_CHUNK and self.model.wide_prefill_supported())
+
     def prefill(self, prompt_ids: torch.Tensor, sigma: int) -> torch.Tensor:
         """The prompt's K/V into history rows [0, len) of segment `sigma`, by replaying the captured
         slab graph once per PREFILL_CHUNK rows (staging, replay, row promotion: three launches + one
