@@ -454,6 +454,7 @@ class Transformer(nn.Module):
             layer.attention.prepare_merged_weights(max_positions, tables=tables)
             layer.feed_forward.prepare_merged_weights()
         self.max_positions = max_positions
+        self.__dict__.get("_prompt_waves", {}).clear()          # captured waves hold the tensors replaced above
 
     def _ar_fused_supported(self, M: int) -> bool:
         a = self.args
@@ -685,8 +686,9 @@ class Transformer(nn.Module):
             kl, vl = _LayerView(k_l, kv_rows), _LayerView(v_l, kv_rows)
             ops.qknorm_rope_kvappend(ws.xqkv[:T], at.q_norm.weight.data, at.k_norm.weight.data, eps, at.rope_cos,
                                      at.rope_sin, pos, a.n_heads, a.n_kv_heads, kl, vl, hist0, pdl=pdl, q_out=ws.qrot[:T])
-            ops.prompt_attention(ws.qrot[:T], kl, vl, hist0, PREFILL_CHUNK, scratch, att=ws.att[:T],
-                                 amax=ws.att_amax[i & 1][:T], pdl=pdl)
+            for a0, a1 in self._prompt_attn_calls(T):
+                ops.prompt_attention(ws.qrot[a0:a1], kl, vl, hist0 + a0, PREFILL_CHUNK, scratch, att=ws.att[a0:a1],
+                                     amax=ws.att_amax[i & 1][a0:a1], pdl=pdl)
             ops.quant_rows_amax(ws.att[:T], ws.att_amax[i & 1][:T], prep=(ws.att_q[:T], ws.att_sum[:T]), s=ws.att_s[:T],
                                 amax_zero=ws.att_amax[(i + 1) & 1][:T], pdl=pdl)
             ops.t2_gemm_wide(ws.att_q[:T], ws.att_sum[:T], at.o_proj.weight.data, ws.att_s[:T], at.o_proj.weight_scale,
@@ -698,24 +700,40 @@ class Transformer(nn.Module):
             ops.t2_gemm_wide(ws.iq[:T], ws.i_sum[:T], ff.down_proj.weight.data, ws.is_[:T], ff.down_proj.weight_scale,
                              out=ws.ffn_out[:T], pdl=pdl)
 
+    def _prompt_attn_calls(self, T: int) -> List[Tuple[int, int]]:
+        """Row ranges of a wave's attention calls.  One call where the head grouping keeps the general kernel: its
+        ticket counters return to zero at places that depend on the number of rows, so calls of different sizes
+        cannot share a scratch."""
+        step = PREFILL_ATTN_ROWS if self.args.n_heads // self.args.n_kv_heads in (1, 2, 4, 8) else T
+        return [(a0, min(T, a0 + step)) for a0 in range(0, T, step)]
+
+    def _prompt_scratch(self, n: int, c0: int, dev) -> torch.Tensor:
+        """Scratch for every attention call of a wave: the calls' rows differ in number only at the end of the wave,
+        and a later call never needs fewer super-chunks, so the largest of the last two is the largest."""
+        a = self.args
+        sizes = [(a1 - a0, c0 + a0) for a0, a1 in self._prompt_attn_calls(n)[-2:]]
+        return max((ops.prompt_attention_scratch(t, h, PREFILL_CHUNK, a.n_heads, a.n_kv_heads, dev) for t, h in sizes),
+                   key=torch.Tensor.numel)
+
     @torch.no_grad()
     def prefill_wide(self, token_values: torch.Tensor, kv_planes: List[SDLMLayerCache], kv_rows: int,
                      logits_buf: Optional[torch.Tensor] = None) -> torch.Tensor:
-        """The whole prompt through prefill_rows_wide in waves of PREFILL_WAVE rows, then the packed head on
+        """The whole prompt through prefill_rows_wide in waves (prompt_waves), then the packed head on
         the last row (the only logit row a decode loop uses).  Returns fp32 logits [1, vocab]."""
         seq = int(token_values.shape[0])
         dev = token_values.device
         a = self.args
         self.prepare_t2_lm_head()
-        wave = min(PREFILL_WAVE, (seq + PREFILL_CHUNK - 1) // PREFILL_CHUNK * PREFILL_CHUNK)
+        waves = prompt_waves(seq)
+        rows = (max(n for _, n in waves) + PREFILL_CHUNK - 1) // PREFILL_CHUNK * PREFILL_CHUNK
         ws = getattr(self, "_prompt_ws", None)
-        if ws is None or ws.T < wave:
-            ws = self._prompt_ws = PromptWorkspace(a, max(wave, PREFILL_WAVE if seq > PREFILL_WAVE else wave), dev)
+        cache = self.__dict__.setdefault("_prompt_waves", {})
+        if ws is None or ws.T < rows:
+            cache.clear()                        # captured waves read and write the workspace they were captured with
+            ws = self._prompt_ws = PromptWorkspace(a, rows, dev)
         ids = token_values.to(torch.int64).contiguous()
         n = 0
-        cache = self.__dict__.setdefault("_prompt_waves", {})
-        for c0 in range(0, seq, wave):
-            n = min(wave, seq - c0)
+        for c0, n in waves:
             # Per (rows, first position, KV buffer): the attention scratch, the position ids and, from the
             # second prompt of that shape on, a CUDA graph of the wave (about 280 launches whose host cost
             # would otherwise exceed their device time).  The graph reads its ids from ws.tokens.
@@ -724,8 +742,7 @@ class Transformer(nn.Module):
             if rec is None:
                 if len(cache) > 32:
                     cache.clear()
-                rec = cache[key] = {"scratch": ops.prompt_attention_scratch(n, c0, PREFILL_CHUNK, a.n_heads,
-                                                                            a.n_kv_heads, dev),
+                rec = cache[key] = {"scratch": self._prompt_scratch(n, c0, dev),
                                     "pos": torch.arange(c0, c0 + n, device=dev, dtype=torch.int64), "uses": 0,
                                     "graph": None}
             rec["uses"] += 1
@@ -791,7 +808,21 @@ class Transformer(nn.Module):
 
 
 PREFILL_CHUNK = 16
-PREFILL_WAVE = 256          # prompt rows one pass of the many-row path takes
+PREFILL_WAVE = 1024         # prompt rows one pass of the many-row path takes
+PREFILL_TAIL = 256          # a last pass shorter than this joins the one before it
+PREFILL_ATTN_ROWS = 512     # rows per attention call: its partials (16 heads, 24 super-chunks: 98 MB) stay in L2
+
+
+def prompt_waves(seq: int) -> List[Tuple[int, int]]:
+    """(first row, rows) of the passes a prompt is cut into.  A pass of 256 rows leaves the 2048-row projections
+    at 128 CTAs, under half of the CTAs the device holds, and pays every launch of a layer four times as often as
+    one of 1024; a short last pass costs most of what a whole one of 256 does."""
+    waves, c0 = [], 0
+    while c0 < seq:
+        n = seq - c0 if seq - c0 < PREFILL_WAVE + PREFILL_TAIL else PREFILL_WAVE
+        waves.append((c0, n))
+        c0 += n
+    return waves
 
 
 class PromptWorkspace:

@@ -172,7 +172,7 @@ def test_atlas_prefill_equals_operator_prefill(geometry, seq, monkeypatch):
     """GraphAtlas.prefill against Transformer.forward_sdlm_prefill (the slab-by-slab prompt forward,
     every operator launched from the host, rows written in place): the prompt's K/V rows in every layer
     and the last row's logits, bit for bit.  Prompts longer than a slab go through the many-row kernels
-    (bm_t2_gemm_wide, bm_prompt_attention; 300 rows = two waves), shorter ones through the captured slab
+    (bm_t2_gemm_wide, bm_prompt_attention), shorter ones through the captured slab
     graph; with BM_WIDE_PREFILL=0 every length goes through the slab graphs."""
     geo = {"tiny": synthetic.TINY, "layers3": dict(synthetic.BONSAI_1P7B, n_layers=3, vocab_size=4096),
            "cut4b": dict(synthetic.BONSAI_4B, n_layers=2, vocab_size=4096)}[geometry]

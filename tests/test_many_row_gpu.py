@@ -1,11 +1,12 @@
 """The many-row paths of a prompt against the decode operators, row for row and bit for bit: the prompt attention
 (history tiles + one merge per slab) against slab-by-slab verify attention, and the packed linear module against the
-GEMV in slabs."""
+GEMV in slabs; whole prompts against the operator-by-operator forward."""
 import pytest
 import torch
 
-from bitmtp_b200 import native, ops, synthetic
-from bitmtp_b200.model import T2LinearKernel
+from bitmtp_b200 import generate, native, ops, synthetic
+from bitmtp_b200.fast_runtime import GraphAtlas
+from bitmtp_b200.model import T2LinearKernel, make_sdlm_cache
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -83,3 +84,36 @@ def test_linear_module_equals_the_gemv_in_slabs(N, K, rows):
     torch.cuda.synchronize()
     assert native.lib().bm_device_error() == 0
     assert got.shape == (1, rows, N) and torch.equal(got[0].view(torch.int16), want.view(torch.int16))
+
+
+def _packed_model(geo, max_positions):
+    cfg = synthetic.make_config(geo, block_size=8)
+    state = synthetic.make_state(cfg, seed=4)
+    model = generate.model_from_state(generate.args_from_config(cfg), state, DEV)
+    model.prepare_merged_weights(max_positions=max_positions)
+    return cfg, model
+
+
+@pytest.mark.parametrize("heads", [(16, 8), (6, 2)])
+def test_long_prompts_equal_the_operator_prefill(heads):
+    """Prompts of one pass with several attention calls (600, 1200 rows) and of two passes (1300), an AR-only atlas,
+    and short prompts before and after the workspace has grown (a pass captured with the old one must not come
+    back): last-row logits and K / V rows bit for bit those of the operator-by-operator forward."""
+    geo = dict(synthetic.TINY, n_heads=heads[0], n_kv_heads=heads[1], dim=512, ffn_dim=512)
+    cfg, model = _packed_model(geo, 1601)
+    sigma = 1600
+    atlas = GraphAtlas(model, model.args, torch.device(DEV), segment_ladder=(sigma,), m_set=(1,), roles=("ar",),
+                       capture_verbose=False)
+    for seq in (40, 40, 600, 40, 1200, 1300, 1300, 40):
+        assert atlas.takes_prompt(seq, sigma)
+        prompt = synthetic.random_prompt(seq, cfg["vocab_size"], seed=seq)[0].to(DEV)
+        cache = make_sdlm_cache(model.args, device=torch.device(DEV))
+        want = model.forward_sdlm_prefill(token_values=prompt, cache=cache)[-1:].clone()
+        atlas.kv_buffers[sigma].zero_()
+        got = atlas.prefill(prompt, sigma)
+        torch.cuda.synchronize()
+        assert native.lib().bm_device_error() == 0
+        assert torch.equal(got.view(torch.int32), want.view(torch.int32)), seq
+        for i, (ck, cv) in enumerate(cache):
+            for j, c in enumerate((ck, cv)):
+                assert torch.equal(atlas.kv_buffers[sigma][j, i, 0, :, :seq].view(torch.int16), c[0].view(torch.int16)), (seq, i)
