@@ -1126,7 +1126,9 @@ bool prompt_attn_plan(int T, int hist0, int slab_rows, int H, int Hkv, PromptAtt
     for (int s = 0; s < pl->n_slabs; ++s) pl->units += (hist0 + s * slab_rows + BM_ATTN_SUPER - 1) / BM_ATTN_SUPER + 1;
     pl->NJ = (hist0 + T + BM_ATTN_SUPER - 1) / BM_ATTN_SUPER + 1;
     bm::attn_query_split((H / Hkv) * slab_rows, &pl->nq, &pl->Z);
-    pl->ticket_bytes = ((size_t)pl->n_slabs * Hkv * pl->Z * 4 + 1023) / 1024 * 1024;
+    // at least 64 KB: calls of different T (up to 512 rows for any head count in use) then keep their counters in one
+    // place, which no call's partials touch, and can share a scratch
+    pl->ticket_bytes = ((size_t)pl->n_slabs * Hkv * pl->Z * 4 + 65535) / 65536 * 65536;
     pl->total = pl->ticket_bytes + (size_t)T * H * pl->NJ * 4 * 2 + (size_t)T * H * pl->NJ * 128 * 4;
     return pl->NJ <= bm::kAttnMaxNJ;
 }
@@ -1159,11 +1161,16 @@ int bm_prompt_attention(const void *q, const void *k_base, const void *v_base, i
     p.pdl = pdl & BM_PDL_OVERLAP;
     p.slab_rows = slab_rows;
     p.slab_hist0 = hist0;
-    if (bm::prompt_hist_fits(slab_rows, H, Hkv)) {
+    // The history by tiles where the general kernel's CTAs would fill the machine (two per SM) more than six times.
+    // Below that a tile's latency is the longer one: 19 rows 28 us against 8, 256 rows 56 against 42, 64 rows behind
+    // 1024 keys 50 against 48; above it, 333 rows 63 against 61, 512 rows 90 against 114, 512 rows behind 2048 keys
+    // 356 against 659 (16 heads; 32 heads change sides at the same fill).
+    const long long general_ctas = (long long)pl.units * Hkv * pl.Z;
+    if (bm::prompt_hist_fits(slab_rows, H, Hkv) && general_ctas > 6LL * 2 * current_device().sm_count) {
         // history super-chunks by tiles of 64 query vectors, then one CTA set per slab for its own rows and the merge
         const int hist_end = hist0 + (pl.n_slabs - 1) * slab_rows, G = H / Hkv;
         if (hist_end > 0) {
-            const bm::PromptHistParams hp{p.q, p.k_base, p.v_base, p.pm, p.pl, p.po, T, H, Hkv, G, kv_rows, hist0, pl.NJ, p.pdl};
+            const bm::PromptHistParams hp{p.q, p.k_base, p.v_base, p.pm, p.pl, p.po, T, H, Hkv, __builtin_ctz(G), kv_rows, hist0, pl.NJ, p.pdl};
             const dim3 hgrid((hist_end + BM_ATTN_SUPER - 1) / BM_ATTN_SUPER, Hkv, (T * G + bm::kPaQueries - 1) / bm::kPaQueries);
             const int rc = launch_ex(bm::prompt_hist_kernel, hgrid, dim3(bm::kPaThreads), bm::kPaSmem,
                                      static_cast<cudaStream_t>(stream), p.pdl, hp);

@@ -12,7 +12,9 @@
 // Bound by the fp32 pipe: 2 * 128 multiply-adds per (query vector, key).  Every one of them is the fma of
 // attn_sub_pass, in the same chain (scores ascending in d, numerators ascending in the key, sub-chunks
 // ascending, the weight sum as the butterfly over the 32 keys), so the partials are the same bits; tensor
-// cores would not give that order.
+// cores would not give that order.  512 rows behind 2048 keys, 16 heads: 659 us by attn_fused_kernel alone, 414 us
+// with scalar fmas (issue slots 56 % busy, a quarter of the instructions not fmas), 356 us with packed ones and
+// bm_expf without branches and conversions; the fmas alone are 134 us at the fp32 rate.
 #pragma once
 
 #include "verify_attn.cuh"
@@ -29,7 +31,7 @@ struct PromptHistParams {
     const uint16_t *q;                   // [T, H, 128] rotated queries
     const uint16_t *k_base, *v_base;     // [Hkv, kv_rows, 128]
     float *pm, *pl, *po;                 // [T, H, NJ] and [T, H, NJ, 128]
-    int T, H, Hkv, G, kv_rows, hist0, NJ, pdl;
+    int T, H, Hkv, log_g, kv_rows, hist0, NJ, pdl;      // 2^log_g heads per kv head
 };
 
 // Q^T fp32 [128][kPaQStride] (after the scores its space holds P^T fp32 [128][64], see pa_weight), K^T bf16
@@ -51,15 +53,26 @@ __device__ __forceinline__ int pa_history(int hist0, int r) { return hist0 + r /
 // threads of a warp, eight keys apart, then store to different banks.  Vectors 8 vg + 4 .. + 7 are at ^ 4 words.
 __device__ __forceinline__ int pa_weight(int key, int vg) { return key * kPaQueries + 4 * ((2 * vg) ^ (key >> 3)); }
 
-// One step of the register-blocked products: acc[t][j] = fma(a[t], b[j], acc[t][j]).
-__device__ __forceinline__ void pa_step(float (&acc)[8][8], const float4 &a0, const float4 &a1, const uint4 &braw) {
+// One step of the register-blocked products: acc[t][j] = fma(a[t], b[j], acc[t][j]), vectors t in pairs: the packed
+// fma rounds each half as the scalar one does, runs at the same rate per value and takes half the issue slots.
+typedef unsigned long long PaPair;
+__device__ __forceinline__ PaPair pa_pack(float lo, float hi) {
+    PaPair v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ void pa_unpack(PaPair v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ void pa_step(PaPair (&acc)[4][8], const float *a, const float *a4, const uint4 &braw) {
     float b[8];
     unpack8(braw, b);
-    const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+    const ulonglong2 lo = *reinterpret_cast<const ulonglong2 *>(a), hi = *reinterpret_cast<const ulonglong2 *>(a4);
+    const PaPair av[4] = {lo.x, lo.y, hi.x, hi.y};
 #pragma unroll
-    for (int t = 0; t < 8; ++t)
+    for (int j = 0; j < 8; ++j) {
+        const PaPair bb = pa_pack(b[j], b[j]);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[t][j] = fmaf(a[t], b[j], acc[t][j]);
+        for (int t = 0; t < 4; ++t) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[t][j]) : "l"(av[t]), "l"(bb));
+    }
 }
 
 // grid (super-chunks of the longest history, Hkv, ceil(T * G / 64)), 128 threads = 8 vector groups x 16 key
@@ -69,7 +82,7 @@ __global__ void __launch_bounds__(kPaThreads, 2) prompt_hist_kernel(const Prompt
     pdl_launch_dependents();
     if (p.pdl) pdl_wait();
     const int J = blockIdx.x, hk = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int rows = kPaQueries / p.G, row0 = blockIdx.z * rows;      // this tile's prompt rows
+    const int gmask = (1 << p.log_g) - 1, rows = kPaQueries >> p.log_g, row0 = blockIdx.z * rows;      // this tile's prompt rows
     const int row_end = min(row0 + rows, p.T);
     const int key0 = J * BM_ATTN_SUPER;
     const int keys_max = min(BM_ATTN_SUPER, pa_history(p.hist0, row_end - 1) - key0);
@@ -102,7 +115,7 @@ __global__ void __launch_bounds__(kPaThreads, 2) prompt_hist_kernel(const Prompt
             }
         }
         const int v = lane + 32 * (warp & 1);                         // vector v of the tile: row v / G, head v % G
-        const int r = row0 + v / p.G, head = hk * p.G + v % p.G;
+        const int r = row0 + (v >> p.log_g), head = (hk << p.log_g) + (v & gmask);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             const int d0 = 8 * ((warp >> 1) + 2 * j);
@@ -118,23 +131,26 @@ __global__ void __launch_bounds__(kPaThreads, 2) prompt_hist_kernel(const Prompt
     const int vgp = tid >> 4, kgp = tid & 15;                         // vector group, key / dim group
     const int v0 = 8 * vgp;
     // keys of this super-chunk that this thread's vectors see (one slab, the same for the whole warp)
-    const int my_row = row0 + v0 / p.G;
+    const int my_row = row0 + (v0 >> p.log_g);
     const int lim = my_row < p.T ? min(BM_ATTN_SUPER, pa_history(p.hist0, my_row) - key0) : 0;
 
-    float acc[8][8];                                                  // [vector][key]
+    PaPair acc2[4][8];                                                // [vector pair][key]
 #pragma unroll
-    for (int t = 0; t < 8; ++t)
+    for (int t = 0; t < 4; ++t)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[t][j] = 0.0f;
+        for (int j = 0; j < 8; ++j) acc2[t][j] = 0ull;
     if (lim > 0) {
         const float *qp = Qt + v0;
         const uint16_t *kp = Kt + 8 * kgp;
 #pragma unroll 4
         for (int d = 0; d < 128; ++d)
-            pa_step(acc, *reinterpret_cast<const float4 *>(qp + d * kPaQStride),
-                    *reinterpret_cast<const float4 *>(qp + d * kPaQStride + 4),
-                    *reinterpret_cast<const uint4 *>(kp + d * kPaKStride));
+            pa_step(acc2, qp + d * kPaQStride, qp + d * kPaQStride + 4, *reinterpret_cast<const uint4 *>(kp + d * kPaKStride));
     }
+    float acc[8][8];                                                  // [vector][key], then [vector][dim]
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) pa_unpack(acc2[t][j], acc[2 * t][j], acc[2 * t + 1][j]);
     __syncthreads();                                                  // Q^T is spent: its space takes P^T
     const int c = kgp >> 2;                                           // sub-chunk of this thread's keys
 #pragma unroll
@@ -184,9 +200,9 @@ __global__ void __launch_bounds__(kPaThreads, 2) prompt_hist_kernel(const Prompt
     }
     for (int s = 0; s < kAttnSub; ++s) {
 #pragma unroll
-        for (int t = 0; t < 8; ++t)
+        for (int t = 0; t < 4; ++t)
 #pragma unroll
-            for (int e = 0; e < 8; ++e) acc[t][e] = 0.0f;
+            for (int e = 0; e < 8; ++e) acc2[t][e] = 0ull;
         const int cn = min(BM_ATTN_CHUNK, lim - s * BM_ATTN_CHUNK);
         for (int k8 = 0; k8 < cn; k8 += 8) {
             const int key = s * BM_ATTN_CHUNK + k8, w = pa_weight(key, vgp);
@@ -194,16 +210,18 @@ __global__ void __launch_bounds__(kPaThreads, 2) prompt_hist_kernel(const Prompt
             if (cn - k8 >= 8) {
 #pragma unroll
                 for (int k = 0; k < 8; ++k)
-                    pa_step(acc, *reinterpret_cast<const float4 *>(Pt + w + k * kPaQueries),
-                            *reinterpret_cast<const float4 *>(Pt + (w ^ 4) + k * kPaQueries),
+                    pa_step(acc2, Pt + w + k * kPaQueries, Pt + (w ^ 4) + k * kPaQueries,
                             *reinterpret_cast<const uint4 *>(vp + k * 128));
             } else {                                                  // a history that ends inside the eight keys
                 for (int k = 0; k < cn - k8; ++k)
-                    pa_step(acc, *reinterpret_cast<const float4 *>(Pt + w + k * kPaQueries),
-                            *reinterpret_cast<const float4 *>(Pt + (w ^ 4) + k * kPaQueries),
+                    pa_step(acc2, Pt + w + k * kPaQueries, Pt + (w ^ 4) + k * kPaQueries,
                             *reinterpret_cast<const uint4 *>(vp + k * 128));
             }
         }
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) pa_unpack(acc2[t][e], acc[2 * t][e], acc[2 * t + 1][e]);
 #pragma unroll
         for (int t = 0; t < 8; ++t) {
             const float m = mc[s * kPaQueries + v0 + t];
@@ -215,7 +233,7 @@ __global__ void __launch_bounds__(kPaThreads, 2) prompt_hist_kernel(const Prompt
     }
 #pragma unroll
     for (int t = 0; t < 8; ++t) {
-        const int r = row0 + (v0 + t) / p.G, head = hk * p.G + (v0 + t) % p.G;
+        const int r = row0 + ((v0 + t) >> p.log_g), head = (hk << p.log_g) + ((v0 + t) & gmask);
         if (r >= p.T) continue;
         const size_t pb = ((size_t)r * p.H + head) * p.NJ + J;
         float *dst = p.po + pb * 128 + 8 * kgp;

@@ -10,7 +10,6 @@ libbitmtp_b200.so; PyTorch only owns the memory and the stream.
 """
 from __future__ import annotations
 
-import ctypes
 import math
 import os
 from dataclasses import dataclass
@@ -41,24 +40,25 @@ def _validate_packed_inputs(a, b, s, ws, *, kind: str = "t2g128", bits: int = 2,
     loaded, so a bad call fails without touching CUDA."""
     if a.dim() not in (2, 3) or b.dim() != 2:
         raise ValueError(f"{kind}: expected rank-2/3 activation and rank-2 weight")
-    m = a.numel() // a.shape[-1] if a.shape[-1] else 0
+    a_k, dev = a.shape[-1], a.device
+    m = a.numel() // a_k if a_k else 0
     n, k = b.shape[0], b.shape[1] * (8 // bits)
     if validate_registry:
         require_kernel_shape(kind, m, n, k)
     else:
         require_native_shape(m, n, k)
-    if a.shape[-1] != k:
-        raise RuntimeError(f"{kind}: activation width mismatch: {a.shape[-1]} != {k}")
-    if tuple(ws.shape) != (n, k // 128):
+    if a_k != k:
+        raise RuntimeError(f"{kind}: activation width mismatch: {a_k} != {k}")
+    if ws.shape != (n, k // 128):
         raise RuntimeError(f"{kind}: invalid weight scale shape {tuple(ws.shape)}")
     if a.dtype != activation_dtype or b.dtype != torch.int8 or ws.dtype != torch.bfloat16:
         raise RuntimeError(f"{kind}: invalid activation, packed-weight, or scale dtype")
     if s.dtype != torch.float32 or s.shape[-1:] != (1,) or s.numel() != m:
         raise RuntimeError(f"{kind}: activation scales must be float32 with one value per row")
-    tensors = (a, b, s, ws)
-    if not all(t.is_cuda and t.is_contiguous() for t in tensors):
+    if not (a.is_cuda and b.is_cuda and s.is_cuda and ws.is_cuda and a.is_contiguous() and b.is_contiguous()
+            and s.is_contiguous() and ws.is_contiguous()):
         raise RuntimeError(f"{kind}: inputs and scales must be contiguous CUDA tensors")
-    if not all(t.device == a.device for t in tensors):
+    if not (b.device == dev and s.device == dev and ws.device == dev):
         raise RuntimeError(f"{kind}: inputs and scales must share one CUDA device")
     return m, n, k
 
@@ -76,13 +76,12 @@ def t2g128_int8xint2_linear(a_int8: torch.Tensor, b_packed: torch.Tensor, s: tor
     m, n, k = _validate_packed_inputs(a_int8, b_packed, s, ws, validate_registry=validate_registry)
     if _t2_lib is None:
         load_t2_kernel()
-    out_shape = (*a_int8.shape[:-1], n)
-    out = torch.empty(out_shape, dtype=torch.bfloat16, device=a_int8.device)
-    stream = torch.cuda.current_stream(a_int8.device)
-    _t2_lib.t2g128_int8xint2_linear(
-        ctypes.c_void_p(a_int8.data_ptr()), ctypes.c_void_p(b_packed.data_ptr()),
-        ctypes.c_void_p(out.data_ptr()), ctypes.c_void_p(s.data_ptr()),
-        ctypes.c_void_p(ws.data_ptr()), m, n, k, ctypes.c_void_p(stream.cuda_stream))
+    dev = a_int8.device
+    out = torch.empty((*a_int8.shape[:-1], n), dtype=torch.bfloat16, device=dev)
+    # plain integers through the declared prototype: this call is bound by the host, and wrapping each pointer and
+    # building a Stream object for its handle cost as much as the launch itself
+    _t2_lib.t2g128_int8xint2_linear(a_int8.data_ptr(), b_packed.data_ptr(), out.data_ptr(), s.data_ptr(), ws.data_ptr(),
+                                    m, n, k, ops._stream(dev))
     return out
 
 
@@ -701,11 +700,8 @@ class Transformer(nn.Module):
                              out=ws.ffn_out[:T], pdl=pdl)
 
     def _prompt_attn_calls(self, T: int) -> List[Tuple[int, int]]:
-        """Row ranges of a wave's attention calls.  One call where the head grouping keeps the general kernel: its
-        ticket counters return to zero at places that depend on the number of rows, so calls of different sizes
-        cannot share a scratch."""
-        step = PREFILL_ATTN_ROWS if self.args.n_heads // self.args.n_kv_heads in (1, 2, 4, 8) else T
-        return [(a0, min(T, a0 + step)) for a0 in range(0, T, step)]
+        """Row ranges of a wave's attention calls."""
+        return [(a0, min(T, a0 + PREFILL_ATTN_ROWS)) for a0 in range(0, T, PREFILL_ATTN_ROWS)]
 
     def _prompt_scratch(self, n: int, c0: int, dev) -> torch.Tensor:
         """Scratch for every attention call of a wave: the calls' rows differ in number only at the end of the wave,

@@ -49,9 +49,11 @@ def _prompt(q, k, v, hist0, calls=1):
     return att[:T]
 
 
-@pytest.mark.parametrize("H,Hkv", [(2, 2), (16, 8), (32, 8), (8, 1), (6, 2)])      # 1, 2, 4, 8 and (general kernel) 3 heads per group
-@pytest.mark.parametrize("T,hist0", [(1, 0), (16, 0), (17, 0), (33, 112), (64, 128), (100, 129), (31, 500), (256, 1024)])
+@pytest.mark.parametrize("H,Hkv", [(2, 2), (8, 8), (16, 8), (32, 8), (8, 1), (6, 2)])      # 1, 1, 2, 4, 8 and (general kernel) 3 heads per group
+@pytest.mark.parametrize("T,hist0", [(1, 0), (16, 0), (17, 0), (33, 112), (64, 128), (100, 129), (31, 500), (256, 1024),
+                                     (500, 129), (1000, 16), (47, 4096)])
 def test_prompt_attention_equals_the_slabs(T, hist0, H, Hkv):
+    """Calls on both sides of the line between the tiles and the general kernel, ragged last tiles and slabs."""
     q, k, v = _attention_inputs(T, hist0, H, Hkv, T + hist0 + H)
     want = _by_slab(q, k, v, hist0)
     assert torch.equal(_prompt(q, k, v, hist0, calls=2).view(torch.int16), want.view(torch.int16))
@@ -59,13 +61,13 @@ def test_prompt_attention_equals_the_slabs(T, hist0, H, Hkv):
 
 def test_rows_past_a_history_do_not_reach_it():
     """Infinities and NaN in K / V rows that a slab may not see stay out of its results."""
-    T, hist0 = 64, 160
-    q, k, v = _attention_inputs(T, hist0, 16, 8, 3)
-    clean = _prompt(q, k, v, hist0)
-    k[:, hist0 + 32:] = float("nan")
-    v[:, hist0 + 32:] = float("inf")
-    got = _prompt(q, k, v, hist0)[:32]
-    assert bool(clean.isfinite().all()) and torch.equal(got.view(torch.int16), clean[:32].view(torch.int16))
+    for T, hist0, keep in ((64, 160, 32), (512, 160, 400)):       # the general kernel, the tiles
+        q, k, v = _attention_inputs(T, hist0, 16, 8, 3)
+        clean = _prompt(q, k, v, hist0)
+        k[:, hist0 + keep:] = float("nan")
+        v[:, hist0 + keep:] = float("inf")
+        got = _prompt(q, k, v, hist0)[:keep]
+        assert bool(clean.isfinite().all()) and torch.equal(got.view(torch.int16), clean[:keep].view(torch.int16))
 
 
 @pytest.mark.parametrize("N,K", [(8, 128), (136, 384), (200, 2048), (504, 2560), (1024, 9728), (512, 2048)])
