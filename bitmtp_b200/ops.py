@@ -6,7 +6,6 @@ of them computes anything in PyTorch.
 """
 from __future__ import annotations
 
-import ctypes
 from typing import Optional, Tuple
 
 import torch
@@ -16,11 +15,13 @@ from .native import check
 
 
 def _ptr(t: Optional[torch.Tensor]):
-    return None if t is None else ctypes.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
-def _stream(device) -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+def _stream(device) -> int:
+    """Handle of torch's current stream on `device`, without the Stream object torch.cuda.current_stream builds."""
+    index = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
 def _require_cuda(*tensors: torch.Tensor) -> None:
