@@ -14,7 +14,7 @@
 // ascending, the weight sum as the butterfly over the 32 keys), so the partials are the same bits; tensor
 // cores would not give that order.  512 rows behind 2048 keys, 16 heads: 659 us by attn_fused_kernel alone, 414 us
 // with scalar fmas (issue slots 56 % busy, a quarter of the instructions not fmas), 356 us with packed ones and
-// bm_expf without branches and conversions; the fmas alone are 134 us at the fp32 rate.
+// an exponential without branches and conversions; the fmas alone are 134 us at the fp32 rate.
 #pragma once
 
 #include "verify_attn.cuh"
@@ -73,6 +73,26 @@ __device__ __forceinline__ void pa_step(PaPair (&acc)[4][8], const float *a, con
 #pragma unroll
         for (int t = 0; t < 4; ++t) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[t][j]) : "l"(av[t]), "l"(bb));
     }
+}
+
+// bm_expf for x <= 0, infinities or NaN, without its branches and the two conversions that issue at a quarter of the
+// rate; the same values: adding 1.5 * 2^23 rounds |t| < 2^22 to the nearest even integer and leaves it in the low bits,
+// and the exponent, -126 .. 0, goes in with one exact step.  Kept here: in the decode kernels, which evaluate a few per
+// thread, the branch is cheaper (whole requests 0.7 % slower without it).
+__device__ __forceinline__ float pa_expf(float x) {
+    const float biased = x * 1.44269504088896341f + 12582912.0f;
+    const float n = biased - 12582912.0f;
+    float r = fmaf(n, -0.693145751953125f, x);
+    r = fmaf(n, -1.42860682030941723e-6f, r);
+    float p = 1.3888889225e-3f;
+    p = fmaf(p, r, 8.3333337680e-3f);
+    p = fmaf(p, r, 4.1666667908e-2f);
+    p = fmaf(p, r, 1.6666667163e-1f);
+    p = fmaf(p, r, 0.5f);
+    p = fmaf(p, r, 1.0f);
+    p = fmaf(p, r, 1.0f);
+    const float e = p * __uint_as_float((__float_as_uint(biased) - 0x4B400000u + 127u) << 23);
+    return x >= -87.0f ? e : (x != x ? x : 0.0f);
 }
 
 // grid (super-chunks of the longest history, Hkv, ceil(T * G / 64)), 128 threads = 8 vector groups x 16 key
@@ -166,7 +186,7 @@ __global__ void __launch_bounds__(kPaThreads, 2) prompt_hist_kernel(const Prompt
         float s[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            const float pr = 8 * kgp + j < lim ? bm_expf(acc[t][j] - mj) : 0.0f;
+            const float pr = 8 * kgp + j < lim ? pa_expf(acc[t][j] - mj) : 0.0f;
             acc[t][j] = bm_bf16_rn(pr);
             // butterfly over the 32 keys of the sub-chunk: offsets 16 and 8 lie across the four threads
             s[j] = pr + __shfl_xor_sync(0xffffffffu, pr, 2);
@@ -225,7 +245,7 @@ __global__ void __launch_bounds__(kPaThreads, 2) prompt_hist_kernel(const Prompt
 #pragma unroll
         for (int t = 0; t < 8; ++t) {
             const float m = mc[s * kPaQueries + v0 + t];
-            const float w = m > -INFINITY ? bm_expf(m - MJ[t]) : 0.0f;
+            const float w = m > -INFINITY ? pa_expf(m - MJ[t]) : 0.0f;
             L[t] = fmaf(lc[s * kPaQueries + v0 + t], w, L[t]);
 #pragma unroll
             for (int e = 0; e < 8; ++e) O[t][e] = fmaf(acc[t][e], w, O[t][e]);
