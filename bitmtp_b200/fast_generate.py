@@ -249,8 +249,10 @@ class _Session:
         shared.zero_()
         takes_prompt = getattr(atlas, "takes_prompt", None)
         if takes_prompt is not None and takes_prompt(self.seq_len, self.sigma):
-            # the prompt's rows go straight into the segment, and only the last one through the head
-            logits = atlas.prefill(self.prompt_ids, self.sigma)
+            # the prompt's rows go straight into the segment, and only the last one through the head.  An atlas without
+            # slab graphs serves requests beside other threads' CUDA work, which a stream in capture would not allow:
+            # its passes are launched
+            logits = atlas.prefill(self.prompt_ids, self.sigma, capture=bool(atlas.prefill_graphs))
         else:
             cache = make_sdlm_cache(self.args, device=self.device)
             logits = self.model.forward_sdlm_prefill(

@@ -272,13 +272,15 @@ class GraphAtlas:
             return False
         return bool(graphs) or (seq > PREFILL_CHUNK and self.model.wide_prefill_supported())
 
-    def prefill(self, prompt_ids: torch.Tensor, sigma: int) -> torch.Tensor:
+    def prefill(self, prompt_ids: torch.Tensor, sigma: int, capture: bool = True) -> torch.Tensor:
         """The prompt's K/V into history rows [0, len) of segment `sigma`, by replaying the captured
         slab graph once per PREFILL_CHUNK rows (staging, replay, row promotion: three launches + one
         graph per slab), then the last row's logits through the packed head.  Same arithmetic as
         Transformer.forward_sdlm_prefill, which launches every operator of every slab from the host
         and computes all rows' logits; the decode loops need only the last row (reference:
-        fast_generate.py:203-222 take `logits[-1]`).  Returns fp32 logits [1, vocab]."""
+        fast_generate.py:203-222 take `logits[-1]`).  `capture` False launches the many-row passes
+        instead of capturing the ones that come back (Transformer.prefill_wide).  Returns fp32 logits
+        [1, vocab]."""
         seq = int(prompt_ids.shape[0])
         if seq < 1 or seq > sigma:
             raise ValueError(f"prompt of {seq} tokens does not fit segment {sigma}")
@@ -288,7 +290,7 @@ class GraphAtlas:
             shared = self.kv_buffers[sigma]
             planes = [(shared[0, i], shared[1, i]) for i in range(self.n_layers)]
             return self.model.prefill_wide(prompt_ids, planes, sigma + self.M_max, self.prefill_logits
-                                           if getattr(self, "prefill_logits", None) is not None else None)
+                                           if getattr(self, "prefill_logits", None) is not None else None, capture)
         g = self.prefill_graphs[sigma]
         ids = prompt_ids.to(torch.int64).contiguous()
         n = 0

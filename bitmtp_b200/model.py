@@ -713,9 +713,14 @@ class Transformer(nn.Module):
 
     @torch.no_grad()
     def prefill_wide(self, token_values: torch.Tensor, kv_planes: List[SDLMLayerCache], kv_rows: int,
-                     logits_buf: Optional[torch.Tensor] = None) -> torch.Tensor:
+                     logits_buf: Optional[torch.Tensor] = None, capture: bool = True) -> torch.Tensor:
         """The whole prompt through prefill_rows_wide in waves (prompt_waves), then the packed head on
-        the last row (the only logit row a decode loop uses).  Returns fp32 logits [1, vocab]."""
+        the last row (the only logit row a decode loop uses).  Returns fp32 logits [1, vocab].
+
+        `capture`: waves of a shape that comes back replay as CUDA graphs (0.5 ms less for 17 rows of the 1.7B
+        geometry, 0.13 ms from 64 rows on).  While a stream is in capture the driver refuses device synchronisations,
+        event queries and copies to the host in every thread of the process, whatever the capture mode, so a program
+        whose other threads use CUDA passes False here or clears `use_prompt_graphs`."""
         seq = int(token_values.shape[0])
         dev = token_values.device
         a = self.args
@@ -730,9 +735,8 @@ class Transformer(nn.Module):
         ids = token_values.to(torch.int64).contiguous()
         n = 0
         for c0, n in waves:
-            # Per (rows, first position, KV buffer): the attention scratch, the position ids and, from the
-            # second prompt of that shape on, a CUDA graph of the wave (about 280 launches whose host cost
-            # would otherwise exceed their device time).  The graph reads its ids from ws.tokens.
+            # Per (rows, first position, KV buffer): the attention scratch, the position ids and, with `capture`, from
+            # the second prompt of that shape on, a CUDA graph of the wave.  The graph reads its ids from ws.tokens.
             key = (n, c0, kv_planes[0][0].data_ptr(), kv_rows)
             rec = cache.get(key)
             if rec is None:
@@ -743,14 +747,14 @@ class Transformer(nn.Module):
                                     "graph": None}
             rec["uses"] += 1
             ws.tokens[:n].copy_(ids[c0:c0 + n])
-            if rec["graph"] is None and rec["uses"] >= 2 and self.use_prompt_graphs \
+            if rec["graph"] is None and rec["uses"] >= 2 and capture and self.use_prompt_graphs \
                     and not torch.cuda.is_current_stream_capturing():
                 torch.cuda.synchronize(dev)
                 g = torch.cuda.CUDAGraph()
                 with torch.cuda.graph(g):
                     self.prefill_rows_wide(ws.tokens[:n], rec["pos"], kv_planes, kv_rows, c0, ws, rec["scratch"])
                 rec["graph"] = g
-            if rec["graph"] is not None:
+            if rec["graph"] is not None and capture:
                 rec["graph"].replay()
             else:
                 self.prefill_rows_wide(ws.tokens[:n], rec["pos"], kv_planes, kv_rows, c0, ws, rec["scratch"])
