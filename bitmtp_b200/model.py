@@ -731,7 +731,10 @@ class Transformer(nn.Module):
         cache = self.__dict__.setdefault("_prompt_waves", {})
         if ws is None or ws.T < rows:
             cache.clear()                        # captured waves read and write the workspace they were captured with
-            ws = self._prompt_ws = PromptWorkspace(a, rows, dev)
+            # the request loops run in inference mode, other callers need not: a tensor made there could not take the
+            # next prompt's ids outside
+            with torch.inference_mode(False):
+                ws = self._prompt_ws = PromptWorkspace(a, rows, dev)
         ids = token_values.to(torch.int64).contiguous()
         n = 0
         for c0, n in waves:

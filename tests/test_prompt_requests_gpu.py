@@ -1,4 +1,4 @@
-"""Prompts of requests beside the rest of a program: other threads' CUDA work."""
+"""Prompts of requests beside the rest of a program: other threads' CUDA work, calls outside inference mode."""
 import threading
 
 import pytest
@@ -34,8 +34,7 @@ def test_requests_of_an_atlas_without_slab_graphs_capture_nothing(kind, monkeypa
     ids = synthetic.random_prompt(40, cfg["vocab_size"], seed=40)[0].to(DEV)
     want = _request(kind, cfg, model, atlas, 40)
     for _ in range(3):
-        with torch.inference_mode():
-            atlas.prefill(ids, SIGMA)
+        atlas.prefill(ids, SIGMA)
 
     def refuse(*args, **kwargs):
         raise AssertionError("a request began a capture")
@@ -44,6 +43,19 @@ def test_requests_of_an_atlas_without_slab_graphs_capture_nothing(kind, monkeypa
     for seq in (40, 57, 57, 57):
         tokens = _request(kind, cfg, model, atlas, seq)
         assert seq != 40 or tokens == want
+
+
+@pytest.mark.parametrize("kind", list(ATLASES))
+@pytest.mark.parametrize("mode", [torch.no_grad, torch.inference_mode])
+def test_prefill_follows_a_request(kind, mode):
+    """Requests run in inference mode; a prompt outside it finds what they left usable, and leaves it so."""
+    cfg, model, atlas = _served(kind)
+    want = _request(kind, cfg, model, atlas, 30)
+    ids = synthetic.random_prompt(30, cfg["vocab_size"], seed=30)[0].to(DEV)
+    with mode():
+        logits = atlas.prefill(ids, SIGMA)
+    assert int(logits.argmax()) == want[0]
+    assert _request(kind, cfg, model, atlas, 30) == want
 
 
 @pytest.mark.parametrize("kind", list(ATLASES))
