@@ -658,7 +658,7 @@ class Transformer(nn.Module):
 
     @torch.no_grad()
     def prefill_rows_wide(self, token_values: torch.Tensor, positions: torch.Tensor, kv_planes: List[SDLMLayerCache],
-                          kv_rows: int, hist0: int, ws: "PromptWorkspace", scratch: torch.Tensor) -> None:
+                          kv_rows: int, hist0: int, ws: "PromptWorkspace") -> None:
         """One wave of the prompt forward on the many-row kernels: T = len(token_values) rows at positions
         hist0 .. hist0 + T - 1, whose K / V rows are written in place at rows [hist0, hist0 + T) of every
         layer's planes (`kv_planes[i]` = (k, v) [1, n_kv, kv_rows, hd]); rows [0, hist0) are history.
@@ -686,7 +686,7 @@ class Transformer(nn.Module):
             ops.qknorm_rope_kvappend(ws.xqkv[:T], at.q_norm.weight.data, at.k_norm.weight.data, eps, at.rope_cos,
                                      at.rope_sin, pos, a.n_heads, a.n_kv_heads, kl, vl, hist0, pdl=pdl, q_out=ws.qrot[:T])
             for a0, a1 in self._prompt_attn_calls(T):
-                ops.prompt_attention(ws.qrot[a0:a1], kl, vl, hist0 + a0, PREFILL_CHUNK, scratch, att=ws.att[a0:a1],
+                ops.prompt_attention(ws.qrot[a0:a1], kl, vl, hist0 + a0, PREFILL_CHUNK, ws.scratch, att=ws.att[a0:a1],
                                      amax=ws.att_amax[i & 1][a0:a1], pdl=pdl)
             ops.quant_rows_amax(ws.att[:T], ws.att_amax[i & 1][:T], prep=(ws.att_q[:T], ws.att_sum[:T]), s=ws.att_s[:T],
                                 amax_zero=ws.att_amax[(i + 1) & 1][:T], pdl=pdl)
@@ -703,13 +703,43 @@ class Transformer(nn.Module):
         """Row ranges of a wave's attention calls."""
         return [(a0, min(T, a0 + PREFILL_ATTN_ROWS)) for a0 in range(0, T, PREFILL_ATTN_ROWS)]
 
-    def _prompt_scratch(self, n: int, c0: int, dev) -> torch.Tensor:
-        """Scratch for every attention call of a wave: the calls' rows differ in number only at the end of the wave,
+    def _prompt_scratch_bytes(self, n: int, c0: int) -> int:
+        """Scratch of the largest attention call of a wave: the calls' rows differ in number only at the end of the wave,
         and a later call never needs fewer super-chunks, so the largest of the last two is the largest."""
         a = self.args
-        sizes = [(a1 - a0, c0 + a0) for a0, a1 in self._prompt_attn_calls(n)[-2:]]
-        return max((ops.prompt_attention_scratch(t, h, PREFILL_CHUNK, a.n_heads, a.n_kv_heads, dev) for t, h in sizes),
-                   key=torch.Tensor.numel)
+        return max(ops.prompt_attention_scratch_bytes(a1 - a0, c0 + a0, PREFILL_CHUNK, a.n_heads, a.n_kv_heads)
+                   for a0, a1 in self._prompt_attn_calls(n)[-2:])
+
+    def _prompt_workspace(self, waves: List[Tuple[int, int]], dev) -> "PromptWorkspace":
+        """The model's workspace and attention scratch, at least as large as these waves need.  A model keeps one: its
+        waves run one after another, and the attention's counters lie at the same place of the scratch for every call.
+        Sizes are rounded up, so that a slightly longer prompt finds it large enough."""
+        rows = max(n for _, n in waves)
+        scratch = max(self._prompt_scratch_bytes(n, c0) for c0, n in waves)
+        ws = self.__dict__.get("_prompt_ws")
+        if ws is not None and ws.T >= rows and ws.scratch.numel() >= scratch:
+            return ws
+        if torch.cuda.is_current_stream_capturing():
+            return PromptWorkspace(self.args, rows, scratch, dev)       # belongs to the caller's graph
+        if ws is not None:
+            # by half at least, so that prompts that get longer one by one drop the captured waves a few times only
+            def grown(need, have):
+                return have if need <= have else max(need, have + have // 2)
+            rows, scratch = min(grown(rows, ws.T), PREFILL_WAVE + PREFILL_TAIL), grown(scratch, ws.scratch.numel())
+            self._drop_prompt_waves(dev)
+            ws = self._prompt_ws = None                                 # given back before the larger one is taken
+        # the request loops run in inference mode, other callers need not: a tensor made there could not take the next
+        # prompt's ids outside
+        with torch.inference_mode(False):
+            self._prompt_ws = PromptWorkspace(self.args, -(-rows // PROMPT_WS_ROWS) * PROMPT_WS_ROWS,
+                                              -(-scratch // PROMPT_WS_SCRATCH) * PROMPT_WS_SCRATCH, dev)
+        return self._prompt_ws
+
+    def _drop_prompt_waves(self, dev) -> None:
+        """Forget the captured waves, which use the workspace that they were captured with; the device may still be
+        reading it, on whatever stream they were launched."""
+        torch.cuda.synchronize(dev)
+        self.__dict__.setdefault("_prompt_waves", {}).clear()
 
     @torch.no_grad()
     def prefill_wide(self, token_values: torch.Tensor, kv_planes: List[SDLMLayerCache], kv_rows: int,
@@ -726,41 +756,33 @@ class Transformer(nn.Module):
         a = self.args
         self.prepare_t2_lm_head()
         waves = prompt_waves(seq)
-        rows = (max(n for _, n in waves) + PREFILL_CHUNK - 1) // PREFILL_CHUNK * PREFILL_CHUNK
-        ws = getattr(self, "_prompt_ws", None)
+        ws = self._prompt_workspace(waves, dev)
         cache = self.__dict__.setdefault("_prompt_waves", {})
-        if ws is None or ws.T < rows:
-            cache.clear()                        # captured waves read and write the workspace they were captured with
-            # the request loops run in inference mode, other callers need not: a tensor made there could not take the
-            # next prompt's ids outside
-            with torch.inference_mode(False):
-                ws = self._prompt_ws = PromptWorkspace(a, rows, dev)
+        capture = capture and self.use_prompt_graphs and not torch.cuda.is_current_stream_capturing()
         ids = token_values.to(torch.int64).contiguous()
         n = 0
         for c0, n in waves:
-            # Per (rows, first position, KV buffer): the attention scratch, the position ids and, with `capture`, from
-            # the second prompt of that shape on, a CUDA graph of the wave.  The graph reads its ids from ws.tokens.
-            key = (n, c0, kv_planes[0][0].data_ptr(), kv_rows)
-            rec = cache.get(key)
-            if rec is None:
-                if len(cache) > 32:
-                    cache.clear()
-                rec = cache[key] = {"scratch": self._prompt_scratch(n, c0, dev),
-                                    "pos": torch.arange(c0, c0 + n, device=dev, dtype=torch.int64), "uses": 0,
-                                    "graph": None}
-            rec["uses"] += 1
+            args = (ws.tokens[:n], ws.positions[c0:c0 + n], kv_planes, kv_rows, c0, ws)
             ws.tokens[:n].copy_(ids[c0:c0 + n])
-            if rec["graph"] is None and rec["uses"] >= 2 and capture and self.use_prompt_graphs \
-                    and not torch.cuda.is_current_stream_capturing():
-                torch.cuda.synchronize(dev)
-                g = torch.cuda.CUDAGraph()
-                with torch.cuda.graph(g):
-                    self.prefill_rows_wide(ws.tokens[:n], rec["pos"], kv_planes, kv_rows, c0, ws, rec["scratch"])
-                rec["graph"] = g
-            if rec["graph"] is not None and capture:
-                rec["graph"].replay()
+            graph = None
+            if capture:
+                # per (rows, first position, KV buffer), from the second wave of that shape on
+                key = (n, c0, kv_planes[0][0].data_ptr(), kv_rows)
+                graph = cache.get(key)
+                if key not in cache:
+                    if len(cache) > 32:
+                        self._drop_prompt_waves(dev)
+                    cache[key] = None
+                elif graph is None:
+                    torch.cuda.synchronize(dev)
+                    graph = torch.cuda.CUDAGraph()
+                    with torch.cuda.graph(graph):
+                        self.prefill_rows_wide(*args)
+                    cache[key] = graph
+            if graph is not None:
+                graph.replay()
             else:
-                self.prefill_rows_wide(ws.tokens[:n], rec["pos"], kv_planes, kv_rows, c0, ws, rec["scratch"])
+                self.prefill_rows_wide(*args)
         if logits_buf is None:
             logits_buf = torch.empty((1, self._lm_head_n_pad), dtype=torch.float32, device=dev)
         # final norm + packed head on the last row of the last wave
@@ -813,6 +835,9 @@ class Transformer(nn.Module):
 PREFILL_CHUNK = 16
 PREFILL_WAVE = 1024         # prompt rows one pass of the many-row path takes
 PREFILL_TAIL = 256          # a last pass shorter than this joins the one before it
+PROMPT_MAX_ROWS = 8064      # longest prompt of bm_prompt_attention
+PROMPT_WS_ROWS = 64         # the prompt workspace's rows and bytes of attention scratch are multiples of these; with
+PROMPT_WS_SCRATCH = 4 << 20 # 256 rows and 32 MB the first prompt of 19 tokens takes 4.7 ms for its allocations, not 4.0
 PREFILL_ATTN_ROWS = 512     # rows per attention call: its partials (16 heads, 24 super-chunks: 98 MB) stay in L2
 
 
@@ -831,7 +856,7 @@ def prompt_waves(seq: int) -> List[Tuple[int, int]]:
 class PromptWorkspace:
     """Intermediates of one wave of the many-row prompt path (Transformer.prefill_rows_wide)."""
 
-    def __init__(self, args: ModelArgs, T: int, device):
+    def __init__(self, args: ModelArgs, T: int, scratch_bytes: int, device):
         bf, i8, f32, i32 = torch.bfloat16, torch.int8, torch.float32, torch.int32
         q_dim = args.n_heads * args.head_dim
         qkv = q_dim + 2 * args.n_kv_heads * args.head_dim
@@ -852,6 +877,9 @@ class PromptWorkspace:
         self.iq, self.i_sum, self.is_ = buf((T, args.ffn_dim), i8), buf((T, args.ffn_dim // 128), i32), buf((T, 1), f32)
         self.ffn_out = buf((T, args.dim), bf)
         self.tokens = torch.zeros(T, dtype=torch.int64, device=device)
+        self.positions = torch.arange(PROMPT_MAX_ROWS, dtype=torch.int64, device=device)
+        # zero before its first use: its head holds the attention's counters, which every call leaves zero
+        self.scratch = torch.zeros(scratch_bytes, dtype=torch.uint8, device=device)
 
 
 class _LayerView:

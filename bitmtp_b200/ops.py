@@ -292,11 +292,15 @@ def t2_linear_rows(x: torch.Tensor, b_packed: torch.Tensor, ws: torch.Tensor) ->
     return t2_gemm_wide(qp, sums, b_packed, s, ws, out=torch.empty((T, N), dtype=torch.bfloat16, device=x.device))
 
 
-def prompt_attention_scratch(T: int, hist0: int, slab_rows: int, H: int, Hkv: int, device) -> torch.Tensor:
+def prompt_attention_scratch_bytes(T: int, hist0: int, slab_rows: int, H: int, Hkv: int) -> int:
     n = int(native.lib().bm_prompt_attention_scratch_bytes(T, hist0, slab_rows, H, Hkv))
     if n < 0:
         raise RuntimeError(f"prompt attention does not take T={T}, hist0={hist0}, slab_rows={slab_rows}")
-    return torch.zeros((n + 15) // 16 * 16, dtype=torch.uint8, device=device)
+    return (n + 15) // 16 * 16
+
+
+def prompt_attention_scratch(T: int, hist0: int, slab_rows: int, H: int, Hkv: int, device) -> torch.Tensor:
+    return torch.zeros(prompt_attention_scratch_bytes(T, hist0, slab_rows, H, Hkv), dtype=torch.uint8, device=device)
 
 
 def prompt_attention(q: torch.Tensor, k_layer, v_layer, hist0: int, slab_rows: int, scratch: torch.Tensor, *,

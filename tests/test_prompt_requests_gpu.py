@@ -1,4 +1,4 @@
-"""Prompts of requests beside the rest of a program: other threads' CUDA work, calls outside inference mode."""
+"""Prompts of requests beside the rest of a program: other threads' CUDA work, calls outside inference mode, memory."""
 import threading
 
 import pytest
@@ -98,3 +98,56 @@ def test_threads_serve_their_own_models(kind):
     other.join(30)
     assert not failures and not any(t.is_alive() for t in (other, *threads))
     assert native.lib().bm_device_error() == 0
+
+
+def test_prompt_lengths_share_one_workspace(monkeypatch):
+    """Prompts of many lengths hold no more memory than the longest one and the longest of one pass, and a prompt of a new
+    length leaves the captured passes of the others alone."""
+    sigma = 1400
+    cfg = synthetic.make_config(dict(synthetic.TINY, n_heads=16, n_kv_heads=8, dim=512, ffn_dim=512), block_size=8)
+    model = generate.model_from_state(generate.args_from_config(cfg), synthetic.make_state(cfg, seed=1), DEV)
+    model.prepare_merged_weights(max_positions=sigma + 1)
+    atlas = GraphAtlas(model, model.args, DEV, segment_ladder=(sigma,), m_set=(1,), roles=("ar",), capture_verbose=False)
+
+    def prefill(seq):
+        logits = atlas.prefill(synthetic.random_prompt(seq, cfg["vocab_size"], seed=seq)[0].to(DEV), sigma).clone()
+        torch.cuda.synchronize()
+        return logits
+
+    want = {seq: prefill(seq) for seq in (300, 1279, sigma)}
+    held = torch.cuda.memory_allocated(DEV)
+    for seq in range(320, sigma, 60):
+        prefill(seq)
+    assert torch.cuda.memory_allocated(DEV) <= held
+    for seq in (300, 300, 1395):
+        prefill(seq)
+
+    def refuse(*args, **kwargs):
+        raise AssertionError("a pass was captured again")
+    monkeypatch.setattr(torch.cuda, "graph", refuse)
+    prefill(301)
+    for _ in range(2):
+        assert torch.equal(prefill(300).view(torch.int32), want[300].view(torch.int32))
+    assert native.lib().bm_device_error() == 0
+
+
+def test_a_pass_captured_by_the_caller_leaves_nothing_behind():
+    """The first prompt of a model under the caller's own capture: its buffers belong to that graph, and prompts before its
+    first replay, after it and beside it come out the same."""
+    cfg, model, atlas = _served("ar")
+    ids = synthetic.random_prompt(40, cfg["vocab_size"], seed=40)[0].to(DEV)
+    _request("ar", cfg, model, atlas, 9)                        # loads what the head needs; too short for a pass
+    with torch.no_grad():
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            captured = atlas.prefill(ids, SIGMA)
+        got = [atlas.prefill(ids, SIGMA).clone() for _ in range(3)]
+        graph.replay()
+        got += [captured.clone(), atlas.prefill(ids, SIGMA).clone()]
+        graph.replay()
+        got.append(captured.clone())
+        cache = model.forward_sdlm_prefill(token_values=ids, cache=[None] * model.args.n_layers)
+    torch.cuda.synchronize()
+    assert native.lib().bm_device_error() == 0
+    for logits in got:
+        assert torch.equal(logits.view(torch.int32), cache[-1:].view(torch.int32))
