@@ -1162,24 +1162,29 @@ int bm_prompt_attention(const void *q, const void *k_base, const void *v_base, i
     p.slab_rows = slab_rows;
     p.slab_hist0 = hist0;
     // The history by tiles where the general kernel's CTAs would fill the machine (two per SM) more than six times.
-    // Below that a tile's latency is the longer one: 19 rows 28 us against 8, 256 rows 56 against 42, 64 rows behind
-    // 1024 keys 50 against 48; above it, 333 rows 63 against 61, 512 rows 90 against 114, 512 rows behind 2048 keys
-    // 356 against 659 (16 heads; 32 heads change sides at the same fill).
+    // Measured over 424 calls of 17 to 512 rows behind 0 to 3000 keys, 8 to 32 heads: below the line a tile's latency is
+    // the longer one (16 heads: 160 rows 39 us against 24, 256 rows 53 against 42, 64 rows behind 512 keys 47 against 31),
+    // above it none is more than 3 % slower by tiles (333 rows 58 against 61, 512 rows 82 against 114, 64 rows behind
+    // 2048 keys 49 against 80, 512 rows behind 2048 keys 338 against 657).  Some calls change sides earlier: a line at
+    // five fills takes the same time in sum, but up to 32 % more for few rows behind a long history.
     const long long general_ctas = (long long)pl.units * Hkv * pl.Z;
+    const size_t smem = bm::attn_smem_bytes(pl.nq);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (bm::prompt_hist_fits(slab_rows, H, Hkv) && general_ctas > 6LL * 2 * current_device().sm_count) {
         // history super-chunks by tiles of 64 query vectors, then one CTA set per slab for its own rows and the merge
         const int hist_end = hist0 + (pl.n_slabs - 1) * slab_rows, G = H / Hkv;
         if (hist_end > 0) {
             const bm::PromptHistParams hp{p.q, p.k_base, p.v_base, p.pm, p.pl, p.po, T, H, Hkv, __builtin_ctz(G), kv_rows, hist0, pl.NJ, p.pdl};
             const dim3 hgrid((hist_end + BM_ATTN_SUPER - 1) / BM_ATTN_SUPER, Hkv, (T * G + bm::kPaQueries - 1) / bm::kPaQueries);
-            const int rc = launch_ex(bm::prompt_hist_kernel, hgrid, dim3(bm::kPaThreads), bm::kPaSmem,
-                                     static_cast<cudaStream_t>(stream), p.pdl, hp);
+            const int rc = launch_ex(bm::prompt_hist_kernel, hgrid, dim3(bm::kPaThreads), bm::kPaSmem, st, p.pdl, hp);
             if (rc != BM_OK) return rc;
         }
-        p.hist_done = 1;
+        // slabs of 16 rows: 16 G query vectors, always eight per CTA (attn_query_split)
+        if (pl.nq != 4) return BM_EINVAL;
+        return launch_ex(bm::attn_fused_kernel<4, false, false, true>, dim3(pl.n_slabs, Hkv, pl.Z), dim3(bm::kAttnThreads), smem,
+                         st, p.pdl, p);
     }
-    const dim3 grid(p.hist_done ? pl.n_slabs : pl.units, Hkv, pl.Z);
-    return launch_attention<false>(pl.nq, grid, bm::attn_smem_bytes(pl.nq), static_cast<cudaStream_t>(stream), p.pdl, p);
+    return launch_attention<false>(pl.nq, dim3(pl.units, Hkv, pl.Z), smem, st, p.pdl, p);
 }
 
 // ---------------------------------------------------------------------------- dense draft heads

@@ -67,9 +67,7 @@ struct AttnParams {
     // sees history [0, slab_hist0 + s * slab_rows) and its own rows.  blockIdx.x runs over the
     // (slab, super-chunk) pairs in slab order; `state` is not read; q, att, amax and the partials are
     // indexed by prompt row; tickets [slabs][Hkv][gridDim.z].
-    // hist_done: the history super-chunks' partials are in pm / pl / po already (prompt_hist_kernel); blockIdx.x is
-    // the slab, its CTAs make the partial of the slab's own rows and merge at once, without a ticket.
-    int slab_rows, slab_hist0, hist_done;
+    int slab_rows, slab_hist0;
     int slots;       // CTAs the device holds at once (0: keep the coarse query split)
 };
 
@@ -240,7 +238,11 @@ __device__ __forceinline__ void attn_sub_pass(const uint16_t *Ks, const uint16_t
 // ticket build, so the fence, the ticket and the read-back from global memory drop out of the chain.  A
 // second barrier keeps the other CTAs' shared memory alive until it has been read.  CTAs of super-chunks
 // without rows take part in both barriers and do nothing else.
-template <int NQ, bool ROPE, bool CLUSTER = false>
+// HIST_DONE (prompt mode only): prompt_hist_kernel has made the partials of the history super-chunks.  blockIdx.x is
+// the slab; its CTAs make the partial of the slab's own rows, keep it in registers and merge at once, without a ticket.
+// A build of its own: as a run-time switch it made every other prompt-mode call 3.6 % slower (1 to 9 % over 117 calls
+// of 17 to 512 rows; 64 rows without history 10.8 us, 10.1 without the switch).
+template <int NQ, bool ROPE, bool CLUSTER = false, bool HIST_DONE = false>
 __global__ void __launch_bounds__(kAttnThreads, 2) attn_fused_kernel(const AttnParams p) {
     extern __shared__ __align__(16) unsigned char dyn[];
     __shared__ unsigned int sh_ticket;
@@ -257,7 +259,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_fused_kernel(const AttnP
     if (!ROPE && p.slab_rows > 0) {
         // prompt mode: find this CTA's slab; a slab with history h has ceil(h / 128) + 1 super-chunks
         int s = 0, rem = J, h = p.slab_hist0;
-        if (p.hist_done) {
+        if (HIST_DONE) {
             s = J;
             h += s * p.slab_rows;
             rem = (h + BM_ATTN_SUPER - 1) / BM_ATTN_SUPER;
@@ -469,7 +471,6 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_fused_kernel(const AttnP
     __syncthreads();
 
     // level 1: the four sub-chunk partials of query vector qi, merged in ascending sub-chunk order
-    const bool merge_now = !ROPE && p.hist_done;       // the partial below stays in this warp's registers
     float MJ = -INFINITY, L = 0.0f, O[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     if (q_live) {
         float mm[kAttnSub];
@@ -490,7 +491,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_fused_kernel(const AttnP
             // vector, both spent since the CTA barrier after level 0
             *reinterpret_cast<float4 *>(Ps + qi * BM_ATTN_SUPER + 4 * lane) = make_float4(O[0], O[1], O[2], O[3]);
             if (lane == 0) *reinterpret_cast<float2 *>(Qs + qi * 128) = make_float2(MJ, L);
-        } else if (!merge_now) {
+        } else if (!HIST_DONE) {
             const size_t pb = ((size_t)(r0 + qm) * p.H + hk * G + qg_) * p.NJ + J;
             *reinterpret_cast<float4 *>(p.po + pb * 128 + 4 * lane) = make_float4(O[0], O[1], O[2], O[3]);
             if (lane == 0) { p.pm[pb] = MJ; p.pl[pb] = L; }
@@ -555,7 +556,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_fused_kernel(const AttnP
         cluster_wait();
         return;
     }
-    if (!merge_now) {
+    if (!HIST_DONE) {
         // ticket: the last CTA of this (kv head, query group) to get here merges the super-chunks
         __threadfence();
         __syncthreads();
@@ -577,12 +578,12 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_fused_kernel(const AttnP
 #pragma unroll
     for (int i = 0; i < kBatch; ++i) {
         const int j = i < n_hs ? i : p.NJ - 1;
-        part[i] = merge_now && i == n_hs ? own_o
+        part[i] = HIST_DONE && i == n_hs ? own_o
                   : i < nv ? __ldcg(reinterpret_cast<const float4 *>(p.po + (pb + j) * 128 + 4 * lane))
                            : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
     float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.0f, l1 = 0.0f;
-    if (merge_now && lane == n_hs) {
+    if (HIST_DONE && lane == n_hs) {
         m0 = MJ;
         l0 = L;
     } else if (lane < nv) {
@@ -590,7 +591,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_fused_kernel(const AttnP
         m0 = __ldcg(p.pm + pb + j);
         l0 = __ldcg(p.pl + pb + j);
     }
-    if (merge_now && lane + 32 == n_hs) {
+    if (HIST_DONE && lane + 32 == n_hs) {
         m1 = MJ;
         l1 = L;
     } else if (lane + 32 < nv) {
@@ -608,7 +609,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_fused_kernel(const AttnP
             for (int i = 0; i < kBatch; ++i) {
                 const int c = b0 + i;
                 const int j = c < n_hs ? c : p.NJ - 1;
-                part[i] = merge_now && c == n_hs ? own_o
+                part[i] = HIST_DONE && c == n_hs ? own_o
                           : c < nv ? __ldcg(reinterpret_cast<const float4 *>(p.po + (pb + j) * 128 + 4 * lane))
                                    : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             }
