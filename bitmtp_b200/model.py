@@ -167,23 +167,19 @@ class T2LinearKernel(nn.Module):
         return q.reshape(x.shape), s.reshape(*x.shape[:-1], 1)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        """Any number of rows.  Up to MAX_ROWS of them are one launch of the decode GEMV; more go through the
-        many-row kernel, which reads each weight byte once per 32 rows (333 rows of 6144 x 2048: 401 us in slabs of
-        MAX_ROWS, 40 us; the slabs remain for K past the many-row kernel's tables).  The reference falls back to a
-        dense bf16 GEMM on unpacked weights for unregistered widths (model.py:650-656); the integer path gives the
-        same quantised product without the bf16 roundings and without the dense copy of the weights."""
+        """Any number of rows.  Up to MAX_ROWS of them are one launch of the decode GEMV; more go where
+        ops.t2_linear_rows takes them, to the many-row kernel, which reads each weight byte once per 32 rows (333 rows of
+        6144 x 2048: 401 us in slabs of MAX_ROWS, 38 us), or, for few rows of a narrow, deep weight, through the GEMV.
+        The reference falls back to a dense bf16 GEMM on unpacked weights for unregistered widths (model.py:650-656);
+        the integer path gives the same quantised product without the bf16 roundings and without the dense copy of the
+        weights."""
         x2 = x.reshape(-1, self.in_features).contiguous()
-        if (self.MAX_ROWS < x2.shape[0] <= ops.GEMM_WIDE_MAX_ROWS and self.in_features <= ops.GEMM_WIDE_MAX_K
-                and self.out_features % 8 == 0 and self.weight.data_ptr() % 16 == 0
-                and self.weight_scale.data_ptr() % 16 == 0):
-            out = ops.t2_linear_rows(x2, self.weight.data, self.weight_scale)
-            return out.reshape(*x.shape[:-1], self.out_features)
-        q, s = ops.quant_rows(x2)
-        out = torch.empty((x2.shape[0], self.out_features), dtype=torch.bfloat16, device=x.device)
-        for r0 in range(0, x2.shape[0], self.MAX_ROWS):
-            r1 = min(r0 + self.MAX_ROWS, x2.shape[0])
-            ops.t2_gemv(q[r0:r1], self.weight.data, s[r0:r1], self.weight_scale, out=out[r0:r1],
-                        ldc=self.out_features)
+        w, ws = self.weight.data, self.weight_scale
+        if x2.shape[0] > self.MAX_ROWS:
+            out = ops.t2_linear_rows(x2, w, ws)
+        else:
+            q, s = ops.quant_rows(x2)
+            out = ops.t2_gemv(q, w, s, ws)
         return out.reshape(*x.shape[:-1], self.out_features)
 
 

@@ -33,20 +33,6 @@ def _require_cuda(*tensors: torch.Tensor) -> None:
             raise RuntimeError("bitmtp_b200 operators need all tensors on one CUDA device")
 
 
-def _check_packed_operands(a_int8: torch.Tensor, b_packed: torch.Tensor, s: torch.Tensor, ws: torch.Tensor):
-    """(W, N, K) of a packed product after the metadata checks."""
-    _require_cuda(a_int8, b_packed, s, ws)
-    W, K = a_int8.shape
-    N = b_packed.shape[0]
-    if b_packed.shape[1] * 4 != K or tuple(ws.shape) != (N, K // 128):
-        raise RuntimeError("t2_gemv: packed weight / scale shape mismatch")
-    if a_int8.dtype != torch.int8 or ws.dtype != torch.bfloat16 or s.dtype != torch.float32:
-        raise RuntimeError("t2_gemv: invalid activation, scale or multiplier dtype")
-    if s.numel() != W:
-        raise RuntimeError("t2_gemv: one activation multiplier per row is required")
-    return W, N, K
-
-
 def t2_gemv(a_int8: torch.Tensor, b_packed: torch.Tensor, s: torch.Tensor, ws: torch.Tensor, *,
             out_kind: int = native.OUT_BF16, path: int = native.PATH_AUTO,
             want_groups: bool = False, pdl: bool = False, out: Optional[torch.Tensor] = None,
@@ -57,7 +43,15 @@ def t2_gemv(a_int8: torch.Tensor, b_packed: torch.Tensor, s: torch.Tensor, ws: t
     ws [N, K/128] bf16.  Returns C ([W, N] bf16 or fp32 per `out_kind`), or
     (C, G) with G int32 [W, N, K/128] when `want_groups`.
     """
-    W, N, K = _check_packed_operands(a_int8, b_packed, s, ws)
+    _require_cuda(a_int8, b_packed, s, ws)
+    W, K = a_int8.shape
+    N = b_packed.shape[0]
+    if b_packed.shape[1] * 4 != K or tuple(ws.shape) != (N, K // 128):
+        raise RuntimeError("t2_gemv: packed weight / scale shape mismatch")
+    if a_int8.dtype != torch.int8 or ws.dtype != torch.bfloat16 or s.dtype != torch.float32:
+        raise RuntimeError("t2_gemv: invalid activation, scale or multiplier dtype")
+    if s.numel() != W:
+        raise RuntimeError("t2_gemv: one activation multiplier per row is required")
     dt = torch.bfloat16 if out_kind == native.OUT_BF16 else torch.float32
     if out is None:
         out = torch.empty((W, N), dtype=dt, device=a_int8.device)
@@ -280,16 +274,56 @@ def t2_gemm_wide(a_prep: torch.Tensor, a_sums: torch.Tensor, b_packed: torch.Ten
     return out
 
 
-GEMM_WIDE_MAX_K = 51200            # its scale and C-operand tables fill the shared memory of an SM there
 GEMM_WIDE_MAX_ROWS = 32 * 65535    # grid.y
+GEMV_MAX_K = 11264                 # 16 INT8 rows and one tile of weights fill the shared memory of an SM there
+
+
+def gemv_serves_rows(T: int, N: int, K: int) -> bool:
+    """Whether 17 to 32 rows are two launches of the decode GEMV instead of one of the many-row kernel.
+
+    The many-row kernel gives 128 weight rows x 32 prompt rows to one CTA, which walks the K / 128 groups in series: with
+    few CTAs its time is that walk, 4 us + 4.2 us per 1024 of K, however small N is.  The GEMV spreads the weight rows over
+    all SMs.  Device us for 17 / 32 rows, GEMV against many-row kernel: 512 x 1024 9.6 / 9.3 - 11.1 / 11.4, 4096 x 1024
+    11.0 / 10.9 - 11.1 / 11.8, 512 x 2048 9.9 / 10.0 - 12.6 / 13.3, 512 x 9728 14.0 / 14.7 - 43.0 / 45.0, 4096 x 9728
+    24.7 / 28.3 - 45.6 / 47.8.  The other side: 6144 x 1024 13.0 / 12.9 - 11.3 / 12.0, 4096 x 512 12.3 / 12.0 - 9.4 / 10.0,
+    12288 x 2048 18.1 / 18.5 - 14.7 / 15.5.  Odd group counts go through the GEMV's slower consumer (512 x 1152, in slabs
+    of 16: 16.8 / 26.9 - 11.6 / 12.1); from 33 rows on the GEMV would read the weights three times (512 x 9728: 44.9 - 45.0,
+    2048 x 2048: 19.1 - 13.7)."""
+    return 16 < T <= 32 and 1024 <= K <= GEMV_MAX_K and K % 256 == 0 and N <= 4096
 
 
 def t2_linear_rows(x: torch.Tensor, b_packed: torch.Tensor, ws: torch.Tensor) -> torch.Tensor:
-    """Quantise bf16 rows [T, K] and multiply them by the packed weight in two launches, whatever T: bf16 [T, N],
-    every row what t2_gemv gives it."""
-    qp, sums, s = quant_rows(x, prepared=True)
-    T, N, _ = _check_packed_operands(qp, b_packed, s, ws)
-    return t2_gemm_wide(qp, sums, b_packed, s, ws, out=torch.empty((T, N), dtype=torch.bfloat16, device=x.device))
+    """Quantise more than 16 bf16 rows [T, K] and multiply them by the packed weight: bf16 [T, N], every row what t2_gemv
+    gives it."""
+    _require_cuda(x, b_packed, ws)
+    T, K = x.shape
+    N = b_packed.shape[0]
+    if b_packed.shape[1] * 4 != K or ws.shape != (N, K // 128):
+        raise RuntimeError("t2_linear_rows: packed weight / scale shape mismatch")
+    if ws.dtype != torch.bfloat16:
+        raise RuntimeError("t2_linear_rows: invalid scale dtype")
+    dev, L = x.device, native.lib()
+    qp = torch.empty((T, K), dtype=torch.int8, device=dev)
+    sums = torch.empty((T, K // 128), dtype=torch.int32, device=dev)
+    s = torch.empty((T, 1), dtype=torch.float32, device=dev)
+    out = torch.empty((T, N), dtype=torch.bfloat16, device=dev)
+    stream, wp = _stream(dev), ws.data_ptr()
+    rc = native.BM_EINVAL if wp % 16 else L.bm_quant_rows(x.data_ptr(), T, K, None, qp.data_ptr(), sums.data_ptr(),
+                                                          s.data_ptr(), 0, stream)
+    if rc == native.BM_OK:
+        if gemv_serves_rows(T, N, K):
+            rc = L.bm_t2_gemv_prepared(qp.data_ptr(), sums.data_ptr(), b_packed.data_ptr(), out.data_ptr(), s.data_ptr(), wp,
+                                       T, N, K, N, native.OUT_BF16, 0, stream)
+        elif T <= GEMM_WIDE_MAX_ROWS:
+            rc = L.bm_t2_gemm_wide(qp.data_ptr(), sums.data_ptr(), b_packed.data_ptr(), out.data_ptr(), s.data_ptr(), wp,
+                                   T, N, K, N, 0, stream)
+        else:
+            for r0 in range(0, T, GEMM_WIDE_MAX_ROWS):
+                r1 = min(r0 + GEMM_WIDE_MAX_ROWS, T)
+                t2_gemm_wide(qp[r0:r1], sums[r0:r1], b_packed, s[r0:r1], ws, out=out[r0:r1])
+    if rc != native.BM_OK:
+        check(rc, f"t2_linear_rows(T={T}, N={N}, K={K})")
+    return out
 
 
 def prompt_attention_scratch_bytes(T: int, hist0: int, slab_rows: int, H: int, Hkv: int) -> int:

@@ -1,12 +1,14 @@
 """The many-row paths of a prompt against the decode operators, row for row and bit for bit: the prompt attention
 (history tiles + one merge per slab) against slab-by-slab verify attention, and the packed linear module against the
 GEMV in slabs; whole prompts against the operator-by-operator forward."""
+import numpy as np
 import pytest
 import torch
 
 from bitmtp_b200 import generate, native, ops, synthetic
 from bitmtp_b200.fast_runtime import GraphAtlas
 from bitmtp_b200.model import T2LinearKernel, make_sdlm_cache
+from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -70,22 +72,88 @@ def test_rows_past_a_history_do_not_reach_it():
         assert bool(clean.isfinite().all()) and torch.equal(got.view(torch.int16), clean[:keep].view(torch.int16))
 
 
+def _module(N, K, rows, seed):
+    gen = torch.Generator(device=DEV).manual_seed(seed)
+    packed, scale = synthetic.device_ternary(N, K, gen, torch.device(DEV))
+    layer = T2LinearKernel(K, N).to(DEV)
+    layer.weight.data, layer.weight_scale = packed, scale
+    return layer, torch.randn(1, rows, K, generator=gen, device=DEV).to(torch.bfloat16)
+
+
+def _gemv_by_row(layer, x):
+    q, s = ops.quant_rows(x)
+    return torch.cat([ops.t2_gemv(q[r:r + 1], layer.weight.data, s[r:r + 1], layer.weight_scale) for r in range(x.shape[0])])
+
+
 @pytest.mark.parametrize("N,K", [(8, 128), (136, 384), (200, 2048), (504, 2560), (1024, 9728), (512, 2048)])
 @pytest.mark.parametrize("rows", [16, 17, 33, 333])
 def test_linear_module_equals_the_gemv_in_slabs(N, K, rows):
     """Row counts on both sides of the module's change to the many-row kernel, weights that end inside one of its
     tiles of 128 rows, K with and without a whole number of its stages."""
-    gen = torch.Generator(device=DEV).manual_seed(N + K + rows)
-    packed, scale = synthetic.device_ternary(N, K, gen, torch.device(DEV))
-    layer = T2LinearKernel(K, N).to(DEV)
-    layer.weight.data, layer.weight_scale = packed, scale
-    x = torch.randn(1, rows, K, generator=gen, device=DEV).to(torch.bfloat16)
+    layer, x = _module(N, K, rows, N + K + rows)
     q, s = ops.quant_rows(x[0])
-    want = torch.cat([ops.t2_gemv(q[r:r + SLAB], packed, s[r:r + SLAB], scale) for r in range(0, rows, SLAB)])
+    want = torch.cat([ops.t2_gemv(q[r:r + SLAB], layer.weight.data, s[r:r + SLAB], layer.weight_scale)
+                      for r in range(0, rows, SLAB)])
     got = layer(x)
     torch.cuda.synchronize()
     assert native.lib().bm_device_error() == 0
     assert got.shape == (1, rows, N) and torch.equal(got[0].view(torch.int16), want.view(torch.int16))
+
+
+@pytest.mark.parametrize("N,K", [(4096, 1024), (4104, 1024), (264, 768), (72, 1152), (72, 2048), (8, ops.GEMV_MAX_K),
+                                 (8, ops.GEMV_MAX_K + 256)])
+@pytest.mark.parametrize("rows", [17, 24, 25, 32, 33])
+def test_linear_module_on_both_sides_of_its_lines(N, K, rows):
+    """The kernel that ops.gemv_serves_rows names is the one that runs (one launch, or two of the GEMV's 16 rows), and the
+    other gives the same bits."""
+    layer, x = _module(N, K, rows, N + K + rows)
+    gemv, before = ops.gemv_serves_rows(rows, N, K), native.lib().bm_launch_count()
+    got = layer(x)[0]
+    assert native.lib().bm_launch_count() - before == (3 if gemv else 2)
+    qp, sums, s = ops.quant_rows(x[0], prepared=True)
+    other = torch.empty_like(got)
+    if gemv:
+        ops.t2_gemm_wide(qp, sums, layer.weight.data, s, layer.weight_scale, out=other)
+    elif K % 256 == 0 and K <= ops.GEMV_MAX_K:
+        for r in range(0, rows, 32):
+            ops.t2_gemv_prepared(qp[r:r + 32], sums[r:r + 32], layer.weight.data, s[r:r + 32], layer.weight_scale,
+                                 out=other[r:r + 32])
+    else:
+        other = _gemv_by_row(layer, x[0])
+    torch.cuda.synchronize()
+    assert native.lib().bm_device_error() == 0
+    assert torch.equal(got.view(torch.int16), other.view(torch.int16))
+
+
+def test_linear_module_at_its_limits():
+    """The largest K of the many-row kernel, more rows than one of its grids has, and what stays refused."""
+    layer, x = _module(8, 51200, 17, 5)
+    got = layer(x)[0]
+    q, s = (t.cpu().numpy() for t in ops.quant_rows(x[0]))
+    _, want, _ = O.t2_gemv(q, layer.weight.data.cpu().numpy(), O.torch_to_u16(layer.weight_scale), s)
+    assert np.array_equal(O.torch_to_u16(got), want)
+    layer, x = _module(8, 51328, 17, 5)
+    with pytest.raises(native.NativeError):
+        layer(x)
+    for N, K in ((12, 1024), (12, 512)):
+        layer, x = _module(N, K, 17, 5)
+        with pytest.raises(native.NativeError):
+            layer(x)
+    layer, x = _module(8, 128, 17, 5)
+    layer.weight_scale = torch.cat([layer.weight_scale.view(-1)[:4], layer.weight_scale.view(-1)])[4:].view(8, 1)
+    assert layer.weight_scale.data_ptr() % 16
+    with pytest.raises(native.NativeError):
+        layer(x)
+    rows = ops.GEMM_WIDE_MAX_ROWS + 33
+    layer, x = _module(8, 128, 1, 5)
+    x = x[0].expand(rows, -1).contiguous()
+    x[-1] *= -3.0
+    got = layer(x)
+    torch.cuda.synchronize()
+    assert native.lib().bm_device_error() == 0
+    ends = torch.cat([x[:1], x[-34:]])
+    assert torch.equal(got[[0, *range(rows - 34, rows)]].view(torch.int16), _gemv_by_row(layer, ends).view(torch.int16))
+    assert bool((got[:-1] == got[0]).all())
 
 
 def _packed_model(geo, max_positions):
