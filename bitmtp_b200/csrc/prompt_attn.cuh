@@ -9,12 +9,14 @@
 // softmax of each 32-key sub-chunk, numerators O = P V and the merge of the four sub-chunks.  It writes the
 // partials (max, sum, 128 numerators) that the slab's own CTA of attn_fused_kernel then merges in order.
 //
-// Bound by the fp32 pipe: 2 * 128 multiply-adds per (query vector, key).  Every one of them is the fma of
+// The work is fp32 arithmetic: 2 * 128 multiply-adds per (query vector, key).  Every one of them is the fma of
 // attn_sub_pass, in the same chain (scores ascending in d, numerators ascending in the key, sub-chunks
 // ascending, the weight sum as the butterfly over the 32 keys), so the partials are the same bits; tensor
-// cores would not give that order.  512 rows behind 2048 keys, 16 heads: 659 us by attn_fused_kernel alone, 414 us
-// with scalar fmas (issue slots 56 % busy, a quarter of the instructions not fmas), 356 us with packed ones and
-// an exponential without branches and conversions; the fmas alone are 134 us at the fp32 rate.
+// cores would not give that order.  512 rows behind 2048 keys, 16 heads: 657 us by attn_fused_kernel alone; called from
+// the host 414 us with scalar fmas and 356 with packed ones and an exponential without branches and conversions; 338 in
+// a captured chain now.  The fmas alone are 134 us at the fp32 rate.  Bound by issue and latency, not by that pipe: it is
+// busy half of the time, 48 % of the issue slots are used, two warps per scheduler have an eligible one in 48 % of the
+// cycles, and nothing is loaded under the multiply.
 #pragma once
 
 #include "verify_attn.cuh"

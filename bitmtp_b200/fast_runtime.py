@@ -273,9 +273,10 @@ class GraphAtlas:
         return bool(graphs) or (seq > PREFILL_CHUNK and self.model.wide_prefill_supported())
 
     def prefill(self, prompt_ids: torch.Tensor, sigma: int, capture: bool = True) -> torch.Tensor:
-        """The prompt's K/V into history rows [0, len) of segment `sigma`, by replaying the captured
-        slab graph once per PREFILL_CHUNK rows (staging, replay, row promotion: three launches + one
-        graph per slab), then the last row's logits through the packed head.  Same arithmetic as
+        """The prompt's K/V into history rows [0, len) of segment `sigma`, then the last row's logits through
+        the packed head: by the many-row kernels for more than PREFILL_CHUNK rows, else, or where a geometry
+        does not fit them, by replaying the captured slab graph once per PREFILL_CHUNK rows (staging, replay,
+        row promotion: three launches + one graph per slab).  Same arithmetic as
         Transformer.forward_sdlm_prefill, which launches every operator of every slab from the host
         and computes all rows' logits; the decode loops need only the last row (reference:
         fast_generate.py:203-222 take `logits[-1]`).  `capture` False launches the many-row passes
@@ -285,8 +286,8 @@ class GraphAtlas:
         if seq < 1 or seq > sigma:
             raise ValueError(f"prompt of {seq} tokens does not fit segment {sigma}")
         if self.model.wide_prefill_supported() and seq > PREFILL_CHUNK:
-            # the many-row kernels: every projection reads its weights once per 32 prompt rows, one
-            # attention launch per layer; K / V rows land in place.  Bit-identical to the slab replays below.
+            # every projection reads its weights once per 32 prompt rows, K / V rows land in place.
+            # Bit-identical to the slab replays below.
             shared = self.kv_buffers[sigma]
             planes = [(shared[0, i], shared[1, i]) for i in range(self.n_layers)]
             return self.model.prefill_wide(prompt_ids, planes, sigma + self.M_max, self.prefill_logits

@@ -645,8 +645,9 @@ class Transformer(nn.Module):
         return logits_buf[:, : self._lm_head_t2_vocab]
 
     def wide_prefill_supported(self) -> bool:
-        """The many-row prompt path needs every projection's row count to be a multiple of 128 and the
-        flat quantisation's K % 256 == 0; every released geometry and the test geometries have both."""
+        """The many-row prompt path needs the flat quantisation's and the RMSNorm's K % 256 == 0 and whole groups of the
+        FFN width; with heads of 128 every projection's row count is a multiple of 128 then.  Every released geometry and
+        the test geometries have both."""
         a = self.args
         q_dim, kv_dim = a.n_heads * a.head_dim, a.n_kv_heads * a.head_dim
         return (all(n % 128 == 0 for n in (q_dim + 2 * kv_dim, a.dim, 2 * a.ffn_dim)) and q_dim % 256 == 0
@@ -660,8 +661,8 @@ class Transformer(nn.Module):
         layer's planes (`kv_planes[i]` = (k, v) [1, n_kv, kv_rows, hd]); rows [0, hist0) are history.
         Same arithmetic, row for row, as the slab-by-slab prefill (forward_sdlm_prefill), so K / V rows and
         the residual stream equal it bit for bit: every projection is bm_t2_gemm_wide (tensor cores, each
-        weight byte read once per 32 rows), the attention one launch over AR-causal slabs of PREFILL_CHUNK
-        rows.  Leaves the residual stream in ws.h / ws.ffn_out (reference: model.py:1306-1340)."""
+        weight byte read once per 32 rows), the attention one call of one or two launches per PREFILL_ATTN_ROWS
+        rows over AR-causal slabs of PREFILL_CHUNK.  Leaves the residual stream in ws.h / ws.ffn_out (reference: model.py:1306-1340)."""
         a = self.args
         T = int(token_values.shape[0])
         eps, pdl = a.norm_eps, self.use_pdl
@@ -834,7 +835,8 @@ PREFILL_TAIL = 256          # a last pass shorter than this joins the one before
 PROMPT_MAX_ROWS = 8064      # longest prompt of bm_prompt_attention
 PROMPT_WS_ROWS = 64         # the prompt workspace's rows and bytes of attention scratch are multiples of these; with
 PROMPT_WS_SCRATCH = 4 << 20 # 256 rows and 32 MB the first prompt of 19 tokens takes 4.7 ms for its allocations, not 4.0
-PREFILL_ATTN_ROWS = 512     # rows per attention call: its partials (16 heads, 24 super-chunks: 98 MB) stay in L2
+PREFILL_ATTN_ROWS = 512     # rows per attention call, which bound its partials: with 16 heads and up to 2944 keys they are
+                            # at most 102 MB and stay in L2, with 32 heads or longer histories they do not
 
 
 def prompt_waves(seq: int) -> List[Tuple[int, int]]:

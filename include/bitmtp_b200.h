@@ -351,14 +351,16 @@ int bm_pack_t2_g128(const void *w, int N, int K, void *packed, void *scale, void
 int bm_t2_gemm_wide(const void *A_prep, const void *a_sums, const void *B, void *C, const void *s, const void *ws,
                     int T, int N, int K, int ldc, int pdl, void *stream);
 
-/* Causal attention of a whole prompt in one launch.  The K / V rows of the T prompt rows already sit at
+/* Causal attention of a whole prompt in one call of one or two launches (long histories of slabs of 16 rows
+ * with 1, 2, 4 or 8 heads per kv head go to a tile kernel first).  The K / V rows of the T prompt rows already sit at
  * rows [hist0, hist0 + T) of the planes (bm_qknorm_rope_kvappend with sigma = hist0); q bf16 [T, H, 128]
  * are the rotated queries.  The rows are served as AR-causal slabs of slab_rows rows (slab s sees rows
  * [0, hist0 + s * slab_rows) as history and its own rows causally), which is exactly what
  * bm_verify_attention computes when called once per slab with sigma = cache_len = the slab's start, so
  * the results equal that slab-by-slab prefill bit for bit.  att_out bf16 [T, H*128]; amax_out uint32 [T]
  * (zero on entry) gathers the row absmax bits for bm_quant_rows_amax.  scratch:
- * bm_prompt_attention_scratch_bytes(...) bytes, zero before first use.  slab_rows <= 32,
+ * bm_prompt_attention_scratch_bytes(...) bytes, zero before first use; calls on one stream may share a
+ * scratch as long as the largest of them has at most 16384 counters (slabs * Hkv * query groups).  slab_rows <= 32,
  * hist0 + T <= 8064.  Replaces the SDPA call of the prompt forward (model.py:797-800). */
 long long bm_prompt_attention_scratch_bytes(int T, int hist0, int slab_rows, int H, int Hkv);
 int bm_prompt_attention(const void *q, const void *k_base, const void *v_base, int T, int hist0, int slab_rows,
