@@ -228,18 +228,38 @@ bool make_mma_plan(int N, int K, bool half, int sms, int force_rb, MmaPlan *out)
     return true;
 }
 
-template <int RB, bool HALF, bool ONECHUNK, bool EMIT_G>
+template <int RB, bool HALF, bool ONECHUNK, bool EMIT_G, int SRC, bool SILU>
 int launch_mma_inst(const MmaPlan &pl, cudaStream_t stream, int pdl, const bm::GemvParams &p) {
-    return launch(bm::t2_gemv_mma_kernel<RB, HALF, ONECHUNK, EMIT_G>, pl.grid, bm::kGemvThreads, pl.smem, stream,
+    return launch(bm::t2_gemv_mma_kernel<RB, HALF, ONECHUNK, EMIT_G, SRC, SILU>, pl.grid, bm::kGemvThreads, pl.smem, stream,
                   pdl, p);
+}
+
+template <bool HALF, bool ONECHUNK, int SRC, bool SILU>
+int launch_mma_src(const MmaPlan &pl, cudaStream_t stream, int pdl, const bm::GemvParams &p) {
+    if (pl.rb == 4) return launch_mma_inst<4, HALF, ONECHUNK, false, SRC, SILU>(pl, stream, pdl, p);
+    if (pl.rb == 2) return launch_mma_inst<2, HALF, ONECHUNK, false, SRC, SILU>(pl, stream, pdl, p);
+    if (SILU && SRC != bm::kSrcRow) return BM_EINVAL;      // bm_t2_gemv_gate_up_silu takes pairs of 8 rows at least
+    return launch_mma_inst<1, HALF, ONECHUNK, false, SRC, SILU && SRC == bm::kSrcRow>(pl, stream, pdl, p);
 }
 
 template <bool HALF, bool ONECHUNK>
 int launch_mma_rb(const MmaPlan &pl, cudaStream_t stream, int pdl, const bm::GemvParams &p) {
-    if (p.G != nullptr) return launch_mma_inst<1, HALF, ONECHUNK, true>(pl, stream, pdl, p);
-    if (pl.rb == 4) return launch_mma_inst<4, HALF, ONECHUNK, false>(pl, stream, pdl, p);
-    if (pl.rb == 2) return launch_mma_inst<2, HALF, ONECHUNK, false>(pl, stream, pdl, p);
-    return launch_mma_inst<1, HALF, ONECHUNK, false>(pl, stream, pdl, p);
+    const bool silu = p.silu_F != 0;
+    if (p.G != nullptr) {
+        if (silu || p.src_mode != 0) return BM_EINVAL;
+        if (p.asum != nullptr) return launch_mma_inst<1, HALF, ONECHUNK, true, bm::kSrcPrepared, false>(pl, stream, pdl, p);
+        return launch_mma_inst<1, HALF, ONECHUNK, true, bm::kSrcNatural, false>(pl, stream, pdl, p);
+    }
+    if (p.src_mode != 0) {
+        if (!HALF) return BM_EINVAL;
+        return silu ? launch_mma_src<true, ONECHUNK, bm::kSrcRow, true>(pl, stream, pdl, p)
+                    : launch_mma_src<true, ONECHUNK, bm::kSrcRow, false>(pl, stream, pdl, p);
+    }
+    if (p.asum != nullptr)
+        return silu ? launch_mma_src<HALF, ONECHUNK, bm::kSrcPrepared, true>(pl, stream, pdl, p)
+                    : launch_mma_src<HALF, ONECHUNK, bm::kSrcPrepared, false>(pl, stream, pdl, p);
+    if (silu) return BM_EINVAL;
+    return launch_mma_src<HALF, ONECHUNK, bm::kSrcNatural, false>(pl, stream, pdl, p);
 }
 
 int gemv_launch_mma(const bm::GemvParams &p0, int sms, int pdl, int force_rb, cudaStream_t stream) {

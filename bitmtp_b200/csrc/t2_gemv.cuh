@@ -129,6 +129,7 @@ __host__ __device__ inline GemvSmem gemv_smem_layout(int W, int K, int RB, int s
 
 // ---- tile producer -----------------------------------------------------------
 // Called by warp 0.  Rows [n0, n0 + rows) with rows a multiple of 8.
+template <bool SILU>
 __device__ __forceinline__ void gemv_issue_tile(const GemvParams &p, unsigned char *stage,
                                                 const GemvSmem &L, uint64_t *bar, int n0,
                                                 int rows, int lane) {
@@ -136,7 +137,7 @@ __device__ __forceinline__ void gemv_issue_tile(const GemvParams &p, unsigned ch
     const uint32_t row_bytes = (uint32_t)(p.K / 4);
     if (lane == 0) mbar_expect_tx(bar, (uint32_t)rows * row_bytes + (uint32_t)(rows * ng * 2));
     __syncwarp();
-    if (p.silu_F == 0) {
+    if (!SILU) {
         for (int r = lane; r < rows; r += 32)
             bulk_g2s(stage + r * L.row_stride, p.B + (size_t)(n0 + r) * row_bytes, row_bytes, bar);
         if (lane == 0)
@@ -157,32 +158,47 @@ __device__ __forceinline__ void gemv_issue_tile(const GemvParams &p, unsigned ch
 }
 
 // ---- activation staging --------------------------------------------------------
-// A (natural order, global) -> shared, 4x4 byte transpose per 16 elements, plus
-// per-(token, group) sums.  `wrows` rows are written; rows >= W are zero.
-__device__ __forceinline__ void gemv_stage_activations(const GemvParams &p, unsigned char *smem,
-                                                       const GemvSmem &L, int wrows) {
-    const int ng = p.K / BM_GROUP;
+// A (natural order, global) -> shared, 4x4 byte transpose per 16 elements, plus per-(token, group) sums, for the W rows
+// that exist.  A row is up to 700 pieces of 16 bytes and every CTA stages all rows, so what counts is how many loads are
+// out at once: one per thread and trip, with the group sums gathered by shared-memory atomics, cost 24 dependent round
+// trips for 9 rows of 6144 (2048 x 6144 at W = 9: 12.3 us a call); now kStageBatch loads per trip, and the eight
+// consecutive lanes that hold a group add its sum by shuffles.
+constexpr int kStageBatch = 8;
+__device__ __forceinline__ void gemv_stage_activations(const GemvParams &p, unsigned char *smem, const GemvSmem &L) {
+    const int ng = p.K / BM_GROUP, units = p.K / 16, total = p.W * units, lane = threadIdx.x & 31;
+    const uint32_t inv_units = 0xffffffffu / (uint32_t)units + 1u;        // i / units = umulhi(i, inv_units): i * units < 2^32
     int *asum = reinterpret_cast<int *>(smem + L.asum_off);
-    for (int i = threadIdx.x; i < wrows * ng; i += blockDim.x) asum[i] = 0;
-    __syncthreads();
-    const int units = p.K / 16;
-    for (int i = threadIdx.x; i < wrows * units; i += blockDim.x) {
-        const int m = i / units, j = i - m * units;
-        uint4 x = make_uint4(0u, 0u, 0u, 0u);
-        if (m < p.W) x = *reinterpret_cast<const uint4 *>(p.A + (size_t)m * p.K + 16 * j);
-        const uint32_t lo01 = __byte_perm(x.x, x.y, 0x5140), lo23 = __byte_perm(x.z, x.w, 0x5140);
-        const uint32_t hi01 = __byte_perm(x.x, x.y, 0x7362), hi23 = __byte_perm(x.z, x.w, 0x7362);
-        uint4 y;
-        y.x = __byte_perm(lo01, lo23, 0x5410);
-        y.y = __byte_perm(lo01, lo23, 0x7632);
-        y.z = __byte_perm(hi01, hi23, 0x5410);
-        y.w = __byte_perm(hi01, hi23, 0x7632);
-        *reinterpret_cast<uint4 *>(smem + L.act_off + m * L.act_stride + 16 * j) = y;
-        int sum = __dp4a((int)x.x, 0x01010101, 0);
-        sum = __dp4a((int)x.y, 0x01010101, sum);
-        sum = __dp4a((int)x.z, 0x01010101, sum);
-        sum = __dp4a((int)x.w, 0x01010101, sum);
-        if (m < p.W) atomicAdd(&asum[m * ng + (j >> 3)], sum);
+    const uint4 *src = reinterpret_cast<const uint4 *>(p.A);
+    for (int b0 = 0; b0 < total; b0 += kStageBatch * kGemvThreads) {
+        uint4 xs[kStageBatch];
+#pragma unroll
+        for (int u = 0; u < kStageBatch; ++u) {
+            const int i = b0 + u * kGemvThreads + (int)threadIdx.x;
+            xs[u] = i < total ? src[i] : make_uint4(0u, 0u, 0u, 0u);
+        }
+#pragma unroll
+        for (int u = 0; u < kStageBatch; ++u) {
+            const int i = b0 + u * kGemvThreads + (int)threadIdx.x;
+            if (b0 + u * kGemvThreads >= total) break;                    // uniform
+            const int m = (int)__umulhi((uint32_t)i, inv_units), j = i - m * units;
+            const uint4 x = xs[u];
+            const uint32_t lo01 = __byte_perm(x.x, x.y, 0x5140), lo23 = __byte_perm(x.z, x.w, 0x5140);
+            const uint32_t hi01 = __byte_perm(x.x, x.y, 0x7362), hi23 = __byte_perm(x.z, x.w, 0x7362);
+            uint4 y;
+            y.x = __byte_perm(lo01, lo23, 0x5410);
+            y.y = __byte_perm(lo01, lo23, 0x7632);
+            y.z = __byte_perm(hi01, hi23, 0x5410);
+            y.w = __byte_perm(hi01, hi23, 0x7632);
+            if (i < total) *reinterpret_cast<uint4 *>(smem + L.act_off + m * L.act_stride + 16 * j) = y;
+            int sum = __dp4a((int)x.x, 0x01010101, 0);
+            sum = __dp4a((int)x.y, 0x01010101, sum);
+            sum = __dp4a((int)x.z, 0x01010101, sum);
+            sum = __dp4a((int)x.w, 0x01010101, sum);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 1);                  // units % 8 == 0: eight lanes hold one group
+            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+            if (i < total && (lane & 7) == 0) asum[m * ng + (j >> 3)] = sum;
+        }
     }
 }
 
@@ -274,13 +290,13 @@ __global__ void __launch_bounds__(kGemvThreads) t2_gemv_dp4a_kernel(const GemvPa
     if (warp == 0) {
         for (int i = 0; i < p.stages - 1 && i < my_tiles; ++i) {
             const int n0 = (blockIdx.x + i * gridDim.x) * R;
-            gemv_issue_tile(p, smem + L.stage_off + i * L.stage_bytes, L, &bars[i], n0,
+            gemv_issue_tile<false>(p, smem + L.stage_off + i * L.stage_bytes, L, &bars[i], n0,
                             min(R, p.N - n0), lane);
         }
     }
     pdl_launch_dependents();
     if (p.pdl) pdl_wait();
-    gemv_stage_activations(p, smem, L, p.W);
+    gemv_stage_activations(p, smem, L);
     __syncthreads();
 
     const int *asum = reinterpret_cast<const int *>(smem + L.asum_off);
@@ -292,7 +308,7 @@ __global__ void __launch_bounds__(kGemvThreads) t2_gemv_dp4a_kernel(const GemvPa
             const int nx = i + p.stages - 1;
             if (nx < my_tiles) {
                 const int n0 = (blockIdx.x + nx * gridDim.x) * R;
-                gemv_issue_tile(p, smem + L.stage_off + (nx % p.stages) * L.stage_bytes, L,
+                gemv_issue_tile<false>(p, smem + L.stage_off + (nx % p.stages) * L.stage_bytes, L,
                                 &bars[nx % p.stages], n0, min(R, p.N - n0), lane);
             }
         }
@@ -556,7 +572,11 @@ __device__ __forceinline__ void mma_group_step(const AFrag<HALF> &f, uint2 w2, f
     }
 }
 
-template <int RB, bool HALF, bool ONECHUNK, bool EMIT_G>
+// Where the activations come from.  A build of its own each, and SILU (the gate|up epilogue) too: a decode launch is a few
+// microseconds over instructions that the previous kernel has evicted, and what it does not run still costs it.
+enum : int { kSrcNatural = 0, kSrcPrepared = 1, kSrcRow = 2 };
+
+template <int RB, bool HALF, bool ONECHUNK, bool EMIT_G, int SRC, bool SILU>
 __global__ void __launch_bounds__(kGemvThreads, 2) t2_gemv_mma_kernel(const GemvParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
     constexpr int R = 8 * RB, RP = R + 8, WROWS = HALF ? 8 : 16;
@@ -565,11 +585,11 @@ __global__ void __launch_bounds__(kGemvThreads, 2) t2_gemv_mma_kernel(const Gemv
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int r = lane >> 2, q = lane & 3;
-    const int R_out = p.silu_F ? R / 2 : R;            // output columns per tile
+    const int R_out = SILU ? R / 2 : R;            // output columns per tile
     const int n_tiles = p.N / R_out;
     const int nch = ONECHUNK ? 1 : (ng + BM_SLOTS - 1) / BM_SLOTS;
     __shared__ unsigned int amax_sh[16];
-    if (p.silu_F && threadIdx.x < 16) amax_sh[threadIdx.x] = 0u;
+    if (SILU && threadIdx.x < 16) amax_sh[threadIdx.x] = 0u;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < p.stages; ++i) mbar_init(&bars[i], 1);
@@ -585,12 +605,11 @@ __global__ void __launch_bounds__(kGemvThreads, 2) t2_gemv_mma_kernel(const Gemv
     LS.scale_off_in_stage = L.scale_off_in_stage;
     if (warp == 0) {
         for (int i = 0; i < p.stages && i < my_tiles; ++i)
-            gemv_issue_tile(p, smem + L.stage_off + i * L.stage_bytes, LS, &bars[i],
+            gemv_issue_tile<SILU>(p, smem + L.stage_off + i * L.stage_bytes, LS, &bars[i],
                             (blockIdx.x + i * gridDim.x) * R_out, R, lane);
     }
     pdl_launch_dependents();
     if (p.pdl) pdl_wait();
-    const bool prepared = p.asum != nullptr;
     // Where fragments come from: the caller's GEMV-ready rows (one chunk: straight from
     // global memory, nothing is staged), or the shared-memory staging area.
     const unsigned char *arows = smem + L.act_off;
@@ -600,16 +619,16 @@ __global__ void __launch_bounds__(kGemvThreads, 2) t2_gemv_mma_kernel(const Gemv
     bool a_ok = true;
     {
         float *invs_w = reinterpret_cast<float *>(smem + L.invs_off);
-        if (p.src_mode == 0 && threadIdx.x < 16) invs_w[threadIdx.x] = threadIdx.x < p.W ? 1.0f / p.s[threadIdx.x] : 0.0f;
-        if (p.src_mode != 0) {
+        if (SRC != kSrcRow && threadIdx.x < 16) invs_w[threadIdx.x] = threadIdx.x < p.W ? 1.0f / p.s[threadIdx.x] : 0.0f;
+        if (SRC == kSrcRow) {
             __shared__ float stage_sh[32];
             gemv_stage_row_from_bf16(p, smem, L.act_off, L.asum_off, L.invs_off, stage_sh);
-        } else if (!prepared) {
+        } else if (SRC == kSrcNatural) {
             GemvSmem LA;
             LA.act_off = L.act_off;
             LA.act_stride = L.act_stride;
             LA.asum_off = L.asum_off;
-            gemv_stage_activations(p, smem, LA, WROWS);
+            gemv_stage_activations(p, smem, LA);
         } else if (ONECHUNK) {
             arows = reinterpret_cast<const unsigned char *>(p.A);
             astride = p.K;
@@ -713,11 +732,11 @@ __global__ void __launch_bounds__(kGemvThreads, 2) t2_gemv_mma_kernel(const Gemv
         }
         // Every warp is done with stage `st`: refill it with the tile `stages` ahead.
         if (warp == 0 && i + p.stages < my_tiles)
-            gemv_issue_tile(p, smem + L.stage_off + st * L.stage_bytes, LS, &bars[st],
+            gemv_issue_tile<SILU>(p, smem + L.stage_off + st * L.stage_bytes, LS, &bars[st],
                             (blockIdx.x + (i + p.stages) * gridDim.x) * R_out, R, lane);
         // Remaining tree levels, reciprocal multiply, store.  Thread = (token, 4 rows).
         const float *pr = part + (i & 1) * L.part_buf_floats;
-        if (p.silu_F) {
+        if (SILU) {
             // rows [0, R/2) of the tile are gate rows, rows [R/2, R) the up rows of the same columns:
             // inner = bf16(silu(bf16 gate) * bf16 up), as the stand-alone SiLU kernel computes it from
             // the bf16 projection outputs
@@ -772,7 +791,7 @@ __global__ void __launch_bounds__(kGemvThreads, 2) t2_gemv_mma_kernel(const Gemv
         }
     }
     (void)failed;
-    if (p.silu_F) {
+    if (SILU) {
         __syncthreads();
         if (threadIdx.x < p.W && amax_sh[threadIdx.x] != 0u) atomicMax(&p.amax_out[threadIdx.x], amax_sh[threadIdx.x]);
     }
