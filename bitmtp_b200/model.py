@@ -73,13 +73,16 @@ def t2g128_int8xint2_linear(a_int8: torch.Tensor, b_packed: torch.Tensor, s: tor
     through the library's drop-in symbol of the same name.  `validate_registry`
     restricts (M, N, K) to the reference's registered triples.
     """
+    if native._host is not None and not validate_registry:
+        # this call is bound by the host: checks, allocation and launch in one native function (None: not such a call)
+        out = native._host.linear(a_int8, b_packed, s, ws)
+        if out is not None:
+            return out
     m, n, k = _validate_packed_inputs(a_int8, b_packed, s, ws, validate_registry=validate_registry)
     if _t2_lib is None:
         load_t2_kernel()
     dev = a_int8.device
     out = torch.empty((*a_int8.shape[:-1], n), dtype=torch.bfloat16, device=dev)
-    # plain integers through the declared prototype: this call is bound by the host, and wrapping each pointer and
-    # building a Stream object for its handle cost as much as the launch itself
     _t2_lib.t2g128_int8xint2_linear(a_int8.data_ptr(), b_packed.data_ptr(), out.data_ptr(), s.data_ptr(), ws.data_ptr(),
                                     m, n, k, ops._stream(dev))
     return out
@@ -173,8 +176,13 @@ class T2LinearKernel(nn.Module):
         The reference falls back to a dense bf16 GEMM on unpacked weights for unregistered widths (model.py:650-656);
         the integer path gives the same quantised product without the bf16 roundings and without the dense copy of the
         weights."""
-        x2 = x.reshape(-1, self.in_features).contiguous()
         w, ws = self.weight.data, self.weight_scale
+        if native._host is not None and x.shape[-1:] == (self.in_features,):
+            # checks, allocations and both launches in one native function (None: not such a call)
+            out = native._host.linear_rows(x, w, ws, ops.gemv_serves_rows, ops.GEMM_WIDE_MAX_ROWS)
+            if out is not None:
+                return out
+        x2 = x.reshape(-1, self.in_features).contiguous()
         if x2.shape[0] > self.MAX_ROWS:
             out = ops.t2_linear_rows(x2, w, ws)
         else:

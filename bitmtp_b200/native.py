@@ -12,10 +12,13 @@ import ctypes
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 SO_PATH = os.path.join(HERE, "libbitmtp_b200.so")
+HOST_SO_PATH = os.path.join(HERE, "_host.so")
+HOST_SOURCE = os.path.join(CSRC, "host_path.cpp")
 SOURCES = ["bm_lib.cu"]
 HEADERS = ["bm_math.h", "bm_common.cuh", "t2_gemv.cuh", "fused_ops.cuh", "verify_attn.cuh", "prompt_attn.cuh", "t2_gemv_rowwarp.cuh",
            "t2_gemv_direct.cuh", "dense_head.cuh", "t2_gemm_wide.cuh"]
@@ -38,20 +41,22 @@ ROLE_DRAFT, ROLE_VERIFY, ROLE_AR = 0, 1, 2
 PDL_OVERLAP, PDL_STABLE_STATE, PDL_STAGED = 1, 2, 4
 
 _lib = None
+_host = None        # the native host path (csrc/host_path.cpp), bound when the library is loaded
 
 
-def _stale() -> bool:
-    if not os.path.exists(SO_PATH):
+def _stale(so: str, deps) -> bool:
+    if not os.path.exists(so):
         return True
-    t = os.path.getmtime(SO_PATH)
-    deps = [os.path.join(CSRC, f) for f in SOURCES + HEADERS]
-    deps.append(os.path.join(HERE, "..", "include", "bitmtp_b200.h"))
+    t = os.path.getmtime(so)
     return any(os.path.exists(p) and os.path.getmtime(p) > t for p in deps)
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile the CUDA library for sm_100a if sources are newer than the .so."""
-    if not force and not _stale():
+    """Compile the CUDA library for sm_100a and the host path's extension module where sources are newer."""
+    if force or _stale(HOST_SO_PATH, [HOST_SOURCE]):
+        _build_host(verbose)
+    deps = [os.path.join(CSRC, f) for f in SOURCES + HEADERS] + [os.path.join(HERE, "..", "include", "bitmtp_b200.h")]
+    if not force and not _stale(SO_PATH, deps):
         return SO_PATH
     nvcc = os.environ.get("NVCC", "nvcc")
     cmd = [nvcc] + NVCC_FLAGS + [os.path.join(CSRC, s) for s in SOURCES] + ["-o", SO_PATH + ".tmp"]
@@ -64,13 +69,41 @@ def build(force: bool = False, verbose: bool = False) -> str:
     return SO_PATH
 
 
+def _build_host(verbose: bool = False) -> None:
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f"-I{root}/include",
+           f"-I{root}/include/torch/csrc/api/include", f"-I{sysconfig.get_paths()['include']}", f"-I{cuda}/include",
+           HOST_SOURCE, "-o", HOST_SO_PATH + ".tmp", f"-L{root}/lib", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+    if verbose:
+        print(" ".join(cmd), file=sys.stderr)
+    subprocess.run(cmd, check=True)
+    os.replace(HOST_SO_PATH + ".tmp", HOST_SO_PATH)
+
+
 class NativeError(RuntimeError):
     pass
 
 
+def _load_host(L):
+    """The extension module of csrc/host_path.cpp, given the library's entry points."""
+    if not os.path.exists(HOST_SO_PATH):
+        raise NativeError(f"{HOST_SO_PATH} is missing: build it with `python -m bitmtp_b200.native`")
+    import importlib.util
+    import torch  # noqa: F401  (its libraries resolve the module's symbols)
+    spec = importlib.util.spec_from_file_location("bitmtp_b200._host", HOST_SO_PATH)
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    mod.bind(*(ctypes.cast(getattr(L, n), ctypes.c_void_p).value
+               for n in ("t2g128_int8xint2_linear", "bm_quant_rows", "bm_t2_gemv", "bm_t2_gemv_prepared", "bm_t2_gemm_wide")))
+    return mod
+
+
 def lib() -> ctypes.CDLL:
     """The loaded library.  Raises if it has not been built: there is no fallback."""
-    global _lib
+    global _lib, _host
     if _lib is not None:
         return _lib
     if not os.path.exists(SO_PATH):
@@ -90,6 +123,7 @@ def lib() -> ctypes.CDLL:
     L.t2g128_int8xint2_linear.argtypes = [vp, vp, vp, vp, vp, ci, ci, ci, vp]
     L.t2g128_int8xint2_linear.restype = None
     _declare_optional(L)
+    _host = _load_host(L)
     _lib = L
     return L
 

@@ -1,0 +1,93 @@
+"""The native host path of single packed products (csrc/host_path.cpp) against the Python path it stands in for: the same
+bits where it takes a call, None - so that the Python path serves or refuses the call - everywhere else."""
+import pytest
+import torch
+
+from bitmtp_b200 import model as BM
+from bitmtp_b200 import native, ops, synthetic
+from bitmtp_b200.model import T2LinearKernel
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda:0")
+
+
+def _operands(rows, n=264, k=768, seed=0):
+    gen = torch.Generator(device=DEV).manual_seed(seed)
+    packed, scale = synthetic.device_ternary(n, k, gen, DEV)
+    x = torch.randn(rows, k, generator=gen, device=DEV).to(torch.bfloat16)
+    native.lib()
+    return x, packed, scale
+
+
+def _without_host(monkeypatch, fn):
+    with monkeypatch.context() as m:
+        m.setattr(native, "_host", None)
+        return fn()
+
+
+@pytest.mark.parametrize("shape", [(1,), (17,), (32,), (1, 1), (2, 5)])
+def test_operator(monkeypatch, shape):
+    rows = shape[0] * (shape[1] if len(shape) == 2 else 1)
+    x, packed, scale = _operands(rows)
+    q, s = ops.quant_rows(x)
+    q, s = q.view(*shape, -1), s.view(*shape, 1)
+    got = native._host.linear(q, packed, s, scale)
+    want = _without_host(monkeypatch, lambda: BM.t2g128_int8xint2_linear(q, packed, s, scale))
+    assert got.shape == want.shape and got.dtype == want.dtype and torch.equal(got.view(torch.int16), want.view(torch.int16))
+    with torch.inference_mode():
+        assert BM.t2g128_int8xint2_linear(q, packed, s, scale).is_inference()
+
+
+@pytest.mark.parametrize("rows", [1, 2, 9, 16, 17, 32, 33, 200])
+@pytest.mark.parametrize("n,k", [(264, 768), (8, 128), (4104, 1024), (520, 384), (2048, 6144)])
+def test_module(monkeypatch, rows, n, k):
+    x, packed, scale = _operands(rows, n, k, seed=rows)
+    layer = T2LinearKernel(k, n).to(DEV)
+    layer.weight.data, layer.weight_scale = packed, scale
+    for xs in (x, x.view(1, rows, k), x[0]):
+        got = native._host.linear_rows(xs, layer.weight.data, scale, ops.gemv_serves_rows, ops.GEMM_WIDE_MAX_ROWS)
+        want = _without_host(monkeypatch, lambda: layer(xs))
+        assert got.shape == want.shape and torch.equal(got.view(torch.int16), want.view(torch.int16))
+        assert torch.equal(layer(xs).view(torch.int16), want.view(torch.int16))
+    # every second column: not contiguous, served by the Python path after a copy
+    wide = torch.stack([x, x], dim=-1)[..., 0]
+    assert native._host.linear_rows(wide, packed, scale, ops.gemv_serves_rows, ops.GEMM_WIDE_MAX_ROWS) is None
+    assert torch.equal(layer(wide).view(torch.int16), layer(x).view(torch.int16))
+
+
+class _Tagged(torch.Tensor):
+    pass
+
+
+def test_what_is_left_to_the_python_path():
+    x, packed, scale = _operands(4)
+    q, s = ops.quant_rows(x)
+    bad = [(q.cpu(), packed, s, scale), (q[:, :640], packed, s, scale), (q, packed.t(), s, scale),
+           (q, packed, s, scale[:, :2]), (q.float(), packed, s, scale), (q, packed, s.double(), scale),
+           (q, packed, s, scale.float()), (q, packed, s[:3], scale), (q, packed, s.view(1, 4), scale), (q, packed, None, scale),
+           (q[None, None], packed, s, scale), (q.as_subclass(_Tagged), packed, s, scale), (q[:0], packed, s[:0], scale),
+           (q, packed[:12], s, scale[:12]), (q.repeat(9, 1), packed, s.repeat(9, 1), scale)]
+    for args in bad:
+        assert native._host.linear(*args) is None
+    for args in (bad[0], bad[1], bad[3], bad[5], bad[13], bad[14]):
+        with pytest.raises((RuntimeError, ValueError)):
+            BM.t2g128_int8xint2_linear(*args)
+    with pytest.raises(RuntimeError):                       # the registry does not list these sizes
+        BM.t2g128_int8xint2_linear(q, packed, s, scale, validate_registry=True)
+
+    class Mode(torch.overrides.TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    with Mode():
+        assert native._host.linear(q, packed, s, scale) is None
+
+    def inside(row):
+        assert native._host.linear_rows(row, packed, scale, ops.gemv_serves_rows, ops.GEMM_WIDE_MAX_ROWS) is None
+        return row
+
+    torch.func.vmap(inside)(x.view(2, 2, -1))
+    torch.func.jvp(inside, (x,), (x,))
+    assert native._host.linear_rows(x.float(), packed, scale, ops.gemv_serves_rows, ops.GEMM_WIDE_MAX_ROWS) is None
+    shifted = torch.cat([scale.view(-1)[:4], scale.view(-1)])[4:].view_as(scale)
+    assert native._host.linear_rows(x, packed, shifted, ops.gemv_serves_rows, ops.GEMM_WIDE_MAX_ROWS) is None
