@@ -18,7 +18,7 @@
 #include "t2_gemv_rowwarp.cuh"
 #include "t2_gemv_direct.cuh"
 #include "dense_head.cuh"
-#include "t2_gemm_wide.cuh"
+#include "t2_gemm_tc.cuh"
 
 #include <cudaTypedefs.h>
 #include <map>
@@ -304,9 +304,32 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t
                                   CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
                                   CUtensorMapFloatOOBfill);
 
+// Descriptor of a byte matrix [rows, row_bytes] for copies of [box_rows, box_bytes].
+int encode_byte_map(const void *base, int rows, int row_bytes, int box_rows, int box_bytes, CUtensorMapSwizzle swizzle,
+                    CUtensorMap *out) {
+    static std::atomic<EncodeTiledFn> encode{nullptr};
+    EncodeTiledFn fn = encode.load(std::memory_order_acquire);
+    if (fn == nullptr) {
+        void *sym = nullptr;
+        cudaDriverEntryPointQueryResult qres;
+        const cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &qres);
+        if (e != cudaSuccess) return cuda_status(e);
+        if (sym == nullptr || qres != cudaDriverEntryPointSuccess) return BM_EINVAL;
+        fn = reinterpret_cast<EncodeTiledFn>(sym);
+        encode.store(fn, std::memory_order_release);
+    }
+    const cuuint64_t dims[2] = {(cuuint64_t)row_bytes, (cuuint64_t)rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)row_bytes};
+    const cuuint32_t box[2] = {(cuuint32_t)box_bytes, (cuuint32_t)box_rows};
+    const cuuint32_t estr[2] = {1, 1};
+    const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(base), dims, strides, box, estr,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? BM_OK : BM_ECUDA_BASE + 999;
+}
+
 int weight_tensor_map(const void *B, int N, int K, CUtensorMap *out) {
     static std::mutex mu;
-    static EncodeTiledFn encode = nullptr;
     static std::map<std::tuple<int, const void *, int, int>, CUtensorMap> cache;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -315,23 +338,9 @@ int weight_tensor_map(const void *B, int N, int K, CUtensorMap *out) {
     const auto key = std::make_tuple(dev, B, N, K);
     auto it = cache.find(key);
     if (it != cache.end()) { *out = it->second; return BM_OK; }
-    if (encode == nullptr) {
-        void *fn = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres);
-        if (e != cudaSuccess) return cuda_status(e);
-        if (fn == nullptr || qres != cudaDriverEntryPointSuccess) return BM_EINVAL;
-        encode = reinterpret_cast<EncodeTiledFn>(fn);
-    }
     CUtensorMap tm;
-    const cuuint64_t dims[2] = {(cuuint64_t)(K / 4), (cuuint64_t)N};
-    const cuuint64_t strides[1] = {(cuuint64_t)(K / 4)};
-    const cuuint32_t box[2] = {(cuuint32_t)bm::kRwPanelBytes, (cuuint32_t)bm::kRwRows};
-    const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = encode(&tm, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(B), dims, strides, box, estr,
-                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return BM_ECUDA_BASE + 999;
+    const int rc = encode_byte_map(B, N, K / 4, bm::kRwRows, bm::kRwPanelBytes, CU_TENSOR_MAP_SWIZZLE_128B, &tm);
+    if (rc != BM_OK) return rc;
     if (cache.size() > 4096) cache.clear();
     cache[key] = tm;
     *out = tm;
@@ -395,6 +404,40 @@ int gemv_launch_rowwarp(const bm::GemvParams &p0, int sms, int pdl, cudaStream_t
     if (ks == 1) return launch_rowwarp<2, 2, 1>(P, c.warps, sms, pdl, stream);
     if (ks == 2) return launch_rowwarp<2, 2, 2>(P, c.warps, sms, pdl, stream);
     return launch_rowwarp<2, 1, 4>(P, c.warps, sms, pdl, stream);
+}
+
+// ---- many-row product ---------------------------------------------------------------
+constexpr int kTcMaxK = 51200;               // part of the interface: what a caller may rely on being refused
+constexpr int kTcMaxRows = 32 * 65535;
+
+// Prompt rows per tile, 32 (two CTAs per SM) or 64 (one).  A wave of 64-row tiles is the unit; one of 32-row tiles takes 0.7
+// (K = 2048) to 0.8 of it while every SM has one CTA and 1.15 to 1.4 when it has two.  us, 32 / 64: 2048 x 2048, 256 rows
+// 10.6 / 12.7; 6144 x 2048, 256 rows 18.8 / 20.7, 333 rows 24.8 / 20.8; 12288 x 2048, 1024 rows 105 / 89; 2560 x 9728,
+// 17 rows 29.8 / 35.2, 256 rows 47 / 36.
+inline int tc_columns(int T, int N, int K, int sms) {
+    const long long rows = (N + bm::kTcRows - 1) / bm::kTcRows;
+    const long long t64 = rows * ((T + 63) / 64), t32 = rows * ((T + 31) / 32);
+    const long long full = K == BM_SLOTS * BM_GROUP ? 115 : 135, half = K == BM_SLOTS * BM_GROUP ? 70 : 75;
+    const long long rest = t32 % (2 * sms);
+    const long long c64 = 100 * ((t64 + sms - 1) / sms);
+    const long long c32 = full * (t32 / (2 * sms)) + (rest == 0 ? 0 : rest <= sms ? half : full);
+    return c32 < c64 ? 32 : 64;
+}
+
+template <int NT>
+int launch_tc(bm::TcParams &p, const void *A, const void *B, cudaStream_t stream) {
+    int rc = encode_byte_map(A, p.T, p.K, NT, BM_GROUP, CU_TENSOR_MAP_SWIZZLE_128B, &p.a_map);
+    if (rc == BM_OK) rc = encode_byte_map(B, p.N, p.K / 4, bm::kTcRows, BM_GROUP / 4, CU_TENSOR_MAP_SWIZZLE_32B, &p.b_map);
+    if (rc != BM_OK) return rc;
+    const int sms = current_device().sm_count;
+    p.t_tiles = (p.T + NT - 1) / NT;
+    const long long tiles = (long long)p.t_tiles * ((p.N + bm::kTcRows - 1) / bm::kTcRows);
+    if (tiles > 0x3fffffffLL) return BM_EINVAL;
+    p.tiles = (int)tiles;
+    const int resident = sms * (NT == 32 ? 2 : 1), grid = p.tiles < resident ? p.tiles : resident;
+    const dim3 block(bm::tc_threads(NT));
+    if (p.K == BM_SLOTS * BM_GROUP) return launch_ex(bm::t2_gemm_tc_kernel<NT, true>, dim3(grid), block, bm::tc_smem_bytes(NT), stream, p.pdl, p);
+    return launch_ex(bm::t2_gemm_tc_kernel<NT, false>, dim3(grid), block, bm::tc_smem_bytes(NT), stream, p.pdl, p);
 }
 
 }  // namespace
@@ -1119,21 +1162,15 @@ int bm_t2_gemm_wide(const void *A_prep, const void *a_sums, const void *B, void 
         K < BM_GROUP || (K % BM_GROUP) != 0 || ldc < N)
         return BM_EINVAL;
     if (!aligned16(A_prep) || !aligned16(B)) return BM_EINVAL;
-    const size_t smem = bm::wide_smem_bytes(K / BM_GROUP, K == BM_SLOTS * BM_GROUP);
-    if (smem > (size_t)kMaxSmemPerCta) return BM_EINVAL;
-    bm::WideParams p;
-    p.A = static_cast<const int8_t *>(A_prep);
+    if (K > kTcMaxK || T > kTcMaxRows) return BM_EINVAL;
+    bm::TcParams p;
     p.asum = static_cast<const int32_t *>(a_sums);
     p.s = static_cast<const float *>(s);
-    p.B = static_cast<const uint8_t *>(B);
     p.ws = static_cast<const uint16_t *>(ws);
     p.C = static_cast<uint16_t *>(C);
     p.T = T; p.N = N; p.K = K; p.ldc = ldc; p.pdl = pdl & BM_PDL_OVERLAP;
-    const dim3 grid((N + bm::kWideRows - 1) / bm::kWideRows, (T + bm::kWideTokens - 1) / bm::kWideTokens);
-    if (grid.y > 65535) return BM_EINVAL;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (K == BM_SLOTS * BM_GROUP) return launch_ex(bm::t2_gemm_wide_kernel<true>, grid, dim3(bm::kWideThreads), smem, st, p.pdl, p);
-    return launch_ex(bm::t2_gemm_wide_kernel<false>, grid, dim3(bm::kWideThreads), smem, st, p.pdl, p);
+    return tc_columns(T, N, K, current_device().sm_count) == 32 ? launch_tc<32>(p, A_prep, B, st) : launch_tc<64>(p, A_prep, B, st);
 }
 
 namespace {

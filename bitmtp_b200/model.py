@@ -171,8 +171,8 @@ class T2LinearKernel(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         """Any number of rows.  Up to MAX_ROWS of them are one launch of the decode GEMV; more go where
-        ops.t2_linear_rows takes them, to the many-row kernel, which reads each weight byte once per 32 rows (333 rows of
-        6144 x 2048: 401 us in slabs of MAX_ROWS, 38 us), or, for few rows of a narrow, deep weight, through the GEMV.
+        ops.t2_linear_rows takes them, to the many-row kernel, which reads each weight byte once per 32 or 64 rows (333 rows
+        of 6144 x 2048: 401 us in slabs of MAX_ROWS, 22.5 us), or, for few rows of a narrow, deep weight, through the GEMV.
         The reference falls back to a dense bf16 GEMM on unpacked weights for unregistered widths (model.py:650-656);
         the integer path gives the same quantised product without the bf16 roundings and without the dense copy of the
         weights."""

@@ -21,7 +21,7 @@ HOST_SO_PATH = os.path.join(HERE, "_host.so")
 HOST_SOURCE = os.path.join(CSRC, "host_path.cpp")
 SOURCES = ["bm_lib.cu"]
 HEADERS = ["bm_math.h", "bm_common.cuh", "t2_gemv.cuh", "fused_ops.cuh", "verify_attn.cuh", "prompt_attn.cuh", "t2_gemv_rowwarp.cuh",
-           "t2_gemv_direct.cuh", "dense_head.cuh", "t2_gemm_wide.cuh"]
+           "t2_gemv_direct.cuh", "dense_head.cuh", "t2_gemm_tc.cuh"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

@@ -281,15 +281,13 @@ GEMV_MAX_K = 11264                 # 16 INT8 rows and one tile of weights fill t
 def gemv_serves_rows(T: int, N: int, K: int) -> bool:
     """Whether 17 to 32 rows are two launches of the decode GEMV instead of one of the many-row kernel.
 
-    The many-row kernel gives 128 weight rows x 32 prompt rows to one CTA, which walks the K / 128 groups in series: with
-    few CTAs its time is that walk, 4 us + 4.2 us per 1024 of K, however small N is.  The GEMV spreads the weight rows over
-    all SMs.  Device us for 17 / 32 rows, GEMV against many-row kernel: 512 x 1024 9.6 / 9.3 - 11.1 / 11.4, 4096 x 1024
-    11.0 / 10.9 - 11.1 / 11.8, 512 x 2048 9.9 / 10.0 - 12.6 / 13.3, 512 x 9728 14.0 / 14.7 - 43.0 / 45.0, 4096 x 9728
-    24.7 / 28.3 - 45.6 / 47.8.  The other side: 6144 x 1024 13.0 / 12.9 - 11.3 / 12.0, 4096 x 512 12.3 / 12.0 - 9.4 / 10.0,
-    12288 x 2048 18.1 / 18.5 - 14.7 / 15.5.  Odd group counts go through the GEMV's slower consumer (512 x 1152, in slabs
-    of 16: 16.8 / 26.9 - 11.6 / 12.1); from 33 rows on the GEMV would read the weights three times (512 x 9728: 44.9 - 45.0,
-    2048 x 2048: 19.1 - 13.7)."""
-    return 16 < T <= 32 and 1024 <= K <= GEMV_MAX_K and K % 256 == 0 and N <= 4096
+    The many-row kernel gives 128 weight rows to one CTA, which walks the K / 128 groups in series: with few CTAs its time is
+    that walk, about 5 us + 2.5 us per 1024 of K, however small N is.  The GEMV spreads the weight rows over all SMs.  Device
+    us for 17 / 32 rows, GEMV - many-row kernel: 512 x 4096 12.1 / 12.2 - 16.6, 512 x 9728 13.5 / 14.0 - 28.9, 2048 x 6144
+    14.5 / 16.5 - 20.7, 4096 x 4096 14.5 / 16.6 - 16.6, 4096 x 9728 23.9 / 26.2 - 29.7 / 30.6.  The other side: 512 x 1024
+    10.7 - 9.8, 4096 x 2048 12.5 - 10.4, 6144 x 4096 18.6 / 20.7 - 16.6, 6144 x 6144 24.8 / 28.9 - 20.7.  Odd group counts go
+    through the GEMV's slower consumer; from 33 rows on the GEMV would read the weights three times."""
+    return 16 < T <= 32 and 2048 < K <= GEMV_MAX_K and K % 256 == 0 and N <= 4096
 
 
 def t2_linear_rows(x: torch.Tensor, b_packed: torch.Tensor, ws: torch.Tensor) -> torch.Tensor:

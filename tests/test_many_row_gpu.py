@@ -156,6 +156,27 @@ def test_linear_module_at_its_limits():
     assert bool((got[:-1] == got[0]).all())
 
 
+@pytest.mark.parametrize("N,K", [(8, 128), (128, 1152), (136, 2048), (128, 2176), (264, 4096), (19000, 2048)])
+@pytest.mark.parametrize("T", [1, 31, 32, 33, 63, 64, 65, 130, 300])
+def test_many_row_product_at_tile_edges(N, K, T):
+    """Row counts and weight rows on both sides of a tile, fewer than 16 groups, an odd number of them, two and three per
+    slot, more tiles than CTAs; scales of either sign, rows of zeros and weights of zeros (the sign of a zero counts)."""
+    gen = torch.Generator(device=DEV).manual_seed(N + K + T)
+    packed, scale = synthetic.device_ternary(N, K, gen, torch.device(DEV))
+    packed[N // 2] = -86                                   # 0b10101010: codes of zero
+    scale[::3] *= -1.0
+    x = torch.randn(T, K, generator=gen, device=DEV).to(torch.bfloat16)
+    x[T // 2] = 0.0
+    qp, sums, s = ops.quant_rows(x, prepared=True)
+    out = torch.full((T + 1, N), 7.0, dtype=torch.bfloat16, device=DEV)
+    ops.t2_gemm_wide(qp, sums, packed, s, scale, out=out[:T])
+    q, s = ops.quant_rows(x)
+    want = torch.cat([ops.t2_gemv(q[r:r + SLAB], packed, s[r:r + SLAB], scale) for r in range(0, T, SLAB)])
+    torch.cuda.synchronize()
+    assert native.lib().bm_device_error() == 0
+    assert torch.equal(out[:T].view(torch.int16), want.view(torch.int16)) and bool((out[T] == 7.0).all())
+
+
 def _packed_model(geo, max_positions):
     cfg = synthetic.make_config(geo, block_size=8)
     state = synthetic.make_state(cfg, seed=4)
