@@ -617,9 +617,11 @@ __global__ void __launch_bounds__(kGemvThreads, 2) t2_gemv_mma_kernel(const Gemv
     const int *asum = reinterpret_cast<const int *>(smem + L.asum_off);
     uint64_t *abar = bars + kMaxStages;
     bool a_ok = true;
+    AFrag<HALF> fA, fB;
     {
+        // what depends on the previous kernel is requested together: one memory round trip
+        const float s_row = SRC != kSrcRow && (int)threadIdx.x < p.W && threadIdx.x < 16 ? p.s[threadIdx.x] : 0.0f;
         float *invs_w = reinterpret_cast<float *>(smem + L.invs_off);
-        if (SRC != kSrcRow && threadIdx.x < 16) invs_w[threadIdx.x] = threadIdx.x < p.W ? 1.0f / p.s[threadIdx.x] : 0.0f;
         if (SRC == kSrcRow) {
             __shared__ float stage_sh[32];
             gemv_stage_row_from_bf16(p, smem, L.act_off, L.asum_off, L.invs_off, stage_sh);
@@ -633,6 +635,8 @@ __global__ void __launch_bounds__(kGemvThreads, 2) t2_gemv_mma_kernel(const Gemv
             arows = reinterpret_cast<const unsigned char *>(p.A);
             astride = p.K;
             asum = p.asum;
+            load_afrag<HALF>(fA, arows, astride, asum, p.W, ng, 2 * warp, r, q);
+            load_afrag<HALF>(fB, arows, astride, asum, p.W, ng, 2 * warp + 1, r, q);
         } else {
             // several chunks: the rows are copied in bulk (no permutation left to do)
             if (warp == 1) {
@@ -643,14 +647,27 @@ __global__ void __launch_bounds__(kGemvThreads, 2) t2_gemv_mma_kernel(const Gemv
                              (uint32_t)p.K, abar);
             }
             int *as = reinterpret_cast<int *>(smem + L.asum_off);
-            for (int i2 = threadIdx.x; i2 < p.W * ng; i2 += kGemvThreads) as[i2] = p.asum[i2];
+            for (int b0 = 0; b0 < p.W * ng; b0 += 4 * kGemvThreads) {
+                int v[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int i2 = b0 + k * kGemvThreads + (int)threadIdx.x;
+                    v[k] = i2 < p.W * ng ? p.asum[i2] : 0;
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int i2 = b0 + k * kGemvThreads + (int)threadIdx.x;
+                    if (i2 < p.W * ng) as[i2] = v[k];
+                }
+            }
             a_ok = mbar_wait_bounded(abar, 0u);
         }
+        // (read after the barrier that ends a tile's sums)
+        if (SRC != kSrcRow && threadIdx.x < 16) invs_w[threadIdx.x] = (int)threadIdx.x < p.W ? 1.0f / s_row : 0.0f;
     }
-    __syncthreads();
+    if (!(ONECHUNK && SRC == kSrcPrepared)) __syncthreads();
 
-    AFrag<HALF> fA, fB;
-    if (ONECHUNK) {
+    if (ONECHUNK && SRC != kSrcPrepared) {
         load_afrag<HALF>(fA, arows, astride, asum, p.W, ng, 2 * warp, r, q);
         load_afrag<HALF>(fB, arows, astride, asum, p.W, ng, 2 * warp + 1, r, q);
     }
