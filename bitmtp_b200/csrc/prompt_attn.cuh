@@ -13,10 +13,10 @@
 // attn_sub_pass, in the same chain (scores ascending in d, numerators ascending in the key, sub-chunks
 // ascending, the weight sum as the butterfly over the 32 keys), so the partials are the same bits; tensor
 // cores would not give that order.  512 rows behind 2048 keys, 16 heads: 657 us by attn_fused_kernel alone; called from
-// the host 414 us with scalar fmas and 356 with packed ones and an exponential without branches and conversions; 338 in
-// a captured chain now.  The fmas alone are 134 us at the fp32 rate.  Bound by issue and latency, not by that pipe: it is
-// busy half of the time, 48 % of the issue slots are used, two warps per scheduler have an eligible one in 48 % of the
-// cycles, and nothing is loaded under the multiply.
+// the host 414 us with scalar fmas and 356 with packed ones and an exponential without branches and conversions; 339 in
+// a captured chain, 310 with every load of a tile out at once and the softmax on pairs too.  The fmas alone are 134 us at
+// the fp32 rate.  Of a tile's 66000 cycles the load took 8000, the scores 19000, the softmax 16000 and the numerators
+// 21000: what is left is latency with two warps per scheduler, and nothing is loaded under the multiply.
 #pragma once
 
 #include "verify_attn.cuh"
@@ -97,6 +97,79 @@ __device__ __forceinline__ float pa_expf(float x) {
     return x >= -87.0f ? e : (x != x ? x : 0.0f);
 }
 
+__device__ __forceinline__ PaPair pa_add2(PaPair a, PaPair b) { PaPair d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ PaPair pa_mul2(PaPair a, PaPair b) { PaPair d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ PaPair pa_fma2(PaPair a, PaPair b, PaPair c) { PaPair d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
+__device__ __forceinline__ PaPair pa_both(float v) { return pa_pack(v, v); }
+
+// pa_expf of two values: the same roundings, two per instruction.  A NaN comes out of the products by itself.
+__device__ __forceinline__ PaPair pa_expf2(PaPair x) {
+    const PaPair biased = pa_add2(pa_mul2(x, pa_both(1.44269504088896341f)), pa_both(12582912.0f));
+    const PaPair n = pa_add2(biased, pa_both(-12582912.0f));
+    PaPair r = pa_fma2(n, pa_both(-0.693145751953125f), x);
+    r = pa_fma2(n, pa_both(-1.42860682030941723e-6f), r);
+    PaPair q = pa_fma2(pa_both(1.3888889225e-3f), r, pa_both(8.3333337680e-3f));
+    q = pa_fma2(q, r, pa_both(4.1666667908e-2f));
+    q = pa_fma2(q, r, pa_both(1.6666667163e-1f));
+    q = pa_fma2(q, r, pa_both(0.5f));
+    q = pa_fma2(q, r, pa_both(1.0f));
+    q = pa_fma2(q, r, pa_both(1.0f));
+    float b0, b1, x0, x1, e0, e1;
+    pa_unpack(biased, b0, b1);
+    pa_unpack(x, x0, x1);
+    const PaPair pw = pa_pack(__uint_as_float((__float_as_uint(b0) - 0x4B400000u + 127u) << 23),
+                              __uint_as_float((__float_as_uint(b1) - 0x4B400000u + 127u) << 23));
+    pa_unpack(pa_mul2(q, pw), e0, e1);
+    return pa_pack(x0 < -87.0f ? 0.0f : e0, x1 < -87.0f ? 0.0f : e1);
+}
+
+// Scores of 4 vector pairs x 8 keys -> bf16-rounded weights in place; maximum and weight sum of every vector's sub-chunk
+// (the four threads of a sub-chunk hold 8 keys each).  FULL: every key is seen.
+template <bool FULL>
+__device__ __forceinline__ void pa_softmax(PaPair (&acc)[4][8], int lim, int kgp, int c, int v0, float *mc, float *lc) {
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+        float m0 = -INFINITY, m1 = -INFINITY;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            acc[t][j] = pa_mul2(acc[t][j], pa_both(0.08838834764831845f));
+            if (!FULL && 8 * kgp + j >= lim) acc[t][j] = pa_both(-INFINITY);
+            float x0, x1;
+            pa_unpack(acc[t][j], x0, x1);
+            m0 = fmaxf(m0, x0);
+            m1 = fmaxf(m1, x1);
+        }
+        m0 = fmaxf(m0, __shfl_xor_sync(0xffffffffu, m0, 1));
+        m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, 1));
+        m0 = fmaxf(m0, __shfl_xor_sync(0xffffffffu, m0, 2));
+        m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, 2));
+        const PaPair minus_m = pa_pack(-m0, -m1);
+        PaPair s[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            PaPair pr = pa_expf2(pa_add2(acc[t][j], minus_m));
+            if (!FULL && 8 * kgp + j >= lim) pr = 0ull;
+            float p0, p1;
+            pa_unpack(pr, p0, p1);
+            // one conversion for both; a NaN is the canonical one, as bm_bf16_rn gives it
+            uint32_t b;
+            asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(b) : "f"(p1), "f"(p0));
+            acc[t][j] = pa_pack(__uint_as_float(b << 16), __uint_as_float(b & 0xffff0000u));
+            // butterfly over the 32 keys of the sub-chunk: offsets 16 and 8 lie across the four threads
+            s[j] = pa_add2(pr, pa_pack(__shfl_xor_sync(0xffffffffu, p0, 2), __shfl_xor_sync(0xffffffffu, p1, 2)));
+            pa_unpack(s[j], p0, p1);
+            s[j] = pa_add2(s[j], pa_pack(__shfl_xor_sync(0xffffffffu, p0, 1), __shfl_xor_sync(0xffffffffu, p1, 1)));
+        }
+        const PaPair l = pa_add2(pa_add2(pa_add2(s[0], s[4]), pa_add2(s[2], s[6])), pa_add2(pa_add2(s[1], s[5]), pa_add2(s[3], s[7])));
+        if ((kgp & 3) == 0) {
+            float l0, l1;
+            pa_unpack(l, l0, l1);
+            *reinterpret_cast<float2 *>(mc + c * kPaQueries + v0 + 2 * t) = make_float2(m0, m1);
+            *reinterpret_cast<float2 *>(lc + c * kPaQueries + v0 + 2 * t) = make_float2(l0, l1);
+        }
+    }
+}
+
 // grid (super-chunks of the longest history, Hkv, ceil(T * G / 64)), 128 threads = 8 vector groups x 16 key
 // (then dim) groups.
 __global__ void __launch_bounds__(kPaThreads, 2) prompt_hist_kernel(const PromptHistParams p) {
@@ -122,27 +195,31 @@ __global__ void __launch_bounds__(kPaThreads, 2) prompt_hist_kernel(const Prompt
         if ((i >> 4) < keys_max) cp_async16(Vs + 8 * i, reinterpret_cast<const uint4 *>(vg) + i);
     }
     {
+        // Every load is out before the first store: the compiler may not move a load over a store to shared memory, and one
+        // round trip per piece cost 8000 cycles of a tile's 66000.
         const int k0 = 2 * (lane + 32 * (warp & 1));                  // keys k0, k0 + 1
+        const int v = lane + 32 * (warp & 1);                         // vector v of the tile: row v / G, head v % G
+        const int r = row0 + (v >> p.log_g), head = (hk << p.log_g) + (v & gmask);
+        uint4 ka[8], kb[8], qv[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             const int d0 = 8 * ((warp >> 1) + 2 * j);
-            uint4 a = make_uint4(0u, 0u, 0u, 0u), b = a;
-            if (k0 < keys_max) a = *reinterpret_cast<const uint4 *>(kg + (size_t)k0 * 128 + d0);
-            if (k0 + 1 < keys_max) b = *reinterpret_cast<const uint4 *>(kg + (size_t)(k0 + 1) * 128 + d0);
-            const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
+            ka[j] = kb[j] = qv[j] = make_uint4(0u, 0u, 0u, 0u);
+            if (k0 < keys_max) ka[j] = *reinterpret_cast<const uint4 *>(kg + (size_t)k0 * 128 + d0);
+            if (k0 + 1 < keys_max) kb[j] = *reinterpret_cast<const uint4 *>(kg + (size_t)(k0 + 1) * 128 + d0);
+            if (r < p.T) qv[j] = *reinterpret_cast<const uint4 *>(p.q + ((size_t)r * p.H + head) * 128 + d0);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int d0 = 8 * ((warp >> 1) + 2 * j);
+            const uint32_t aw[4] = {ka[j].x, ka[j].y, ka[j].z, ka[j].w}, bw[4] = {kb[j].x, kb[j].y, kb[j].z, kb[j].w};
 #pragma unroll
             for (int w = 0; w < 4; ++w) {
                 *reinterpret_cast<uint32_t *>(Kt + (d0 + 2 * w) * kPaKStride + k0) = __byte_perm(aw[w], bw[w], 0x5410);
                 *reinterpret_cast<uint32_t *>(Kt + (d0 + 2 * w + 1) * kPaKStride + k0) = __byte_perm(aw[w], bw[w], 0x7632);
             }
-        }
-        const int v = lane + 32 * (warp & 1);                         // vector v of the tile: row v / G, head v % G
-        const int r = row0 + (v >> p.log_g), head = (hk << p.log_g) + (v & gmask);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int d0 = 8 * ((warp >> 1) + 2 * j);
-            float f[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-            if (r < p.T) unpack8(*reinterpret_cast<const uint4 *>(p.q + ((size_t)r * p.H + head) * 128 + d0), f);
+            float f[8];
+            unpack8(qv[j], f);
 #pragma unroll
             for (int e = 0; e < 8; ++e) Qt[(d0 + e) * kPaQStride + v] = f[e];
         }
@@ -168,47 +245,20 @@ __global__ void __launch_bounds__(kPaThreads, 2) prompt_hist_kernel(const Prompt
         for (int d = 0; d < 128; ++d)
             pa_step(acc2, qp + d * kPaQStride, qp + d * kPaQStride + 4, *reinterpret_cast<const uint4 *>(kp + d * kPaKStride));
     }
-    float acc[8][8];                                                  // [vector][key], then [vector][dim]
-#pragma unroll
-    for (int t = 0; t < 4; ++t)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) pa_unpack(acc2[t][j], acc[2 * t][j], acc[2 * t + 1][j]);
     __syncthreads();                                                  // Q^T is spent: its space takes P^T
     const int c = kgp >> 2;                                           // sub-chunk of this thread's keys
-#pragma unroll
-    for (int t = 0; t < 8; ++t) {
-        float mj = -INFINITY;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            acc[t][j] = 8 * kgp + j < lim ? acc[t][j] * 0.08838834764831845f : -INFINITY;
-            mj = fmaxf(mj, acc[t][j]);
-        }
-        mj = fmaxf(mj, __shfl_xor_sync(0xffffffffu, mj, 1));
-        mj = fmaxf(mj, __shfl_xor_sync(0xffffffffu, mj, 2));
-        float s[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const float pr = 8 * kgp + j < lim ? pa_expf(acc[t][j] - mj) : 0.0f;
-            acc[t][j] = bm_bf16_rn(pr);
-            // butterfly over the 32 keys of the sub-chunk: offsets 16 and 8 lie across the four threads
-            s[j] = pr + __shfl_xor_sync(0xffffffffu, pr, 2);
-            s[j] = s[j] + __shfl_xor_sync(0xffffffffu, s[j], 1);
-        }
-        const float lj = ((s[0] + s[4]) + (s[2] + s[6])) + ((s[1] + s[5]) + (s[3] + s[7]));
-        if ((kgp & 3) == 0) {
-            mc[c * kPaQueries + v0 + t] = mj;
-            lc[c * kPaQueries + v0 + t] = lj;
-        }
-    }
+    if (lim >= BM_ATTN_SUPER) pa_softmax<true>(acc2, lim, kgp, c, v0, mc, lc);
+    else pa_softmax<false>(acc2, lim, kgp, c, v0, mc, lc);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
         const int w = pa_weight(8 * kgp + j, vgp);
-        *reinterpret_cast<float4 *>(Pt + w) = make_float4(acc[0][j], acc[1][j], acc[2][j], acc[3][j]);
-        *reinterpret_cast<float4 *>(Pt + (w ^ 4)) = make_float4(acc[4][j], acc[5][j], acc[6][j], acc[7][j]);
+        *reinterpret_cast<ulonglong2 *>(Pt + w) = make_ulonglong2(acc2[0][j], acc2[1][j]);
+        *reinterpret_cast<ulonglong2 *>(Pt + (w ^ 4)) = make_ulonglong2(acc2[2][j], acc2[3][j]);
     }
     __syncthreads();
     if (lim <= 0) return;
 
+    float acc[8][8];                                                  // [vector][dim]
     // numerators: this thread's 8 vectors x dims 8 kgp .. 8 kgp + 7, one chain per sub-chunk, then the merge
     float O[8][8], L[8], MJ[8];
 #pragma unroll

@@ -72,6 +72,17 @@ def test_rows_past_a_history_do_not_reach_it():
         assert bool(clean.isfinite().all()) and torch.equal(got.view(torch.int16), clean[:keep].view(torch.int16))
 
 
+@pytest.mark.parametrize("what", [float("nan"), float("inf"), float("-inf"), 3.0e38])
+def test_odd_values_in_a_history(what):
+    """Infinities, NaN and the largest values in K rows that the slabs see: the same bits as slab by slab."""
+    T, hist0 = 512, 176
+    q, k, v = _attention_inputs(T, hist0, 16, 8, 9)
+    k[0, 40:44], k[1, 0:160], k[2, 5, 7] = what, what, what
+    q[8, 6] = 0.0
+    want, got = _by_slab(q, k, v, hist0), _prompt(q, k, v, hist0)
+    assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+
+
 def _module(N, K, rows, seed):
     gen = torch.Generator(device=DEV).manual_seed(seed)
     packed, scale = synthetic.device_ternary(N, K, gen, torch.device(DEV))
