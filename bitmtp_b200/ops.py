@@ -284,10 +284,12 @@ def gemv_serves_rows(T: int, N: int, K: int) -> bool:
     The many-row kernel gives 128 weight rows to one CTA, which walks the K / 128 groups in series: with few CTAs its time is
     that walk, about 5 us + 2.5 us per 1024 of K, however small N is.  The GEMV spreads the weight rows over all SMs.  Device
     us for 17 / 32 rows, GEMV - many-row kernel: 512 x 4096 12.1 / 12.2 - 16.6, 512 x 9728 13.5 / 14.0 - 28.9, 2048 x 6144
-    14.5 / 16.5 - 20.7, 4096 x 4096 14.5 / 16.6 - 16.6, 4096 x 9728 23.9 / 26.2 - 29.7 / 30.6.  The other side: 512 x 1024
-    10.7 - 9.8, 4096 x 2048 12.5 - 10.4, 6144 x 4096 18.6 / 20.7 - 16.6, 6144 x 6144 24.8 / 28.9 - 20.7.  Odd group counts go
-    through the GEMV's slower consumer; from 33 rows on the GEMV would read the weights three times."""
-    return 16 < T <= 32 and 2048 < K <= GEMV_MAX_K and K % 256 == 0 and N <= 4096
+    14.5 / 16.5 - 20.7, 4096 x 4096 14.5 / 16.6 - 16.6, 4096 x 9728 23.9 / 26.2 - 29.7 / 30.6.  Between K = 1024 and 2048 the
+    two are level for narrow weights (512 x 1024 10.7 / 10.4 - 9.8 / 10.4, 512 x 2048 10.4 / 12.2 - 10.4) and the many-row
+    kernel is 2 us ahead at N = 4096 (12.5 - 10.4); the line stays where shapes were first sorted.  The other side:
+    512 x 512 12.5 - 8.4, 6144 x 4096 18.6 / 20.7 - 16.6, 6144 x 6144 24.8 / 28.9 - 20.7.  Odd group counts go through the
+    GEMV's slower consumer; from 33 rows on the GEMV would read the weights three times."""
+    return 16 < T <= 32 and 1024 <= K <= GEMV_MAX_K and K % 256 == 0 and N <= 4096
 
 
 def t2_linear_rows(x: torch.Tensor, b_packed: torch.Tensor, ws: torch.Tensor) -> torch.Tensor:
