@@ -59,7 +59,8 @@ int bm_sm_count(void);
 unsigned long long bm_launch_count(void);
 
 /* Reads and clears the per-device error word that kernels set when a bounded
- * wait runs out (0 = none, 1 = a GEMV weight tile never arrived). Synchronises
+ * wait runs out (0 = none, 1 = a GEMV weight tile never arrived,
+ * 4 = a peer of a split layer, 5 = a copy or product of the many-row kernel). Synchronises
  * the device. */
 int bm_device_error(void);
 
@@ -343,9 +344,9 @@ int bm_draft_chain_split(const void *logits, int D, int vocab, int ld, float tau
 int bm_pack_t2_g128(const void *w, int N, int K, void *packed, void *scale, void *frozen, void *stream);
 
 /* The packed product for MANY rows at once (a prompt): C bf16 [T, ldc] = the value bm_t2_gemv_prepared
- * gives every row alone, bit for bit, with each weight byte read once per 32 rows instead of once per
+ * gives every row alone, bit for bit, with each weight byte read once per 32 or 64 rows instead of once per
  * GEMV launch.  A_prep / a_sums / s: GEMV-ready INT8 rows, their group sums and multipliers for T rows;
- * N % 8 == 0, K % 128 == 0.  Tensor-core kernel (mma.sync int8, exact int32 group sums, the GEMV's
+ * N % 8 == 0, K % 128 == 0.  Tensor-core kernel (tcgen05 int8, exact int32 group sums, the GEMV's
  * fp32 order).  Replaces the dense bf16 fallback of T2LinearKernel.forward behind forward_sdlm_prefill
  * (src/bonsai_sft/gpu/model.py:650-656, 1306-1340). */
 int bm_t2_gemm_wide(const void *A_prep, const void *a_sums, const void *B, void *C, const void *s, const void *ws,
