@@ -1143,16 +1143,13 @@ int bm_pack_t2_g128(const void *w, int N, int K, void *packed, void *scale, void
     const int per_cta = bm::kPackThreads / 32 * 2 * bm::kPackGroupPairs;
     const long long blocks = (groups + per_cta - 1) / per_cta;
     if (blocks > 0x7fffffffLL) return BM_EINVAL;
-    count_launch();
     const uint16_t *src = static_cast<const uint16_t *>(w);
+    uint8_t *codes = static_cast<uint8_t *>(packed);
+    uint16_t *sc = static_cast<uint16_t *>(scale), *fr = static_cast<uint16_t *>(frozen);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (frozen)
-        bm::pack_t2_g128_kernel<true><<<(unsigned)blocks, bm::kPackThreads, 0, st>>>(
-            src, groups, static_cast<uint8_t *>(packed), static_cast<uint16_t *>(scale), static_cast<uint16_t *>(frozen));
-    else
-        bm::pack_t2_g128_kernel<false><<<(unsigned)blocks, bm::kPackThreads, 0, st>>>(
-            src, groups, static_cast<uint8_t *>(packed), static_cast<uint16_t *>(scale), nullptr);
-    return cuda_status(cudaGetLastError());
+    const dim3 grid((unsigned)blocks), block(bm::kPackThreads);
+    if (frozen) return launch_ex(bm::pack_t2_g128_kernel<true>, grid, block, 0, st, 1, src, groups, codes, sc, fr);
+    return launch_ex(bm::pack_t2_g128_kernel<false>, grid, block, 0, st, 1, src, groups, codes, sc, fr);
 }
 
 // ---------------------------------------------------------------------------- prompt (many-row) path

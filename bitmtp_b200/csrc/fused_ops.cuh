@@ -482,8 +482,9 @@ __global__ void kv_copy_rows_kernel(uint16_t *kv, int planes, int kv_rows, int s
 //     rounding cannot reach one half), i.e. when 2|w| > s;
 //   * the scale is a function of the group's absmax alone (the absmax element itself rounds to +-1), so the
 //     second reduction, over the frozen values, and the packer's second division (exact +-1 or 0) drop out.
-// 12288 x 2048, one call: 88.1 us with two IEEE divisions per weight and one 512-byte request per warp, 16.4 us now
-// (57 MB: 8.7 us at the measured copy rate; the rest is mostly the host's launch interval).
+// 12288 x 2048, one call after another: 88.1 us with two IEEE divisions per weight and one 512-byte request per warp, 16.4
+// without, 14.0 with programmatic dependency between calls (57 MB: 8.7 us at the measured copy rate; two or eight pairs a
+// warp 15.0 and 14.9).
 // NaN weights pack as 0 and are ignored by the absmax; a group with an infinity has scale 0 and all codes 0, as
 // `inf / inf` and `0 * inf` of the expressions above give.
 // =============================================================================
@@ -495,6 +496,9 @@ __global__ void __launch_bounds__(kPackThreads) pack_t2_g128_kernel(const uint16
                                                                     uint8_t *__restrict__ packed,
                                                                     uint16_t *__restrict__ scale,
                                                                     uint16_t *__restrict__ frozen) {
+    // the next call's CTAs may take their places while this one drains; nothing is read or written before the wait
+    pdl_launch_dependents();
+    pdl_wait();
     const int lane = threadIdx.x & 31, sub = lane & 15;
     const long long u0 = ((long long)blockIdx.x * (kPackThreads / 32) + (threadIdx.x >> 5)) * (2 * kPackGroupPairs) + (lane >> 4);
     uint4 raw[kPackGroupPairs];
