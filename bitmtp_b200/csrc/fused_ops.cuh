@@ -514,8 +514,9 @@ __global__ void kv_copy_rows_kernel(uint16_t *kv, int planes, int kv_rows, int s
 //   * the scale is a function of the group's absmax alone (the absmax element itself rounds to +-1), so the
 //     second reduction, over the frozen values, and the packer's second division (exact +-1 or 0) drop out.
 // 12288 x 2048, one call after another: 88.1 us with two IEEE divisions per weight and one 512-byte request per warp, 16.4
-// without, 14.0 with programmatic dependency between calls (57 MB: 8.7 us at the measured copy rate; two or eight pairs a
-// warp 15.0 and 14.9).
+// without, 13.6 where a launch overlaps the end of the one before (57 MB: 8.7 us at the measured copy rate; two or eight
+// pairs a warp about 1 us more).  Letting the next launch start with this one's first block was no faster (13.7), and products
+// behind it then requested codes that were not there yet.
 // NaN weights pack as 0 and are ignored by the absmax; a group with an infinity has scale 0 and all codes 0, as
 // `inf / inf` and `0 * inf` of the expressions above give.
 // =============================================================================
@@ -527,8 +528,8 @@ __global__ void __launch_bounds__(kPackThreads) pack_t2_g128_kernel(const uint16
                                                                     uint8_t *__restrict__ packed,
                                                                     uint16_t *__restrict__ scale,
                                                                     uint16_t *__restrict__ frozen) {
-    // the next call's CTAs may take their places while this one drains; nothing is read or written before the wait
-    pdl_launch_dependents();
+    // No launch_dependents: every product requests its weights before its own wait, and these are what is written here.  The
+    // launch itself overlaps the previous one; nothing is read or written before this wait.
     pdl_wait();
     const int lane = threadIdx.x & 31, sub = lane & 15;
     const long long u0 = ((long long)blockIdx.x * (kPackThreads / 32) + (threadIdx.x >> 5)) * (2 * kPackGroupPairs) + (lane >> 4);

@@ -32,7 +32,10 @@ extern "C" {
 
 /* consumer selection for bm_t2_gemv */
 /* `pdl` values (bit mask).  BM_PDL_OVERLAP: the launch may start before the previous kernel
- * of the stream has finished and waits for it on the device before reading its output.
+ * of the stream has finished and waits for it on the device before reading its output.  Weights and
+ * their scales are the exception: products request them before that wait.  So they must not be written
+ * by a launch that lets its successor start early, nor by one that such a launch itself overlaps;
+ * bm_pack_t2_g128 does not let its successor start before its last block has ended.
  * BM_PDL_STABLE_STATE (bm_verify_attention only, with BM_PDL_OVERLAP): the caller promises
  * that the step record and the history rows [0, cache_len) were written by launches that
  * completed before the current run of overlapped launches began (true for a captured
@@ -107,7 +110,8 @@ int64_t bm_t2_gemv_bytes(int W, int N, int K, int out_kind);
 /* ------------------------------------------------------------------ fused operators
  * `pdl` on every call below has the meaning given at bm_t2_gemv: the kernel is
  * launched with programmatic stream serialisation and waits for its
- * predecessor before its first read of a tensor the predecessor writes. */
+ * predecessor before its first read of a tensor the predecessor writes
+ * (weights and scales: see BM_PDL_OVERLAP). */
 
 /* Per-row absmax INT8 quantisation: x bf16 [M, K] -> q int8 [M, K], s fp32 [M]
  * with s = 127 / max(absmax, 1e-5), q = clamp(rint(x * s), -128, 127).
@@ -340,7 +344,8 @@ int bm_draft_chain_split(const void *logits, int D, int vocab, int ld, float tau
  * weights on the {-s, 0, +s} grid.  The arithmetic of freeze_quantize_to_ternary_g128
  * (src/bonsai_sft/ternary_modules.py:86-93) followed by _pack_t2_g128
  * (src/bonsai_sft/gpu/convert_bonsai_mtp_to_gpu.py:127-144), which the reference's converter runs on the
- * CPU; same bytes.  K % 128 == 0; w and frozen 16-byte aligned. */
+ * CPU; same bytes.  K % 128 == 0; w and frozen 16-byte aligned.  The launch overlaps the previous one's end
+ * and waits for it; a product may follow it with or without BM_PDL_OVERLAP. */
 int bm_pack_t2_g128(const void *w, int N, int K, void *packed, void *scale, void *frozen, void *stream);
 
 /* The packed product for MANY rows at once (a prompt): C bf16 [T, ldc] = the value bm_t2_gemv_prepared

@@ -86,6 +86,35 @@ def test_tail_groups_and_values_that_are_not_finite():
     assert bool((codes[2].view(torch.uint8) == 0xAA).all()) and float(scale[2]) == 0.0
 
 
+@pytest.mark.parametrize("W,N,K", [(1, 1024, 2048), (9, 2048, 2048), (8, 2048, 6144), (8, 19200, 512), (3, 264, 384), (16, 520, 768)])
+def test_an_overlapped_product_right_after_the_packer(W, N, K):
+    """Codes and scales that replace others, multiplied at once by a launch that may overlap its predecessor, directly and
+    behind an overlapped quantisation: the direct, cooperative, row-per-warp and lanes-across-K kernels."""
+    gen = torch.Generator(device=DEV).manual_seed(W + N + K)
+    ws = [(0.02 * torch.randn(N, K, generator=gen, device=DEV)).to(torch.bfloat16) for _ in range(2)]
+    x = torch.randn(W, K, generator=gen, device=DEV).to(torch.bfloat16)
+    q, s = ops.quant_rows(x)
+    refs = []
+    for w in ws:
+        codes, scale = ops.pack_t2_g128(w)
+        torch.cuda.synchronize()
+        refs.append(ops.t2_gemv(q, codes, s, scale))
+    codes, scale = torch.empty_like(codes), torch.empty_like(scale)
+    stream = torch.cuda.current_stream().cuda_stream
+    got = []
+    for i in range(24):
+        native.check(native.lib().bm_pack_t2_g128(ws[i & 1].data_ptr(), N, K, codes.data_ptr(), scale.data_ptr(), None, stream), "pack")
+        if i % 3 == 2:
+            q2, s2 = ops.quant_rows(x, pdl=True)
+            got.append(ops.t2_gemv(q2, codes, s2, scale, pdl=True))
+        else:
+            got.append(ops.t2_gemv(q, codes, s, scale, pdl=True))
+    torch.cuda.synchronize()
+    for i, y in enumerate(got):
+        assert torch.equal(y.view(torch.int16), refs[i & 1].view(torch.int16)), i
+    assert native.lib().bm_device_error() == 0
+
+
 def test_rejects_what_the_packer_cannot_take():
     w = torch.zeros(4, 128, dtype=torch.bfloat16, device=DEV)
     with pytest.raises(RuntimeError):
