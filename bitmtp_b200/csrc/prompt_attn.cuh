@@ -51,6 +51,12 @@ __host__ __device__ inline bool prompt_hist_fits(int slab_rows, int H, int Hkv) 
 // History length of the slab that holds prompt row r.
 __device__ __forceinline__ int pa_history(int hist0, int r) { return hist0 + r / kPaSlab * kPaSlab; }
 
+// Keys of the super-chunk at key0 that the 16 vectors of a warp see; 0 where the warp has no row of the prompt.
+__device__ __forceinline__ int pa_tile_keys(int hist0, int T, int row0, int log_g, int warp, int key0) {
+    const int r = row0 + ((16 * warp) >> log_g);
+    return r < T ? min(BM_ATTN_SUPER, pa_history(hist0, r) - key0) : 0;
+}
+
 // Word of weight (key, vector 8 vg) in P^T, whose 16-byte pieces are swizzled by the key's group of eight: the
 // threads of a warp, eight keys apart, then store to different banks.  Vectors 8 vg + 4 .. + 7 are at ^ 4 words.
 __device__ __forceinline__ int pa_weight(int key, int vg) { return key * kPaQueries + 4 * ((2 * vg) ^ (key >> 3)); }
@@ -229,9 +235,9 @@ __global__ void __launch_bounds__(kPaThreads, 2) prompt_hist_kernel(const Prompt
 
     const int vgp = tid >> 4, kgp = tid & 15;                         // vector group, key / dim group
     const int v0 = 8 * vgp;
-    // keys of this super-chunk that this thread's vectors see (one slab, the same for the whole warp)
-    const int my_row = row0 + (v0 >> p.log_g);
-    const int lim = my_row < p.T ? min(BM_ATTN_SUPER, pa_history(p.hist0, my_row) - key0) : 0;
+    // Keys of this super-chunk that the warp's 16 vectors see: one slab, so one number, and the same in every lane also where
+    // the prompt ends between the warp's two vector groups (the shuffles of the softmax take whole warps).
+    const int lim = pa_tile_keys(p.hist0, p.T, row0, p.log_g, warp, key0);
 
     PaPair acc2[4][8];                                                // [vector pair][key]
 #pragma unroll

@@ -61,6 +61,13 @@ def test_prompt_attention_equals_the_slabs(T, hist0, H, Hkv):
     assert torch.equal(_prompt(q, k, v, hist0, calls=2).view(torch.int16), want.view(torch.int16))
 
 
+@pytest.mark.parametrize("T,H,Hkv", [(357, 8, 8), (340, 16, 8), (341, 32, 8), (511, 8, 1)])
+def test_prompts_that_end_inside_a_warp(T, H, Hkv):
+    """The last warp with rows holds one vector group of the prompt and one past its end, behind whole super-chunks."""
+    q, k, v = _attention_inputs(T, 2560, H, Hkv, T)
+    assert torch.equal(_prompt(q, k, v, 2560).view(torch.int16), _by_slab(q, k, v, 2560).view(torch.int16))
+
+
 def test_rows_past_a_history_do_not_reach_it():
     """Infinities and NaN in K / V rows that a slab may not see stay out of its results."""
     for T, hist0, keep in ((64, 160, 32), (512, 160, 400)):       # the general kernel, the tiles

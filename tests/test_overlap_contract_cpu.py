@@ -1,4 +1,5 @@
-"""Launch order that no run can show reliably: what the kernel sources say about overlapped launches."""
+"""What no run can show reliably, from the kernel sources: the order of overlapped launches, and which lanes of a warp meet
+in a shuffle."""
 import os
 import re
 
@@ -20,3 +21,18 @@ def test_the_packer_never_lets_a_product_start_early():
     assert "launch_dependents" not in body
     statements = [s.strip() for s in body.lstrip("{").split(";")]
     assert statements[0] == "pdl_wait()"
+
+
+def test_the_prompt_softmax_takes_whole_warps():
+    """The tile kernel's two softmax builds shuffle over whole warps, so the number that chooses between them may depend on
+    the warp but on nothing finer.  And one number is enough: the rows of a warp's 16 vectors lie in one slab."""
+    source = open(os.path.join(native.CSRC, "prompt_attn.cuh")).read()
+    body = _body(source, "prompt_hist_kernel")
+    assert "if (lim >= BM_ATTN_SUPER) pa_softmax<true>" in body
+    assert re.findall(r"\blim\s*=[^=][^;]*;", body) == ["lim = pa_tile_keys(p.hist0, p.T, row0, p.log_g, warp, key0);"]
+    slab, vectors = (int(re.search(rf"{n} = (\d+)", source).group(1)) for n in ("kPaSlab", "kPaQueries"))
+    for log_g in range(4):
+        for warp in range(vectors // 16):
+            for row0 in range(0, 40 * slab, vectors >> log_g):
+                rows = [row0 + (v >> log_g) for v in range(16 * warp, 16 * warp + 16)]
+                assert rows[0] == row0 + ((16 * warp) >> log_g) and len({r // slab for r in rows}) == 1
