@@ -20,7 +20,6 @@
 
 namespace {
 
-typedef void (*LinearFn)(const void *, const void *, void *, const void *, const void *, int, int, int, void *);
 typedef int (*QuantFn)(const void *, int, int, void *, void *, void *, void *, int, void *);
 typedef int (*GemvFn)(const void *, const void *, void *, const void *, const void *, int, int, int, int, int, int, void *,
                       int, void *);
@@ -30,7 +29,6 @@ typedef int (*GemmFn)(const void *, const void *, const void *, void *, const vo
                       void *);
 
 // Entry points of the library, set once by bind() before the first call.
-LinearFn g_linear = nullptr;
 QuantFn g_quant = nullptr;
 GemvFn g_gemv = nullptr;
 GemvPreparedFn g_gemv_prepared = nullptr;
@@ -56,19 +54,18 @@ bool modes_active() {
 }
 
 PyObject *bind(PyObject *, PyObject *args) {
-    unsigned long long f[5];
-    if (!PyArg_ParseTuple(args, "KKKKK", &f[0], &f[1], &f[2], &f[3], &f[4])) return nullptr;
-    g_linear = reinterpret_cast<LinearFn>(f[0]);
-    g_quant = reinterpret_cast<QuantFn>(f[1]);
-    g_gemv = reinterpret_cast<GemvFn>(f[2]);
-    g_gemv_prepared = reinterpret_cast<GemvPreparedFn>(f[3]);
-    g_gemm = reinterpret_cast<GemmFn>(f[4]);
+    unsigned long long f[4];
+    if (!PyArg_ParseTuple(args, "KKKK", &f[0], &f[1], &f[2], &f[3])) return nullptr;
+    g_quant = reinterpret_cast<QuantFn>(f[0]);
+    g_gemv = reinterpret_cast<GemvFn>(f[1]);
+    g_gemv_prepared = reinterpret_cast<GemvPreparedFn>(f[2]);
+    g_gemm = reinterpret_cast<GemmFn>(f[3]);
     Py_RETURN_NONE;
 }
 
 // linear(a, b, s, ws): t2g128_int8xint2_linear without the registry check.
 PyObject *linear(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
-    if (nargs != 4 || g_linear == nullptr || modes_active()) Py_RETURN_NONE;
+    if (nargs != 4 || g_gemv == nullptr || modes_active()) Py_RETURN_NONE;
     const at::Tensor *a = plain_cuda(args[0]), *b = plain_cuda(args[1]), *s = plain_cuda(args[2]), *ws = plain_cuda(args[3]);
     if (!a || !b || !s || !ws || (a->dim() != 2 && a->dim() != 3) || b->dim() != 2 || ws->dim() != 2 || s->dim() < 1)
         Py_RETURN_NONE;
@@ -87,9 +84,11 @@ PyObject *linear(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
         void *stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
         const void *ap = a->const_data_ptr(), *bp = b->const_data_ptr(), *sp = s->const_data_ptr(), *wp = ws->const_data_ptr();
         void *op = out.mutable_data_ptr();
+        int rc;
         Py_BEGIN_ALLOW_THREADS
-        g_linear(ap, bp, op, sp, wp, (int)m, (int)n, (int)k, stream);
+        rc = g_gemv(ap, bp, op, sp, wp, (int)m, (int)n, (int)k, (int)n, 0, 0, nullptr, 0, stream);
         Py_END_ALLOW_THREADS
+        if (rc != 0) Py_RETURN_NONE;                       // the Python path reports it
         return THPVariable_Wrap(std::move(out));
     } catch (const std::exception &e) {
         PyErr_SetString(PyExc_RuntimeError, e.what());

@@ -69,8 +69,10 @@ def t2g128_int8xint2_linear(a_int8: torch.Tensor, b_packed: torch.Tensor, s: tor
 
     Same call as the reference wrapper (src/bonsai_sft/gpu/model.py:222-256):
     a_int8 `[M, K]` or `[B, S, K]` int8, b_packed `[N, K/4]` int8, s `[..., 1]`
-    fp32 (127/absmax, the output is divided by it), ws `[N, K/128]` bf16.  It goes
-    through the library's drop-in symbol of the same name.  `validate_registry`
+    fp32 (127/absmax, the output is divided by it), ws `[N, K/128]` bf16.  It is
+    bm_t2_gemv, the form of the library's drop-in symbol of the same name that
+    returns a status: a call that the library refuses (operands off a 16-byte
+    boundary, a K whose rows do not fit shared memory) raises.  `validate_registry`
     restricts (M, N, K) to the reference's registered triples.
     """
     if native._host is not None and not validate_registry:
@@ -83,8 +85,10 @@ def t2g128_int8xint2_linear(a_int8: torch.Tensor, b_packed: torch.Tensor, s: tor
         load_t2_kernel()
     dev = a_int8.device
     out = torch.empty((*a_int8.shape[:-1], n), dtype=torch.bfloat16, device=dev)
-    _t2_lib.t2g128_int8xint2_linear(a_int8.data_ptr(), b_packed.data_ptr(), out.data_ptr(), s.data_ptr(), ws.data_ptr(),
-                                    m, n, k, ops._stream(dev))
+    rc = _t2_lib.bm_t2_gemv(a_int8.data_ptr(), b_packed.data_ptr(), out.data_ptr(), s.data_ptr(), ws.data_ptr(), m, n, k, n,
+                            native.OUT_BF16, native.PATH_AUTO, None, 0, ops._stream(dev))
+    if rc != native.BM_OK:
+        native.check(rc, f"t2g128_int8xint2_linear(M={m}, N={n}, K={k})")
     return out
 
 

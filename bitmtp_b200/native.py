@@ -97,7 +97,7 @@ def _load_host(L):
     mod = importlib.util.module_from_spec(spec)
     spec.loader.exec_module(mod)
     mod.bind(*(ctypes.cast(getattr(L, n), ctypes.c_void_p).value
-               for n in ("t2g128_int8xint2_linear", "bm_quant_rows", "bm_t2_gemv", "bm_t2_gemv_prepared", "bm_t2_gemm_wide")))
+               for n in ("bm_quant_rows", "bm_t2_gemv", "bm_t2_gemv_prepared", "bm_t2_gemm_wide")))
     return mod
 
 

@@ -91,3 +91,28 @@ def test_what_is_left_to_the_python_path():
     assert native._host.linear_rows(x.float(), packed, scale, ops.gemv_serves_rows, ops.GEMM_WIDE_MAX_ROWS) is None
     shifted = torch.cat([scale.view(-1)[:4], scale.view(-1)])[4:].view_as(scale)
     assert native._host.linear_rows(x, packed, shifted, ops.gemv_serves_rows, ops.GEMM_WIDE_MAX_ROWS) is None
+
+
+def _shifted(t, elements):
+    """The same values, contiguous, off a 16-byte boundary."""
+    return torch.cat([t.reshape(-1)[:elements], t.reshape(-1)])[elements:].view_as(t)
+
+
+@pytest.mark.parametrize("host", [True, False])
+def test_a_call_that_the_library_refuses_raises(monkeypatch, host):
+    """Operands off a 16-byte boundary, and rows too long for the shared memory of the lanes-across-K kernel: an error and no
+    tensor of whatever memory held, by the native host path and by the Python path behind it."""
+    x, packed, scale = _operands(4)
+    q, s = ops.quant_rows(x)
+    long_x, long_packed, long_scale = _operands(16, 8, 16512)
+    long_q, long_s = ops.quant_rows(long_x)
+    if not host:
+        monkeypatch.setattr(native, "_host", None)
+    for args in ((_shifted(q, 8), packed, s, scale), (q, _shifted(packed, 8), s, scale), (q, packed, s, _shifted(scale, 4)),
+                 (long_q, long_packed, long_s, long_scale)):
+        assert all(t.is_contiguous() for t in args)
+        with pytest.raises(native.NativeError):
+            BM.t2g128_int8xint2_linear(*args)
+    torch.cuda.synchronize()
+    got = BM.t2g128_int8xint2_linear(q, packed, _shifted(s, 1), scale)       # multipliers need no more than their own size
+    assert torch.equal(got, BM.t2g128_int8xint2_linear(q, packed, s, scale))
