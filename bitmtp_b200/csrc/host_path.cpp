@@ -34,11 +34,12 @@ GemvFn g_gemv = nullptr;
 GemvPreparedFn g_gemv_prepared = nullptr;
 GemmFn g_gemm = nullptr;
 
-// The tensor behind `o` when its data pointer may be handed to a kernel, else null.
+// The tensor behind `o` when its data pointer may be handed to a kernel, else null.  (Strided nested tensors are exact
+// torch.Tensor objects too, without one size per dimension.)
 const at::Tensor *plain_cuda(PyObject *o) {
     if (!THPVariable_CheckExact(o) && Py_TYPE(o) != reinterpret_cast<PyTypeObject *>(ParameterClass)) return nullptr;
     const at::Tensor &t = THPVariable_Unpack(o);
-    if (!t.defined() || !t.is_cuda() || t.layout() != at::kStrided || !t.has_storage()) return nullptr;
+    if (!t.defined() || !t.is_cuda() || t.layout() != at::kStrided || t.is_nested() || !t.has_storage()) return nullptr;
     constexpr c10::DispatchKeySet kWrapped({c10::DispatchKey::Python, c10::DispatchKey::Functionalize,
                                             c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper,
                                             c10::DispatchKey::Conjugate, c10::DispatchKey::Negative,
@@ -66,19 +67,19 @@ PyObject *bind(PyObject *, PyObject *args) {
 // linear(a, b, s, ws): t2g128_int8xint2_linear without the registry check.
 PyObject *linear(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     if (nargs != 4 || g_gemv == nullptr || modes_active()) Py_RETURN_NONE;
-    const at::Tensor *a = plain_cuda(args[0]), *b = plain_cuda(args[1]), *s = plain_cuda(args[2]), *ws = plain_cuda(args[3]);
-    if (!a || !b || !s || !ws || (a->dim() != 2 && a->dim() != 3) || b->dim() != 2 || ws->dim() != 2 || s->dim() < 1)
-        Py_RETURN_NONE;
-    const int64_t k = a->size(-1), n = b->size(0);
-    if (k < 128 || k % 128 || b->size(1) * 4 != k || n < 8 || n % 8 || k > INT32_MAX || n > INT32_MAX) Py_RETURN_NONE;
-    const int64_t m = a->numel() / k;
-    if (m < 1 || m > 32 || ws->size(0) != n || ws->size(1) != k / 128 || s->size(-1) != 1 || s->numel() != m) Py_RETURN_NONE;
-    if (a->scalar_type() != at::kChar || b->scalar_type() != at::kChar || ws->scalar_type() != at::kBFloat16 ||
-        s->scalar_type() != at::kFloat)
-        Py_RETURN_NONE;
-    const c10::Device dev = a->device();
-    if (b->device() != dev || s->device() != dev || ws->device() != dev) Py_RETURN_NONE;
-    try {
+    try {                                                  // sizes too: they throw for tensors without plain ones
+        const at::Tensor *a = plain_cuda(args[0]), *b = plain_cuda(args[1]), *s = plain_cuda(args[2]), *ws = plain_cuda(args[3]);
+        if (!a || !b || !s || !ws || (a->dim() != 2 && a->dim() != 3) || b->dim() != 2 || ws->dim() != 2 || s->dim() < 1)
+            Py_RETURN_NONE;
+        const int64_t k = a->size(-1), n = b->size(0);
+        if (k < 128 || k % 128 || b->size(1) * 4 != k || n < 8 || n % 8 || k > INT32_MAX || n > INT32_MAX) Py_RETURN_NONE;
+        const int64_t m = a->numel() / k;
+        if (m < 1 || m > 32 || ws->size(0) != n || ws->size(1) != k / 128 || s->size(-1) != 1 || s->numel() != m) Py_RETURN_NONE;
+        if (a->scalar_type() != at::kChar || b->scalar_type() != at::kChar || ws->scalar_type() != at::kBFloat16 ||
+            s->scalar_type() != at::kFloat)
+            Py_RETURN_NONE;
+        const c10::Device dev = a->device();
+        if (b->device() != dev || s->device() != dev || ws->device() != dev) Py_RETURN_NONE;
         at::Tensor out = a->dim() == 2 ? at::empty({m, n}, a->options().dtype(at::kBFloat16))
                                        : at::empty({a->size(0), a->size(1), n}, a->options().dtype(at::kBFloat16));
         void *stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
@@ -103,25 +104,25 @@ inline int64_t up16(int64_t v) { return (v + 15) & ~int64_t(15); }
 // for the rows' codes).
 PyObject *linear_rows(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     if (nargs != 5 || g_quant == nullptr || modes_active()) Py_RETURN_NONE;
-    const at::Tensor *x = plain_cuda(args[0]), *w = plain_cuda(args[1]), *ws = plain_cuda(args[2]);
-    if (!x || !w || !ws || x->dim() < 1 || w->dim() != 2 || ws->dim() != 2) Py_RETURN_NONE;
-    const int64_t k = x->size(-1), n = w->size(0), wide_max = PyLong_AsLongLong(args[4]);
-    if (k < 128 || k % 128 || w->size(1) * 4 != k || n < 8 || n % 8 || k > INT32_MAX || n > INT32_MAX) Py_RETURN_NONE;
-    const int64_t t = x->numel() / k;
-    if (t < 1 || t > wide_max || ws->size(0) != n || ws->size(1) != k / 128) Py_RETURN_NONE;
-    if (x->scalar_type() != at::kBFloat16 || w->scalar_type() != at::kChar || ws->scalar_type() != at::kBFloat16)
-        Py_RETURN_NONE;
-    const c10::Device dev = x->device();
-    const void *xp = x->const_data_ptr(), *bp = w->const_data_ptr(), *wp = ws->const_data_ptr();
-    if (w->device() != dev || ws->device() != dev || (reinterpret_cast<uintptr_t>(wp) & 15)) Py_RETURN_NONE;
-    bool gemv = t <= 16;
-    if (t > 16 && t <= 32) {
-        PyObject *r = PyObject_CallFunction(args[3], "LLL", (long long)t, (long long)n, (long long)k);
-        if (r == nullptr) return nullptr;
-        gemv = PyObject_IsTrue(r);
-        Py_DECREF(r);
-    }
     try {
+        const at::Tensor *x = plain_cuda(args[0]), *w = plain_cuda(args[1]), *ws = plain_cuda(args[2]);
+        if (!x || !w || !ws || x->dim() < 1 || w->dim() != 2 || ws->dim() != 2) Py_RETURN_NONE;
+        const int64_t k = x->size(-1), n = w->size(0), wide_max = PyLong_AsLongLong(args[4]);
+        if (k < 128 || k % 128 || w->size(1) * 4 != k || n < 8 || n % 8 || k > INT32_MAX || n > INT32_MAX) Py_RETURN_NONE;
+        const int64_t t = x->numel() / k;
+        if (t < 1 || t > wide_max || ws->size(0) != n || ws->size(1) != k / 128) Py_RETURN_NONE;
+        if (x->scalar_type() != at::kBFloat16 || w->scalar_type() != at::kChar || ws->scalar_type() != at::kBFloat16)
+            Py_RETURN_NONE;
+        const c10::Device dev = x->device();
+        const void *xp = x->const_data_ptr(), *bp = w->const_data_ptr(), *wp = ws->const_data_ptr();
+        if (w->device() != dev || ws->device() != dev || (reinterpret_cast<uintptr_t>(wp) & 15)) Py_RETURN_NONE;
+        bool gemv = t <= 16;
+        if (t > 16 && t <= 32) {
+            PyObject *r = PyObject_CallFunction(args[3], "LLL", (long long)t, (long long)n, (long long)k);
+            if (r == nullptr) return nullptr;
+            gemv = PyObject_IsTrue(r);
+            Py_DECREF(r);
+        }
         c10::DimVector shape(x->sizes());
         shape.back() = n;
         // codes, group sums and multipliers of the rows in one allocation

@@ -116,3 +116,21 @@ def test_a_call_that_the_library_refuses_raises(monkeypatch, host):
     torch.cuda.synchronize()
     got = BM.t2g128_int8xint2_linear(q, packed, _shifted(s, 1), scale)       # multipliers need no more than their own size
     assert torch.equal(got, BM.t2g128_int8xint2_linear(q, packed, s, scale))
+
+
+def test_nested_tensors_are_left_to_the_python_path():
+    """Strided nested tensors are exact torch.Tensor objects on a CUDA device, but asking them for a ragged size throws."""
+    x, packed, scale = _operands(4)
+    q, s = ops.quant_rows(x)
+    for widths in ((768, 768), (768, 640)):
+        nq, ns, nx = (torch.nested.nested_tensor([t[:2, :w], t[2:, :w]], layout=torch.strided)
+                      for t, w in ((q, widths[1]), (s, 1), (x, widths[1])))
+        ragged = torch.nested.nested_tensor([q[:3, :widths[0]], q[3:, :widths[1]]], layout=torch.strided)
+        assert type(ragged) is torch.Tensor and ragged.is_cuda and ragged.layout == torch.strided
+        for args in ((nq, packed, s, scale), (ragged, packed, s, scale), (q, ragged, s, scale), (q, packed, ns, scale),
+                     (q, packed, s, ragged)):
+            assert native._host.linear(*args) is None
+        for args in ((nx, packed, scale), (ragged, packed, scale), (x, ragged, scale), (x, packed, ragged)):
+            assert native._host.linear_rows(*args, ops.gemv_serves_rows, ops.GEMM_WIDE_MAX_ROWS) is None
+        with pytest.raises(RuntimeError):
+            BM.t2g128_int8xint2_linear(ragged, packed, s, scale)
