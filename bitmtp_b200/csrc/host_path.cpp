@@ -14,9 +14,11 @@
 #include <ATen/ATen.h>
 #include <ATen/PythonTorchFunctionTLS.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cstdint>
+#include <exception>
 
 namespace {
 
@@ -46,6 +48,13 @@ const at::Tensor *plain_cuda(PyObject *o) {
                                             c10::DispatchKey::ZeroTensor});
     if (t.key_set().has_any(kWrapped) || !t.is_contiguous()) return nullptr;
     return &t;
+}
+
+// The exception in flight as the Python error that torch's own calls raise for it (torch.OutOfMemoryError for an allocation
+// that fails, an error that Python has already set as it is).
+PyObject *raise_as_torch_does() {
+    torch::translate_exception_to_python(std::current_exception());
+    return nullptr;
 }
 
 bool modes_active() {
@@ -91,9 +100,8 @@ PyObject *linear(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
         Py_END_ALLOW_THREADS
         if (rc != 0) Py_RETURN_NONE;                       // the Python path reports it
         return THPVariable_Wrap(std::move(out));
-    } catch (const std::exception &e) {
-        PyErr_SetString(PyExc_RuntimeError, e.what());
-        return nullptr;
+    } catch (...) {
+        return raise_as_torch_does();
     }
 }
 
@@ -147,9 +155,8 @@ PyObject *linear_rows(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
         Py_END_ALLOW_THREADS
         if (rc != 0) Py_RETURN_NONE;                       // the Python path reports it
         return THPVariable_Wrap(std::move(out));
-    } catch (const std::exception &e) {
-        PyErr_SetString(PyExc_RuntimeError, e.what());
-        return nullptr;
+    } catch (...) {
+        return raise_as_torch_does();
     }
 }
 

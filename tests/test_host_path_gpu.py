@@ -134,3 +134,18 @@ def test_nested_tensors_are_left_to_the_python_path():
             assert native._host.linear_rows(*args, ops.gemv_serves_rows, ops.GEMM_WIDE_MAX_ROWS) is None
         with pytest.raises(RuntimeError):
             BM.t2g128_int8xint2_linear(ragged, packed, s, scale)
+
+
+@pytest.mark.parametrize("host", [True, False])
+def test_running_out_of_memory_is_torchs_own_error(monkeypatch, host):
+    """A product whose output (256 GiB) fits no device: torch.OutOfMemoryError, which callers catch to retry with less."""
+    n, rows = 1 << 22, 1 << 15
+    layer = T2LinearKernel(128, 8).to(DEV)
+    layer.weight.data = torch.zeros(n, 32, dtype=torch.int8, device=DEV)
+    layer.weight_scale = torch.zeros(n, 1, dtype=torch.bfloat16, device=DEV)
+    layer.out_features = n
+    native.lib()
+    if not host:
+        monkeypatch.setattr(native, "_host", None)
+    with pytest.raises(torch.OutOfMemoryError):
+        layer(torch.zeros(rows, 128, dtype=torch.bfloat16, device=DEV))
