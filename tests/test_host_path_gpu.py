@@ -149,3 +149,19 @@ def test_running_out_of_memory_is_torchs_own_error(monkeypatch, host):
         monkeypatch.setattr(native, "_host", None)
     with pytest.raises(torch.OutOfMemoryError):
         layer(torch.zeros(rows, 128, dtype=torch.bfloat16, device=DEV))
+
+
+def test_the_drop_in_symbol():
+    """The C symbol that programs written for the reference bind: the operator's bits, and nothing written on refusal."""
+    x, packed, scale = _operands(9)
+    q, s = ops.quant_rows(x)
+    out = torch.full((9, 264), 7.0, dtype=torch.bfloat16, device=DEV)
+    call = native.lib().t2g128_int8xint2_linear
+    stream = torch.cuda.current_stream().cuda_stream
+    call(q.data_ptr() + 8, packed.data_ptr(), out.data_ptr(), s.data_ptr(), scale.data_ptr(), 9, 264, 768, stream)
+    torch.cuda.synchronize()
+    assert bool((out == 7.0).all())
+    call(q.data_ptr(), packed.data_ptr(), out.data_ptr(), s.data_ptr(), scale.data_ptr(), 9, 264, 768, stream)
+    want = BM.t2g128_int8xint2_linear(q, packed, s, scale)
+    torch.cuda.synchronize()
+    assert torch.equal(out.view(torch.int16), want.view(torch.int16))

@@ -195,6 +195,24 @@ def test_many_row_product_at_tile_edges(N, K, T):
     assert torch.equal(out[:T].view(torch.int16), want.view(torch.int16)) and bool((out[T] == 7.0).all())
 
 
+@pytest.mark.parametrize("N,K,T", [(40008, 384, 17), (40008, 2176, 17), (19000, 1152, 130), (19000, 2176, 130)])
+def test_many_row_product_over_several_tiles_with_an_odd_step(N, K, T):
+    """CTAs that walk several tiles whose last step holds one group of its two, so that the rings and the prefetch go on from
+    it: tiles of 32 and of 64 prompt rows, one and several groups per slot."""
+    gen = torch.Generator(device=DEV).manual_seed(N + K + T)
+    packed, scale = synthetic.device_ternary(N, K, gen, torch.device(DEV))
+    x = torch.randn(T, K, generator=gen, device=DEV).to(torch.bfloat16)
+    qp, sums, s = ops.quant_rows(x, prepared=True)
+    q, _ = ops.quant_rows(x)
+    want = torch.cat([ops.t2_gemv(q[r:r + SLAB], packed, s[r:r + SLAB], scale) for r in range(0, T, SLAB)])
+    out = torch.full((T + 1, N), 7.0, dtype=torch.bfloat16, device=DEV)
+    for _ in range(2):
+        ops.t2_gemm_wide(qp, sums, packed, s, scale, out=out[:T])
+    torch.cuda.synchronize()
+    assert native.lib().bm_device_error() == 0
+    assert torch.equal(out[:T].view(torch.int16), want.view(torch.int16)) and bool((out[T] == 7.0).all())
+
+
 def _packed_model(geo, max_positions):
     cfg = synthetic.make_config(geo, block_size=8)
     state = synthetic.make_state(cfg, seed=4)

@@ -45,7 +45,7 @@ def test_gemv_agrees_with_reference_cuda_kernel(ref_lib, W, N, K):
     ref_lib.t2g128_int8xint2_linear(A.data_ptr(), B.data_ptr(), ref.data_ptr(), s.data_ptr(), ws.data_ptr(), W, N, K,
                                     torch.cuda.current_stream().cuda_stream)
     ours = ops.t2_gemv(A, B, s, ws, out_kind=native.OUT_BF16)
-    # the drop-in symbol of the same name, through the reference-facing wrapper
+    # the reference-facing wrapper of the same name
     shim = BM.t2g128_int8xint2_linear(A, B, s.view(W, 1), ws)
     torch.cuda.synchronize()
     assert native.lib().bm_device_error() == 0
