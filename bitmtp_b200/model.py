@@ -673,7 +673,7 @@ class Transformer(nn.Module):
         layer's planes (`kv_planes[i]` = (k, v) [1, n_kv, kv_rows, hd]); rows [0, hist0) are history.
         Same arithmetic, row for row, as the slab-by-slab prefill (forward_sdlm_prefill), so K / V rows and
         the residual stream equal it bit for bit: every projection is bm_t2_gemm_wide (tensor cores, each
-        weight byte read once per 32 rows), the attention one call of one or two launches per PREFILL_ATTN_ROWS
+        weight byte read once per 32 or 64 rows), the attention one call of one or two launches per PREFILL_ATTN_ROWS
         rows over AR-causal slabs of PREFILL_CHUNK.  Leaves the residual stream in ws.h / ws.ffn_out (reference: model.py:1306-1340)."""
         a = self.args
         T = int(token_values.shape[0])

@@ -274,7 +274,7 @@ def t2_gemm_wide(a_prep: torch.Tensor, a_sums: torch.Tensor, b_packed: torch.Ten
     return out
 
 
-GEMM_WIDE_MAX_ROWS = 32 * 65535    # grid.y
+GEMM_WIDE_MAX_ROWS = 32 * 65535    # what one call of bm_t2_gemm_wide takes
 GEMV_MAX_K = 11264                 # 16 INT8 rows and one tile of weights fill the shared memory of an SM there
 
 
@@ -282,13 +282,15 @@ def gemv_serves_rows(T: int, N: int, K: int) -> bool:
     """Whether 17 to 32 rows are two launches of the decode GEMV instead of one of the many-row kernel.
 
     The many-row kernel gives 128 weight rows to one CTA, which walks the K / 128 groups in series: with few CTAs its time is
-    that walk, about 5 us + 2.5 us per 1024 of K, however small N is.  The GEMV spreads the weight rows over all SMs.  Device
-    us for 17 / 32 rows, GEMV - many-row kernel: 512 x 4096 12.1 / 12.2 - 16.6, 512 x 9728 13.5 / 14.0 - 28.9, 2048 x 6144
-    14.5 / 16.5 - 20.7, 4096 x 4096 14.5 / 16.6 - 16.6, 4096 x 9728 23.9 / 26.2 - 29.7 / 30.6.  Between K = 1024 and 2048 the
-    two are level for narrow weights (512 x 1024 10.7 / 10.4 - 9.8 / 10.4, 512 x 2048 10.4 / 12.2 - 10.4) and the many-row
-    kernel is 2 us ahead at N = 4096 (12.5 - 10.4); the line stays where shapes were first sorted.  The other side:
-    512 x 512 12.5 - 8.4, 6144 x 4096 18.6 / 20.7 - 16.6, 6144 x 6144 24.8 / 28.9 - 20.7.  Odd group counts go through the
-    GEMV's slower consumer; from 33 rows on the GEMV would read the weights three times."""
+    that walk, about 5 us + 2.5 us per 1024 of K, however small N is.  The GEMV spreads the weight rows over all SMs.
+    us for 17 rows with the quantisation, in a captured chain over weights that rotate through more than L2, GEMV - many-row
+    kernel (32 rows: within 0.3): 512 x 1024 7.6 - 8.6, 4096 x 1024 8.7 - 9.2, 4096 x 1536 10.6 - 10.5, 512 x 2048 7.1 - 9.5,
+    4096 x 2048 8.4 - 10.1, 2048 x 2560 9.4 - 12.9, 4096 x 2560 11.8 - 13.0, 4096 x 4096 12.1 - 16.4.  Called from the host
+    back to back the GEMV's second launch shows: 512 x 1024 11.6 - 10.3, 4096 x 1024 14.4 - 11.6, 512 x 2048 11.6 - 12.3,
+    4096 x 2048 13.3 - 12.3, 4096 x 2560 15.6 - 14.4, 4096 x 4096 16.4 - 18.5 (32 rows: 18.5 - 18.5).  The line is the
+    device's.  The other side (product alone): 512 x 512 12.5 - 8.4, 6144 x 4096 18.6 / 20.7 - 16.6, 6144 x 6144
+    24.8 / 28.9 - 20.7.  Odd group counts go through the GEMV's slower consumer; from 33 rows on the GEMV would read the
+    weights three times."""
     return 16 < T <= 32 and 1024 <= K <= GEMV_MAX_K and K % 256 == 0 and N <= 4096
 
 
