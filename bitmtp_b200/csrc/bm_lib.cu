@@ -5,6 +5,7 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <algorithm>
 #include <atomic>
 #include <mutex>
 
@@ -891,30 +892,31 @@ int launch_attention_cluster(dim3 grid, size_t smem, cudaStream_t st, int pdl, c
     return cuda_status(cudaLaunchKernelEx(&cfg, kernel, p));
 }
 
-template <bool ROPE>
-int launch_attention(int nq, dim3 grid, size_t smem, cudaStream_t st, int pdl, const bm::AttnParams &p) {
+template <bool ROPE, int MERGE>
+int launch_attention(int nv, dim3 grid, size_t smem, cudaStream_t st, int pdl, const bm::AttnParams &p) {
     const dim3 block(bm::kAttnThreads);
-    // Cluster build where a (kv head, query group)'s super-chunks fit one cluster.  Same arithmetic, same order.
-    if (p.slab_rows == 0 && p.slots > 0 && grid.x <= (unsigned)bm::kAttnMaxCluster) {
-        int rc;
-        switch (nq) {
-            case 1: rc = launch_attention_cluster<bm::attn_fused_kernel<1, ROPE, true>>(grid, smem, st, pdl, p); break;
-            case 2: rc = launch_attention_cluster<bm::attn_fused_kernel<2, ROPE, true>>(grid, smem, st, pdl, p); break;
-            case 3: rc = launch_attention_cluster<bm::attn_fused_kernel<3, ROPE, true>>(grid, smem, st, pdl, p); break;
-            default: rc = launch_attention_cluster<bm::attn_fused_kernel<4, ROPE, true>>(grid, smem, st, pdl, p); break;
-        }
-        if (rc >= 0) return rc;
-    }
-    switch (nq) {
-        case 1: return launch_ex(bm::attn_fused_kernel<1, ROPE>, grid, block, smem, st, pdl, p);
-        case 2: return launch_ex(bm::attn_fused_kernel<2, ROPE>, grid, block, smem, st, pdl, p);
-        case 3: return launch_ex(bm::attn_fused_kernel<3, ROPE>, grid, block, smem, st, pdl, p);
-        default: return launch_ex(bm::attn_fused_kernel<4, ROPE>, grid, block, smem, st, pdl, p);
+    switch (nv) {
+        case 1: return launch_ex(bm::attn_fused_kernel<1, ROPE, MERGE>, grid, block, smem, st, pdl, p);
+        case 2: return launch_ex(bm::attn_fused_kernel<2, ROPE, MERGE>, grid, block, smem, st, pdl, p);
+        case 3: return launch_ex(bm::attn_fused_kernel<3, ROPE, MERGE>, grid, block, smem, st, pdl, p);
+        default: return launch_ex(bm::attn_fused_kernel<4, ROPE, MERGE>, grid, block, smem, st, pdl, p);
     }
 }
 
-// One attention launch (scores, softmax, numerators, merge: bf16 rows + row absmax bits), followed by the
-// flat quantisation launch unless the caller asked for rows only (`amax_rows` != null).
+// Cluster build where a (kv head, query group)'s super-chunks fit one cluster; -1: not taken.  Same arithmetic, same order.
+int launch_attention_clusters(int nv, dim3 grid, size_t smem, cudaStream_t st, int pdl, const bm::AttnParams &p) {
+    using namespace bm;
+    switch (nv) {
+        case 1: return launch_attention_cluster<attn_fused_kernel<1, true, kMergeCluster>>(grid, smem, st, pdl, p);
+        case 2: return launch_attention_cluster<attn_fused_kernel<2, true, kMergeCluster>>(grid, smem, st, pdl, p);
+        case 3: return launch_attention_cluster<attn_fused_kernel<3, true, kMergeCluster>>(grid, smem, st, pdl, p);
+        default: return launch_attention_cluster<attn_fused_kernel<4, true, kMergeCluster>>(grid, smem, st, pdl, p);
+    }
+}
+
+// Rows wanted (`amax_rows` != null): one attention launch, bf16 rows + row absmax bits.  Codes wanted: an attention launch
+// that leaves its super-chunk partials to the launch that merges and quantises them (up to 32 heads: one warp each), else
+// an attention launch that merges, and the flat quantisation.
 int verify_attention_impl(const void *q, const RopeInputs *rope, const void *k_base, const void *v_base, int M, int H,
                           int Hkv, int kv_rows, int sigma, const void *state, void *scratch, void *att_out,
                           void *q_out, void *q_prep, void *asum, void *s_out, int pdl, void *stream,
@@ -940,14 +942,13 @@ int verify_attention_impl(const void *q, const RopeInputs *rope, const void *k_b
     const int NJ = (sigma + BM_ATTN_SUPER - 1) / BM_ATTN_SUPER + 1;
     if (NJ > bm::kAttnMaxNJ) return BM_EINVAL;
     const int G = H / Hkv, QV = G * M;
-    int nq = 1, Z = 1;
-    bm::attn_query_split(QV, &nq, &Z);
-    // more z-slices than the coarse split needs: every CTA picks the split for the history length it reads
-    Z = bm::attn_zmax(QV, nq);
+    const int nv = bm::attn_nv(QV), Z = bm::attn_groups(QV, 1);   // every CTA picks its split between the two
     if (Hkv * Z > bm::kAttnTickets) return BM_EINVAL;
     if ((H * 128) % 256 != 0 && amax_rows == nullptr) return BM_EINVAL;   // the flat quantisation wants K % 256 == 0
     bm::AttnParams p = {};
-    p.slots = 2 * current_device().sm_count;                     // two CTAs of this kernel per SM (shared memory)
+    const int sms = current_device().sm_count;
+    p.z_max = Z;
+    const bool single = bm::attn_fill_pick(p.pick, NJ, QV, Hkv, sms);
     p.q = static_cast<const uint16_t *>(q);
     p.k_base = static_cast<const uint16_t *>(k_base);
     p.v_base = static_cast<const uint16_t *>(v_base);
@@ -964,16 +965,20 @@ int verify_attention_impl(const void *q, const RopeInputs *rope, const void *k_b
     p.amax = amax_rows ? static_cast<unsigned int *>(amax_rows) : own_amax;
     p.pdl = pdl & (BM_PDL_OVERLAP | BM_PDL_STABLE_STATE);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (amax_rows == nullptr) {
-        // this call gathers the row absmax in the scratch header: clear it first (stream-ordered)
+    const bool later = amax_rows == nullptr && H <= 32;
+    int attn_pdl = pdl & BM_PDL_OVERLAP;
+    if (amax_rows == nullptr && !later) {
+        // this call gathers the row absmax in the scratch header: clear it first (stream-ordered); after a memset node the
+        // launch cannot overlap its predecessor programmatically
         const cudaError_t e = cudaMemsetAsync(own_amax, 0, BM_MAX_W * sizeof(unsigned int), st);
         if (e != cudaSuccess) return cuda_status(e);
+        attn_pdl = p.pdl = 0;
     }
-    const size_t smem = bm::attn_smem_bytes(nq);
-    const dim3 grid(NJ, Hkv, Z);
-    // after a memset node the launch cannot overlap its predecessor programmatically
-    const int attn_pdl = amax_rows ? (pdl & BM_PDL_OVERLAP) : 0;
-    if (amax_rows == nullptr) p.pdl = 0;
+    // Where the working CTAs never exceed the SMs, one CTA per SM: two would share the first SM that the predecessor leaves
+    // while others stay empty.
+    size_t smem = bm::attn_smem_bytes(nv);
+    if (single) smem = std::max(smem, (size_t)kMaxSmemPerCta / 2 + 1024);
+    const dim3 grid(Hkv, NJ * Z);
     int rc;
     if (rope != nullptr) {
         p.xqkv = static_cast<const uint16_t *>(rope->xqkv);
@@ -985,11 +990,21 @@ int verify_attention_impl(const void *q, const RopeInputs *rope, const void *k_b
         p.k_out = const_cast<uint16_t *>(p.k_base);
         p.v_out = const_cast<uint16_t *>(p.v_base);
         p.eps = rope->eps;
-        rc = launch_attention<true>(nq, grid, smem, st, attn_pdl, p);
+        rc = later ? launch_attention<true, bm::kMergeLater>(nv, grid, smem, st, attn_pdl, p)
+                   : launch_attention_clusters(nv, dim3(NJ, Hkv, Z), smem, st, attn_pdl, p);
+        if (rc < 0) rc = launch_attention<true, bm::kMergeTicket>(nv, grid, smem, st, attn_pdl, p);
     } else {
-        rc = launch_attention<false>(nq, grid, smem, st, attn_pdl, p);
+        rc = later ? launch_attention<false, bm::kMergeLater>(nv, grid, smem, st, attn_pdl, p)
+                   : launch_attention<false, bm::kMergeTicket>(nv, grid, smem, st, attn_pdl, p);
     }
     if (rc != BM_OK || amax_rows != nullptr) return rc;
+    if (later) {
+        const bm::AttnMergeParams mp{p.pm, p.pl, p.po, p.state, H, NJ, sigma, p.pdl, static_cast<uint16_t *>(att_out),
+                                     bm::QuantSink{static_cast<int8_t *>(q_out), static_cast<int8_t *>(q_prep),
+                                                   static_cast<int32_t *>(asum)},
+                                     static_cast<float *>(s_out)};
+        return launch_ex(bm::attn_merge_quant_kernel, dim3(M), dim3(32 * H), 0, st, attn_pdl, mp);
+    }
     // INT8 codes of the rows from the flat grid, with the absmax the merge gathered
     bm::QuantSink sink{static_cast<int8_t *>(q_out), static_cast<int8_t *>(q_prep), static_cast<int32_t *>(asum)};
     const int K = H * 128, units = M * (K / 8);
@@ -1172,14 +1187,16 @@ int bm_t2_gemm_wide(const void *A_prep, const void *a_sums, const void *B, void 
 
 namespace {
 // Slabs, grid.x and scratch layout of the prompt-mode attention.
-struct PromptAttnPlan { int n_slabs, units, NJ, nq, Z; size_t ticket_bytes, total; };
+struct PromptAttnPlan { int n_slabs, units, NJ, nv, Z; size_t ticket_bytes, total; };
 bool prompt_attn_plan(int T, int hist0, int slab_rows, int H, int Hkv, PromptAttnPlan *pl) {
     if (T < 1 || hist0 < 0 || slab_rows < 1 || slab_rows > BM_MAX_W || H < 1 || Hkv < 1 || (H % Hkv) != 0) return false;
     pl->n_slabs = (T + slab_rows - 1) / slab_rows;
     pl->units = 0;
     for (int s = 0; s < pl->n_slabs; ++s) pl->units += (hist0 + s * slab_rows + BM_ATTN_SUPER - 1) / BM_ATTN_SUPER + 1;
     pl->NJ = (hist0 + T + BM_ATTN_SUPER - 1) / BM_ATTN_SUPER + 1;
-    bm::attn_query_split((H / Hkv) * slab_rows, &pl->nq, &pl->Z);
+    // at most eight query vectors per CTA: a slab has few, and its CTAs are many
+    pl->nv = std::min(bm::attn_nv((H / Hkv) * slab_rows), 2);
+    pl->Z = bm::attn_groups((H / Hkv) * slab_rows, pl->nv);
     // at least 64 KB: calls of different T (up to 512 rows for any head count in use) then keep their counters in one
     // place, which no call's partials touch, and can share a scratch
     pl->ticket_bytes = ((size_t)pl->n_slabs * Hkv * pl->Z * 4 + 65535) / 65536 * 65536;
@@ -1222,7 +1239,8 @@ int bm_prompt_attention(const void *q, const void *k_base, const void *v_base, i
     // 2048 keys 49 against 80, 512 rows behind 2048 keys 338 against 657).  Some calls change sides earlier: a line at
     // five fills takes the same time in sum, but up to 32 % more for few rows behind a long history.
     const long long general_ctas = (long long)pl.units * Hkv * pl.Z;
-    const size_t smem = bm::attn_smem_bytes(pl.nq);
+    const size_t smem = bm::attn_smem_bytes(pl.nv);
+    p.z_max = pl.Z;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (bm::prompt_hist_fits(slab_rows, H, Hkv) && general_ctas > 6LL * 2 * current_device().sm_count) {
         // history super-chunks by tiles of 64 query vectors, then one CTA set per slab for its own rows and the merge
@@ -1233,12 +1251,12 @@ int bm_prompt_attention(const void *q, const void *k_base, const void *v_base, i
             const int rc = launch_ex(bm::prompt_hist_kernel, hgrid, dim3(bm::kPaThreads), bm::kPaSmem, st, p.pdl, hp);
             if (rc != BM_OK) return rc;
         }
-        // slabs of 16 rows: 16 G query vectors, always eight per CTA (attn_query_split)
-        if (pl.nq != 4) return BM_EINVAL;
-        return launch_ex(bm::attn_fused_kernel<4, false, false, true>, dim3(pl.n_slabs, Hkv, pl.Z), dim3(bm::kAttnThreads), smem,
+        return launch_ex(bm::attn_fused_kernel<2, false, bm::kMergeHistory>, dim3(pl.n_slabs, Hkv, pl.Z), dim3(bm::kAttnThreads), smem,
                          st, p.pdl, p);
     }
-    return launch_attention<false>(pl.nq, dim3(pl.units, Hkv, pl.Z), smem, st, p.pdl, p);
+    const dim3 grid(pl.units, Hkv, pl.Z);
+    return pl.nv == 1 ? launch_ex(bm::attn_fused_kernel<1, false>, grid, dim3(bm::kAttnThreads), smem, st, p.pdl, p)
+                      : launch_ex(bm::attn_fused_kernel<2, false>, grid, dim3(bm::kAttnThreads), smem, st, p.pdl, p);
 }
 
 // ---------------------------------------------------------------------------- dense draft heads

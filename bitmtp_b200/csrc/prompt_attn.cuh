@@ -63,13 +63,6 @@ __device__ __forceinline__ int pa_weight(int key, int vg) { return key * kPaQuer
 
 // One step of the register-blocked products: acc[t][j] = fma(a[t], b[j], acc[t][j]), vectors t in pairs: the packed
 // fma rounds each half as the scalar one does, runs at the same rate per value and takes half the issue slots.
-typedef unsigned long long PaPair;
-__device__ __forceinline__ PaPair pa_pack(float lo, float hi) {
-    PaPair v;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
-    return v;
-}
-__device__ __forceinline__ void pa_unpack(PaPair v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
 __device__ __forceinline__ void pa_step(PaPair (&acc)[4][8], const float *a, const float *a4, const uint4 &braw) {
     float b[8];
     unpack8(braw, b);
@@ -82,31 +75,6 @@ __device__ __forceinline__ void pa_step(PaPair (&acc)[4][8], const float *a, con
         for (int t = 0; t < 4; ++t) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[t][j]) : "l"(av[t]), "l"(bb));
     }
 }
-
-// bm_expf for x <= 0, infinities or NaN, without its branches and the two conversions that issue at a quarter of the
-// rate; the same values: adding 1.5 * 2^23 rounds |t| < 2^22 to the nearest even integer and leaves it in the low bits,
-// and the exponent, -126 .. 0, goes in with one exact step.  Kept here: in the decode kernels, which evaluate a few per
-// thread, the branch is cheaper (whole requests 0.7 % slower without it).
-__device__ __forceinline__ float pa_expf(float x) {
-    const float biased = x * 1.44269504088896341f + 12582912.0f;
-    const float n = biased - 12582912.0f;
-    float r = fmaf(n, -0.693145751953125f, x);
-    r = fmaf(n, -1.42860682030941723e-6f, r);
-    float p = 1.3888889225e-3f;
-    p = fmaf(p, r, 8.3333337680e-3f);
-    p = fmaf(p, r, 4.1666667908e-2f);
-    p = fmaf(p, r, 1.6666667163e-1f);
-    p = fmaf(p, r, 0.5f);
-    p = fmaf(p, r, 1.0f);
-    p = fmaf(p, r, 1.0f);
-    const float e = p * __uint_as_float((__float_as_uint(biased) - 0x4B400000u + 127u) << 23);
-    return x >= -87.0f ? e : (x != x ? x : 0.0f);
-}
-
-__device__ __forceinline__ PaPair pa_add2(PaPair a, PaPair b) { PaPair d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
-__device__ __forceinline__ PaPair pa_mul2(PaPair a, PaPair b) { PaPair d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
-__device__ __forceinline__ PaPair pa_fma2(PaPair a, PaPair b, PaPair c) { PaPair d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
-__device__ __forceinline__ PaPair pa_both(float v) { return pa_pack(v, v); }
 
 // pa_expf of two values: the same roundings, two per instruction.  A NaN comes out of the products by itself.
 __device__ __forceinline__ PaPair pa_expf2(PaPair x) {

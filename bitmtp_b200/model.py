@@ -512,8 +512,6 @@ class Transformer(nn.Module):
         fused_ffn = self.fused_ffn and M <= 16 and a.ffn_dim % 16 == 0 and a.dim % 256 == 0
         if fused_ffn:
             ops.zero_words(W.inner_amax[0])           # slot of layer 0; every layer clears the next one's
-        if self.fused_rope:
-            ops.zero_words(W.att_amax[0])
         ops.rmsnorm_fused(self.embed_tokens.weight.data, L0.input_layernorm.weight.data, eps, M=M,
                           gather=token_values, pdl=pdl, out=qsink)
         for i, layer in enumerate(self.layers):
@@ -525,15 +523,12 @@ class Transformer(nn.Module):
                                  ldc=W.xqkv.shape[1], pdl=pdl)
             k_l, v_l = kv_full[i]
             if self.fused_rope:
-                # one attention launch (q/k norm, RoPE and KV append folded in; the last CTA of a query group
-                # merges the split-KV partials and gathers the row absmax by atomic max), then the INT8 codes
-                # from the flat quantisation kernel
-                ops.rope_verify_attention_rows(W.xqkv, at.q_norm.weight.data, at.k_norm.weight.data, eps,
-                                               at.rope_cos, at.rope_sin, positions, a.n_heads, a.n_kv_heads,
-                                               _LayerView(k_l, kv_rows), _LayerView(v_l, kv_rows), sigma, attn_mask,
-                                               attn_scratch, att=W.att, amax=W.att_amax[i & 1], pdl=attn_pdl)
-                ops.quant_rows_amax(W.att, W.att_amax[i & 1], prep=(W.att_q, W.att_sum), s=W.att_s,
-                                    amax_zero=W.att_amax[(i + 1) & 1], pdl=pdl)
+                # one attention launch (q/k norm, RoPE and KV append folded in) that leaves split-KV partials, and one
+                # that merges them and writes the rows as INT8 codes
+                ops.rope_verify_attention(W.xqkv, at.q_norm.weight.data, at.k_norm.weight.data, eps, at.rope_cos,
+                                          at.rope_sin, positions, a.n_heads, a.n_kv_heads, _LayerView(k_l, kv_rows),
+                                          _LayerView(v_l, kv_rows), sigma, attn_mask, attn_scratch,
+                                          out=(None, None, W.att_s), prep=(W.att_q, W.att_sum), pdl=attn_pdl)
             else:
                 ops.qknorm_rope_kvappend(W.xqkv, at.q_norm.weight.data, at.k_norm.weight.data, eps,
                                          at.rope_cos, at.rope_sin, positions, a.n_heads, a.n_kv_heads,

@@ -405,6 +405,45 @@ def test_rope_folded_into_attention(oracle, M, H, Hkv, sigma, cache_len, n_pend,
     assert native.lib().bm_device_error() == 0
 
 
+@pytest.mark.parametrize("M,H,Hkv,sigma,cache_len,n_pend,role", [
+    # every split (4, 8, 12, 16 query vectors per CTA; one or several CTAs per SM) and the edges of sub- and super-chunks
+    (2, 4, 4, 128, 127, 0, "ar"), (4, 2, 1, 256, 128, 0, "draft"), (3, 12, 4, 256, 129, 1, "draft"), (9, 10, 5, 256, 31, 0, "verify"),
+    (16, 16, 8, 1024, 385, 8, "draft"), (16, 16, 8, 1024, 1024, 0, "draft"), (32, 8, 8, 512, 33, 0, "ar"), (17, 32, 8, 2048, 1537, 9, "draft"),
+    # one warp per head ends at 32 heads: the general merge and the flat quantisation
+    (3, 34, 17, 128, 65, 0, "ar"), (2, 32, 32, 128, 1, 1, "verify"),
+])
+def test_attention_codes_equal_rows_then_quantisation(oracle, M, H, Hkv, sigma, cache_len, n_pend, role):
+    """Codes merged and quantised from the partials (GEMV-ready order, group sums, multipliers) against the rows-only call
+    followed by the flat quantisation: the same bits, also with a launch that may overlap its predecessor."""
+    gen = torch.Generator().manual_seed(M * 7 + cache_len + H)
+    xqkv = _bf16(gen, M, (H + 2 * Hkv) * 128, scale=2.0).to(DEV)
+    w = (1.0 + 0.1 * torch.randn(128, generator=gen)).to(torch.bfloat16).to(DEV)
+    cos, sin = (oracle.u16_to_torch(t).to(DEV) for t in _rope_tables(oracle, sigma + 40))
+    pos = (torch.arange(M) + max(cache_len - 1, 0)).to(torch.int64).to(DEV)
+    kv = _bf16(gen, 2, Hkv, sigma + M, 128, scale=1.5).to(DEV)
+    state = ops.new_step_state(DEV)
+    ops.set_step_state(state, cache_len, n_pend, oracle.ROLE_IDS[role], max(M - 8, 0))
+    scratch = ops.attention_scratch(M, H, sigma, DEV)
+    amax = torch.zeros(M, dtype=torch.int32, device=DEV)
+    att = torch.empty(M, H * 128, dtype=torch.bfloat16, device=DEV)
+
+    def sink():
+        return (torch.empty(M, H * 128, dtype=torch.int8, device=DEV), torch.empty(M, H, dtype=torch.int32, device=DEV),
+                torch.empty(M, 1, dtype=torch.float32, device=DEV))
+    qa, suma, sa = sink()
+    ka, va = kv[0].clone(), kv[1].clone()
+    ops.rope_verify_attention_rows(xqkv, w, w, 1e-6, cos, sin, pos, H, Hkv, ka, va, sigma, state, scratch, att=att, amax=amax)
+    ops.quant_rows_amax(att, amax, prep=(qa, suma), s=sa)
+    for pdl in (0, native.PDL_OVERLAP | native.PDL_STABLE_STATE):
+        qb, sumb, sb = sink()
+        kb, vb = kv[0].clone(), kv[1].clone()
+        ops.rope_verify_attention(xqkv, w, w, 1e-6, cos, sin, pos, H, Hkv, kb, vb, sigma, state, scratch,
+                                  out=(None, None, sb), prep=(qb, sumb), pdl=pdl)
+        torch.cuda.synchronize()
+        assert torch.equal(qa, qb) and torch.equal(suma, sumb) and torch.equal(sa.view(torch.int32), sb.view(torch.int32))
+        assert torch.equal(ka.view(torch.int16), kb.view(torch.int16)) and torch.equal(va.view(torch.int16), vb.view(torch.int16))
+
+
 @pytest.mark.parametrize("M,D,n_pend,cache_len", [(9, 8, 1, 40), (10, 8, 2, 7), (12, 8, 3, 100), (16, 8, 8, 300),
                                                   (17, 8, 9, 12), (16, 8, 5, 1), (5, 4, 1, 9), (9, 4, 5, 64)])
 def test_stage_replay_inputs_matches_the_tensor_fills(M, D, n_pend, cache_len):
