@@ -551,21 +551,26 @@ static int gemv_common(const void *A, const void *a_sums, const void *B, void *C
     if (path < BM_PATH_AUTO || path > BM_PATH_DIRECT) return BM_EINVAL;
     const int force_rb = 0;                           // tile height chosen by make_mma_plan
     if (path == BM_PATH_AUTO) {
-        // Measured on B200 (one call after the other over weights that rotate through more than L2):
+        // Measured on B200 (one call after the other over weights that rotate through more than L2), us at the sizes named:
         //  * many rows and at most 8 tokens: every warp streams its own 16-row blocks (row-per-warp kernel);
-        //  * one token over up to 4 MB of weights (two over up to 2 MB): the launch is latency-bound and the
-        //    kernel with a single memory round trip wins (3.3-5.3 us against 5.2-8.4 us); for three or four
-        //    tokens it still does up to 1 MB (2048 x 2048: 5.2 against 5.6 us, 1024 x 2048: 4.4 against 5.6 us);
-        //  * otherwise, up to 8 tokens and K a multiple of 2048: the row-per-warp kernel with two or four warps
-        //    sharing a block (2048 x 6144 at W = 8: 9.7 against 11.2 us; a 14336 x 8192 shard: 14.7 against 28.8 us);
-        //  * everything else (more than 8 tokens, odd K): the cooperative tiles.
+        //  * one token over up to 4 MB of weights, two over up to 1 MB: the launch is latency-bound and the kernel with a
+        //    single memory round trip wins (two tokens: 2048 x 2048 3.5 against 3.8 by cooperative tiles; 4096 x 2048 4.7
+        //    against 4.4).  Three and four tokens: level at 512 x 2048, 4.7 against 3.9 at 2048 x 2048;
+        //  * up to 8 tokens and K a multiple of 2048: the row-per-warp kernel with two or four warps sharing a block from
+        //    48 rows per SM on (8 tokens: 8192 x 2048 6.2 against 6.5, 12288 x 2048 6.8 against 7.9, 14336 x 8192 15.9
+        //    against 20.3); below, its few blocks leave SMs idle (2048 x 6144 8.8 against 6.5, 4096 x 2048 5.6 against 4.7,
+        //    4096 x 4096 7.6 against 6.4, 6144 x 2048 6.0 against 5.9);
+        //  * everything else (more than 8 tokens, other K): the cooperative tiles.
+        // One token, and a K that the tiles do not take, keep the limits that do not look at the tiles.
         const bool rw = rowwarp_fits(W, N, K);
-        const size_t wbytes = (size_t)N * K / 4;
-        const bool direct_ok = p.world <= 1 && bm::direct_fits(W, N, K) &&
-                               wbytes <= (W == 1 ? (size_t)4 << 20 : (W == 2 ? (size_t)2 << 20 : (size_t)1 << 20));
+        MmaPlan pl;
+        const bool tiles = W > 1 && (K % 256) == 0 && make_mma_plan(N, K, W <= 8, sms, 0, &pl);
+        const size_t wbytes = (size_t)N * K / 4, mb = (size_t)1 << 20;
+        const size_t direct_max = W == 1 ? 4 * mb : (W == 2 ? (tiles ? mb : 2 * mb) : (tiles ? 0 : mb));
+        const bool direct_ok = p.world <= 1 && bm::direct_fits(W, N, K) && wbytes <= direct_max;
         if (rw && N / bm::kRwRows >= 8 * sms) path = BM_PATH_ROWWARP;
         else if (direct_ok) path = BM_PATH_DIRECT;
-        else if (rw && (K % 2048) == 0) path = BM_PATH_ROWWARP;
+        else if (rw && (K % 2048) == 0 && (!tiles || N >= 48 * sms)) path = BM_PATH_ROWWARP;
         else path = (K % 256) == 0 ? BM_PATH_MMA : BM_PATH_DP4A;
     }
     if (path == BM_PATH_DIRECT) return gemv_launch_direct(p, pdl, st);

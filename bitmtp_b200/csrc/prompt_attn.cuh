@@ -39,7 +39,8 @@ struct PromptHistParams {
 // Q^T fp32 [128][kPaQStride] (after the scores its space holds P^T fp32 [128][64], see pa_weight), K^T bf16
 // [128][kPaKStride], V bf16 [128][128], m and l fp32 [4][64].
 constexpr int kPaQBytes = 128 * kPaQStride * 4, kPaKBytes = 128 * kPaKStride * 2, kPaVBytes = BM_ATTN_SUPER * 256;
-constexpr int kPaSmem = kPaQBytes + kPaKBytes + kPaVBytes + 2 * kAttnSub * kPaQueries * 4;
+static_assert(kPaVBytes <= kPaKBytes, "V takes the space of K^T");
+constexpr int kPaSmem = kPaQBytes + kPaKBytes + 2 * kAttnSub * kPaQueries * 4;
 
 // Whether the tile kernel takes a call; the launcher keeps attn_fused_kernel for every other slab height or
 // head grouping.
@@ -146,7 +147,7 @@ __device__ __forceinline__ void pa_softmax(PaPair (&acc)[4][8], int lim, int kgp
 
 // grid (super-chunks of the longest history, Hkv, ceil(T * G / 64)), 128 threads = 8 vector groups x 16 key
 // (then dim) groups.
-__global__ void __launch_bounds__(kPaThreads, 2) prompt_hist_kernel(const PromptHistParams p) {
+__global__ void __launch_bounds__(kPaThreads, 3) prompt_hist_kernel(const PromptHistParams p) {
     extern __shared__ __align__(16) unsigned char pa_smem[];
     pdl_launch_dependents();
     if (p.pdl) pdl_wait();
@@ -158,16 +159,13 @@ __global__ void __launch_bounds__(kPaThreads, 2) prompt_hist_kernel(const Prompt
     if (keys_max <= 0) return;
     float *Qt = reinterpret_cast<float *>(pa_smem), *Pt = Qt;
     uint16_t *Kt = reinterpret_cast<uint16_t *>(pa_smem + kPaQBytes);
-    uint16_t *Vs = reinterpret_cast<uint16_t *>(pa_smem + kPaQBytes + kPaKBytes);
-    float *mc = reinterpret_cast<float *>(pa_smem + kPaQBytes + kPaKBytes + kPaVBytes), *lc = mc + kAttnSub * kPaQueries;
+    uint16_t *Vs = Kt;
+    float *mc = reinterpret_cast<float *>(pa_smem + kPaQBytes + kPaKBytes), *lc = mc + kAttnSub * kPaQueries;
 
-    // V as it is (16-byte asynchronous copies); K two rows per lane, transposed as bf16 pairs; Q one vector per
+    // K two rows per lane, transposed as bf16 pairs; Q one vector per
     // lane, transposed as fp32.  Consecutive lanes store consecutive words: no bank conflicts.
     const uint16_t *kg = p.k_base + ((size_t)hk * p.kv_rows + key0) * 128;
     const uint16_t *vg = p.v_base + ((size_t)hk * p.kv_rows + key0) * 128;
-    for (int i = tid; i < BM_ATTN_SUPER * 16; i += kPaThreads) {
-        if ((i >> 4) < keys_max) cp_async16(Vs + 8 * i, reinterpret_cast<const uint4 *>(vg) + i);
-    }
     {
         // Every load is out before the first store: the compiler may not move a load over a store to shared memory, and one
         // round trip per piece cost 8000 cycles of a tile's 66000.
@@ -198,7 +196,6 @@ __global__ void __launch_bounds__(kPaThreads, 2) prompt_hist_kernel(const Prompt
             for (int e = 0; e < 8; ++e) Qt[(d0 + e) * kPaQStride + v] = f[e];
         }
     }
-    cp_async_wait_all();
     __syncthreads();
 
     const int vgp = tid >> 4, kgp = tid & 15;                         // vector group, key / dim group
@@ -219,7 +216,8 @@ __global__ void __launch_bounds__(kPaThreads, 2) prompt_hist_kernel(const Prompt
         for (int d = 0; d < 128; ++d)
             pa_step(acc2, qp + d * kPaQStride, qp + d * kPaQStride + 4, *reinterpret_cast<const uint4 *>(kp + d * kPaKStride));
     }
-    __syncthreads();                                                  // Q^T is spent: its space takes P^T
+    __syncthreads();                                                  // Q^T and K^T are spent: P^T and V take their space
+    for (int i = tid; i < keys_max * 16; i += kPaThreads) cp_async16(Vs + 8 * i, reinterpret_cast<const uint4 *>(vg) + i);
     const int c = kgp >> 2;                                           // sub-chunk of this thread's keys
     if (lim >= BM_ATTN_SUPER) pa_softmax<true>(acc2, lim, kgp, c, v0, mc, lc);
     else pa_softmax<false>(acc2, lim, kgp, c, v0, mc, lc);
@@ -229,21 +227,35 @@ __global__ void __launch_bounds__(kPaThreads, 2) prompt_hist_kernel(const Prompt
         *reinterpret_cast<ulonglong2 *>(Pt + w) = make_ulonglong2(acc2[0][j], acc2[1][j]);
         *reinterpret_cast<ulonglong2 *>(Pt + (w ^ 4)) = make_ulonglong2(acc2[2][j], acc2[3][j]);
     }
+    cp_async_wait_all();
+    __syncthreads();
+    // level 1 of a vector by one thread: maximum of its four sub-chunks, their weights (over the maxima) and the weight sum
+    if (tid < kPaQueries) {
+        float m[kAttnSub], MJ = -INFINITY, L = 0.0f;
+#pragma unroll
+        for (int s = 0; s < kAttnSub; ++s) { m[s] = mc[s * kPaQueries + tid]; MJ = fmaxf(MJ, m[s]); }
+#pragma unroll
+        for (int s = 0; s < kAttnSub; ++s) {
+            const float w = m[s] > -INFINITY ? pa_expf(m[s] - MJ) : 0.0f;
+            L = fmaf(lc[s * kPaQueries + tid], w, L);
+            mc[s * kPaQueries + tid] = w;
+        }
+        const int r = row0 + (tid >> p.log_g), head = (hk << p.log_g) + (tid & gmask);
+        if (r < p.T && pa_history(p.hist0, r) > key0) {
+            const size_t pb = ((size_t)r * p.H + head) * p.NJ + J;
+            p.pm[pb] = MJ;
+            p.pl[pb] = L;
+        }
+    }
     __syncthreads();
     if (lim <= 0) return;
 
-    float acc[8][8];                                                  // [vector][dim]
     // numerators: this thread's 8 vectors x dims 8 kgp .. 8 kgp + 7, one chain per sub-chunk, then the merge
-    float O[8][8], L[8], MJ[8];
+    PaPair O[4][8];                                                   // [vector pair][dim]
 #pragma unroll
-    for (int t = 0; t < 8; ++t) {
-        L[t] = 0.0f;
-        MJ[t] = -INFINITY;
+    for (int t = 0; t < 4; ++t)
 #pragma unroll
-        for (int s = 0; s < kAttnSub; ++s) MJ[t] = fmaxf(MJ[t], mc[s * kPaQueries + v0 + t]);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) O[t][e] = 0.0f;
-    }
+        for (int e = 0; e < 8; ++e) O[t][e] = 0ull;
     for (int s = 0; s < kAttnSub; ++s) {
 #pragma unroll
         for (int t = 0; t < 4; ++t)
@@ -265,27 +277,26 @@ __global__ void __launch_bounds__(kPaThreads, 2) prompt_hist_kernel(const Prompt
             }
         }
 #pragma unroll
-        for (int t = 0; t < 4; ++t)
+        for (int t = 0; t < 4; ++t) {
+            const PaPair w = *reinterpret_cast<const PaPair *>(mc + s * kPaQueries + v0 + 2 * t);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) pa_unpack(acc2[t][e], acc[2 * t][e], acc[2 * t + 1][e]);
-#pragma unroll
-        for (int t = 0; t < 8; ++t) {
-            const float m = mc[s * kPaQueries + v0 + t];
-            const float w = m > -INFINITY ? pa_expf(m - MJ[t]) : 0.0f;
-            L[t] = fmaf(lc[s * kPaQueries + v0 + t], w, L[t]);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) O[t][e] = fmaf(acc[t][e], w, O[t][e]);
+            for (int e = 0; e < 8; ++e) O[t][e] = pa_fma2(acc2[t][e], w, O[t][e]);
         }
     }
 #pragma unroll
-    for (int t = 0; t < 8; ++t) {
-        const int r = row0 + ((v0 + t) >> p.log_g), head = (hk << p.log_g) + ((v0 + t) & gmask);
-        if (r >= p.T) continue;
-        const size_t pb = ((size_t)r * p.H + head) * p.NJ + J;
-        float *dst = p.po + pb * 128 + 8 * kgp;
-        *reinterpret_cast<float4 *>(dst) = make_float4(O[t][0], O[t][1], O[t][2], O[t][3]);
-        *reinterpret_cast<float4 *>(dst + 4) = make_float4(O[t][4], O[t][5], O[t][6], O[t][7]);
-        if (kgp == 0) { p.pm[pb] = MJ[t]; p.pl[pb] = L[t]; }
+    for (int t = 0; t < 4; ++t) {
+        float lo[8], hi[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) pa_unpack(O[t][e], lo[e], hi[e]);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int v = v0 + 2 * t + i, r = row0 + (v >> p.log_g), head = (hk << p.log_g) + (v & gmask);
+            if (r >= p.T) continue;
+            const float *o = i ? hi : lo;
+            float *dst = p.po + (((size_t)r * p.H + head) * p.NJ + J) * 128 + 8 * kgp;
+            *reinterpret_cast<float4 *>(dst) = make_float4(o[0], o[1], o[2], o[3]);
+            *reinterpret_cast<float4 *>(dst + 4) = make_float4(o[4], o[5], o[6], o[7]);
+        }
     }
 }
 

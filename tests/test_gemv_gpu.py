@@ -289,3 +289,11 @@ def test_many_row_product_equals_the_gemv_row_for_row(T, N, K):
     assert native.lib().bm_device_error() == 0
     assert torch.equal(got[:T, :N].view(torch.int16), want.view(torch.int16))
     assert bool((got[T] == 7.0).all()) and bool((got[:, N:] == 7.0).all()), "wrote outside the output"
+
+
+# around 48 rows per SM (148 SMs: 7104 rows), where a K that is a multiple of 2048 goes from the cooperative tiles to the
+# row-per-warp kernel; two tokens over 1 MB; a K whose tiles do not fit shared memory
+@pytest.mark.parametrize("W,N,K", [(8, 7088, 2048), (8, 7104, 2048), (5, 7120, 2048), (2, 4096, 2048), (2, 4112, 2048), (3, 1040, 2048),
+                                   (4, 16, 4096), (7, 24, 2048), (2, 64, 24576), (4, 32, 10496)])
+def test_auto_path_at_its_lines(oracle, W, N, K):
+    _check(oracle, synthetic.gemv_case(W, N, K, seed=W + N + K), native.PATH_AUTO)
