@@ -71,6 +71,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
 // try_wait itself blocks for a hardware-defined slice, so 1<<22 polls is on the
 // order of seconds, far beyond any healthy copy.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity) {
+#pragma unroll 1
     for (int it = 0; it < (1 << 22); ++it) {
         if (mbar_try_wait(bar, parity)) return true;
         if (it > 64) __nanosleep(64);
@@ -87,6 +88,7 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
 // out its own full limit in turn.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity,
                                                   volatile int *abort_flag) {
+#pragma unroll 1
     for (int it = 0; it < (1 << 22); ++it) {
         if (mbar_try_wait(bar, parity)) return true;
         if (it > 32) {
@@ -149,6 +151,32 @@ __device__ __forceinline__ void cluster_st_f32(uint32_t a, float v) {
 }
 __device__ __forceinline__ void cluster_st_s32(uint32_t a, int v) {
     asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+
+// ---- conversions, several at once ------------------------------------------------
+// Two fp32 values to bf16, `lo` in the low half: the roundings of bm_f32_to_bf16 in one instruction.
+__device__ __forceinline__ uint32_t bf16_pair(float lo, float hi) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+// Two values after one bf16 rounding each (bm_bf16_rn).
+__device__ __forceinline__ void bf16_round_pair(float &a, float &b) {
+    const uint32_t r = bf16_pair(a, b);
+    a = __uint_as_float(r << 16);
+    b = __uint_as_float(r & 0xffff0000u);
+}
+// Four INT8 codes (bm_quant_i8), a in the lowest byte: the packing conversions saturate.
+__device__ __forceinline__ uint32_t quant_quad(float a, float b, float c, float d, float s) {
+    int x, y, z, w;
+    asm("cvt.rni.s32.f32 %0, %1;" : "=r"(x) : "f"(a * s));
+    asm("cvt.rni.s32.f32 %0, %1;" : "=r"(y) : "f"(b * s));
+    asm("cvt.rni.s32.f32 %0, %1;" : "=r"(z) : "f"(c * s));
+    asm("cvt.rni.s32.f32 %0, %1;" : "=r"(w) : "f"(d * s));
+    uint32_t hi, r;
+    asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, 0;" : "=r"(hi) : "r"(w), "r"(z));
+    asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(y), "r"(x), "r"(hi));
+    return r;
 }
 
 // ---- warp reductions in the oracle's butterfly order -------------------------

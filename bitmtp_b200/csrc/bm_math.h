@@ -52,15 +52,16 @@ BM_HD float bm_bits_f32(uint32_t u) {
 BM_HD float bm_bf16_to_f32(uint16_t h) { return bm_bits_f32(((uint32_t)h) << 16); }
 
 BM_HD uint16_t bm_f32_to_bf16(float f) {
-    uint32_t u = bm_f32_bits(f);
-    if ((u & 0x7fffffffu) > 0x7f800000u) return (uint16_t)((u >> 16) | 0x0040u);  // NaN stays NaN
 #if defined(__CUDA_ARCH__)
-    // the hardware conversion rounds to nearest even exactly as the integer form below does
-    // (denormals and the overflow to infinity included); one instruction instead of five
+    // the hardware conversion rounds to nearest even exactly as the integer form below does (denormals and the overflow to
+    // infinity included).  A NaN becomes 0x7fff, which is also what the integer form makes of the only NaN that the device's
+    // arithmetic gives (0x7fffffff): one instruction instead of the five around the branch that kept other payloads.
     unsigned short r;
     asm("cvt.rn.bf16.f32 %0, %1;" : "=h"(r) : "f"(f));
     return r;
 #else
+    uint32_t u = bm_f32_bits(f);
+    if ((u & 0x7fffffffu) > 0x7f800000u) return (uint16_t)((u >> 16) | 0x0040u);  // NaN stays NaN
     u += 0x7fffu + ((u >> 16) & 1u);
     return (uint16_t)(u >> 16);
 #endif
@@ -131,10 +132,17 @@ BM_HD float bm_rsqrtf(float v) { return 1.0f / sqrtf(v); }
 // Per-token symmetric INT8 quantisation of one value (model.py:632-636):
 // round-half-to-even of x*s, clamped to [-128, 127].
 BM_HD int bm_quant_i8(float x, float s) {
+#if defined(__CUDA_ARCH__)
+    // one conversion that rounds to nearest even, saturates and gives 0 for a NaN, as the four steps below do
+    int r;
+    asm("cvt.rni.s32.f32 %0, %1;" : "=r"(r) : "f"(x * s));
+    return r < -128 ? -128 : (r > 127 ? 127 : r);
+#else
     float r = rintf(x * s);
     r = r < -128.0f ? -128.0f : r;
     r = r > 127.0f ? 127.0f : r;
     return (int)r;
+#endif
 }
 
 // Activation multiplier s = 127 / max(absmax, 1e-5) (model.py:635).  torch evaluates

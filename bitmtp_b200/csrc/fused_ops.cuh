@@ -84,18 +84,36 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
     uint32_t w[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
-        w[i] = (uint32_t)bm_f32_to_bf16(f[2 * i]) | ((uint32_t)bm_f32_to_bf16(f[2 * i + 1]) << 16);
+        w[i] = bf16_pair(f[2 * i], f[2 * i + 1]);
     return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-__device__ __forceinline__ uint2 quant8(const float (&f)[8], float s) {
-    uint32_t lo = 0, hi = 0;
+// h = bf16(h + r), the rounded sums also as they are stored.
+__device__ __forceinline__ uint4 add8(float (&h)[8], const float (&r)[8]) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        lo |= ((uint32_t)(bm_quant_i8(f[i], s) & 0xff)) << (8 * i);
-        hi |= ((uint32_t)(bm_quant_i8(f[4 + i], s) & 0xff)) << (8 * i);
+    for (int i = 0; i < 8; ++i) h[i] = h[i] + r[i];
+    const uint4 v = pack8(h);
+    unpack8(v, h);
+    return v;
+}
+
+// n = bf16(w * bf16(h * r)); returns the largest |n| (a NaN is passed over).
+__device__ __forceinline__ float norm8(const float (&h)[8], const float (&w)[8], float r, float (&n)[8]) {
+    float amax = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; i += 2) {
+        float a = h[i] * r, b = h[i + 1] * r;
+        bf16_round_pair(a, b);
+        n[i] = w[i] * a;
+        n[i + 1] = w[i + 1] * b;
+        bf16_round_pair(n[i], n[i + 1]);
+        amax = fmaxf(fmaxf(amax, fabsf(n[i])), fabsf(n[i + 1]));
     }
-    return make_uint2(lo, hi);
+    return amax;
+}
+
+__device__ __forceinline__ uint2 quant8(const float (&f)[8], float s) {
+    return make_uint2(quant_quad(f[0], f[1], f[2], f[3], s), quant_quad(f[4], f[5], f[6], f[7], s));
 }
 
 // Where the INT8 codes of a row go.  `nat` is the natural-order row the reference's
@@ -251,14 +269,14 @@ __global__ void __launch_bounds__(1024) rmsnorm_kernel(const NormParams p) {
     if (p.pdl) pdl_wait();
     const size_t src_row = p.gather ? gather_row(p.gather[m], p.gather_rows) : (size_t)(p.row0 + m);
     float h[8];
-    unpack8(reinterpret_cast<const uint4 *>(p.x + src_row * p.dim)[t], h);
+    uint4 hraw = reinterpret_cast<const uint4 *>(p.x + src_row * p.dim)[t];
+    unpack8(hraw, h);
     if (p.res) {
         float r[8];
         unpack8(reinterpret_cast<const uint4 *>(p.res + (size_t)(p.row0 + m) * p.dim)[t], r);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) h[i] = bm_bf16_rn(h[i] + r[i]);
+        hraw = add8(h, r);
     }
-    if (p.h_out) reinterpret_cast<uint4 *>(p.h_out + (size_t)m * p.dim)[t] = pack8(h);
+    if (p.h_out) reinterpret_cast<uint4 *>(p.h_out + (size_t)m * p.dim)[t] = hraw;
     float acc = 0.0f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) acc = fmaf(h[i], h[i], acc);
@@ -266,15 +284,10 @@ __global__ void __launch_bounds__(1024) rmsnorm_kernel(const NormParams p) {
     const float r = bm_rsqrtf(mean_of(total, p.dim) + p.eps);
     float wv[8], n[8];
     unpack8(wraw, wv);
-    float amax = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        n[i] = bm_bf16_rn(wv[i] * bm_bf16_rn(h[i] * r));
-        amax = fmaxf(amax, fabsf(n[i]));
-    }
+    const float amax_row = norm8(h, wv, r, n);
     if (p.n_out) reinterpret_cast<uint4 *>(p.n_out + (size_t)m * p.dim)[t] = pack8(n);
     if (p.s) {
-        amax = block_absmax(amax, sh + 32, lane, warp, nwarps);
+        const float amax = block_absmax(amax_row, sh + 32, lane, warp, nwarps);
         const float s = bm_act_scale(amax);
         emit_codes(p.q, (size_t)m * p.dim, p.dim, t, quant8(n, s), true, lane);
         if (t == 0) p.s[m] = s;
@@ -379,7 +392,13 @@ __global__ void __launch_bounds__(128) qknorm_rope_kvappend_kernel(const RopePar
                          __uint_as_float(sraw.y << 16), __uint_as_float(sraw.y & 0xffff0000u)};
     float n[4], o[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) n[i] = bm_bf16_rn(w[i] * bm_bf16_rn(x[i] * r));
+    for (int i = 0; i < 4; i += 2) {
+        float a = x[i] * r, b = x[i + 1] * r;
+        bf16_round_pair(a, b);
+        n[i] = w[i] * a;
+        n[i + 1] = w[i + 1] * b;
+        bf16_round_pair(n[i], n[i + 1]);
+    }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const float partner = __shfl_xor_sync(0xffffffffu, n[i], 16);
@@ -387,8 +406,7 @@ __global__ void __launch_bounds__(128) qknorm_rope_kvappend_kernel(const RopePar
         o[i] = bm_bf16_rn(n[i] * c[i]) + bm_bf16_rn(rot * sn[i]);
     }
     const uint2 packed = make_uint2(
-        (uint32_t)bm_f32_to_bf16(o[0]) | ((uint32_t)bm_f32_to_bf16(o[1]) << 16),
-        (uint32_t)bm_f32_to_bf16(o[2]) | ((uint32_t)bm_f32_to_bf16(o[3]) << 16));
+        bf16_pair(o[0], o[1]), bf16_pair(o[2], o[3]));
     uint16_t *dst = hd < p.H
                         ? p.q_out + ((size_t)m * p.H + hd) * 128
                         : p.k_base + ((size_t)(hd - p.H) * p.kv_rows + p.sigma + m) * 128;

@@ -39,8 +39,7 @@ struct PromptHistParams {
 // Q^T fp32 [128][kPaQStride] (after the scores its space holds P^T fp32 [128][64], see pa_weight), K^T bf16
 // [128][kPaKStride], V bf16 [128][128], m and l fp32 [4][64].
 constexpr int kPaQBytes = 128 * kPaQStride * 4, kPaKBytes = 128 * kPaKStride * 2, kPaVBytes = BM_ATTN_SUPER * 256;
-static_assert(kPaVBytes <= kPaKBytes, "V takes the space of K^T");
-constexpr int kPaSmem = kPaQBytes + kPaKBytes + 2 * kAttnSub * kPaQueries * 4;
+constexpr int kPaSmem = kPaQBytes + kPaKBytes + kPaVBytes + 2 * kAttnSub * kPaQueries * 4;
 
 // Whether the tile kernel takes a call; the launcher keeps attn_fused_kernel for every other slab height or
 // head grouping.
@@ -147,7 +146,7 @@ __device__ __forceinline__ void pa_softmax(PaPair (&acc)[4][8], int lim, int kgp
 
 // grid (super-chunks of the longest history, Hkv, ceil(T * G / 64)), 128 threads = 8 vector groups x 16 key
 // (then dim) groups.
-__global__ void __launch_bounds__(kPaThreads, 3) prompt_hist_kernel(const PromptHistParams p) {
+__global__ void __launch_bounds__(kPaThreads, 2) prompt_hist_kernel(const PromptHistParams p) {
     extern __shared__ __align__(16) unsigned char pa_smem[];
     pdl_launch_dependents();
     if (p.pdl) pdl_wait();
@@ -159,13 +158,14 @@ __global__ void __launch_bounds__(kPaThreads, 3) prompt_hist_kernel(const Prompt
     if (keys_max <= 0) return;
     float *Qt = reinterpret_cast<float *>(pa_smem), *Pt = Qt;
     uint16_t *Kt = reinterpret_cast<uint16_t *>(pa_smem + kPaQBytes);
-    uint16_t *Vs = Kt;
-    float *mc = reinterpret_cast<float *>(pa_smem + kPaQBytes + kPaKBytes), *lc = mc + kAttnSub * kPaQueries;
+    uint16_t *Vs = reinterpret_cast<uint16_t *>(pa_smem + kPaQBytes + kPaKBytes);
+    float *mc = reinterpret_cast<float *>(pa_smem + kPaQBytes + kPaKBytes + kPaVBytes), *lc = mc + kAttnSub * kPaQueries;
 
-    // K two rows per lane, transposed as bf16 pairs; Q one vector per
+    // V as it is (16-byte asynchronous copies); K two rows per lane, transposed as bf16 pairs; Q one vector per
     // lane, transposed as fp32.  Consecutive lanes store consecutive words: no bank conflicts.
     const uint16_t *kg = p.k_base + ((size_t)hk * p.kv_rows + key0) * 128;
     const uint16_t *vg = p.v_base + ((size_t)hk * p.kv_rows + key0) * 128;
+    for (int i = tid; i < keys_max * 16; i += kPaThreads) cp_async16(Vs + 8 * i, reinterpret_cast<const uint4 *>(vg) + i);
     {
         // Every load is out before the first store: the compiler may not move a load over a store to shared memory, and one
         // round trip per piece cost 8000 cycles of a tile's 66000.
@@ -216,8 +216,7 @@ __global__ void __launch_bounds__(kPaThreads, 3) prompt_hist_kernel(const Prompt
         for (int d = 0; d < 128; ++d)
             pa_step(acc2, qp + d * kPaQStride, qp + d * kPaQStride + 4, *reinterpret_cast<const uint4 *>(kp + d * kPaKStride));
     }
-    __syncthreads();                                                  // Q^T and K^T are spent: P^T and V take their space
-    for (int i = tid; i < keys_max * 16; i += kPaThreads) cp_async16(Vs + 8 * i, reinterpret_cast<const uint4 *>(vg) + i);
+    __syncthreads();                                                  // Q^T is spent: its space takes P^T
     const int c = kgp >> 2;                                           // sub-chunk of this thread's keys
     if (lim >= BM_ATTN_SUPER) pa_softmax<true>(acc2, lim, kgp, c, v0, mc, lc);
     else pa_softmax<false>(acc2, lim, kgp, c, v0, mc, lc);

@@ -138,6 +138,7 @@ __device__ __forceinline__ void gemv_issue_tile(const GemvParams &p, unsigned ch
     if (lane == 0) mbar_expect_tx(bar, (uint32_t)rows * row_bytes + (uint32_t)(rows * ng * 2));
     __syncwarp();
     if (!SILU) {
+#pragma unroll 1
         for (int r = lane; r < rows; r += 32)
             bulk_g2s(stage + r * L.row_stride, p.B + (size_t)(n0 + r) * row_bytes, row_bytes, bar);
         if (lane == 0)
@@ -145,6 +146,7 @@ __device__ __forceinline__ void gemv_issue_tile(const GemvParams &p, unsigned ch
     } else {
         // paired tile: rows [0, rows/2) are gate rows n0.., rows [rows/2, rows) the up rows of the same columns
         const int half = rows >> 1;
+#pragma unroll 1
         for (int r = lane; r < rows; r += 32) {
             const size_t src = r < half ? (size_t)(n0 + r) : (size_t)(p.silu_F + n0 + r - half);
             bulk_g2s(stage + r * L.row_stride, p.B + src * row_bytes, row_bytes, bar);
@@ -207,6 +209,7 @@ __device__ __forceinline__ void gemv_store(const GemvParams &p, int m, int n, fl
         const uint16_t v = bm_f32_to_bf16(y);
         if (p.world > 1) {
             const int b = (int)((p.done[1] + 1u) & 1u);       // buffer of this call
+#pragma unroll 1
             for (int r = 0; r < p.world; ++r) p.peer_C[b][r][(size_t)m * p.ldc + n] = v;
         } else {
             reinterpret_cast<uint16_t *>(p.C)[(size_t)m * p.ldc + n] = v;
@@ -237,9 +240,11 @@ __device__ __forceinline__ void gemv_peer_finish(const GemvParams &p) {
     atomicExch(&p.done[0], 0u);
     const unsigned int epoch = p.done[1] + 1u;
     __threadfence_system();
+#pragma unroll 1
     for (int r = 0; r < p.world; ++r)
         if (r != p.rank)
             asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(p.peer_flags[r] + p.rank), "r"(epoch) : "memory");
+#pragma unroll 1
     for (int r = 0; r < p.world; ++r) {
         if (r == p.rank) continue;
         const unsigned int *flag = p.peer_flags[p.rank] + r;
@@ -424,14 +429,14 @@ __device__ __forceinline__ void gemv_stage_row_from_bf16(const GemvParams &p, un
         const uint4 wraw = reinterpret_cast<const uint4 *>(p.norm_w)[t];
         const size_t src_row = p.gather ? gather_row(p.gather[0], p.gather_rows) : 0;
         float h[8];
-        unpack8(reinterpret_cast<const uint4 *>(p.xb + src_row * p.K)[t], h);
+        uint4 hraw = reinterpret_cast<const uint4 *>(p.xb + src_row * p.K)[t];
+        unpack8(hraw, h);
         if (p.res) {
             float rr[8];
             unpack8(reinterpret_cast<const uint4 *>(p.res)[t], rr);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) h[i] = bm_bf16_rn(h[i] + rr[i]);
+            hraw = add8(h, rr);
         }
-        if (blockIdx.x == 0 && p.h_out) reinterpret_cast<uint4 *>(p.h_out)[t] = pack8(h);
+        if (blockIdx.x == 0 && p.h_out) reinterpret_cast<uint4 *>(p.h_out)[t] = hraw;
         float acc = 0.0f;
 #pragma unroll
         for (int i = 0; i < 8; ++i) acc = fmaf(h[i], h[i], acc);
@@ -439,13 +444,7 @@ __device__ __forceinline__ void gemv_stage_row_from_bf16(const GemvParams &p, un
         const float rs = bm_rsqrtf(total / (float)p.K + p.eps);
         float wv[8], n[8];
         unpack8(wraw, wv);
-        float amax = 0.0f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            n[i] = bm_bf16_rn(wv[i] * bm_bf16_rn(h[i] * rs));
-            amax = fmaxf(amax, fabsf(n[i]));
-        }
-        amax = block_max(amax, sh, lane, warp, nwarps);
+        const float amax = block_max(norm8(h, wv, rs, n), sh, lane, warp, nwarps);
         s = bm_act_scale(amax);
         emit_codes(sink, 0, p.K, t, quant8(n, s), true, lane);
     } else {
@@ -592,6 +591,7 @@ __global__ void __launch_bounds__(kGemvThreads, 2) t2_gemv_mma_kernel(const Gemv
     if (SILU && threadIdx.x < 16) amax_sh[threadIdx.x] = 0u;
 
     if (threadIdx.x == 0) {
+#pragma unroll 1
         for (int i = 0; i < p.stages; ++i) mbar_init(&bars[i], 1);
         mbar_init(&bars[kMaxStages], 1);              // activation rows (several-chunk, prepared)
         mbar_fence_init();
@@ -604,6 +604,7 @@ __global__ void __launch_bounds__(kGemvThreads, 2) t2_gemv_mma_kernel(const Gemv
     LS.row_stride = L.row_stride;
     LS.scale_off_in_stage = L.scale_off_in_stage;
     if (warp == 0) {
+#pragma unroll 1
         for (int i = 0; i < p.stages && i < my_tiles; ++i)
             gemv_issue_tile<SILU>(p, smem + L.stage_off + i * L.stage_bytes, LS, &bars[i],
                             (blockIdx.x + i * gridDim.x) * R_out, R, lane);
@@ -647,6 +648,7 @@ __global__ void __launch_bounds__(kGemvThreads, 2) t2_gemv_mma_kernel(const Gemv
                              (uint32_t)p.K, abar);
             }
             int *as = reinterpret_cast<int *>(smem + L.asum_off);
+#pragma unroll 1
             for (int b0 = 0; b0 < p.W * ng; b0 += 4 * kGemvThreads) {
                 int v[4];
 #pragma unroll
@@ -679,6 +681,7 @@ __global__ void __launch_bounds__(kGemvThreads, 2) t2_gemv_mma_kernel(const Gemv
     const int soff = L.scale_off_in_stage + (2 * q * ng + 2 * warp) * 2;
     bool failed = false;
 
+#pragma unroll 1
     for (int i = 0; i < my_tiles; ++i) {
         const int st = i % p.stages;
         const bool ok = mbar_wait_bounded(&bars[st], (uint32_t)((i / p.stages) & 1)) && a_ok;
@@ -694,6 +697,7 @@ __global__ void __launch_bounds__(kGemvThreads, 2) t2_gemv_mma_kernel(const Gemv
                 for (int e = 0; e < 4; ++e) acc[rb][sl][e] = 0.0f;
 
         if (ok) {
+#pragma unroll 1
             for (int c = 0; c < nch; ++c) {
                 const int g0 = c * BM_SLOTS + 2 * warp;
                 if (!ONECHUNK) {
@@ -741,7 +745,9 @@ __global__ void __launch_bounds__(kGemvThreads, 2) t2_gemv_mma_kernel(const Gemv
             failed = true;
             if (threadIdx.x == 0) {
                 report_error(kErrGemvWaitTimeout);
+#pragma unroll 1
                 for (int j = i; j < my_tiles && j < i + p.stages; ++j)
+#pragma unroll 1
                     for (int it = 0; it < (1 << 12); ++it)
                         if (mbar_try_wait(&bars[j % p.stages], (uint32_t)((j / p.stages) & 1))) break;
             }
@@ -758,6 +764,7 @@ __global__ void __launch_bounds__(kGemvThreads, 2) t2_gemv_mma_kernel(const Gemv
             // inner = bf16(silu(bf16 gate) * bf16 up), as the stand-alone SiLU kernel computes it from
             // the bf16 projection outputs
             // one output element per thread: the SiLU (own exp, IEEE division) is a long dependent chain
+#pragma unroll 1
             for (int o = threadIdx.x; o < p.W * (R / 2); o += kGemvThreads) {
                 const int m = o / (R / 2), c = o - m * (R / 2);
                 float vg[kGemvWarps], vu[kGemvWarps];
@@ -775,6 +782,7 @@ __global__ void __launch_bounds__(kGemvThreads, 2) t2_gemv_mma_kernel(const Gemv
             }
             continue;
         }
+#pragma unroll 1
         for (int o = threadIdx.x; o < p.W * (R / 4); o += kGemvThreads) {
             const int m = o / (R / 4), rq = o - m * (R / 4);
             float4 v[kGemvWarps];
@@ -788,10 +796,10 @@ __global__ void __launch_bounds__(kGemvThreads, 2) t2_gemv_mma_kernel(const Gemv
 #undef BM_TREE
             const size_t dst = (size_t)m * p.ldc + n0 + 4 * rq;
             if (p.out_kind == 0) {
-                const uint32_t lo = (uint32_t)bm_f32_to_bf16(y[0]) | ((uint32_t)bm_f32_to_bf16(y[1]) << 16);
-                const uint32_t hi = (uint32_t)bm_f32_to_bf16(y[2]) | ((uint32_t)bm_f32_to_bf16(y[3]) << 16);
+                const uint32_t lo = bf16_pair(y[0], y[1]), hi = bf16_pair(y[2], y[3]);
                 if (p.world > 1) {
                     const int b = (int)((p.done[1] + 1u) & 1u);   // buffer of this call
+#pragma unroll 1
                     for (int pr = 0; pr < p.world; ++pr)
                         *reinterpret_cast<uint2 *>(p.peer_C[b][pr] + dst) = make_uint2(lo, hi);
                 } else {

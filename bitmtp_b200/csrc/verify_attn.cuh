@@ -139,7 +139,13 @@ __device__ __noinline__ float4 rope_head_vector(uint2 raw, uint2 wraw, uint2 cra
                          __uint_as_float(sraw.y << 16), __uint_as_float(sraw.y & 0xffff0000u)};
     float n[4], o[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) n[i] = bm_bf16_rn(wv[i] * bm_bf16_rn(x[i] * r));
+    for (int i = 0; i < 4; i += 2) {
+        float a = x[i] * r, b = x[i + 1] * r;
+        bf16_round_pair(a, b);
+        n[i] = wv[i] * a;
+        n[i + 1] = wv[i + 1] * b;
+        bf16_round_pair(n[i], n[i + 1]);
+    }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const float partner = __shfl_xor_sync(0xffffffffu, n[i], 16);
@@ -385,8 +391,7 @@ __device__ __forceinline__ void attn_merge_vector(const float *pm, const float *
     for (int e = 0; e < 4; ++e) v[e] = bm_bf16_rn(o[e] / l);
 }
 __device__ __forceinline__ uint2 attn_pack_row(const float (&v)[4]) {
-    return make_uint2((uint32_t)bm_f32_to_bf16(v[0]) | ((uint32_t)bm_f32_to_bf16(v[1]) << 16),
-                      (uint32_t)bm_f32_to_bf16(v[2]) | ((uint32_t)bm_f32_to_bf16(v[3]) << 16));
+    return make_uint2(bf16_pair(v[0], v[1]), bf16_pair(v[2], v[3]));
 }
 __device__ __forceinline__ float attn_row_amax(const float (&v)[4]) {
     return warp_max(fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))));
@@ -773,9 +778,7 @@ __global__ void __launch_bounds__(1024) attn_merge_quant_kernel(const AttnMergeP
     if (lane == 0) sh[head] = amax != 0.0f ? __float_as_uint(amax) : 0u;
     __syncthreads();
     const float s = bm_act_scale(__uint_as_float(__reduce_max_sync(0xffffffffu, lane < p.H ? sh[lane] : 0u)));
-    uint32_t codes = 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) codes |= ((uint32_t)(bm_quant_i8(v[i], s) & 0xff)) << (8 * i);
+    const uint32_t codes = quant_quad(v[0], v[1], v[2], v[3], s);
     if (p.q.nat) reinterpret_cast<uint32_t *>(p.q.nat + at)[lane] = codes;
     if (p.q.prep) {
         // GEMV-ready order: the 4 x 4 bytes of four consecutive lanes transposed in two exchanges

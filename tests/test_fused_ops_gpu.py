@@ -596,3 +596,36 @@ def test_commit_and_stage_draft_in_one_launch(M, D, n_commit, verified, cache_le
     pend_c = torch.full((18,), -2, dtype=torch.int64, device=DEV)
     ops.commit_stage_draft(src, n_commit, verified, gen_c[5:], pend_c)
     assert torch.equal(gen_c, gen_a) and torch.equal(pend_c, pend_a)
+
+
+@pytest.mark.parametrize("K", [256, 2048])
+def test_quantisation_of_rows_with_infinities_nans_and_extremes(K):
+    """Codes and multipliers of rows that hold infinities, NaNs, the largest and the smallest bf16 values, against the
+    definition evaluated by numpy: round half to even of x * s, clamped to [-128, 127], 0 for a NaN; a NaN does not count
+    for the row's absmax."""
+    rng = np.random.default_rng(K)
+    rows = rng.standard_normal((9, K)).astype(np.float32)
+    rows[1, 5] = np.inf
+    rows[2, 7], rows[2, 8] = -np.inf, np.nan
+    rows[3, ::3] = np.nan
+    rows[4] = np.nan
+    rows[5] = 0.0
+    rows[6, 1], rows[6, 2] = 3.3895e38, -3.3895e38
+    rows[7] = rows[7] * np.float32(1e-39)
+    rows[8, :4] = (127.5, -127.5, 63.5, -0.5)              # with an absmax of 127 * 2: ties at half
+    rows[8, 4:] = 254.0
+    x = torch.from_numpy(rows).to(torch.bfloat16).to(DEV)
+    q, s = ops.quant_rows(x)
+    qp, asum, sp = ops.quant_rows(x, prepared=True)
+    xf = x.float().cpu().numpy()
+    with np.errstate(all="ignore"):
+        absmax = np.nan_to_num(np.fmax.reduce(np.abs(xf), axis=1, initial=0.0), nan=0.0, posinf=np.inf).astype(np.float32)
+        s_ref = (np.float32(1.0) / np.where(absmax < np.float32(1e-5), np.float32(1e-5), absmax)) * np.float32(127.0)
+        prod = np.rint(xf * s_ref[:, None].astype(np.float32))
+        want = np.where(np.isnan(prod), 0.0, np.clip(prod, -128, 127)).astype(np.int8)
+    assert np.array_equal(s.cpu().numpy().reshape(-1).view(np.uint32), s_ref.astype(np.float32).view(np.uint32))
+    assert np.array_equal(q.cpu().numpy(), want)
+    perm = np.array([4 * (k & 3) + (k >> 2) for k in range(16)])
+    back = qp.cpu().numpy().reshape(9, K // 16, 16)[:, :, perm].reshape(9, K)
+    assert np.array_equal(back, want)
+    assert np.array_equal(asum.cpu().numpy(), want.astype(np.int32).reshape(9, K // 128, 128).sum(-1))
