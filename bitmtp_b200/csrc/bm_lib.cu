@@ -755,12 +755,13 @@ int bm_t2_gemv_row_fused(int src_mode, const void *x, const void *gather, int ga
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // A few MB of weights: the register-only kernel (one memory round trip after the row is staged).
     if (!staged && bm::direct_row_fits(N, K) && (size_t)(silu ? 2 : 1) * N * K / 4 <= kDirectMaxBytes) {
-        const dim3 grid((unsigned)(N / bm::kDirectWarps)), block(bm::kGemvThreads);
-        const int maxp = K <= 2048 ? 1 : (K <= 6144 ? 3 : 5);
-#define BM_ROW_CASE(S_, MP_) \
-        if (silu == S_ && maxp == MP_) return launch_ex(bm::t2_gemv_direct_row_kernel<S_, MP_>, grid, block, 0, st, pdl, p);
-        BM_ROW_CASE(false, 1) BM_ROW_CASE(false, 3) BM_ROW_CASE(false, 5)
-        BM_ROW_CASE(true, 1) BM_ROW_CASE(true, 3) BM_ROW_CASE(true, 5)
+        const int maxp = K <= 2048 ? 1 : (K <= 6144 ? 3 : 5), cols = bm::direct_row_cols(N, K, sms);
+        const dim3 grid((unsigned)((N + cols * bm::kDirectWarps - 1) / (cols * bm::kDirectWarps))), block(bm::kGemvThreads);
+#define BM_ROW_CASE(S_, MP_, C_)                                                                                        \
+        if (silu == S_ && maxp == MP_ && cols == C_)                                                                    \
+            return launch_ex(bm::t2_gemv_direct_row_kernel<S_, MP_, C_>, grid, block, 0, st, pdl, p);
+        BM_ROW_CASE(false, 1, 1) BM_ROW_CASE(false, 1, 2) BM_ROW_CASE(false, 1, 3) BM_ROW_CASE(false, 3, 1) BM_ROW_CASE(false, 5, 1)
+        BM_ROW_CASE(true, 1, 1) BM_ROW_CASE(true, 1, 2) BM_ROW_CASE(true, 1, 3) BM_ROW_CASE(true, 3, 1) BM_ROW_CASE(true, 5, 1)
 #undef BM_ROW_CASE
     }
     const bool one = K == 2048;

@@ -199,6 +199,11 @@ __global__ void __launch_bounds__(kDirectWarps * 32) t2_gemv_direct_kernel(const
 // rows (B holds silu_F gate rows, then silu_F up rows) and stores bf16(silu(bf16 gate) * bf16 up); the
 // row's max |output| goes to p.amax_out by atomic max.  Weight rows are requested before the wait on
 // the previous kernel.  Same results as t2_gemv_mma_kernel with src_mode != 0, bit for bit.
+//
+// What bounds it is the row's preparation, which every CTA repeats: some 600 instructions in each of its 8 warps.  So a warp
+// computes COLS columns, as many as leave two CTAs per SM (direct_row_cols): with one column and five CTAs per SM the
+// preparation alone was 3 us of a gate|up launch (6144 columns), and 28 of its 768 CTAs were a wave of their own.  In a
+// width-1 replay gate|up takes 6.4 us with one column, 4.7 with three; the whole replay 686 us, now 645.
 constexpr int kDirectRowAsumOff = 2048 * kDirectMaxPasses;                 // int32 [K/128]
 constexpr int kDirectRowInvsOff = kDirectRowAsumOff + 4 * 16 * kDirectMaxPasses;   // float [16]
 constexpr int kDirectRowShOff = kDirectRowInvsOff + 64;                    // float [32]
@@ -208,13 +213,20 @@ __host__ __device__ inline bool direct_row_fits(int N, int K) {
     return K >= 256 && (K % 256) == 0 && K <= 2048 * kDirectMaxPasses && N >= 8 && (N % 8) == 0;
 }
 
-template <bool SILU, int MAXP>
+// Columns per warp for N output columns: more than one only where a row's weights are one pass (K <= 2048), whose registers
+// leave room for them.
+__host__ __device__ inline int direct_row_cols(int N, int K, int sms) {
+    const int c = K <= 2048 ? (N + 16 * sms - 1) / (16 * sms) : 1;
+    return c < 1 ? 1 : (c > 3 ? 3 : c);
+}
+
+template <bool SILU, int MAXP, int COLS>
 __global__ void __launch_bounds__(kGemvThreads) t2_gemv_direct_row_kernel(const GemvParams p) {
     __shared__ __align__(16) unsigned char smem[kDirectRowSmem];
     __shared__ unsigned int amax_sh;
-    constexpr int NR = SILU ? 2 : 1;                    // weight rows per output column
+    constexpr int NR = (SILU ? 2 : 1) * COLS;           // weight rows of this warp: COLS columns, then their up rows
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int n = blockIdx.x * kDirectWarps + warp;     // output column; N % 8 == 0, so every warp has one
+    const int n = (blockIdx.x * kDirectWarps + warp) * COLS;     // first output column; columns past N are not stored
     const int ng = p.K >> 7;
     const int passes = (p.K + 2047) >> 11;
     pdl_launch_dependents();
@@ -224,7 +236,7 @@ __global__ void __launch_bounds__(kGemvThreads) t2_gemv_direct_row_kernel(const 
     float sc[NR][MAXP][4];
 #pragma unroll
     for (int r = 0; r < NR; ++r) {
-        const size_t row = (size_t)n + (size_t)r * p.silu_F;
+        const size_t row = (size_t)min(n + r % COLS, p.N - 1) + (size_t)(r / COLS) * p.silu_F;
         const uint32_t *wrow = reinterpret_cast<const uint32_t *>(p.B + row * (p.K >> 2));
 #pragma unroll
         for (int ps = 0; ps < MAXP; ++ps)
@@ -272,16 +284,26 @@ __global__ void __launch_bounds__(kGemvThreads) t2_gemv_direct_row_kernel(const 
     float y[NR];
 #pragma unroll
     for (int r = 0; r < NR; ++r) y[r] = direct_slot_tree(acc[r]) * inv_s;
+    // the tree leaves every sum in all lanes: lane c stores column c
+    if (COLS > 1) {
+#pragma unroll
+        for (int c = 1; c < COLS; ++c)
+            if (lane == c) {
+                y[0] = y[c];
+                if (SILU) y[COLS] = y[COLS + c];
+            }
+    }
+    const bool stores = lane < COLS && n + lane < p.N;
     if (SILU) {
-        if (lane == 0) {
-            const float v = bm_bf16_rn(bm_silu_bf16(bm_bf16_rn(y[0])) * bm_bf16_rn(y[NR - 1]));
-            reinterpret_cast<uint16_t *>(p.C)[n] = bm_f32_to_bf16(v);
+        if (stores) {
+            const float v = bm_bf16_rn(bm_silu_bf16(bm_bf16_rn(y[0])) * bm_bf16_rn(y[NR / 2]));
+            reinterpret_cast<uint16_t *>(p.C)[n + lane] = bm_f32_to_bf16(v);
             atomicMax(&amax_sh, __float_as_uint(fabsf(v)));
         }
         __syncthreads();
         if (threadIdx.x == 0 && amax_sh != 0u) atomicMax(&p.amax_out[0], amax_sh);
-    } else if (lane == 0) {
-        gemv_store(p, 0, n, y[0]);
+    } else if (stores) {
+        gemv_store(p, 0, n + lane, y[0]);
     }
 }
 

@@ -492,7 +492,9 @@ def test_stage_replay_inputs_matches_the_tensor_fills(M, D, n_pend, cache_len):
 
 
 ROW_FUSED = [(1, 2048, 2048, False), (1, 2048, 6144, False), (1, 2560, 9728, False), (1, 1024, 2560, False),
-             (2, 4096, 2048, False), (2, 2048, 2048, False), (2, 6144, 2048, True), (2, 512, 2048, True)]
+             (2, 4096, 2048, False), (2, 2048, 2048, False), (2, 6144, 2048, True), (2, 512, 2048, True),
+             # two and three columns per warp, the last CTA with fewer; the last size with one
+             (2, 2376, 2048, False), (1, 2376, 1024, False), (2, 4768, 2048, True), (1, 7112, 2048, False), (2, 2368, 2048, True)]
 
 
 @pytest.mark.parametrize("src_mode,N,K,silu", ROW_FUSED)
