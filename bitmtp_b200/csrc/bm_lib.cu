@@ -1257,8 +1257,8 @@ int bm_prompt_attention(const void *q, const void *k_base, const void *v_base, i
             const int rc = launch_ex(bm::prompt_hist_kernel, hgrid, dim3(bm::kPaThreads), bm::kPaSmem, st, p.pdl, hp);
             if (rc != BM_OK) return rc;
         }
-        return launch_ex(bm::attn_fused_kernel<2, false, bm::kMergeHistory>, dim3(pl.n_slabs, Hkv, pl.Z), dim3(bm::kAttnThreads), smem,
-                         st, p.pdl, p);
+        return launch_ex(bm::attn_fused_kernel<2, false, bm::kMergeHistory>, dim3(pl.n_slabs, Hkv, pl.Z), dim3(bm::kAttnThreads),
+                         bm::attn_smem_bytes(pl.nv, true), st, p.pdl, p);
     }
     const dim3 grid(pl.units, Hkv, pl.Z);
     return pl.nv == 1 ? launch_ex(bm::attn_fused_kernel<1, false>, grid, dim3(bm::kAttnThreads), smem, st, p.pdl, p)

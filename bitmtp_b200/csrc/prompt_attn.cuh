@@ -15,8 +15,11 @@
 // cores would not give that order.  512 rows behind 2048 keys, 16 heads: 657 us by attn_fused_kernel alone; called from
 // the host 414 us with scalar fmas and 356 with packed ones and an exponential without branches and conversions; 339 in
 // a captured chain, 310 with every load of a tile out at once and the softmax on pairs too.  The fmas alone are 134 us at
-// the fp32 rate.  Of a tile's 66000 cycles the load took 8000, the scores 19000, the softmax 16000 and the numerators
-// 21000: what is left is latency with two warps per scheduler, and nothing is loaded under the multiply.
+// the fp32 rate.  Of a tile's 66000 cycles then the load took 8000, the scores 19000, the softmax 16000 and the numerators
+// 21000: what is left is latency with two warps per scheduler, and nothing is loaded under the multiply.  Later: the merge
+// weights of a vector made by one thread, not by each of its 16, and a slab kernel that stages 16 keys: 512 rows behind 2400
+// keys 359 -> 327.  Three CTAs per SM (V over K^T, 168 registers) gave 330 there and lost 8 to 14 us a call where the tiles are
+// few; 256 threads with 8 x 4 outputs each were level (their loads from shared memory then bind).
 #pragma once
 
 #include "verify_attn.cuh"

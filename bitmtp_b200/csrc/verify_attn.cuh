@@ -104,11 +104,17 @@ inline bool attn_fill_pick(uint8_t *pick, int NJ, int QV, int Hkv, int sms) {
 }
 
 // K (padded rows; after level 0 its space takes the sub-chunk numerators), V, queries, weights, sub-chunk max / sum.
-__host__ __device__ inline size_t attn_smem_bytes(int nv) {
+// `slab`: kMergeHistory, whose own rows are one sub-chunk (the K rows' space is then that of the numerators).
+__host__ __device__ constexpr int attn_key_bytes(int nv, bool slab) {
+    return slab ? kAttnSub * 4 * nv * 128 * 4 : BM_ATTN_SUPER * kKeyStride * 2;
+}
+__host__ __device__ constexpr int attn_value_bytes(bool slab) { return (slab ? BM_ATTN_CHUNK : BM_ATTN_SUPER) * 128 * 2; }
+__host__ __device__ inline size_t attn_smem_bytes(int nv, bool slab = false) {
     const size_t QC = 4 * (size_t)nv;
-    return (size_t)BM_ATTN_SUPER * kKeyStride * 2 + (size_t)BM_ATTN_SUPER * 128 * 2 + QC * kKeyStride * 2 +
+    return (size_t)attn_key_bytes(nv, slab) + attn_value_bytes(slab) + QC * kKeyStride * 2 +
            (size_t)kAttnWarps * BM_ATTN_CHUNK * kWeightStride * 4 + (size_t)kAttnSub * QC * 2 * 4;
 }
+static_assert(BM_ATTN_CHUNK * kKeyStride * 2 <= attn_key_bytes(2, true), "a slab's K rows fit");
 static_assert(kAttnSub * 4 * kAttnMaxNV * 128 * 4 <= BM_ATTN_SUPER * kKeyStride * 2, "sub-chunk numerators fit the K rows");
 
 // History length of this replay.  The record is written by other launches (or by the caller through
@@ -408,7 +414,7 @@ __device__ __forceinline__ float attn_row_amax(const float (&v)[4]) {
 //   kMergeHistory  prompt mode only: prompt_hist_kernel has made the partials of the history super-chunks.  blockIdx.x is
 //                  the slab; its CTAs make the partial of the slab's own rows, keep it in registers and merge at once.  A
 //                  build of its own: as a run-time switch it made every other prompt-mode call 3.6 % slower (1 to 9 % over
-//                  117 calls of 17 to 512 rows).
+//                  117 calls of 17 to 512 rows).  It stages 16 keys, not 128, so four CTAs share an SM (512 rows of 16 heads: 70.5 us a call without history, now 62.3).
 //   kMergeLater    the next launch (attn_merge_quant_kernel): this one ends with its partials.  A replay wants the rows as
 //                  INT8 codes, for which a launch has to follow anyway; the end of a launch is then the only hand-over
 //                  (fence, ticket, read-back and row-absmax atomics took 3.4 us of 12.4 at width 16).
@@ -422,7 +428,7 @@ enum : int { kMergeTicket = 0, kMergeCluster = 1, kMergeHistory = 2, kMergeLater
 // work are the first in y, so that working CTAs are spread over the SMs and the rest leave; clusters and prompt mode
 // (super-chunks or (slab, super-chunk) pairs, Hkv, query groups).
 template <int NV, bool ROPE, int MERGE = kMergeTicket>
-__global__ void __launch_bounds__(kAttnThreads, 2) attn_fused_kernel(const __grid_constant__ AttnParams p) {
+__global__ void __launch_bounds__(kAttnThreads, MERGE == kMergeHistory ? 4 : 2) attn_fused_kernel(const __grid_constant__ AttnParams p) {
     extern __shared__ __align__(16) unsigned char dyn[];
     __shared__ unsigned int sh_ticket;
     constexpr int QC = 4 * NV, NQW = (QC + kAttnWarps - 1) / kAttnWarps;      // vectors per CTA; per warp outside level 0
@@ -497,8 +503,8 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_fused_kernel(const __gri
 
     uint16_t *Ks = reinterpret_cast<uint16_t *>(dyn);                              // [128][136]
     float *oc = reinterpret_cast<float *>(dyn);                                    // [4][QC][128], over the K rows
-    uint16_t *Vs = Ks + BM_ATTN_SUPER * kKeyStride;                                 // [128][128]
-    uint16_t *Qs = Vs + BM_ATTN_SUPER * 128;                                        // [QC][136]
+    uint16_t *Vs = Ks + attn_key_bytes(NV, HIST_DONE) / 2;                          // [128][128], a slab's [32][128]
+    uint16_t *Qs = Vs + attn_value_bytes(HIST_DONE) / 2;                            // [QC][136]
     float *Ps = reinterpret_cast<float *>(Qs + QC * kKeyStride);                    // [8 warps][32 keys][8]
     float *mc = Ps + kAttnWarps * BM_ATTN_CHUNK * kWeightStride;                    // [4][QC]
     float *lc = mc + kAttnSub * QC;                                                 // [4][QC]
