@@ -172,8 +172,8 @@ __device__ __forceinline__ PaPair pa_pack(float lo, float hi) {
 __device__ __forceinline__ void pa_unpack(PaPair v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
 // bm_expf for x <= 0, infinities or NaN, without its branches and the two conversions that issue at a quarter of the
 // rate; the same values: adding 1.5 * 2^23 rounds |t| < 2^22 to the nearest even integer and leaves it in the low bits,
-// and the exponent, -126 .. 0, goes in with one exact step.  Kept here: in the decode kernels, which evaluate a few per
-// thread, the branch is cheaper (whole requests 0.7 % slower without it).
+// and the exponent, -126 .. 0, goes in with one exact step.  For the attention, whose
+// arguments are differences from a maximum.
 __device__ __forceinline__ float pa_expf(float x) {
     const float biased = x * 1.44269504088896341f + 12582912.0f;
     const float n = biased - 12582912.0f;
@@ -365,8 +365,8 @@ __device__ __forceinline__ void attn_merge_vector(const float *pm, const float *
         l1 = __ldcg(pl + pb + j);
     }
     const float gmax = warp_max(fmaxf(m0, m1));
-    const float w0 = m0 > -INFINITY ? bm_expf(m0 - gmax) : 0.0f;
-    const float w1 = m1 > -INFINITY ? bm_expf(m1 - gmax) : 0.0f;
+    const float w0 = m0 > -INFINITY ? pa_expf(m0 - gmax) : 0.0f;
+    const float w1 = m1 > -INFINITY ? pa_expf(m1 - gmax) : 0.0f;
     float l = 0.0f, o[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     for (int b0 = 0; b0 < nv; b0 += kBatch) {
         if (b0 > 0) {
@@ -649,7 +649,7 @@ __global__ void __launch_bounds__(kAttnThreads, MERGE == kMergeHistory ? 4 : 2) 
         for (int c = 0; c < kAttnSub; ++c) { mm[c] = mc[c * QC + qi]; MJ[k] = fmaxf(MJ[k], mm[c]); }
 #pragma unroll
         for (int c = 0; c < kAttnSub; ++c) {
-            const float w = mm[c] > -INFINITY ? bm_expf(mm[c] - MJ[k]) : 0.0f;
+            const float w = mm[c] > -INFINITY ? pa_expf(mm[c] - MJ[k]) : 0.0f;
             L[k] = fmaf(lc[c * QC + qi], w, L[k]);
             const float4 o = *reinterpret_cast<const float4 *>(oc + ((size_t)c * QC + qi) * 128 + 4 * lane);
             O[k][0] = fmaf(o.x, w, O[k][0]);
@@ -691,7 +691,7 @@ __global__ void __launch_bounds__(kAttnThreads, MERGE == kMergeHistory ? 4 : 2) 
                               : i == n_hs ? *reinterpret_cast<const float4 *>(own_o)
                                           : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                 const float gmax = warp_max(ml.x);
-                const float w0 = ml.x > -INFINITY ? bm_expf(ml.x - gmax) : 0.0f;
+                const float w0 = ml.x > -INFINITY ? pa_expf(ml.x - gmax) : 0.0f;
                 float l = 0.0f, o[4] = {0.0f, 0.0f, 0.0f, 0.0f};
                 for (int b0 = 0; b0 < np; b0 += kBatch) {
                     if (b0 > 0) {
