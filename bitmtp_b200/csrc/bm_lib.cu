@@ -860,7 +860,8 @@ struct RopeInputs {
 // Launch of the cluster build of the attention kernel: the grid's x extent is one thread-block cluster.
 // Returns -1 (and launches nothing) unless the device holds all of the grid's clusters at once - a
 // cluster that has to wait for a place costs more than the shorter merge saves - so that the caller takes
-// the ticket build; the device is asked once per kernel, cluster size and device.
+// the ticket build; the device is asked once per kernel, cluster size and device, so `smem` is the kernel's own, the same in
+// every call.
 template <void (*kernel)(const bm::AttnParams)>
 int launch_attention_cluster(dim3 grid, size_t smem, cudaStream_t st, int pdl, const bm::AttnParams &p) {
     static std::atomic<int> resident[bm::kAttnMaxCluster + 1][8];    // clusters the device holds, +1 (0: not asked yet)
@@ -997,7 +998,7 @@ int verify_attention_impl(const void *q, const RopeInputs *rope, const void *k_b
         p.v_out = const_cast<uint16_t *>(p.v_base);
         p.eps = rope->eps;
         rc = later ? launch_attention<true, bm::kMergeLater>(nv, grid, smem, st, attn_pdl, p)
-                   : launch_attention_clusters(nv, dim3(NJ, Hkv, Z), smem, st, attn_pdl, p);
+                   : launch_attention_clusters(nv, dim3(NJ, Hkv, Z), bm::attn_smem_bytes(nv), st, attn_pdl, p);
         if (rc < 0) rc = launch_attention<true, bm::kMergeTicket>(nv, grid, smem, st, attn_pdl, p);
     } else {
         rc = later ? launch_attention<false, bm::kMergeLater>(nv, grid, smem, st, attn_pdl, p)

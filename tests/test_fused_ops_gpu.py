@@ -444,6 +444,31 @@ def test_attention_codes_equal_rows_then_quantisation(oracle, M, H, Hkv, sigma, 
         assert torch.equal(ka.view(torch.int16), kb.view(torch.int16)) and torch.equal(va.view(torch.int16), vb.view(torch.int16))
 
 
+def test_cluster_merge_for_several_head_counts_in_one_process(oracle):
+    """The cluster build is asked about once per cluster size: calls whose grids differ (more heads than SMs take one by one,
+    then fewer, and back) share that answer and all run.  Rows equal those of the launch that merges later."""
+    M, sigma, cache_len = 1, 1152, 1000
+    cos, sin = (oracle.u16_to_torch(t).to(DEV) for t in _rope_tables(oracle, sigma + 40))
+    pos = torch.tensor([cache_len], dtype=torch.int64, device=DEV)
+    for H, Hkv in ((32, 16), (16, 8), (32, 16), (4, 2)):
+        gen = torch.Generator().manual_seed(H)
+        xqkv = _bf16(gen, M, (H + 2 * Hkv) * 128, scale=2.0).to(DEV)
+        w = (1.0 + 0.1 * torch.randn(128, generator=gen)).to(torch.bfloat16).to(DEV)
+        kv = _bf16(gen, 2, Hkv, sigma + M, 128, scale=1.5).to(DEV)
+        state = ops.new_step_state(DEV)
+        ops.set_step_state(state, cache_len, 0, oracle.ROLE_IDS["ar"], 0)
+        scratch = ops.attention_scratch(M, H, sigma, DEV)
+        att_a, att_b = (torch.empty(M, H * 128, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+        amax = torch.zeros(M, dtype=torch.int32, device=DEV)
+        ops.rope_verify_attention_rows(xqkv, w, w, 1e-6, cos, sin, pos, H, Hkv, kv[0].clone(), kv[1].clone(), sigma, state, scratch,
+                                       att=att_a, amax=amax)
+        q, s = torch.empty(M, H * 128, dtype=torch.int8, device=DEV), torch.empty(M, 1, dtype=torch.float32, device=DEV)
+        ops.rope_verify_attention(xqkv, w, w, 1e-6, cos, sin, pos, H, Hkv, kv[0].clone(), kv[1].clone(), sigma, state, scratch,
+                                  out=(att_b, q, s))
+        torch.cuda.synchronize()
+        assert torch.equal(att_a.view(torch.int16), att_b.view(torch.int16)), (H, Hkv)
+
+
 @pytest.mark.parametrize("M,D,n_pend,cache_len", [(9, 8, 1, 40), (10, 8, 2, 7), (12, 8, 3, 100), (16, 8, 8, 300),
                                                   (17, 8, 9, 12), (16, 8, 5, 1), (5, 4, 1, 9), (9, 4, 5, 64)])
 def test_stage_replay_inputs_matches_the_tensor_fills(M, D, n_pend, cache_len):
