@@ -53,12 +53,28 @@ inline int cuda_status(cudaError_t e) { return e == cudaSuccess ? BM_OK : BM_ECU
 std::atomic<unsigned long long> g_launches{0};
 inline void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 
+// Dynamic shared memory that a kernel may be launched with: all that its own variables leave.  The limit is an attribute of the
+// kernel, not of a launch, so it is never set to what one call needs: a call with less in another thread, between this one's
+// setting and its launch, would have this launch refused.
+template <auto kernel>
+cudaError_t allow_smem() {
+    static std::atomic<int> most{0};
+    int n = most.load(std::memory_order_relaxed);
+    if (n == 0) {
+        cudaFuncAttributes a;
+        const cudaError_t e = cudaFuncGetAttributes(&a, kernel);
+        if (e != cudaSuccess) return e;
+        n = kMaxSmemPerCta - (int)a.sharedSizeBytes;
+        most.store(n, std::memory_order_relaxed);
+    }
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, n);
+}
+
 // Generic launch with the optional programmatic-serialisation attribute.
-template <typename Kernel, typename... Args>
-int launch_ex(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int pdl,
-              Args... args) {
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+template <auto kernel, typename... Args>
+int launch_ex(dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int pdl, Args... args) {
+    if (smem > 32 * 1024) {                   // (48 KB, the kernel's own variables included, go without asking)
+        const cudaError_t e = allow_smem<kernel>();
         if (e != cudaSuccess) return cuda_status(e);
     }
     cudaLaunchConfig_t cfg = {};
@@ -73,25 +89,6 @@ int launch_ex(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t st
     cfg.numAttrs = pdl ? 1 : 0;
     count_launch();
     return cuda_status(cudaLaunchKernelEx(&cfg, kernel, args...));
-}
-
-template <typename Kernel>
-int launch(Kernel kernel, int grid, int block, int smem, cudaStream_t stream, int pdl,
-           const bm::GemvParams &p) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return cuda_status(e);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid, 1, 1);
-    cfg.blockDim = dim3((unsigned)block, 1, 1);
-    cfg.dynamicSmemBytes = (size_t)smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    count_launch();
-    return cuda_status(cudaLaunchKernelEx(&cfg, kernel, p));
 }
 
 // Rows per tile: the largest of 32/16/8 that still leaves two tiles per SM, so
@@ -141,8 +138,7 @@ int gemv_launch_dp4a(const bm::GemvParams &p0, int sms, int pdl, cudaStream_t st
     const int wb = p.W == 1 ? 1 : (p.W == 2 ? 2 : 4);
 #define BM_DP4A_CASE(WB_, RB_)                                                               \
     if (wb == WB_ && pl.rb == RB_)                                                           \
-        return launch(bm::t2_gemv_dp4a_kernel<WB_, RB_>, pl.grid, bm::kGemvThreads, pl.smem, \
-                      stream, pdl, p);
+        return launch_ex<bm::t2_gemv_dp4a_kernel<WB_, RB_>>(dim3(pl.grid), dim3(bm::kGemvThreads), pl.smem, stream, pdl, p);
     BM_DP4A_CASE(1, 1) BM_DP4A_CASE(1, 2) BM_DP4A_CASE(1, 4)
     BM_DP4A_CASE(2, 1) BM_DP4A_CASE(2, 2) BM_DP4A_CASE(2, 4)
     BM_DP4A_CASE(4, 1) BM_DP4A_CASE(4, 2) BM_DP4A_CASE(4, 4)
@@ -160,7 +156,7 @@ int gemv_launch_direct(const bm::GemvParams &p0, int pdl, cudaStream_t stream) {
     const int maxp = p.K <= 2048 ? 1 : (p.K <= 6144 ? 3 : 5);
     const int wt = p.W == 1 ? 1 : (p.W == 2 ? 2 : 4);
 #define BM_DIRECT_CASE(WT_, MP_) \
-    if (wt == WT_ && maxp == MP_) return launch_ex(bm::t2_gemv_direct_kernel<WT_, MP_>, grid, block, 0, stream, pdl, p);
+    if (wt == WT_ && maxp == MP_) return launch_ex<bm::t2_gemv_direct_kernel<WT_, MP_>>(grid, block, 0, stream, pdl, p);
     BM_DIRECT_CASE(1, 1) BM_DIRECT_CASE(1, 3) BM_DIRECT_CASE(1, 5)
     BM_DIRECT_CASE(2, 1) BM_DIRECT_CASE(2, 3) BM_DIRECT_CASE(2, 5)
     BM_DIRECT_CASE(4, 1) BM_DIRECT_CASE(4, 3) BM_DIRECT_CASE(4, 5)
@@ -231,8 +227,8 @@ bool make_mma_plan(int N, int K, bool half, int sms, int force_rb, MmaPlan *out)
 
 template <int RB, bool HALF, bool ONECHUNK, bool EMIT_G, int SRC, bool SILU>
 int launch_mma_inst(const MmaPlan &pl, cudaStream_t stream, int pdl, const bm::GemvParams &p) {
-    return launch(bm::t2_gemv_mma_kernel<RB, HALF, ONECHUNK, EMIT_G, SRC, SILU>, pl.grid, bm::kGemvThreads, pl.smem, stream,
-                  pdl, p);
+    return launch_ex<bm::t2_gemv_mma_kernel<RB, HALF, ONECHUNK, EMIT_G, SRC, SILU>>(dim3(pl.grid), dim3(bm::kGemvThreads), pl.smem,
+                                                                                    stream, pdl, p);
 }
 
 template <bool HALF, bool ONECHUNK, int SRC, bool SILU>
@@ -383,8 +379,8 @@ int launch_rowwarp(const bm::RowWarpParams &P, int warps, int sms, int pdl, cuda
     if (grid > sms) grid = sms;
     const size_t smem = (size_t)L.total + 1024;
     if (P.g.G != nullptr)
-        return launch_ex(bm::t2_gemv_rowwarp_kernel<NTOK, PB, true, KS>, dim3(grid), dim3(warps * 32), smem, stream, pdl, P);
-    return launch_ex(bm::t2_gemv_rowwarp_kernel<NTOK, PB, false, KS>, dim3(grid), dim3(warps * 32), smem, stream, pdl, P);
+        return launch_ex<bm::t2_gemv_rowwarp_kernel<NTOK, PB, true, KS>>(dim3(grid), dim3(warps * 32), smem, stream, pdl, P);
+    return launch_ex<bm::t2_gemv_rowwarp_kernel<NTOK, PB, false, KS>>(dim3(grid), dim3(warps * 32), smem, stream, pdl, P);
 }
 
 int gemv_launch_rowwarp(const bm::GemvParams &p0, int sms, int pdl, cudaStream_t stream) {
@@ -437,8 +433,8 @@ int launch_tc(bm::TcParams &p, const void *A, const void *B, cudaStream_t stream
     p.tiles = (int)tiles;
     const int resident = sms * (NT == 32 ? 2 : 1), grid = p.tiles < resident ? p.tiles : resident;
     const dim3 block(bm::tc_threads(NT));
-    if (p.K == BM_SLOTS * BM_GROUP) return launch_ex(bm::t2_gemm_tc_kernel<NT, true>, dim3(grid), block, bm::tc_smem_bytes(NT), stream, p.pdl, p);
-    return launch_ex(bm::t2_gemm_tc_kernel<NT, false>, dim3(grid), block, bm::tc_smem_bytes(NT), stream, p.pdl, p);
+    if (p.K == BM_SLOTS * BM_GROUP) return launch_ex<bm::t2_gemm_tc_kernel<NT, true>>(dim3(grid), block, bm::tc_smem_bytes(NT), stream, p.pdl, p);
+    return launch_ex<bm::t2_gemm_tc_kernel<NT, false>>(dim3(grid), block, bm::tc_smem_bytes(NT), stream, p.pdl, p);
 }
 
 }  // namespace
@@ -592,7 +588,7 @@ int bm_quant_rows(const void *x, int M, int K, void *q, void *q_prep, void *asum
     if ((q_prep == nullptr) != (asum == nullptr) || (q_prep && (K % BM_GROUP) != 0)) return BM_EINVAL;
     if ((reinterpret_cast<uintptr_t>(q) & 7u) || (reinterpret_cast<uintptr_t>(q_prep) & 7u)) return BM_EINVAL;
     bm::QuantSink sink{static_cast<int8_t *>(q), static_cast<int8_t *>(q_prep), static_cast<int32_t *>(asum)};
-    return launch_ex(bm::quant_rows_kernel, dim3(M), dim3(bm::kRowThreads), 0, static_cast<cudaStream_t>(stream), pdl,
+    return launch_ex<bm::quant_rows_kernel>(dim3(M), dim3(bm::kRowThreads), 0, static_cast<cudaStream_t>(stream), pdl,
                      static_cast<const uint16_t *>(x), K, sink, static_cast<float *>(s), pdl);
 }
 
@@ -618,7 +614,7 @@ int bm_rmsnorm_fused(const void *x, const void *gather, int gather_rows, const v
     p.dim = dim;
     p.row0 = row0;
     p.pdl = pdl;
-    return launch_ex(bm::rmsnorm_kernel, dim3(M), dim3(dim / 8), 0, static_cast<cudaStream_t>(stream), pdl, p);
+    return launch_ex<bm::rmsnorm_kernel>(dim3(M), dim3(dim / 8), 0, static_cast<cudaStream_t>(stream), pdl, p);
 }
 
 int bm_t2_gemv_gate_up_silu(const void *A_prep, const void *a_sums, const void *B, const void *ws, const void *s, int W,
@@ -759,7 +755,7 @@ int bm_t2_gemv_row_fused(int src_mode, const void *x, const void *gather, int ga
         const dim3 grid((unsigned)((N + cols * bm::kDirectWarps - 1) / (cols * bm::kDirectWarps))), block(bm::kGemvThreads);
 #define BM_ROW_CASE(S_, MP_, C_)                                                                                        \
         if (silu == S_ && maxp == MP_ && cols == C_)                                                                    \
-            return launch_ex(bm::t2_gemv_direct_row_kernel<S_, MP_, C_>, grid, block, 0, st, pdl, p);
+            return launch_ex<bm::t2_gemv_direct_row_kernel<S_, MP_, C_>>(grid, block, 0, st, pdl, p);
         BM_ROW_CASE(false, 1, 1) BM_ROW_CASE(false, 1, 2) BM_ROW_CASE(false, 1, 3) BM_ROW_CASE(false, 3, 1) BM_ROW_CASE(false, 5, 1)
         BM_ROW_CASE(true, 1, 1) BM_ROW_CASE(true, 1, 2) BM_ROW_CASE(true, 1, 3) BM_ROW_CASE(true, 3, 1) BM_ROW_CASE(true, 5, 1)
 #undef BM_ROW_CASE
@@ -785,7 +781,7 @@ int bm_quant_rows_amax(const void *x, const void *amax_in, void *amax_zero, int 
     bm::QuantSink sink{static_cast<int8_t *>(q), static_cast<int8_t *>(q_prep), static_cast<int32_t *>(asum)};
     const int units = M * (K / 8);
     const int grid = (units + bm::kQuantAmaxThreads - 1) / bm::kQuantAmaxThreads;
-    return launch_ex(bm::quant_rows_amax_kernel, dim3(grid), dim3(bm::kQuantAmaxThreads), 0,
+    return launch_ex<bm::quant_rows_amax_kernel>(dim3(grid), dim3(bm::kQuantAmaxThreads), 0,
                      static_cast<cudaStream_t>(stream), pdl, static_cast<const uint16_t *>(x),
                      static_cast<const unsigned int *>(amax_in), static_cast<unsigned int *>(amax_zero), M, K, sink,
                      static_cast<float *>(s), pdl);
@@ -798,7 +794,7 @@ int bm_silu_mul_quant(const void *gu, int M, int F, void *q, void *q_prep, void 
     const size_t smem = (size_t)F * 2;
     if (smem > 200 * 1024) return BM_EINVAL;
     bm::QuantSink sink{static_cast<int8_t *>(q), static_cast<int8_t *>(q_prep), static_cast<int32_t *>(asum)};
-    return launch_ex(bm::silu_mul_quant_kernel, dim3(M), dim3(bm::kRowThreads), smem, static_cast<cudaStream_t>(stream),
+    return launch_ex<bm::silu_mul_quant_kernel>(dim3(M), dim3(bm::kRowThreads), smem, static_cast<cudaStream_t>(stream),
                      pdl, static_cast<const uint16_t *>(gu), F, sink, static_cast<float *>(s),
                      static_cast<uint16_t *>(inner_out), pdl);
 }
@@ -821,7 +817,7 @@ int bm_qknorm_rope_kvappend(const void *xqkv, const void *q_w, const void *k_w, 
     p.eps = eps;
     p.M = M; p.H = H; p.Hkv = Hkv; p.kv_rows = kv_rows; p.sigma = sigma; p.pdl = pdl;
     const int heads = H + 2 * Hkv;
-    return launch_ex(bm::qknorm_rope_kvappend_kernel, dim3((heads + 3) / 4, M), dim3(128), 0,
+    return launch_ex<bm::qknorm_rope_kvappend_kernel>(dim3((heads + 3) / 4, M), dim3(128), 0,
                      static_cast<cudaStream_t>(stream), pdl, p);
 }
 
@@ -884,7 +880,7 @@ int launch_attention_cluster(dim3 grid, size_t smem, cudaStream_t st, int pdl, c
     int held = known.load(std::memory_order_relaxed) - 1;
     if (held < 0) {
         int clusters = 0;
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = allow_smem<kernel>();
         if (e == cudaSuccess && grid.x > 8)
             e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         cfg.numAttrs = 1;
@@ -903,10 +899,10 @@ template <bool ROPE, int MERGE>
 int launch_attention(int nv, dim3 grid, size_t smem, cudaStream_t st, int pdl, const bm::AttnParams &p) {
     const dim3 block(bm::kAttnThreads);
     switch (nv) {
-        case 1: return launch_ex(bm::attn_fused_kernel<1, ROPE, MERGE>, grid, block, smem, st, pdl, p);
-        case 2: return launch_ex(bm::attn_fused_kernel<2, ROPE, MERGE>, grid, block, smem, st, pdl, p);
-        case 3: return launch_ex(bm::attn_fused_kernel<3, ROPE, MERGE>, grid, block, smem, st, pdl, p);
-        default: return launch_ex(bm::attn_fused_kernel<4, ROPE, MERGE>, grid, block, smem, st, pdl, p);
+        case 1: return launch_ex<bm::attn_fused_kernel<1, ROPE, MERGE>>(grid, block, smem, st, pdl, p);
+        case 2: return launch_ex<bm::attn_fused_kernel<2, ROPE, MERGE>>(grid, block, smem, st, pdl, p);
+        case 3: return launch_ex<bm::attn_fused_kernel<3, ROPE, MERGE>>(grid, block, smem, st, pdl, p);
+        default: return launch_ex<bm::attn_fused_kernel<4, ROPE, MERGE>>(grid, block, smem, st, pdl, p);
     }
 }
 
@@ -1010,13 +1006,13 @@ int verify_attention_impl(const void *q, const RopeInputs *rope, const void *k_b
                                      bm::QuantSink{static_cast<int8_t *>(q_out), static_cast<int8_t *>(q_prep),
                                                    static_cast<int32_t *>(asum)},
                                      static_cast<float *>(s_out)};
-        return launch_ex(bm::attn_merge_quant_kernel, dim3(M), dim3(32 * H), 0, st, attn_pdl, mp);
+        return launch_ex<bm::attn_merge_quant_kernel>(dim3(M), dim3(32 * H), 0, st, attn_pdl, mp);
     }
     // INT8 codes of the rows from the flat grid, with the absmax the merge gathered
     bm::QuantSink sink{static_cast<int8_t *>(q_out), static_cast<int8_t *>(q_prep), static_cast<int32_t *>(asum)};
     const int K = H * 128, units = M * (K / 8);
     const int qgrid = (units + bm::kQuantAmaxThreads - 1) / bm::kQuantAmaxThreads;
-    return launch_ex(bm::quant_rows_amax_kernel, dim3(qgrid), dim3(bm::kQuantAmaxThreads), 0, st, pdl & BM_PDL_OVERLAP,
+    return launch_ex<bm::quant_rows_amax_kernel>(dim3(qgrid), dim3(bm::kQuantAmaxThreads), 0, st, pdl & BM_PDL_OVERLAP,
                      static_cast<const uint16_t *>(p.att), static_cast<const unsigned int *>(own_amax),
                      static_cast<unsigned int *>(nullptr), M, K, sink, static_cast<float *>(s_out), pdl & BM_PDL_OVERLAP);
 }
@@ -1170,8 +1166,8 @@ int bm_pack_t2_g128(const void *w, int N, int K, void *packed, void *scale, void
     uint16_t *sc = static_cast<uint16_t *>(scale), *fr = static_cast<uint16_t *>(frozen);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const dim3 grid((unsigned)blocks), block(bm::kPackThreads);
-    if (frozen) return launch_ex(bm::pack_t2_g128_kernel<true>, grid, block, 0, st, 1, src, groups, codes, sc, fr);
-    return launch_ex(bm::pack_t2_g128_kernel<false>, grid, block, 0, st, 1, src, groups, codes, sc, fr);
+    if (frozen) return launch_ex<bm::pack_t2_g128_kernel<true>>(grid, block, 0, st, 1, src, groups, codes, sc, fr);
+    return launch_ex<bm::pack_t2_g128_kernel<false>>(grid, block, 0, st, 1, src, groups, codes, sc, fr);
 }
 
 // ---------------------------------------------------------------------------- prompt (many-row) path
@@ -1255,15 +1251,15 @@ int bm_prompt_attention(const void *q, const void *k_base, const void *v_base, i
         if (hist_end > 0) {
             const bm::PromptHistParams hp{p.q, p.k_base, p.v_base, p.pm, p.pl, p.po, T, H, Hkv, __builtin_ctz(G), kv_rows, hist0, pl.NJ, p.pdl};
             const dim3 hgrid((hist_end + BM_ATTN_SUPER - 1) / BM_ATTN_SUPER, Hkv, (T * G + bm::kPaQueries - 1) / bm::kPaQueries);
-            const int rc = launch_ex(bm::prompt_hist_kernel, hgrid, dim3(bm::kPaThreads), bm::kPaSmem, st, p.pdl, hp);
+            const int rc = launch_ex<bm::prompt_hist_kernel>(hgrid, dim3(bm::kPaThreads), bm::kPaSmem, st, p.pdl, hp);
             if (rc != BM_OK) return rc;
         }
-        return launch_ex(bm::attn_fused_kernel<2, false, bm::kMergeHistory>, dim3(pl.n_slabs, Hkv, pl.Z), dim3(bm::kAttnThreads),
+        return launch_ex<bm::attn_fused_kernel<2, false, bm::kMergeHistory>>(dim3(pl.n_slabs, Hkv, pl.Z), dim3(bm::kAttnThreads),
                          bm::attn_smem_bytes(pl.nv, true), st, p.pdl, p);
     }
     const dim3 grid(pl.units, Hkv, pl.Z);
-    return pl.nv == 1 ? launch_ex(bm::attn_fused_kernel<1, false>, grid, dim3(bm::kAttnThreads), smem, st, p.pdl, p)
-                      : launch_ex(bm::attn_fused_kernel<2, false>, grid, dim3(bm::kAttnThreads), smem, st, p.pdl, p);
+    return pl.nv == 1 ? launch_ex<bm::attn_fused_kernel<1, false>>(grid, dim3(bm::kAttnThreads), smem, st, p.pdl, p)
+                      : launch_ex<bm::attn_fused_kernel<2, false>>(grid, dim3(bm::kAttnThreads), smem, st, p.pdl, p);
 }
 
 // ---------------------------------------------------------------------------- dense draft heads
@@ -1289,8 +1285,8 @@ int bm_dense_head(const void *h, const void *W, int fp8, const void *w_scale, in
     const dim3 g(grid), b(bm::kDenseThreads);
     const int nb = (R + 7) / 8;
 #define BM_DENSE_CASE(NB_) \
-    if (nb == NB_) return fp8 ? launch_ex(bm::dense_head_kernel<NB_, true>, g, b, smem, st, p.pdl, p) \
-                             : launch_ex(bm::dense_head_kernel<NB_, false>, g, b, smem, st, p.pdl, p);
+    if (nb == NB_) return fp8 ? launch_ex<bm::dense_head_kernel<NB_, true>>(g, b, smem, st, p.pdl, p) \
+                             : launch_ex<bm::dense_head_kernel<NB_, false>>(g, b, smem, st, p.pdl, p);
     BM_DENSE_CASE(1) BM_DENSE_CASE(2) BM_DENSE_CASE(3)
 #undef BM_DENSE_CASE
     return BM_EINVAL;

@@ -656,3 +656,63 @@ def test_quantisation_of_rows_with_infinities_nans_and_extremes(K):
     back = qp.cpu().numpy().reshape(9, K // 16, 16)[:, :, perm].reshape(9, K)
     assert np.array_equal(back, want)
     assert np.array_equal(asum.cpu().numpy(), want.astype(np.int32).reshape(9, K // 128, 128).sum(-1))
+
+
+def _attention_call(gen, oracle, sigma):
+    """Arguments of one attention call to codes (16 rows behind 130 keys of a segment), and what it reads and writes."""
+    M, H, Hkv, cache_len = 16, 16, 8, 130
+    xqkv = _bf16(gen, M, (H + 2 * Hkv) * 128, scale=2.0).to(DEV)
+    w = (1.0 + 0.1 * torch.randn(128, generator=gen)).to(torch.bfloat16).to(DEV)
+    cos, sin = (oracle.u16_to_torch(t).to(DEV) for t in _rope_tables(oracle, sigma + 40))
+    pos = (torch.arange(M) + cache_len).to(torch.int64).to(DEV)
+    kv = _bf16(gen, 2, Hkv, sigma + M, 128, scale=1.5).to(DEV)
+    state = ops.new_step_state(DEV)
+    ops.set_step_state(state, cache_len, 0, oracle.ROLE_IDS["ar"], 0)
+    scratch = ops.attention_scratch(M, H, sigma, DEV)
+    q, s = torch.empty(M, H * 128, dtype=torch.int8, device=DEV), torch.empty(M, 1, dtype=torch.float32, device=DEV)
+    p = [t.data_ptr() for t in (xqkv, w, w, cos, sin, pos, kv[0], kv[1], state, scratch, q, s)]
+    args = p[:3] + [1e-6] + p[3:8] + [M, H, Hkv, sigma + M, sigma] + p[8:10] + [None, p[10], None, None, p[11], 0]
+    return native.lib().bm_rope_verify_attention, args, (xqkv, w, cos, sin, pos, kv, state, scratch), (q, s)
+
+
+def _gemv_call(gen, oracle, K):
+    from bitmtp_b200 import synthetic
+    W, N = 9, 2048
+    case = {k: v.to(DEV) for k, v in synthetic.gemv_case(W, N, K, seed=K).items() if torch.is_tensor(v)}
+    out = torch.empty(W, N, dtype=torch.bfloat16, device=DEV)
+    args = [case["A"].data_ptr(), case["B"].data_ptr(), out.data_ptr(), case["s"].data_ptr(), case["ws"].data_ptr(), W, N, K, N,
+            native.OUT_BF16, native.PATH_MMA, None, 0]
+    return native.lib().bm_t2_gemv, args, case, (out,)
+
+
+@pytest.mark.parametrize("make,sizes", [(_attention_call, (1024, 4096)), (_gemv_call, (5120, 6144))], ids=["attention", "gemv"])
+def test_threads_with_different_sizes_launch_one_kernel(oracle, make, sizes):
+    """Two threads launch the same kernel with different amounts of shared memory (two segments of one model, two weights):
+    no launch is refused for what the other thread needs, and each gets its own results.  The loops run in C (map over a
+    function that gives the interpreter's lock back), so that the calls do overlap."""
+    import itertools
+    import threading
+    gen = torch.Generator().manual_seed(11)
+    calls = [make(gen, oracle, size) for size in sizes]
+    streams = [torch.cuda.Stream() for _ in calls]
+    torch.cuda.synchronize()
+    want = []
+    for fn, args, _, out in calls:
+        assert fn(*args, torch.cuda.current_stream().cuda_stream) == native.BM_OK
+        torch.cuda.synchronize()
+        want.append([t.clone() for t in out])
+    status, start = [None] * len(calls), threading.Barrier(len(calls))
+
+    def work(i):
+        fn, args = calls[i][:2]
+        start.wait()
+        status[i] = set(map(fn, *(itertools.repeat(a, 20000) for a in args + [streams[i].cuda_stream])))
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(calls))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert status == [{native.BM_OK}] * len(calls)
+    for (_, _, _, out), ref in zip(calls, want):
+        assert all(torch.equal(a.view(torch.uint8), b.view(torch.uint8)) for a, b in zip(out, ref))
