@@ -128,8 +128,7 @@ __device__ __forceinline__ int attn_cache_len(const AttnParams &p) {
 // lane l owns elements 4l..4l+3 (`raw`: its four bf16 inputs, `wraw`: its norm weights, `craw` / `sraw`:
 // its cos / sin table entries), the RoPE partner lives in lane l ^ 16.  Returns the sums before
 // the final bf16 rounding.
-// A call, not inlined: up to six vectors a warp would be 30 KB of instructions that every launch fetches anew.
-__device__ __noinline__ float4 rope_head_vector(uint2 raw, uint2 wraw, uint2 craw, uint2 sraw, float eps, int lane) {
+__device__ __forceinline__ float4 rope_head_vector(uint2 raw, uint2 wraw, uint2 craw, uint2 sraw, float eps, int lane) {
     const float x[4] = {__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u),
                         __uint_as_float(raw.y << 16), __uint_as_float(raw.y & 0xffff0000u)};
     float acc = 0.0f;
@@ -159,6 +158,11 @@ __device__ __noinline__ float4 rope_head_vector(uint2 raw, uint2 wraw, uint2 cra
         o[i] = bm_bf16_rn(n[i] * c[i]) + bm_bf16_rn(rot * sn[i]);
     }
     return make_float4(o[0], o[1], o[2], o[3]);
+}
+// The same as a call, for the builds of more than four query vectors: up to six vectors a warp would be 30 KB of instructions
+// that every launch fetches anew.
+__device__ __noinline__ float4 rope_head_vector_call(uint2 raw, uint2 wraw, uint2 craw, uint2 sraw, float eps, int lane) {
+    return rope_head_vector(raw, wraw, craw, sraw, eps, lane);
 }
 
 // Two fp32 values in a register pair, and the packed arithmetic on them: each half rounds as the scalar instruction does,
@@ -328,6 +332,56 @@ __device__ __forceinline__ void attn_level0(const uint16_t *Ks, const uint16_t *
         *reinterpret_cast<float4 *>(oc + (2 * i) * 128 + 4 * lane) = make_float4(x[0], x[1], x[2], x[3]);
         *reinterpret_cast<float4 *>(oc + (2 * i + 1) * 128 + 4 * lane) = make_float4(y[0], y[1], y[2], y[3]);
     }
+}
+
+// Level 0 where a CTA has one or two query vectors (width 1 of the 1.7B geometry): a warp serves one, a lane holds one key.
+// attn_level0 would put both on the first four warps, a half warp each with two keys a lane, and have the others compute
+// nothing: twice the chain.  Rows by clusters, 16 / 8 heads, width 1, us that way and this: 5.0 and 4.5 behind 20 keys, 5.7 and
+// 5.0 behind 600, 6.3 and 5.6 behind 1000.  Same scores, same sums: the butterfly 16, 8, 4, 2, 1 now crosses lanes in its first
+// step too.  a.q_lo: the vector; Qs its row; Pw 32 weights; oc one row.
+__device__ __forceinline__ void attn_level0_one(const uint16_t *Ks, const uint16_t *Vs, const uint16_t *Qs, float *Pw,
+                                                const AttnView &a, int cn, int hidden, int lane, float *mc, float *lc, float *oc) {
+    float o[4] = {0.0f, 0.0f, 0.0f, 0.0f};                             // dims 4 lane + e
+    if (cn > 0) {
+        float s = 0.0f;
+        const uint16_t *kr = Ks + (lane < cn ? lane : 0) * kKeyStride;
+#pragma unroll 4
+        for (int u = 0; u < 16; ++u) {
+            float k[8], q[8];
+            unpack8(*reinterpret_cast<const uint4 *>(kr + 8 * u), k);
+            unpack8(*reinterpret_cast<const uint4 *>(Qs + 8 * u), q);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) s = fmaf(q[e], k[e], s);
+        }
+        const bool seen = lane < cn && (a.fresh ? bm_visible(a.role, a.q_lo - a.q_lo / a.M * a.M, a.key0 + lane, a.sigma,
+                                                             a.cache_len, a.n_pend, a.P)
+                                                : lane != hidden);
+        s = seen ? s * 0.08838834764831845f : -INFINITY;
+        const float m = warp_max(s), e = pa_expf(s - m), w = seen ? e : 0.0f, l = warp_sum_butterfly(w);
+        Pw[lane] = bm_bf16_rn(w);
+        if (lane == 0) { mc[0] = m; lc[0] = l; }
+        __syncwarp();
+        for (int cb = 0; cb < cn; cb += 4) {
+            uint2 raw[4];
+#pragma unroll
+            for (int cc = 0; cc < 4; ++cc)
+                raw[cc] = cb + cc < cn ? *reinterpret_cast<const uint2 *>(Vs + (cb + cc) * 128 + 4 * lane) : make_uint2(0u, 0u);
+            const float4 w4 = *reinterpret_cast<const float4 *>(Pw + cb);
+            const float wk[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+            for (int cc = 0; cc < 4; ++cc) {
+                const float v[4] = {__uint_as_float(raw[cc].x << 16), __uint_as_float(raw[cc].x & 0xffff0000u),
+                                    __uint_as_float(raw[cc].y << 16), __uint_as_float(raw[cc].y & 0xffff0000u)};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) o[i] = fmaf(wk[cc], v[i], o[i]);
+            }
+        }
+    } else if (lane == 0) {
+        mc[0] = -INFINITY;
+        lc[0] = 0.0f;
+    }
+    __syncthreads();                                                   // every warp is done with the K rows
+    *reinterpret_cast<float4 *>(oc + 4 * lane) = make_float4(o[0], o[1], o[2], o[3]);
 }
 
 // Level 2 of one query vector by one warp: super-chunk partials in ascending order (history chunks 0 .. n_hs - 1, then the
@@ -579,7 +633,8 @@ __global__ void __launch_bounds__(kAttnThreads, MERGE == kMergeHistory ? 4 : 2) 
             if (qi >= qc) break;                                          // warp-uniform
             uint2 bits = make_uint2(0u, 0u);
             if (q_live[k]) {
-                const float4 r = rope_head_vector(qraw[k], qw, qcos[k], qsin[k], p.eps, lane);
+                const float4 r = NV == 1 ? rope_head_vector(qraw[k], qw, qcos[k], qsin[k], p.eps, lane)
+                                         : rope_head_vector_call(qraw[k], qw, qcos[k], qsin[k], p.eps, lane);
                 bits = attn_pack_row({r.x, r.y, r.z, r.w});
             }
             *reinterpret_cast<uint2 *>(Qs + qi * kKeyStride + 4 * lane) = bits;
@@ -590,7 +645,8 @@ __global__ void __launch_bounds__(kAttnThreads, MERGE == kMergeHistory ? 4 : 2) 
             for (int k = 0; k < kFreshPerWarp; ++k) {
                 const int m = warp + k * kAttnWarps;
                 if (m >= M_) break;                                       // warp-uniform
-                const float4 r = rope_head_vector(kraw[k], kw, kcos[k], ksin[k], p.eps, lane);
+                const float4 r = NV == 1 ? rope_head_vector(kraw[k], kw, kcos[k], ksin[k], p.eps, lane)
+                                         : rope_head_vector_call(kraw[k], kw, kcos[k], ksin[k], p.eps, lane);
                 const uint2 kbits = attn_pack_row({r.x, r.y, r.z, r.w});
                 *reinterpret_cast<uint2 *>(Ks + m * kKeyStride + 4 * lane) = kbits;
                 *reinterpret_cast<uint2 *>(Vs + m * 128 + 4 * lane) = vraw[k];
@@ -623,7 +679,8 @@ __global__ void __launch_bounds__(kAttnThreads, MERGE == kMergeHistory ? 4 : 2) 
         // rows: the last committed token, which such a replay appends again
         const bool hides = role == BM_ROLE_VERIFY || (role == BM_ROLE_DRAFT && min(max(n_pend, 0), P_) == 0);
         const int hidden = hides && !fresh ? cache_len - 1 - key0 - c * BM_ATTN_CHUNK : -1;
-        const AttnView a{fresh, role, sigma_, cache_len, n_pend, P_, M_, q_lo + 2 * nv * g, key0 + c * BM_ATTN_CHUNK};
+        const bool one = NV == 1 && QV - q_lo <= 2;                       // one vector per warp
+        const AttnView a{fresh, role, sigma_, cache_len, n_pend, P_, M_, q_lo + (one ? 1 : 2 * nv) * g, key0 + c * BM_ATTN_CHUNK};
         const uint16_t *Kc = Ks + c * BM_ATTN_CHUNK * kKeyStride, *Vc = Vs + c * BM_ATTN_CHUNK * 128;
 #define BM_ATTN_LEVEL0(N_)                                                                                                    \
     attn_level0<N_>(Kc, Vc, Qs + 2 * N_ * g * kKeyStride, Ps + warp * BM_ATTN_CHUNK * kWeightStride, a, cn, hidden, lane,       \
@@ -631,6 +688,9 @@ __global__ void __launch_bounds__(kAttnThreads, MERGE == kMergeHistory ? 4 : 2) 
         if (NV >= 4 && nv == 4) BM_ATTN_LEVEL0(4);
         else if (NV >= 3 && nv == 3) BM_ATTN_LEVEL0(3);
         else if (NV >= 2 && nv == 2) BM_ATTN_LEVEL0(2);
+        else if (one)
+            attn_level0_one(Kc, Vc, Qs + g * kKeyStride, Ps + warp * BM_ATTN_CHUNK * kWeightStride, a, cn, hidden, lane, mc + c * QC + g,
+                            lc + c * QC + g, oc + ((size_t)c * QC + g) * 128);
         else BM_ATTN_LEVEL0(1);
 #undef BM_ATTN_LEVEL0
     }

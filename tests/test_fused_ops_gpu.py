@@ -137,6 +137,12 @@ ATTN_CASES = [
     (8, 16, 8, 1024, 700, 0, 8, "draft"),      # 288 CTAs in 32 clusters, three of nine CTAs without rows
     (4, 16, 8, 1920, 1901, 0, 4, "draft"),     # the largest cluster (16)
     (4, 16, 8, 1920, 0, 0, 4, "ar"),           # only the CTA of the replay's own rows works
+    # one or two query vectors per kv head (one per warp), at the edges of sub- and super-chunks, with a hidden key too
+    (1, 4, 4, 128, 33, 0, 1, "ar"),
+    (1, 4, 2, 384, 256, 0, 1, "ar"),
+    (1, 4, 2, 256, 161, 0, 1, "verify"),
+    (2, 4, 4, 256, 128, 0, 1, "verify"),
+    (2, 4, 4, 256, 129, 1, 1, "draft"),
 ]
 
 
