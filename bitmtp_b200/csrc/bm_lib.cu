@@ -945,13 +945,13 @@ int verify_attention_impl(const void *q, const RopeInputs *rope, const void *k_b
     const int NJ = (sigma + BM_ATTN_SUPER - 1) / BM_ATTN_SUPER + 1;
     if (NJ > bm::kAttnMaxNJ) return BM_EINVAL;
     const int G = H / Hkv, QV = G * M;
-    const int nv = bm::attn_nv(QV), Z = bm::attn_groups(QV, 1);   // every CTA picks its split between the two
-    if (Hkv * Z > bm::kAttnTickets) return BM_EINVAL;
+    if (Hkv * bm::attn_groups(QV, 1) > bm::kAttnTickets) return BM_EINVAL;
     if ((H * 128) % 256 != 0 && amax_rows == nullptr) return BM_EINVAL;   // the flat quantisation wants K % 256 == 0
     bm::AttnParams p = {};
-    const int sms = current_device().sm_count;
-    p.z_max = Z;
-    const bool single = bm::attn_fill_pick(p.pick, NJ, QV, Hkv, sms);
+    const bm::AttnSplit split = bm::attn_split(NJ, QV, Hkv, current_device().sm_count);
+    const int nv = bm::attn_nv(QV);                               // widest split: the kernel's build
+    std::copy(split.pick, split.pick + NJ, p.pick);
+    p.z_max = split.groups;
     p.q = static_cast<const uint16_t *>(q);
     p.k_base = static_cast<const uint16_t *>(k_base);
     p.v_base = static_cast<const uint16_t *>(v_base);
@@ -980,8 +980,8 @@ int verify_attention_impl(const void *q, const RopeInputs *rope, const void *k_b
     // Where the working CTAs never exceed the SMs, one CTA per SM: two would share the first SM that the predecessor leaves
     // while others stay empty.
     size_t smem = bm::attn_smem_bytes(nv);
-    if (single) smem = std::max(smem, (size_t)kMaxSmemPerCta / 2 + 1024);
-    const dim3 grid(Hkv, NJ * Z);
+    if (split.single) smem = std::max(smem, (size_t)kMaxSmemPerCta / 2 + 1024);
+    const dim3 grid(Hkv, split.pairs);
     int rc;
     if (rope != nullptr) {
         p.xqkv = static_cast<const uint16_t *>(rope->xqkv);
@@ -994,7 +994,7 @@ int verify_attention_impl(const void *q, const RopeInputs *rope, const void *k_b
         p.v_out = const_cast<uint16_t *>(p.v_base);
         p.eps = rope->eps;
         rc = later ? launch_attention<true, bm::kMergeLater>(nv, grid, smem, st, attn_pdl, p)
-                   : launch_attention_clusters(nv, dim3(NJ, Hkv, Z), bm::attn_smem_bytes(nv), st, attn_pdl, p);
+                   : launch_attention_clusters(nv, dim3(NJ, Hkv, split.groups), bm::attn_smem_bytes(nv), st, attn_pdl, p);
         if (rc < 0) rc = launch_attention<true, bm::kMergeTicket>(nv, grid, smem, st, attn_pdl, p);
     } else {
         rc = later ? launch_attention<false, bm::kMergeLater>(nv, grid, smem, st, attn_pdl, p)

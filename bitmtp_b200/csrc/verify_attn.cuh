@@ -29,6 +29,8 @@
 //   NJ = ceil(sigma/128) + 1; super-chunk NJ-1 holds the rows appended by this replay.
 #pragma once
 
+#include <algorithm>
+
 #include "bm_common.cuh"
 #include "fused_ops.cuh"
 
@@ -50,7 +52,7 @@ struct AttnParams {
     const uint16_t *v_base;
     const StepState *state;
     int M, H, Hkv, kv_rows, sigma, NJ;
-    unsigned int *tickets;    // [Hkv * gridDim.z], zero between launches
+    unsigned int *tickets;    // [Hkv * z_max] a replay or slab, zero between launches
     unsigned int *amax;       // [M] row absmax bits, gathered by atomic max (zero on entry)
     float *pm, *pl, *po;
     uint16_t *att;            // [M, H*128] bf16 attention output
@@ -66,10 +68,10 @@ struct AttnParams {
     // [slab_hist0, slab_hist0 + M) of the planes are served as AR-causal slabs of slab_rows rows: slab s
     // sees history [0, slab_hist0 + s * slab_rows) and its own rows.  blockIdx.x runs over the
     // (slab, super-chunk) pairs in slab order; `state` is not read; q, att, amax and the partials are
-    // indexed by prompt row; tickets [slabs][Hkv][gridDim.z].
+    // indexed by prompt row.
     int slab_rows, slab_hist0;
-    int z_max;       // query groups the tickets are laid out for: gridDim.z, or the finest split of a flat grid
-    uint8_t pick[kAttnMaxNJ];        // replays: query vectors per half warp for n history super-chunks (attn_fill_pick)
+    int z_max;       // query groups the tickets are laid out for
+    uint8_t pick[kAttnMaxNJ];        // replays: query vectors per half warp for n history super-chunks (attn_split)
 };
 
 __host__ __device__ inline size_t attn_scratch_bytes(int M, int H, int sigma) {
@@ -85,22 +87,37 @@ __host__ __device__ inline size_t attn_scratch_bytes(int M, int H, int sigma) {
 __host__ __device__ inline int attn_nv(int QV) { return QV >= 4 * kAttnMaxNV ? kAttnMaxNV : (QV + 3) / 4; }
 __host__ __device__ inline int attn_groups(int QV, int nv) { return (QV + 4 * nv - 1) / (4 * nv); }
 
-// pick[n]: split for n history super-chunks, NJ - 1 at most.  A CTA costs about its vectors plus four more (loading and
-// unpacking its keys).  Returns whether the working CTAs never exceed the SMs; where the widest split allows that, only
-// splits that do are taken.
-inline bool attn_fill_pick(uint8_t *pick, int NJ, int QV, int Hkv, int sms) {
-    const bool single = NJ * Hkv * attn_groups(QV, attn_nv(QV)) <= sms;
+// The splits of a replay over a segment of NJ - 1 history super-chunks.  The cost of n of them at a split is the time of the
+// fullest SM, in units of about half a microsecond: a CTA alone takes 2 nv + 5 (7.4 us to codes with nv = 2, 9.2 with 3, 10.5
+// with 4); two that share an SM overlap, 3 nv + 5 for the pair; an odd one after pairs takes 0.6 of a pair.  Where no split
+// needs more CTAs than SMs, only such are taken and each CTA gets an SM to itself.  The grid is that of the largest pick, not
+// of the finest split: CTAs without work delayed the others by up to 2.6 us (2112 CTAs, 256 of them working).
+// Fitted to the attention to codes for every nv, over 1566 calls (five head counts, 2 to 32 rows, 1 to 32 super-chunks, segments of
+// 256 to 4096): 0.2 % over the fastest split on average, where the rule before (w (2 nv + 3) for w CTAs, grid of the finest split) was
+// 6 % over it.  us then / now: 16 / 8 heads, width 9 behind 6 super-chunks of 1024 keys 9.1 / 9.1, behind 8 of 4096 13.2 / 10.9; width 16
+// behind 8 of 1024 12.6 / 11.6, behind 8 of 4096 15.5 / 11.6; 32 / 8 heads, width 9 behind 3 of 1024 11.4 / 9.3, width 16 13.7 / 10.6.
+struct AttnSplit {
+    uint8_t pick[kAttnMaxNJ];   // nv for n history super-chunks
+    bool single;                // the working CTAs never exceed the SMs
+    int groups, pairs;          // most query groups, most (super-chunk, query group) pairs of any n
+};
+inline AttnSplit attn_split(int NJ, int QV, int Hkv, int sms) {
+    AttnSplit r = {};
+    const int widest = attn_nv(QV);
+    r.single = NJ * Hkv * attn_groups(QV, widest) <= sms;
     for (int n = 0; n < NJ; ++n) {
         int best = 0, cost = 0;
-        for (int nv = 1; nv <= attn_nv(QV); ++nv) {
-            const int ctas = (n + 1) * Hkv * attn_groups(QV, nv);
-            if (single && ctas > sms) continue;
-            const int c = (ctas + sms - 1) / sms * (2 * nv + 3);
+        for (int nv = 1; nv <= widest; ++nv) {
+            const int ctas = (n + 1) * Hkv * attn_groups(QV, nv), w = (ctas + sms - 1) / sms;      // CTAs of the fullest SM
+            if (r.single && ctas > sms) continue;
+            const int c = w == 1 ? 10 * (2 * nv + 5) : (3 * nv + 5) * (w / 2 * 10 + w % 2 * 6);
             if (best == 0 || c < cost) { best = nv; cost = c; }
         }
-        pick[n] = (uint8_t)best;
+        r.pick[n] = (uint8_t)best;
+        r.groups = std::max(r.groups, attn_groups(QV, best));
+        r.pairs = std::max(r.pairs, (n + 1) * attn_groups(QV, best));
     }
-    return single;
+    return r;
 }
 
 // K (padded rows; after level 0 its space takes the sub-chunk numerators), V, queries, weights, sub-chunk max / sum.
