@@ -918,8 +918,7 @@ int launch_attention_clusters(int nv, dim3 grid, size_t smem, cudaStream_t st, i
 }
 
 // Rows wanted (`amax_rows` != null): one attention launch, bf16 rows + row absmax bits.  Codes wanted: an attention launch
-// that leaves its super-chunk partials to the launch that merges and quantises them (up to 32 heads: one warp each), else
-// an attention launch that merges, and the flat quantisation.
+// that leaves its super-chunk partials, and one that merges and quantises them.
 int verify_attention_impl(const void *q, const RopeInputs *rope, const void *k_base, const void *v_base, int M, int H,
                           int Hkv, int kv_rows, int sigma, const void *state, void *scratch, void *att_out,
                           void *q_out, void *q_prep, void *asum, void *s_out, int pdl, void *stream,
@@ -945,10 +944,12 @@ int verify_attention_impl(const void *q, const RopeInputs *rope, const void *k_b
     const int NJ = (sigma + BM_ATTN_SUPER - 1) / BM_ATTN_SUPER + 1;
     if (NJ > bm::kAttnMaxNJ) return BM_EINVAL;
     const int G = H / Hkv, QV = G * M;
-    if (Hkv * bm::attn_groups(QV, 1) > bm::kAttnTickets) return BM_EINVAL;
-    if ((H * 128) % 256 != 0 && amax_rows == nullptr) return BM_EINVAL;   // the flat quantisation wants K % 256 == 0
+    // rows: a counter per kv head and query group; codes: none, but the product that takes them wants K % 256 == 0
+    if (H > bm::kAttnMaxHeads) return BM_EINVAL;
+    if (amax_rows != nullptr ? Hkv * bm::attn_groups(QV, 1) > bm::kAttnTickets : (H % 2) != 0) return BM_EINVAL;
     bm::AttnParams p = {};
     const bm::AttnSplit split = bm::attn_split(NJ, QV, Hkv, current_device().sm_count);
+    if (split.pairs > 65535) return BM_EINVAL;                    // one grid dimension
     const int nv = bm::attn_nv(QV);                               // widest split: the kernel's build
     std::copy(split.pick, split.pick + NJ, p.pick);
     p.z_max = split.groups;
@@ -959,24 +960,15 @@ int verify_attention_impl(const void *q, const RopeInputs *rope, const void *k_b
     p.M = M; p.H = H; p.Hkv = Hkv; p.kv_rows = kv_rows; p.sigma = sigma; p.NJ = NJ;
     char *sc = static_cast<char *>(scratch);
     p.tickets = reinterpret_cast<unsigned int *>(sc);
-    unsigned int *own_amax = reinterpret_cast<unsigned int *>(sc) + bm::kAttnTickets;
     p.pm = reinterpret_cast<float *>(sc + bm::kAttnHeaderBytes);
     p.pl = p.pm + (size_t)M * H * NJ;
     p.po = p.pl + (size_t)M * H * NJ;
-    uint16_t *own_rows = reinterpret_cast<uint16_t *>(p.po + (size_t)M * H * NJ * 128);
-    p.att = att_out ? static_cast<uint16_t *>(att_out) : own_rows;
-    p.amax = amax_rows ? static_cast<unsigned int *>(amax_rows) : own_amax;
+    p.att = static_cast<uint16_t *>(att_out);
+    p.amax = static_cast<unsigned int *>(amax_rows);
     p.pdl = pdl & (BM_PDL_OVERLAP | BM_PDL_STABLE_STATE);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const bool later = amax_rows == nullptr && H <= 32;
-    int attn_pdl = pdl & BM_PDL_OVERLAP;
-    if (amax_rows == nullptr && !later) {
-        // this call gathers the row absmax in the scratch header: clear it first (stream-ordered); after a memset node the
-        // launch cannot overlap its predecessor programmatically
-        const cudaError_t e = cudaMemsetAsync(own_amax, 0, BM_MAX_W * sizeof(unsigned int), st);
-        if (e != cudaSuccess) return cuda_status(e);
-        attn_pdl = p.pdl = 0;
-    }
+    const bool codes = amax_rows == nullptr;
+    const int attn_pdl = pdl & BM_PDL_OVERLAP;
     // Where the working CTAs never exceed the SMs, one CTA per SM: two would share the first SM that the predecessor leaves
     // while others stay empty.
     size_t smem = bm::attn_smem_bytes(nv);
@@ -993,28 +985,21 @@ int verify_attention_impl(const void *q, const RopeInputs *rope, const void *k_b
         p.k_out = const_cast<uint16_t *>(p.k_base);
         p.v_out = const_cast<uint16_t *>(p.v_base);
         p.eps = rope->eps;
-        rc = later ? launch_attention<true, bm::kMergeLater>(nv, grid, smem, st, attn_pdl, p)
+        rc = codes ? launch_attention<true, bm::kMergeLater>(nv, grid, smem, st, attn_pdl, p)
                    : launch_attention_clusters(nv, dim3(NJ, Hkv, split.groups), bm::attn_smem_bytes(nv), st, attn_pdl, p);
         if (rc < 0) rc = launch_attention<true, bm::kMergeTicket>(nv, grid, smem, st, attn_pdl, p);
     } else {
-        rc = later ? launch_attention<false, bm::kMergeLater>(nv, grid, smem, st, attn_pdl, p)
-                   : launch_attention<false, bm::kMergeTicket>(nv, grid, smem, st, attn_pdl, p);
+        rc = launch_attention<false, bm::kMergeLater>(nv, grid, smem, st, attn_pdl, p);
     }
-    if (rc != BM_OK || amax_rows != nullptr) return rc;
-    if (later) {
-        const bm::AttnMergeParams mp{p.pm, p.pl, p.po, p.state, H, NJ, sigma, p.pdl, static_cast<uint16_t *>(att_out),
-                                     bm::QuantSink{static_cast<int8_t *>(q_out), static_cast<int8_t *>(q_prep),
-                                                   static_cast<int32_t *>(asum)},
-                                     static_cast<float *>(s_out)};
-        return launch_ex<bm::attn_merge_quant_kernel>(dim3(M), dim3(32 * H), 0, st, attn_pdl, mp);
-    }
-    // INT8 codes of the rows from the flat grid, with the absmax the merge gathered
-    bm::QuantSink sink{static_cast<int8_t *>(q_out), static_cast<int8_t *>(q_prep), static_cast<int32_t *>(asum)};
-    const int K = H * 128, units = M * (K / 8);
-    const int qgrid = (units + bm::kQuantAmaxThreads - 1) / bm::kQuantAmaxThreads;
-    return launch_ex<bm::quant_rows_amax_kernel>(dim3(qgrid), dim3(bm::kQuantAmaxThreads), 0, st, pdl & BM_PDL_OVERLAP,
-                     static_cast<const uint16_t *>(p.att), static_cast<const unsigned int *>(own_amax),
-                     static_cast<unsigned int *>(nullptr), M, K, sink, static_cast<float *>(s_out), pdl & BM_PDL_OVERLAP);
+    if (rc != BM_OK || !codes) return rc;
+    const bool many = H > 32;
+    uint16_t *own_rows = reinterpret_cast<uint16_t *>(p.po + (size_t)M * H * NJ * 128);
+    const bm::AttnMergeParams mp{p.pm, p.pl, p.po, p.state, H, NJ, sigma, p.pdl, many && !att_out ? own_rows : p.att,
+                                 bm::QuantSink{static_cast<int8_t *>(q_out), static_cast<int8_t *>(q_prep), static_cast<int32_t *>(asum)},
+                                 static_cast<float *>(s_out)};
+    const dim3 rows(M), block(32 * std::min(H, 32));
+    return many ? launch_ex<bm::attn_merge_quant_kernel<true>>(rows, block, 0, st, attn_pdl, mp)
+                : launch_ex<bm::attn_merge_quant_kernel<false>>(rows, block, 0, st, attn_pdl, mp);
 }
 }  // namespace
 

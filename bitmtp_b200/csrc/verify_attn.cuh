@@ -41,7 +41,8 @@ constexpr int kAttnSub = BM_ATTN_SUPER / BM_ATTN_CHUNK;   // sub-chunks per supe
 constexpr int kKeyStride = 136;        // bf16 elements per staged key row (128 + 8 pad = 272 bytes)
 constexpr int kWeightStride = 8;        // fp32 softmax weights per key and warp (a warp serves up to 8 query vectors)
 constexpr int kAttnHeaderBytes = 1024;
-constexpr int kAttnTickets = 224;      // counters in the header; the row absmax words follow
+constexpr int kAttnTickets = 224;      // counters in the header
+constexpr int kAttnMaxHeads = 1024;    // heads of one call (keeps the split's products in an int)
 constexpr int kAttnMaxNV = 4;          // query vectors per half warp; a CTA serves up to 4 * kAttnMaxNV
 constexpr int kAttnMaxNJ = 64;         // super-chunk partials one merging warp handles (2 per lane)
 constexpr int kAttnMaxCluster = 16;    // super-chunks (CTAs) of one cluster in the cluster build
@@ -831,7 +832,8 @@ __global__ void __launch_bounds__(kAttnThreads, MERGE == kMergeHistory ? 4 : 2) 
 }
 
 // =============================================================================
-// Level 2 and the INT8 quantisation of the attention rows in one launch: one CTA per row, one warp per head (H <= 32).
+// Level 2 and the INT8 quantisation of the attention rows in one launch: one CTA per row, one warp per head; above 32
+// heads (MANY) a warp takes every 32nd, and the rows go through memory between the merge and the codes.
 // Follows attn_fused_kernel<.., kMergeLater>; replaces its ticket merge, the absmax atomics and the flat quantisation
 // launch that had to read the rows again.  Same merge, same codes.
 // =============================================================================
@@ -839,37 +841,63 @@ struct AttnMergeParams {
     const float *pm, *pl, *po;
     const StepState *state;
     int H, NJ, sigma, pdl;
-    uint16_t *att;            // optional bf16 rows
+    uint16_t *att;            // bf16 rows; optional up to 32 heads
     QuantSink q;
     float *s;
 };
 
+// Codes of the row's group `group` (row * H + head) by one warp; lane: dims 4 lane .. 4 lane + 3.
+__device__ __forceinline__ void attn_emit_codes(const QuantSink &q, int group, const float (&v)[4], float s, int lane) {
+    const size_t at = (size_t)group * 128;
+    const uint32_t codes = quant_quad(v[0], v[1], v[2], v[3], s);
+    if (q.nat) reinterpret_cast<uint32_t *>(q.nat + at)[lane] = codes;
+    if (q.prep) {
+        // GEMV-ready order: the 4 x 4 bytes of four consecutive lanes transposed in two exchanges
+        const uint32_t x = __shfl_xor_sync(0xffffffffu, codes, 1), t = __byte_perm(codes, x, (lane & 1) ? 0x3715u : 0x6240u);
+        const uint32_t y = __shfl_xor_sync(0xffffffffu, t, 2);
+        reinterpret_cast<uint32_t *>(q.prep + at)[lane] = __byte_perm(t, y, (lane & 2) ? 0x3276u : 0x5410u);
+        const int sum = __reduce_add_sync(0xffffffffu, __dp4a((int)codes, 0x01010101, 0));
+        if (lane == 0) q.asum[group] = sum;
+    }
+}
+
+template <bool MANY>
 __global__ void __launch_bounds__(1024) attn_merge_quant_kernel(const AttnMergeParams p) {
     __shared__ unsigned int sh[32];
     pdl_launch_dependents();
     const bool early = (p.pdl & BM_PDL_STABLE_STATE) != 0;
     if (p.pdl && !early) pdl_wait();
     const int cache_len = min(max(p.state->cache_len, 0), p.sigma), n_hs = (cache_len + BM_ATTN_SUPER - 1) / BM_ATTN_SUPER;
-    const int m = blockIdx.x, lane = threadIdx.x & 31, head = threadIdx.x >> 5;
+    const int m = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (early) pdl_wait();
-    float v[4];
-    attn_merge_vector<false>(p.pm, p.pl, p.po, ((size_t)m * p.H + head) * p.NJ, n_hs, p.NJ, lane, 0.0f, 0.0f,
-                             make_float4(0.0f, 0.0f, 0.0f, 0.0f), v);
-    const size_t at = ((size_t)m * p.H + head) * 128;
-    if (p.att) *reinterpret_cast<uint2 *>(p.att + at + 4 * lane) = attn_pack_row(v);
-    const float amax = attn_row_amax(v);
-    if (lane == 0) sh[head] = amax != 0.0f ? __float_as_uint(amax) : 0u;
+    // one head: merged rows (stored if asked for) and their absmax
+    auto merge = [&](int head, float (&v)[4]) {
+        const size_t row = (size_t)m * p.H + head;
+        attn_merge_vector<false>(p.pm, p.pl, p.po, row * p.NJ, n_hs, p.NJ, lane, 0.0f, 0.0f, make_float4(0.0f, 0.0f, 0.0f, 0.0f), v);
+        if (MANY || p.att) *reinterpret_cast<uint2 *>(p.att + row * 128 + 4 * lane) = attn_pack_row(v);
+        return attn_row_amax(v);
+    };
+    float v[4], amax;
+    if (MANY) {
+        amax = 0.0f;
+        for (int head = warp; head < p.H; head += 32) amax = fmaxf(amax, merge(head, v));
+    } else {
+        amax = merge(warp, v);
+    }
+    if (lane == 0) sh[warp] = __float_as_uint(amax);
     __syncthreads();
-    const float s = bm_act_scale(__uint_as_float(__reduce_max_sync(0xffffffffu, lane < p.H ? sh[lane] : 0u)));
-    const uint32_t codes = quant_quad(v[0], v[1], v[2], v[3], s);
-    if (p.q.nat) reinterpret_cast<uint32_t *>(p.q.nat + at)[lane] = codes;
-    if (p.q.prep) {
-        // GEMV-ready order: the 4 x 4 bytes of four consecutive lanes transposed in two exchanges
-        const uint32_t x = __shfl_xor_sync(0xffffffffu, codes, 1), t = __byte_perm(codes, x, (lane & 1) ? 0x3715u : 0x6240u);
-        const uint32_t y = __shfl_xor_sync(0xffffffffu, t, 2);
-        reinterpret_cast<uint32_t *>(p.q.prep + at)[lane] = __byte_perm(t, y, (lane & 2) ? 0x3276u : 0x5410u);
-        const int sum = __reduce_add_sync(0xffffffffu, __dp4a((int)codes, 0x01010101, 0));
-        if (lane == 0) p.q.asum[m * p.H + head] = sum;
+    const int nwarps = MANY ? 32 : p.H;
+    const float s = bm_act_scale(__uint_as_float(__reduce_max_sync(0xffffffffu, lane < nwarps ? sh[lane] : 0u)));
+    if (MANY) {
+        for (int head = warp; head < p.H; head += 32) {
+            const int row = m * p.H + head;
+            const uint2 raw = *reinterpret_cast<const uint2 *>(p.att + (size_t)row * 128 + 4 * lane);   // (as this lane wrote it)
+            const float u[4] = {__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u), __uint_as_float(raw.y << 16),
+                                __uint_as_float(raw.y & 0xffff0000u)};
+            attn_emit_codes(p.q, row, u, s, lane);
+        }
+    } else {
+        attn_emit_codes(p.q, m * p.H + warp, v, s, lane);
     }
     if (threadIdx.x == 0) p.s[m] = s;
 }

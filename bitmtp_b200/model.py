@@ -512,6 +512,12 @@ class Transformer(nn.Module):
         fused_ffn = self.fused_ffn and M <= 16 and a.ffn_dim % 16 == 0 and a.dim % 256 == 0
         if fused_ffn:
             ops.zero_words(W.inner_amax[0])           # slot of layer 0; every layer clears the next one's
+        # Above 32 heads a warp of the launch that merges to codes takes two heads or more in turn, and a single row does not
+        # pay for that (40 / 8 heads, width 1 behind 20 keys: 8.0 us to codes, 6.6 to rows and then codes; width 9 level,
+        # width 16 behind 600 17.9 against 19.1).
+        rows_first = self.fused_rope and M == 1 and a.n_heads > 32 and a.n_heads % 4 == 0
+        if rows_first:
+            ops.zero_words(W.att_amax[0])
         ops.rmsnorm_fused(self.embed_tokens.weight.data, L0.input_layernorm.weight.data, eps, M=M,
                           gather=token_values, pdl=pdl, out=qsink)
         for i, layer in enumerate(self.layers):
@@ -522,7 +528,14 @@ class Transformer(nn.Module):
             ops.t2_gemv_prepared(W.q, W.q_sum, at.wqkv_weight, W.s, at.wqkv_scale, out=W.xqkv,
                                  ldc=W.xqkv.shape[1], pdl=pdl)
             k_l, v_l = kv_full[i]
-            if self.fused_rope:
+            if rows_first:
+                ops.rope_verify_attention_rows(W.xqkv, at.q_norm.weight.data, at.k_norm.weight.data, eps, at.rope_cos,
+                                               at.rope_sin, positions, a.n_heads, a.n_kv_heads, _LayerView(k_l, kv_rows),
+                                               _LayerView(v_l, kv_rows), sigma, attn_mask, attn_scratch, att=W.att,
+                                               amax=W.att_amax[i & 1], pdl=attn_pdl)
+                ops.quant_rows_amax(W.att, W.att_amax[i & 1], prep=(W.att_q, W.att_sum), s=W.att_s,
+                                    amax_zero=W.att_amax[(i + 1) & 1], pdl=pdl)
+            elif self.fused_rope:
                 # one attention launch (q/k norm, RoPE and KV append folded in) that leaves split-KV partials, and one
                 # that merges them and writes the rows as INT8 codes
                 ops.rope_verify_attention(W.xqkv, at.q_norm.weight.data, at.k_norm.weight.data, eps, at.rope_cos,

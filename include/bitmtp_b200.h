@@ -183,10 +183,9 @@ int64_t bm_verify_attention_scratch_bytes(int M, int H, int sigma);
  *   first use (its first KiB holds counters that every call leaves zero again); not
  *   shared by calls that may execute at the same time;
  *   att_out bf16 [M, H*128] or NULL; q_out / q_prep / asum: the quantised rows (see
- *   bm_quant_rows); s_out fp32 [M].  H*128 a multiple of 256; sigma <= 8064.
+ *   bm_quant_rows); s_out fp32 [M].  H*128 a multiple of 256, H <= 1024; sigma <= 8064.
  * Two launches: the attention's split-KV partials (scores, softmax, numerators), then their merge
- * and the quantisation of the merged rows, one warp per head (more than 32 heads: merge by the last
- * CTA to finish, then the flat quantisation; same order, same bits).
+ * and the quantisation of the merged rows.
  * Visibility follows the reference's draft / verify / ar masks.  Replaces the
  * attention and o-projection input quantisation of
  * Attention.forward_sdlm_graph_kernel (src/bonsai_sft/gpu/model.py:989-1005) and the
@@ -307,7 +306,7 @@ int bm_rope_verify_attention(const void *xqkv, const void *q_w, const void *k_w,
  * CTA to finish, or, where the device holds the whole grid as thread-block clusters, through distributed shared memory:
  * writes the bf16 rows att_out [M, H*128] and folds each row's absmax into amax_out uint32 [M] by atomic
  * max (float bits; zero on entry).  bm_quant_rows_amax(att_out, amax_out, ...) then yields exactly the
- * codes and multipliers of bm_rope_verify_attention.  H % 4 == 0. */
+ * codes and multipliers of bm_rope_verify_attention.  H % 4 == 0, Hkv * ceil(M * H / Hkv / 4) <= 224 (the counters). */
 int bm_rope_verify_attention_rows(const void *xqkv, const void *q_w, const void *k_w, float eps,
                                   const void *cos_t, const void *sin_t, const void *positions, void *k_base,
                                   void *v_base, int M, int H, int Hkv, int kv_rows, int sigma,

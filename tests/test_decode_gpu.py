@@ -66,6 +66,35 @@ def test_forward_matches_oracle(oracle, geom, role, M, cache_len, n_pend):
     assert np.array_equal(oracle.torch_to_u16(kvd.cpu()), kv_np), "KV buffer differs"
 
 
+@pytest.mark.parametrize("role,M,cache_len,n_pend", [("ar", 1, 0, 0), ("ar", 1, 33, 0), ("verify", 9, 30, 0), ("draft", 16, 40, 8)])
+@pytest.mark.parametrize("pdl_stable", [False, True])
+def test_forward_of_more_than_32_heads_matches_oracle(oracle, role, M, cache_len, n_pend, pdl_stable):
+    """40 query heads: the merge to codes with two heads a warp, and the rows form of a single row."""
+    cfg = synthetic.make_config(dict(synthetic.TINY, n_heads=40, n_kv_heads=8, dim=512, ffn_dim=768), block_size=8)
+    sigma, m_max = 64, 17
+    model, state = _model(cfg, 4, sigma + m_max)
+    om = oracle.OracleModel(cfg, state, max_positions=sigma + m_max)
+    D, L, Hkv = 8, cfg["n_layers"], cfg["n_kv_heads"]
+    gen = torch.Generator().manual_seed(M + cache_len)
+    kv = (torch.randn(2, L, 1, Hkv, sigma + m_max, 128, generator=gen) * 0.5).to(torch.bfloat16)
+    tokens = torch.randint(0, cfg["vocab_size"], (M,), generator=gen)
+    positions = torch.arange(max(cache_len - 1, 0), max(cache_len - 1, 0) + M)
+    rid = oracle.ROLE_IDS[role]
+    ls, le = {"ar": (0, M), "verify": (0, min(D + 1, M)), "draft": (M - D, M)}[role]
+    kv_np = oracle.torch_to_u16(kv).copy()
+    want = om.forward(tokens.numpy(), positions.numpy(), kv_np, sigma, rid, cache_len, n_pend, ls, le)
+    kvd, tok, pos = kv.to(DEV), tokens.to(DEV), positions.to(DEV)
+    state_t = ops.new_step_state(DEV)
+    ops.set_step_state(state_t, cache_len, min(n_pend, max(M - D, 0)), rid, M - D)
+    kv_full = [(kvd[0, i][:, :, : sigma + M, :], kvd[1, i][:, :, : sigma + M, :]) for i in range(L)]
+    torch.cuda.synchronize()
+    logits = model.forward_sdlm_decode_graph_kernel(tok, pos, kv_full, M, state_t, ls, le, "t2", stable_state=pdl_stable)
+    torch.cuda.synchronize()
+    assert native.lib().bm_device_error() == 0
+    assert np.array_equal(logits.cpu().numpy().view(np.uint32), want.view(np.uint32)), "logits differ"
+    assert np.array_equal(oracle.torch_to_u16(kvd.cpu()), kv_np), "KV buffer differs"
+
+
 @pytest.mark.parametrize("rec", RECORDS, ids=lambda r: f"{r['geometry']}-D{r['cfg']['block_size']}-{r['mode']}-"
                                                          f"{r['accept']}" + ("-eos" if r.get("eos_ids") else "") +
                                                          ("-m1verify" if r.get("exact_m1_verify") else ""))

@@ -722,3 +722,54 @@ def test_threads_with_different_sizes_launch_one_kernel(oracle, make, sizes):
     assert status == [{native.BM_OK}] * len(calls)
     for (_, _, _, out), ref in zip(calls, want):
         assert all(torch.equal(a.view(torch.uint8), b.view(torch.uint8)) for a, b in zip(out, ref))
+
+
+@pytest.mark.parametrize("M,H,Hkv,sigma,cache_len,n_pend,D,role", [
+    (32, 32, 32, 256, 200, 0, 8, "ar"),        # 256 groups of four vectors
+    (32, 32, 8, 640, 513, 9, 8, "draft"),
+    (16, 40, 8, 512, 385, 8, 8, "draft"),      # above 32 heads some warps of the merge take two heads, or every warp
+    (9, 48, 16, 256, 129, 0, 8, "verify"),
+    (2, 64, 8, 128, 33, 0, 1, "ar"),
+    (3, 98, 14, 256, 256, 0, 1, "ar"),
+])
+def test_attention_codes_for_any_number_of_heads(oracle, M, H, Hkv, sigma, cache_len, n_pend, D, role):
+    """Codes take no counter and no row-absmax word of the scratch, whatever the number of heads: rows, codes, group sums and
+    multipliers against the oracle, from rotated queries and from the projection's output, the scratch's header untouched."""
+    gen = torch.Generator().manual_seed(H * 3 + M)
+    kv_rows, rid = sigma + M, oracle.ROLE_IDS[role]
+    xqkv = _bf16(gen, M, (H + 2 * Hkv) * 128, scale=2.0).to(DEV)
+    w = (1.0 + 0.1 * torch.randn(128, generator=gen)).to(torch.bfloat16).to(DEV)
+    cos, sin = (oracle.u16_to_torch(t).to(DEV) for t in _rope_tables(oracle, sigma + 40))
+    pos = (torch.arange(M) + max(cache_len - 1, 0)).to(torch.int64).to(DEV)
+    kv = _bf16(gen, 2, Hkv, kv_rows, 128, scale=1.5).to(DEV)
+    state = ops.new_step_state(DEV)
+    ops.set_step_state(state, cache_len, n_pend, rid, M - D)
+    scratch = ops.attention_scratch(M, H, sigma, DEV)
+    ka, va = kv[0].clone(), kv[1].clone()
+    q = ops.qknorm_rope_kvappend(xqkv, w, w, 1e-6, cos, sin, pos, H, Hkv, ka, va, sigma)
+    want = oracle.attention(_u16(oracle, q), _u16(oracle, ka), _u16(oracle, va), sigma, cache_len, n_pend, M - D, rid)
+    codes, mult = oracle.quant_rows(want)
+    sums = codes.astype(np.int32).reshape(M, H, 128).sum(-1)
+
+    def sink():
+        return [torch.empty(M, H * 128, dtype=dt, device=DEV) for dt in (torch.int8, torch.int8)] + [
+            torch.empty(M, H, dtype=torch.int32, device=DEV), torch.empty(M, 1, dtype=torch.float32, device=DEV)]
+    for pdl in (0, native.PDL_OVERLAP | native.PDL_STABLE_STATE):
+        for rope in (False, True):
+            for rows in (None, torch.empty(M, H * 128, dtype=torch.bfloat16, device=DEV)):
+                nat, prep, asum, s = sink()
+                kb, vb = kv[0].clone(), kv[1].clone()
+                torch.cuda.synchronize()               # (what a call reads early was written by launches that have completed)
+                if rope:
+                    ops.rope_verify_attention(xqkv, w, w, 1e-6, cos, sin, pos, H, Hkv, kb, vb, sigma, state, scratch,
+                                              out=(rows, nat, s), prep=(prep, asum), pdl=pdl)
+                else:
+                    ops.verify_attention(q, ka, va, sigma, state, scratch, out=(rows, nat, s), prep=(prep, asum), pdl=pdl)
+                torch.cuda.synchronize()
+                assert rows is None or np.array_equal(_u16(oracle, rows), want)
+                assert np.array_equal(nat.cpu().numpy(), codes)
+                assert np.array_equal(prep.cpu().numpy(), _permute16(codes))
+                assert np.array_equal(asum.cpu().numpy(), sums)
+                assert np.array_equal(s.cpu().numpy().reshape(-1).view(np.uint32), mult.reshape(-1).view(np.uint32))
+    assert int(scratch[:1024].sum().item()) == 0
+    assert native.lib().bm_device_error() == 0
