@@ -105,6 +105,9 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity
 // are visible.  launch_dependents: allow the next grid in the stream to start
 // its own prologue.  Both are no-ops for a kernel launched without the
 // programmatic-serialisation attribute.
+// A kernel that waits takes no `const ... *__restrict__`: that promises memory which nobody writes while the kernel runs, and
+// such a load may be made by the read-only path and moved ahead of the wait, but what the previous grid writes it may still be
+// writing when this one starts.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -158,10 +158,7 @@ __device__ __forceinline__ void emit_codes(const QuantSink &sink, size_t row_off
 // =============================================================================
 constexpr int kRowThreads = 512;
 
-__global__ void __launch_bounds__(kRowThreads) quant_rows_kernel(const uint16_t *__restrict__ x,
-                                                                 int K, QuantSink sink,
-                                                                 float *__restrict__ s_out,
-                                                                 int pdl) {
+__global__ void __launch_bounds__(kRowThreads) quant_rows_kernel(const uint16_t *x, int K, QuantSink sink, float *s_out, int pdl) {
     __shared__ float sh[kRowThreads / 32];
     pdl_launch_dependents();
     if (pdl) pdl_wait();
@@ -198,8 +195,7 @@ __global__ void __launch_bounds__(kRowThreads) quant_rows_kernel(const uint16_t 
 constexpr int kQuantAmaxThreads = 256;
 
 __global__ void __launch_bounds__(kQuantAmaxThreads) quant_rows_amax_kernel(
-    const uint16_t *__restrict__ x, const unsigned int *__restrict__ amax_in, unsigned int *amax_zero, int M, int K,
-    QuantSink sink, float *__restrict__ s_out, int pdl) {
+    const uint16_t *x, const unsigned int *amax_in, unsigned int *amax_zero, int M, int K, QuantSink sink, float *s_out, int pdl) {
     pdl_launch_dependents();
     if (pdl) pdl_wait();
     const int units = K / 8, lane = threadIdx.x & 31;
@@ -301,8 +297,7 @@ __global__ void __launch_bounds__(1024) rmsnorm_kernel(const NormParams p) {
 // shared memory between the absmax pass and the quantisation pass.
 // =============================================================================
 __global__ void __launch_bounds__(kRowThreads) silu_mul_quant_kernel(
-    const uint16_t *__restrict__ gu, int F, QuantSink sink, float *__restrict__ s_out,
-    uint16_t *__restrict__ inner_out, int pdl) {
+    const uint16_t *gu, int F, QuantSink sink, float *s_out, uint16_t *inner_out, int pdl) {
     extern __shared__ __align__(16) unsigned char dyn[];
     __shared__ float sh[kRowThreads / 32];
     pdl_launch_dependents();
@@ -542,10 +537,8 @@ constexpr int kPackGroupPairs = 4;       // pairs of groups per warp
 constexpr int kPackThreads = 256;
 
 template <bool FROZEN>
-__global__ void __launch_bounds__(kPackThreads) pack_t2_g128_kernel(const uint16_t *__restrict__ w, long long groups,
-                                                                    uint8_t *__restrict__ packed,
-                                                                    uint16_t *__restrict__ scale,
-                                                                    uint16_t *__restrict__ frozen) {
+__global__ void __launch_bounds__(kPackThreads) pack_t2_g128_kernel(const uint16_t *w, long long groups, uint8_t *packed,
+                                                                    uint16_t *scale, uint16_t *frozen) {
     // No launch_dependents: every product requests its weights before its own wait, and these are what is written here.  The
     // launch itself overlaps the previous one; nothing is read or written before this wait.
     pdl_wait();

@@ -36,3 +36,20 @@ def test_the_prompt_softmax_takes_whole_warps():
             for row0 in range(0, 40 * slab, vectors >> log_g):
                 rows = [row0 + (v >> log_g) for v in range(16 * warp, 16 * warp + 16)]
                 assert rows[0] == row0 + ((16 * warp) >> log_g) and len({r // slab for r in rows}) == 1
+
+
+def test_kernels_that_wait_promise_no_read_only_memory():
+    """A kernel that may start before its predecessor has finished reads memory that is written while it runs, so none of its
+    parameters may be declared read-only and unaliased: a load through one may be moved ahead of the wait."""
+    seen = 0
+    for name in sorted(os.listdir(native.CSRC)):
+        if not name.endswith((".cu", ".cuh")):
+            continue
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(native.CSRC, name)).read())
+        for m in re.finditer(r"__global__[^;{]*\{", text):
+            body = text[m.end():text.index("\n}\n", m.end())]
+            if "pdl_wait()" in body:
+                seen += 1
+                assert "__restrict__" not in m.group(0), f"{name}: {m.group(0)}"
+                assert not re.search(r"const[^;=]*__restrict__", body), f"{name}: {m.group(0)}"
+    assert seen >= 10
