@@ -88,6 +88,14 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
     return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
+// Eight bf16 values as they are stored: a signalling NaN becomes a quiet one (bm_f32_to_bf16 of a value from memory).
+__device__ __forceinline__ uint4 quiet8(uint4 v) {
+    uint32_t *w = &v.x;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] |= __vcmpgtu2(w[i] & 0x7fff7fffu, 0x7f807f80u) & 0x00400040u;
+    return v;
+}
+
 // h = bf16(h + r), the rounded sums also as they are stored.
 __device__ __forceinline__ uint4 add8(float (&h)[8], const float (&r)[8]) {
 #pragma unroll
@@ -271,6 +279,8 @@ __global__ void __launch_bounds__(1024) rmsnorm_kernel(const NormParams p) {
         float r[8];
         unpack8(reinterpret_cast<const uint4 *>(p.res + (size_t)(p.row0 + m) * p.dim)[t], r);
         hraw = add8(h, r);
+    } else {
+        hraw = quiet8(hraw);
     }
     if (p.h_out) reinterpret_cast<uint4 *>(p.h_out + (size_t)m * p.dim)[t] = hraw;
     float acc = 0.0f;

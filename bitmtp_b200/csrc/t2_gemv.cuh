@@ -435,6 +435,8 @@ __device__ __forceinline__ void gemv_stage_row_from_bf16(const GemvParams &p, un
             float rr[8];
             unpack8(reinterpret_cast<const uint4 *>(p.res)[t], rr);
             hraw = add8(h, rr);
+        } else {
+            hraw = quiet8(hraw);
         }
         if (blockIdx.x == 0 && p.h_out) reinterpret_cast<uint4 *>(p.h_out)[t] = hraw;
         float acc = 0.0f;

@@ -773,3 +773,25 @@ def test_attention_codes_for_any_number_of_heads(oracle, M, H, Hkv, sigma, cache
                 assert np.array_equal(s.cpu().numpy().reshape(-1).view(np.uint32), mult.reshape(-1).view(np.uint32))
     assert int(scratch[:1024].sum().item()) == 0
     assert native.lib().bm_device_error() == 0
+
+
+def test_a_gathered_row_is_kept_with_its_nans_quiet():
+    """The residual row that the first norm of a replay keeps, of a table row with NaNs: quiet ones keep their bits, signalling
+    ones become quiet with sign and payload kept, infinities stay (the conversion's host form), for both launches that gather."""
+    from bitmtp_b200 import synthetic
+    dim = 2048
+    table = torch.randn(4, dim, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).view(torch.int16)
+    odd = torch.tensor([0x7f81, 0x7fa0, 0x7fc0, 0x7fff, 0x7f80, 0x7f7f, 0x0001, 0xff81, 0xffbf, 0xffc1, 0xff80, 0xffff], dtype=torch.int32)
+    table[2, 5:17] = odd.to(torch.int16)
+    bits = table[2].numpy().view(np.uint16)
+    want = np.where((bits & 0x7fff) > 0x7f80, bits | 0x40, bits)
+    assert not np.array_equal(want, bits)
+    x = table.view(torch.bfloat16).to(DEV)
+    ids, w = torch.tensor([2], dtype=torch.int64, device=DEV), torch.ones(dim, dtype=torch.bfloat16, device=DEV)
+    out = ops.rmsnorm_fused(x, w, 1e-6, gather=ids, want_h=True)
+    B, ws = synthetic.device_ternary(256, dim, torch.Generator(device=DEV).manual_seed(2), DEV)
+    h = torch.empty(1, dim, dtype=torch.bfloat16, device=DEV)
+    y = torch.empty(1, 256, dtype=torch.bfloat16, device=DEV)
+    ops.gemv_row_fused(2, x, B, ws, out=y, gather=ids, norm_w=w, eps=1e-6, h_out=h)
+    for got in (out["h"], h):
+        assert np.array_equal(got.cpu().view(torch.int16).numpy().reshape(-1).view(np.uint16), want)
