@@ -1239,8 +1239,14 @@ int bm_prompt_attention(const void *q, const void *k_base, const void *v_base, i
             const int rc = launch_ex<bm::prompt_hist_kernel>(hgrid, dim3(bm::kPaThreads), bm::kPaSmem, st, p.pdl, hp);
             if (rc != BM_OK) return rc;
         }
-        return launch_ex<bm::attn_fused_kernel<2, false, bm::kMergeHistory>>(dim3(pl.n_slabs, Hkv, pl.Z), dim3(bm::kAttnThreads),
-                         bm::attn_smem_bytes(pl.nv, true), st, p.pdl, p);
+        const dim3 sgrid(pl.n_slabs, Hkv, pl.Z), block(bm::kAttnThreads);
+        const size_t ssmem = bm::attn_smem_bytes(pl.nv, true);
+        // Three CTAs an SM at most: the build with the registers that a thread wants, else the one of which an SM holds four.
+        // us by the first and the second, 16 / 8 heads: 64 rows behind 2048 keys (128 CTAs) 47.1 and 49.4, 128 behind 1024 (256)
+        // 45.5 and 46.9, 192 behind 1024 (384) 68.6 and 69.9, 256 behind 1024 (512) 90.5 and 87.0, 512 without history 66.7 and 61.7.
+        if ((long long)pl.n_slabs * Hkv * pl.Z <= 3 * current_device().sm_count)
+            return launch_ex<bm::attn_fused_kernel<2, false, bm::kMergeHistoryFew>>(sgrid, block, ssmem, st, p.pdl, p);
+        return launch_ex<bm::attn_fused_kernel<2, false, bm::kMergeHistory>>(sgrid, block, ssmem, st, p.pdl, p);
     }
     const dim3 grid(pl.units, Hkv, pl.Z);
     return pl.nv == 1 ? launch_ex<bm::attn_fused_kernel<1, false>>(grid, dim3(bm::kAttnThreads), smem, st, p.pdl, p)

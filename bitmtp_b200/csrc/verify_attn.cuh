@@ -122,7 +122,7 @@ inline AttnSplit attn_split(int NJ, int QV, int Hkv, int sms) {
 }
 
 // K (padded rows; after level 0 its space takes the sub-chunk numerators), V, queries, weights, sub-chunk max / sum.
-// `slab`: kMergeHistory, whose own rows are one sub-chunk (the K rows' space is then that of the numerators).
+// `slab`: kMergeHistory and kMergeHistoryFew, whose own rows are one sub-chunk (the K rows' space is then that of the numerators).
 __host__ __device__ constexpr int attn_key_bytes(int nv, bool slab) {
     return slab ? kAttnSub * 4 * nv * 128 * 4 : BM_ATTN_SUPER * kKeyStride * 2;
 }
@@ -486,14 +486,16 @@ __device__ __forceinline__ float attn_row_amax(const float (&v)[4]) {
 //   kMergeHistory  prompt mode only: prompt_hist_kernel has made the partials of the history super-chunks.  blockIdx.x is
 //                  the slab; its CTAs make the partial of the slab's own rows, keep it in registers and merge at once.  A
 //                  build of its own: as a run-time switch it made every other prompt-mode call 3.6 % slower (1 to 9 % over
-//                  117 calls of 17 to 512 rows).  It stages 16 keys, not 128, so four CTAs share an SM (512 rows of 16 heads: 70.5 us a call without history, now 62.3).
+//                  117 calls of 17 to 512 rows).  It stages 16 keys, not 128, so four CTAs share an SM (512 rows of 16 heads: 70.5
+//                  us a call without history, now 62.3), which leaves a thread 64 registers and costs a call of few CTAs 2 us.
+//   kMergeHistoryFew  the same, for few CTAs: 79 registers, three CTAs per SM
 //   kMergeLater    the next launch (attn_merge_quant_kernel): this one ends with its partials.  A replay wants the rows as
 //                  INT8 codes, for which a launch has to follow anyway; the end of a launch is then the only hand-over
 //                  (fence, ticket, read-back and row-absmax atomics took 3.4 us of 12.4 at width 16).
 // Attention to codes in a chain of such launches, 16 / 8 heads, before (ticket, up to 8 vectors a CTA, two CTAs per SM) and
 // now, us: width 16 behind 120 / 300 / 600 / 900 keys 11.0 / 11.4 / 13.4 / 15.8, now 7.6 / 8.4 / 10.8 / 12.9; width 9 behind
 // 120 / 600 10.2 / 10.9, now 6.5 / 8.3; 32 / 8 heads, width 16 behind 1100 keys 34.4, now 25.6.
-enum : int { kMergeTicket = 0, kMergeCluster = 1, kMergeHistory = 2, kMergeLater = 3 };
+enum : int { kMergeTicket = 0, kMergeCluster = 1, kMergeHistory = 2, kMergeLater = 3, kMergeHistoryFew = 4 };
 
 // 256 threads.  NV: widest split (4 * NV query vectors per CTA); ROPE: queries and the replay's own K/V rows are made here
 // from the qkv projection output.  Grid: replays (Hkv, NJ * finest query groups) - the (super-chunk, query group) pairs with
@@ -504,7 +506,7 @@ __global__ void __launch_bounds__(kAttnThreads, MERGE == kMergeHistory ? 4 : 2) 
     extern __shared__ __align__(16) unsigned char dyn[];
     __shared__ unsigned int sh_ticket;
     constexpr int QC = 4 * NV, NQW = (QC + kAttnWarps - 1) / kAttnWarps;      // vectors per CTA; per warp outside level 0
-    constexpr bool CLUSTER = MERGE == kMergeCluster, HIST_DONE = MERGE == kMergeHistory;
+    constexpr bool CLUSTER = MERGE == kMergeCluster, HIST_DONE = MERGE == kMergeHistory || MERGE == kMergeHistoryFew;
     pdl_launch_dependents();
     // BM_PDL_STABLE_STATE: the step record, the positions and the history rows were written by launches
     // that had completed before this call's chain of overlapped launches began, so they may be read

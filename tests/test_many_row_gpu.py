@@ -68,6 +68,14 @@ def test_prompts_that_end_inside_a_warp(T, H, Hkv):
     assert torch.equal(_prompt(q, k, v, 2560).view(torch.int16), _by_slab(q, k, v, 2560).view(torch.int16))
 
 
+@pytest.mark.parametrize("T,hist0,H,Hkv", [(64, 2048, 16, 8), (207, 1025, 16, 8), (209, 1025, 16, 8), (96, 1300, 32, 8), (97, 1300, 32, 8),
+                                           (432, 1100, 8, 1), (433, 1100, 8, 1)])
+def test_tiles_then_few_or_many_slab_blocks(T, hist0, H, Hkv):
+    """Both builds of the slab kernel behind the tiles, next to the line between them (three blocks per SM)."""
+    q, k, v = _attention_inputs(T, hist0, H, Hkv, T)
+    assert torch.equal(_prompt(q, k, v, hist0, calls=2).view(torch.int16), _by_slab(q, k, v, hist0).view(torch.int16))
+
+
 def test_rows_past_a_history_do_not_reach_it():
     """Infinities and NaN in K / V rows that a slab may not see stay out of its results."""
     for T, hist0, keep in ((64, 160, 32), (512, 160, 400)):       # the general kernel, the tiles
