@@ -118,6 +118,10 @@ inline AttnSplit attn_split(int NJ, int QV, int Hkv, int sms) {
         r.groups = std::max(r.groups, attn_groups(QV, best));
         r.pairs = std::max(r.pairs, (n + 1) * attn_groups(QV, best));
     }
+    // Up to 16 vectors a kv head, a CTA an SM: the finest split's grid, CTAs without work and all.  1.7B replays in a segment of
+    // 1024 with the smaller grid / this, us: width 5 behind 300 and 500 keys 807 / 803 and 819 / 809, width 6 behind 300 827 / 815,
+    // width 8 behind 120 830 / 824, behind 300 847 / 842.  Wider ones: level (width 9), or now one, now the other (width 16).
+    if (r.single && attn_groups(QV, widest) == 1) r.pairs = NJ * attn_groups(QV, 1);
     return r;
 }
 
