@@ -795,3 +795,32 @@ def test_a_gathered_row_is_kept_with_its_nans_quiet():
     ops.gemv_row_fused(2, x, B, ws, out=y, gather=ids, norm_w=w, eps=1e-6, h_out=h)
     for got in (out["h"], h):
         assert np.array_equal(got.cpu().view(torch.int16).numpy().reshape(-1).view(np.uint16), want)
+
+
+@pytest.mark.parametrize("M,H,Hkv,sigma,cache_len", [(1, 40, 8, 1024, 1000), (6, 16, 8, 4096, 2100), (9, 40, 8, 1024, 513),
+                                                     (16, 32, 8, 2048, 2000)])
+def test_rows_leave_the_counters_zero(oracle, M, H, Hkv, sigma, cache_len):
+    """The rows call where its grid does not go as clusters (merge by the last block to draw a ticket), for 4 to 16 vectors a
+    block: several histories over one scratch, rows against the codes call's, every counter back at zero."""
+    gen = torch.Generator().manual_seed(M + H)
+    xqkv = _bf16(gen, M, (H + 2 * Hkv) * 128, scale=2.0).to(DEV)
+    w = (1.0 + 0.1 * torch.randn(128, generator=gen)).to(torch.bfloat16).to(DEV)
+    cos, sin = (oracle.u16_to_torch(t).to(DEV) for t in _rope_tables(oracle, sigma + 40))
+    kv = _bf16(gen, 2, Hkv, sigma + M, 128, scale=1.5).to(DEV)
+    state = ops.new_step_state(DEV)
+    scratch, other = (ops.attention_scratch(M, H, sigma, DEV) for _ in range(2))
+    for cl in (cache_len, 1, cache_len // 2, sigma):
+        pos = (torch.arange(M) + cl).clamp(max=sigma + 39).to(torch.int64).to(DEV)
+        ops.set_step_state(state, cl, 0, oracle.ROLE_IDS["ar"], M)
+        rows, want = (torch.empty(M, H * 128, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+        amax = torch.zeros(M, dtype=torch.int32, device=DEV)
+        ops.rope_verify_attention_rows(xqkv, w, w, 1e-6, cos, sin, pos, H, Hkv, kv[0], kv[1], sigma, state, scratch, att=rows,
+                                       amax=amax)
+        ops.rope_verify_attention(xqkv, w, w, 1e-6, cos, sin, pos, H, Hkv, kv[0], kv[1], sigma, state, other,
+                                  out=(want, torch.empty(M, H * 128, dtype=torch.int8, device=DEV),
+                                       torch.empty(M, 1, dtype=torch.float32, device=DEV)))
+        torch.cuda.synchronize()
+        assert torch.equal(rows.view(torch.int16), want.view(torch.int16)), cl
+        assert torch.equal(amax.view(torch.float32), want.float().abs().amax(dim=1)), cl
+        assert int(scratch[:1024].sum().item()) == 0, cl
+    assert native.lib().bm_device_error() == 0
