@@ -44,16 +44,6 @@ constexpr int kRwSmemBudget = 226 * 1024;   // 1 KB of the 227 KB is run-time al
 
 enum : int { kErrRowWarpWaitTimeout = 2 };  // a weight panel never arrived
 
-// mbar_wait_bounded with its loop left to the compiler, which unrolls it: here the wait is the main loop's, not code that runs
-// once (28672 x 8192 at eight tokens 24.8 us, with the rolled loop 25.0).
-__device__ __forceinline__ bool rowwarp_wait(uint64_t *bar, uint32_t parity) {
-    for (int it = 0; it < (1 << 22); ++it) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if (it > 64) __nanosleep(64);
-    }
-    return false;
-}
-
 struct RowWarpParams {
     CUtensorMap tmap;       // uint8 [N, K/4], box [16 rows, 128 bytes], 128-byte swizzle
     GemvParams g;
@@ -307,7 +297,7 @@ __global__ void __launch_bounds__(kRwMaxWarps * 32, 1) t2_gemv_rowwarp_kernel(co
                 const unsigned char *arow = arow0 + (size_t)pan * 4 * BM_GROUP, *nbp = nb_base + (size_t)pan * 4 * 64;
                 const int G = 4 * pan;
                 if (pp % PB == 0) {
-                    ok = __all_sync(0xffffffffu, rowwarp_wait(&bars[cst], cpar));
+                    ok = __all_sync(0xffffffffu, mbar_wait_bounded<4>(&bars[cst], cpar));
                     if (!ok) break;
                 }
                 const unsigned char *stage = ring + cst * kStage + (pp % PB) * kRwStageBytes;
