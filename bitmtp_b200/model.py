@@ -324,7 +324,6 @@ class StepWorkspace:
         self.s = buf((M, 1), f32)
         self.xqkv = buf((M, qkv), bf)
         self.qrot = buf((M, args.n_heads, args.head_dim), bf)
-        self.att = buf((M, q_dim), bf)
         self.att_q = buf((M, q_dim), i8)
         self.att_s = buf((M, 1), f32)
         self.attn_out = buf((M, args.dim), bf)
@@ -343,8 +342,11 @@ class StepWorkspace:
         self.h_sum = buf((M, args.dim // 128), i32)
         self.inner = buf((M, args.ffn_dim), bf)
         self.inner_amax = torch.zeros((2, M), dtype=i32, device=device)   # row absmax bits, two slots used in turn
-        self.att_amax = torch.zeros((2, M), dtype=i32, device=device)
-        self.h2 = buf((M, args.dim), bf)            # second residual buffer of the width-1 fused path
+        if M == 1:
+            # attention rows and their absmax bits, and the second residual buffer of the width-1 fused path
+            self.att = buf((M, q_dim), bf)
+            self.att_amax = torch.zeros((2, M), dtype=i32, device=device)
+            self.h2 = buf((M, args.dim), bf)
         self.n_pad = n_pad
 
 
@@ -371,8 +373,8 @@ class Transformer(nn.Module):
         self.fused_ffn = os.environ.get("BM_FUSED_FFN", "1") != "0"
         # q/k norm + RoPE + KV append folded into the attention kernel (BM_FUSED_ROPE=0: own launch)
         self.fused_rope = os.environ.get("BM_FUSED_ROPE", "1") != "0"
-        # width-1 replays: RMSNorm / quantisation inside the consuming GEMV, 6 launches per layer instead
-        # of 10 (BM_FUSED_AR=0: the general sequence)
+        # width-1 replays: RMSNorm / quantisation inside the consuming GEMV, 5 launches per layer instead
+        # of 9 (BM_FUSED_AR=0: the general sequence)
         self.fused_ar = os.environ.get("BM_FUSED_AR", "1") != "0"
 
     def tie_weights(self) -> None:
@@ -470,7 +472,7 @@ class Transformer(nn.Module):
 
     def _layers_ar_fused(self, W, token_values, positions, kv_full, kv_rows, sigma, attn_mask, attn_scratch,
                          pdl, attn_pdl) -> None:
-        """Width-1 layer stack in six launches per layer: each projection quantises (and, for qkv and
+        """Width-1 layer stack in five launches per layer: each projection quantises (and, for qkv and
         gate|up, normalises) its own input row.  The residual stream alternates between W.h2 and W.h and
         ends in W.h, where the final norm expects it."""
         a = self.args
@@ -501,7 +503,7 @@ class Transformer(nn.Module):
 
     def _layers_by_operator(self, W, token_values, positions, kv_full, kv_rows, sigma, attn_mask, attn_scratch,
                             pdl, attn_pdl) -> None:
-        """The layer stack as ten launches per layer (every geometry, every width)."""
+        """The layer stack as nine launches per layer (every geometry, every width; ten where the rotation has its own)."""
         a = self.args
         M = W.M
         eps = a.norm_eps
