@@ -63,7 +63,7 @@ def parse_args():
     ap.add_argument("--shape", default="151936x2048", help="gemv-one: NxK")
     ap.add_argument("--w", type=int, default=1, help="gemv-one, attention: width")
     ap.add_argument("--cache-len", type=int, default=700, help="attention: history rows")
-    ap.add_argument("--layers", type=int, default=28, help="attention: dependent launches per graph, one K/V plane each")
+    ap.add_argument("--layers", type=int, default=28, help="attention: dependent calls per graph, one K/V plane each")
     ap.add_argument("--rows", type=int, default=256, help="prompt-gemm: prompt rows")
     ap.add_argument("--path", default="auto", choices=["auto", "dp4a", "mma", "rowwarp", "direct"])
     ap.add_argument("--calls", type=int, default=0, help="gemv-one: launches per step")
@@ -1172,8 +1172,9 @@ def run_reference_decode(args) -> dict:
 
 # ----------------------------------------------------------------------------- single-kernel workloads
 def run_kernel(args, world, rank, local, dist):
-    """`attention`: the replay's attention launch (q/k norm, RoPE, KV append, split-KV, merge) on the 1.7B head
-    geometry, `--layers` dependent launches per graph over distinct K/V planes.  `prompt-gemm`: the many-row
+    """`attention`: the replay's attention (q/k norm, RoPE, KV append, split-KV, merge) on the 1.7B head geometry as a
+    replay of that width calls it - width 1 to rows in one launch, wider to INT8 codes in two -, `--layers` dependent
+    calls per graph over distinct K/V planes.  `prompt-gemm`: the many-row
     T2 x int8 GEMM of the prompt forward over weight copies that exceed L2.  One JSON line each; these are the
     commands the ncu summaries under profiles/ were captured from."""
     import torch
@@ -1202,14 +1203,24 @@ def run_kernel(args, world, rank, local, dist):
         ops.set_step_state(state, cl, min(8, max(M - 8, 0)), role, max(M - 8, 0))
         pdl = native.PDL_OVERLAP | native.PDL_STABLE_STATE
 
+        codes = torch.empty(M, H * 128, dtype=torch.int8, device=device)
+        sums = torch.empty(M, H, dtype=torch.int32, device=device)
+        mult = torch.empty(M, 1, dtype=torch.float32, device=device)
+
         def chain():
             for i in range(L):
-                ops.rope_verify_attention_rows(xqkv, qw, qw, 1e-6, cos, sin, pos, H, Hkv, _LayerView(kvb[0, i], kv_rows),
-                                               _LayerView(kvb[1, i], kv_rows), sigma, state, scratch, att=att,
-                                               amax=amax[i & 1], pdl=pdl)
-        calls = L
-        alg = 2 * Hkv * (cl + M) * 256 + M * (H + 2 * Hkv) * 256 + M * H * 256      # live K/V rows + qkv in + rows out
-        label = f"attention launch, 16/8 heads, width {M}, cache_len {cl}, segment {sigma}, {L} dependent launches per graph"
+                planes = _LayerView(kvb[0, i], kv_rows), _LayerView(kvb[1, i], kv_rows)
+                if M == 1:
+                    ops.rope_verify_attention_rows(xqkv, qw, qw, 1e-6, cos, sin, pos, H, Hkv, *planes, sigma, state, scratch,
+                                                   att=att, amax=amax[i & 1], pdl=pdl)
+                else:
+                    ops.rope_verify_attention(xqkv, qw, qw, 1e-6, cos, sin, pos, H, Hkv, *planes, sigma, state, scratch,
+                                              out=(None, None, mult), prep=(codes, sums), pdl=pdl)
+        calls, launches = L, L if M == 1 else 2 * L
+        # live K/V rows + qkv in + rows or codes out
+        alg = 2 * Hkv * (cl + M) * 256 + M * (H + 2 * Hkv) * 256 + M * H * (256 if M == 1 else 128)
+        label = (f"attention to {'rows' if M == 1 else 'codes'}, 16/8 heads, width {M}, cache_len {cl}, segment {sigma}, "
+                 f"{L} dependent calls of {launches // L} launch(es) per graph")
         bound, unit, scale, pk = "hbm", "GB/s", 1e9, peak
     else:
         n, k = (int(x) for x in args.shape.lower().split("x"))
@@ -1224,7 +1235,7 @@ def run_kernel(args, world, rank, local, dist):
         def chain():
             for B, ws in Bs:
                 ops.t2_gemm_wide(A, asum, B, sc, ws, out=C)
-        calls = copies
+        calls = launches = copies
         alg = 2 * T * n * k                                                             # integer multiply-adds x 2
         label = f"prompt GEMM {n}x{k}, {T} rows, {copies} weight copies (> L2) per graph"
         bound, unit, scale = "tensor", "TOP/s", 1e12
@@ -1240,15 +1251,15 @@ def run_kernel(args, world, rank, local, dist):
         raise RuntimeError(f"device error word = {err}")
     us = ms * 1e3 / (steps * calls)
     achieved = alg / (us * 1e-6) / scale
-    return {"metric": f"{args.workload} us per launch", "value": round(us, 3), "unit": "us", "n_gpus": world, "steps": steps,
+    return {"metric": f"{args.workload} us per {'call' if args.workload == 'attention' else 'launch'}", "value": round(us, 3), "unit": "us", "n_gpus": world, "steps": steps,
             "warmup": warmup, "ms_per_step": round(ms / steps, 5), "higher_is_better": False, "scaling": "weak",
             "vs_baseline": None, "dtype": "bf16 -> fp32" if args.workload == "attention" else "s8 x ternary -> s32",
             "data": "synthetic", "config": {"workload": label, "timing": "CUDA events around graph replays"},
-            "gpu_launches": steps * calls, "clocks": clocks,
+            "gpu_launches": steps * launches, "clocks": clocks,
             "roofline": {"bound": bound, "achieved": round(achieved, 3), "peak": pk, "unit": unit,
                          "frac": round(achieved / pk, 5), "traffic": None, "peak_kind": peak_kind,
                          "note": "peak = measured bf16 cuBLAS rate; the int8 tensor path is nominally 2x that"
-                         if bound == "tensor" else "algorithmic bytes = live K/V rows + the replay's qkv rows in and attention rows out"}}
+                         if bound == "tensor" else "algorithmic bytes = live K/V rows + the replay's qkv rows in and attention rows or codes out"}}
 
 
 def main():
