@@ -70,8 +70,9 @@ BM_HD uint16_t bm_f32_to_bf16(float f) {
 // fp32 value after one bf16 rounding.
 BM_HD float bm_bf16_rn(float f) { return bm_bf16_to_f32(bm_f32_to_bf16(f)); }
 
-// e^x.  Range reduction x = n*ln2 + r with a split ln2, degree-6 polynomial
-// for e^r on |r| <= ln2/2, exponent inserted with integer arithmetic.
+// e^x.  Range reduction x = n*ln2 + r with ln2 in two parts (Cody and Waite, Software Manual for the Elementary
+// Functions; the parts as in Moshier's Cephes library, exp.c), the Taylor polynomial of degree 6 for e^r on
+// |r| <= ln2/2, exponent inserted with integer arithmetic.
 // Below -87 the result is 0, above 88 it is +inf (callers: softmax weights with
 // x <= 0, SiLU with any x, confidence with x <= 0).
 BM_HD float bm_expf(float x) {

@@ -10,7 +10,7 @@
 // partials (max, sum, 128 numerators) that the slab's own CTA of attn_fused_kernel then merges in order.
 //
 // The work is fp32 arithmetic: 2 * 128 multiply-adds per (query vector, key).  Every one of them is the fma of
-// attn_sub_pass, in the same chain (scores ascending in d, numerators ascending in the key, sub-chunks
+// attn_level0, in the same chain (scores ascending in d, numerators ascending in the key, sub-chunks
 // ascending, the weight sum as the butterfly over the 32 keys), so the partials are the same bits; tensor
 // cores would not give that order.  512 rows behind 2048 keys, 16 heads: 657 us by attn_fused_kernel alone; called from
 // the host 414 us with scalar fmas and 356 with packed ones and an exponential without branches and conversions; 339 in

@@ -22,10 +22,10 @@
 //
 // Scratch (caller-allocated, bm_verify_attention_scratch_bytes; zero before the first call, the
 // kernel leaves its counters zero):
-//   1024 bytes                 224 ticket counters, then 32 row-absmax words
+//   1024 bytes                 224 ticket counters (rows wanted)
 //   pm, pl fp32 [M, H, NJ]      super-chunk max / sum
 //   po   fp32 [M, H, NJ, 128]   super-chunk numerators
-//   rows bf16 [M, H*128]        attention rows when the caller passes no att_out
+//   rows bf16 [M, H*128]        attention rows between merge and codes (above 32 heads) when the caller passes no att_out
 //   NJ = ceil(sigma/128) + 1; super-chunk NJ-1 holds the rows appended by this replay.
 #pragma once
 
@@ -497,8 +497,8 @@ __device__ __forceinline__ float attn_row_amax(const float (&v)[4]) {
 //                  INT8 codes, for which a launch has to follow anyway; the end of a launch is then the only hand-over
 //                  (fence, ticket, read-back and row-absmax atomics took 3.4 us of 12.4 at width 16).
 // Attention to codes in a chain of such launches, 16 / 8 heads, before (ticket, up to 8 vectors a CTA, two CTAs per SM) and
-// now, us: width 16 behind 120 / 300 / 600 / 900 keys 11.0 / 11.4 / 13.4 / 15.8, now 7.6 / 8.4 / 10.8 / 12.9; width 9 behind
-// 120 / 600 10.2 / 10.9, now 6.5 / 8.3; 32 / 8 heads, width 16 behind 1100 keys 34.4, now 25.6.
+// now, us: width 16 behind 120 / 300 / 600 / 900 keys 11.0 / 11.4 / 13.4 / 15.8, now 6.3 / 7.7 / 9.4 / 11.6; width 9 behind
+// 120 / 600 10.2 / 10.9, now 6.2 / 7.6; 32 / 8 heads, width 16 behind 1100 keys 34.4, now 23.8.
 enum : int { kMergeTicket = 0, kMergeCluster = 1, kMergeHistory = 2, kMergeLater = 3, kMergeHistoryFew = 4 };
 
 // 256 threads.  NV: widest split (4 * NV query vectors per CTA); ROPE: queries and the replay's own K/V rows are made here
