@@ -751,7 +751,7 @@ int bm_t2_gemv_row_fused(int src_mode, const void *x, const void *gather, int ga
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // A few MB of weights: the register-only kernel (one memory round trip after the row is staged).
     if (!staged && bm::direct_row_fits(N, K) && (size_t)(silu ? 2 : 1) * N * K / 4 <= kDirectMaxBytes) {
-        const int maxp = K <= 2048 ? 1 : (K <= 6144 ? 3 : 5), cols = bm::direct_row_cols(N, K, sms);
+        const int maxp = K <= 2048 ? 1 : (K <= 6144 ? 3 : 5), cols = bm::direct_row_cols(N, K, silu, src_mode == 2, sms);
         const dim3 grid((unsigned)((N + cols * bm::kDirectWarps - 1) / (cols * bm::kDirectWarps))), block(bm::kGemvThreads);
 #define BM_ROW_CASE(S_, MP_, C_)                                                                                        \
         if (silu == S_ && maxp == MP_ && cols == C_)                                                                    \

@@ -201,9 +201,9 @@ __global__ void __launch_bounds__(kDirectWarps * 32) t2_gemv_direct_kernel(const
 // the previous kernel.  Same results as t2_gemv_mma_kernel with src_mode != 0, bit for bit.
 //
 // What bounds it is the row's preparation, which every CTA repeats: some 600 instructions in each of its 8 warps.  So a warp
-// computes COLS columns, as many as leave two CTAs per SM (direct_row_cols): with one column and five CTAs per SM the
-// preparation alone was 3 us of a gate|up launch (6144 columns), and 28 of its 768 CTAs were a wave of their own.  In a
-// width-1 replay gate|up takes 6.4 us with one column, 4.7 with three; the whole replay 686 us, now 645.
+// computes COLS columns (direct_row_cols): with one column and five CTAs per SM the preparation alone was 3 us of a gate|up
+// launch (6144 columns), and 28 of its 768 CTAs were a wave of their own.  In a width-1 replay gate|up takes 6.4 us with one
+// column, 4.7 with three.
 constexpr int kDirectRowAsumOff = 2048 * kDirectMaxPasses;                 // int32 [K/128]
 constexpr int kDirectRowInvsOff = kDirectRowAsumOff + 4 * 16 * kDirectMaxPasses;   // float [16]
 constexpr int kDirectRowShOff = kDirectRowInvsOff + 64;                    // float [32]
@@ -214,10 +214,16 @@ __host__ __device__ inline bool direct_row_fits(int N, int K) {
 }
 
 // Columns per warp for N output columns: more than one only where a row's weights are one pass (K <= 2048), whose registers
-// leave room for them.
-__host__ __device__ inline int direct_row_cols(int N, int K, int sms) {
-    const int c = K <= 2048 ? (N + 16 * sms - 1) / (16 * sms) : 1;
-    return c < 1 ? 1 : (c > 3 ? 3 : c);
+// leave room for them.  Forced to 1 / 2 / 3 in chains of overlapped calls over weights that exceed L2, us: three are best from 1024
+// columns on, though they leave most SMs without a CTA at first (o projection, 2048 x 2048 with known absmax, 2.9 / 2.7 / 2.3;
+// with a norm 4.3 / 3.8 / 2.7, its SiLU form 5.0 / 4.6 / 3.4; 4096 x 2048 with a norm 4.6 / 4.4 / 4.3).  Below, level (512 x 2048 2.0 /
+// 2.1 / 2.2).  Half a row without norm or SiLU is little to prepare: one column up to 41 an SM (3072 x 1024 2.6 / 3.1 / 3.1, 6144 level),
+// then two (8192 x 1024 4.6 / 3.3 / 3.4).  SiLU with three columns holds two CTAs an SM, so two columns where they would not all
+// be resident (8192 x 2048 7.8 / 6.0 / 7.7).
+inline int direct_row_cols(int N, int K, bool silu, bool norm, int sms) {
+    if (K > 2048 || N < 1024) return 1;
+    if (K <= 1024 && !silu && !norm) return N <= 41 * sms ? 1 : 2;
+    return silu && N > 48 * sms ? 2 : 3;
 }
 
 template <bool SILU, int MAXP, int COLS>

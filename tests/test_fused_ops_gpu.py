@@ -824,3 +824,11 @@ def test_rows_leave_the_counters_zero(oracle, M, H, Hkv, sigma, cache_len):
         assert torch.equal(amax.view(torch.float32), want.float().abs().amax(dim=1)), cl
         assert int(scratch[:1024].sum().item()) == 0, cl
     assert native.lib().bm_device_error() == 0
+
+
+@pytest.mark.parametrize("src_mode,N,K,silu", [(2, 1016, 2048, False), (2, 1024, 2048, False), (1, 1032, 2048, False), (1, 2048, 2048, False),
+                                               (2, 2048, 2048, True), (1, 1040, 1024, True), (1, 3072, 1024, False), (1, 6064, 1024, False),
+                                               (1, 6072, 1024, False), (1, 8192, 512, False), (2, 7104, 2048, True), (1, 7120, 1024, True)])
+def test_width1_row_fused_columns_at_the_lines(src_mode, N, K, silu):
+    """One to three columns a warp, on both sides of each line of the rule that picks them, the last block full and not."""
+    test_width1_row_fused_register_kernel_equals_staged_kernel(src_mode, N, K, silu)
