@@ -948,7 +948,7 @@ int verify_attention_impl(const void *q, const RopeInputs *rope, const void *k_b
     if (H > bm::kAttnMaxHeads) return BM_EINVAL;
     if (amax_rows != nullptr ? Hkv * bm::attn_groups(QV, 1) > bm::kAttnTickets : (H % 2) != 0) return BM_EINVAL;
     bm::AttnParams p = {};
-    const bm::AttnSplit split = bm::attn_split(NJ, QV, Hkv, current_device().sm_count);
+    const bm::AttnSplit split = bm::attn_split(NJ, QV, Hkv, current_device().sm_count, amax_rows != nullptr);
     if (split.pairs > 65535) return BM_EINVAL;                    // one grid dimension
     const int nv = bm::attn_nv(QV);                               // widest split: the kernel's build
     std::copy(split.pick, split.pick + NJ, p.pick);

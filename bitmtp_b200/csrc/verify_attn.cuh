@@ -91,7 +91,9 @@ __host__ __device__ inline int attn_groups(int QV, int nv) { return (QV + 4 * nv
 // The splits of a replay over a segment of NJ - 1 history super-chunks.  The cost of n of them at a split is the time of the
 // fullest SM, in units of about half a microsecond: a CTA alone takes 2 nv + 5 (7.4 us to codes with nv = 2, 9.2 with 3, 10.5
 // with 4); two that share an SM overlap, 3 nv + 5 for the pair; an odd one after pairs takes 0.6 of a pair.  Where no split
-// needs more CTAs than SMs, only such are taken and each CTA gets an SM to itself.  The grid is that of the largest pick, not
+// needs more CTAs than SMs, only such are taken and each CTA gets an SM to itself (codes only: `rows` calls, whose last launch
+// merges, do better with two narrow CTAs an SM; held to one, 50 of 781 of them were 3 to 28 % slower than before there were wide
+// CTAs, now 15, by 10 % at most).  The grid is that of the largest pick, not
 // of the finest split: CTAs without work delayed the others by up to 2.6 us (2112 CTAs, 256 of them working).
 // Fitted to the attention to codes for every nv, over 1566 calls (five head counts, 2 to 32 rows, 1 to 32 super-chunks, segments of
 // 256 to 4096): 0.2 % over the fastest split on average, where the rule before (w (2 nv + 3) for w CTAs, grid of the finest split) was
@@ -102,10 +104,10 @@ struct AttnSplit {
     bool single;                // the working CTAs never exceed the SMs
     int groups, pairs;          // most query groups, most (super-chunk, query group) pairs of any n
 };
-inline AttnSplit attn_split(int NJ, int QV, int Hkv, int sms) {
+inline AttnSplit attn_split(int NJ, int QV, int Hkv, int sms, bool rows) {
     AttnSplit r = {};
     const int widest = attn_nv(QV);
-    r.single = NJ * Hkv * attn_groups(QV, widest) <= sms;
+    r.single = !rows && NJ * Hkv * attn_groups(QV, widest) <= sms;
     for (int n = 0; n < NJ; ++n) {
         int best = 0, cost = 0;
         for (int nv = 1; nv <= widest; ++nv) {
