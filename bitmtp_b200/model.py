@@ -305,6 +305,15 @@ class TransformerBlock(nn.Module):
 # ===========================================================================
 # Transformer: the captured forward
 # ===========================================================================
+def attention_rows_first(args: ModelArgs, M: int) -> bool:
+    """Whether a replay of width M (other than the fused width-1 one) takes its attention as bf16 rows, quantised by the next
+    launch, instead of as codes.  Above 32 heads a warp of the launch that merges to codes takes two heads or more in turn, which
+    few rows do not pay for: codes against rows and quantisation, 40 / 8 and 48 / 16 heads over segments of 256 to 4096, 1.15 and 1.16
+    at width 1, 1.00 and 1.06 at 4, 1.03 and 1.02 at 8, 1.00 at 9, 0.97 and 0.98 at 16.  The rows form has 224 counters."""
+    groups = (M * (args.n_heads // args.n_kv_heads) + 3) // 4
+    return M <= 8 and args.n_heads > 32 and args.n_heads % 4 == 0 and args.n_kv_heads * groups <= 224
+
+
 class StepWorkspace:
     """Every intermediate of one replay width M, allocated once.  A captured graph bakes
     these addresses in; graphs of the same width share one workspace because replays on
@@ -342,11 +351,11 @@ class StepWorkspace:
         self.h_sum = buf((M, args.dim // 128), i32)
         self.inner = buf((M, args.ffn_dim), bf)
         self.inner_amax = torch.zeros((2, M), dtype=i32, device=device)   # row absmax bits, two slots used in turn
-        if M == 1:
-            # attention rows and their absmax bits, and the second residual buffer of the width-1 fused path
-            self.att = buf((M, q_dim), bf)
+        if M == 1 or attention_rows_first(args, M):
+            self.att = buf((M, q_dim), bf)          # attention rows and their absmax bits
             self.att_amax = torch.zeros((2, M), dtype=i32, device=device)
-            self.h2 = buf((M, args.dim), bf)
+        if M == 1:
+            self.h2 = buf((M, args.dim), bf)        # second residual buffer of the width-1 fused path
         self.n_pad = n_pad
 
 
@@ -514,10 +523,7 @@ class Transformer(nn.Module):
         fused_ffn = self.fused_ffn and M <= 16 and a.ffn_dim % 16 == 0 and a.dim % 256 == 0
         if fused_ffn:
             ops.zero_words(W.inner_amax[0])           # slot of layer 0; every layer clears the next one's
-        # Above 32 heads a warp of the launch that merges to codes takes two heads or more in turn, and a single row does not
-        # pay for that (40 / 8 heads, width 1 behind 20 keys: 8.0 us to codes, 6.6 to rows and then codes; width 9 level,
-        # width 16 behind 600 17.9 against 19.1).
-        rows_first = self.fused_rope and M == 1 and a.n_heads > 32 and a.n_heads % 4 == 0
+        rows_first = self.fused_rope and attention_rows_first(a, M)
         if rows_first:
             ops.zero_words(W.att_amax[0])
         ops.rmsnorm_fused(self.embed_tokens.weight.data, L0.input_layernorm.weight.data, eps, M=M,

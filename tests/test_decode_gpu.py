@@ -66,10 +66,11 @@ def test_forward_matches_oracle(oracle, geom, role, M, cache_len, n_pend):
     assert np.array_equal(oracle.torch_to_u16(kvd.cpu()), kv_np), "KV buffer differs"
 
 
-@pytest.mark.parametrize("role,M,cache_len,n_pend", [("ar", 1, 0, 0), ("ar", 1, 33, 0), ("verify", 9, 30, 0), ("draft", 16, 40, 8)])
+@pytest.mark.parametrize("role,M,cache_len,n_pend", [("ar", 1, 0, 0), ("ar", 1, 33, 0), ("ar", 7, 48, 0), ("draft", 8, 31, 0),
+                                                     ("verify", 9, 30, 0), ("draft", 16, 40, 8)])
 @pytest.mark.parametrize("pdl_stable", [False, True])
 def test_forward_of_more_than_32_heads_matches_oracle(oracle, role, M, cache_len, n_pend, pdl_stable):
-    """40 query heads: the merge to codes with two heads a warp, and the rows form of a single row."""
+    """40 query heads: the merge to codes with two heads a warp, and the rows form of up to eight rows."""
     cfg = synthetic.make_config(dict(synthetic.TINY, n_heads=40, n_kv_heads=8, dim=512, ffn_dim=768), block_size=8)
     sigma, m_max = 64, 17
     model, state = _model(cfg, 4, sigma + m_max)
