@@ -165,3 +165,34 @@ def test_the_drop_in_symbol():
     want = BM.t2g128_int8xint2_linear(q, packed, s, scale)
     torch.cuda.synchronize()
     assert torch.equal(out.view(torch.int16), want.view(torch.int16))
+
+
+def test_the_operators_output_is_an_ordinary_tensor(monkeypatch):
+    """What the host path allocates is what torch.empty gives in each setting: shape, strides, type, device, inference tensor or
+    not, in a memory pool of its own under capture, and the same bits where uninitialised memory is filled."""
+    x, packed, scale = _operands(6)
+    q, s = ops.quant_rows(x)
+    want = _without_host(monkeypatch, lambda: BM.t2g128_int8xint2_linear(q, packed, s, scale))
+    for inference in (False, True):
+        with torch.inference_mode(inference):
+            for view in ((6,), (2, 3)):
+                got = native._host.linear(q.view(*view, -1), packed, s.view(*view, 1), scale)
+                ref = torch.empty((*view, 264), dtype=torch.bfloat16, device=DEV)
+                for name in ("shape", "dtype", "device", "layout", "requires_grad"):
+                    assert getattr(got, name) == getattr(ref, name), name
+                assert got.stride() == ref.stride() and got.is_inference() == ref.is_inference() == inference
+                assert torch.equal(got.view(6, -1).view(torch.int16), want.view(torch.int16))
+    torch.use_deterministic_algorithms(True)
+    try:
+        assert torch.equal(native._host.linear(q, packed, s, scale).view(torch.int16), want.view(torch.int16))
+    finally:
+        torch.use_deterministic_algorithms(False)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = BM.t2g128_int8xint2_linear(q, packed, s, scale)
+    out.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out.view(torch.int16), want.view(torch.int16))
+    traced = torch.jit.trace(lambda a: BM.t2g128_int8xint2_linear(a, packed, s, scale), (q,), check_trace=False)
+    assert traced(q).shape == want.shape
